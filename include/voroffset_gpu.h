@@ -155,7 +155,7 @@ int vo_morph_batched(vo_ctx *ctx, int n, const int *ops, const double *radii, in
  * plans the chains of every volume (erosion -> dilation for opening and
  * closing), sizes the output slots (from the attached sizer, see
  * vo_set_sizer, or a fixed capacity), orders the persistent work queue,
- * chooses the block shape with the autotuner (cached per context), and
+ * chooses the lanes per column with the autotuner (cached per context), and
  * captures all device steps into one CUDA graph; it keeps pointers to `ins`,
  * which must outlive the plan and keep their contents. Run replays the graph
  * and re-runs, one by one through vo_morph's path, the volumes whose output
@@ -164,10 +164,10 @@ typedef struct vo_batch vo_batch;
 typedef struct {
   int64_t slot_bytes;   /* output slot memory of the dilations */
   int32_t tiles;        /* work-queue items over all rounds */
-  int32_t tile_rows;    /* warps (8 x 4 column patches) per block chosen by the autotuner (last round): 1, 2 or 4 */
-  int32_t union_cap;    /* union slots per column of the main kernel (last round): 24, 32, 48 or 64; one holds a sentinel */
-  int32_t persistent;   /* 1: one wave of blocks pulling queue items; 0: one block per item (last round) */
-  int32_t regs;         /* register budget per thread of the batch kernel (last round): 64 or 80 */
+  int32_t tile_rows;    /* lanes per column of the patch kernel (last round): 1 or 4 */
+  int32_t union_cap;    /* union slots per column of the patch kernel's first tier: 64, one of them spare */
+  int32_t persistent;   /* 1: one wave of blocks pulling queue items */
+  int32_t regs;         /* register budget per thread of the patch kernel */
   int32_t graph_nodes;  /* nodes of the captured graph */
   int32_t graph_kernels;/* kernel launches per replay */
   int32_t learned;      /* 1 when slots and queue came from a sizer */
@@ -177,8 +177,8 @@ typedef struct {
   double spill_peak;    /* largest fraction of a dilation's spill region used by the last run (> 1: exhausted) */
   int32_t spill_peak_round; /* its dilation round */
   double plan_ms;       /* host time of vo_batch_create */
-  double tune_ms[4];    /* autotuner sample times for 1, 2, 4 rows (persistent, 64 registers, the largest union
-                           capacity tried; 0: cached); [3] unused */
+  double tune_ms[4];    /* autotuner times of the last tuned round with 1 ([0]) and 4 ([2]) lanes per column
+                           (0: cached, or a round whose size decides); the others unused */
 } vo_batch_stats;
 int vo_batch_create(vo_ctx *ctx, int n, const int *ops, const double *radii, int method,
                     const vo_volume *const *ins, vo_batch **out);

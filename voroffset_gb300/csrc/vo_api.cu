@@ -30,43 +30,6 @@ void dfree(vo_ctx *ctx, void *p) {
   if (p) cudaFreeAsync(p, ctx->stream);
 }
 
-// FP32 lower bound of a - b as the device computes it
-// (__double2float_rd(__dsub_rd(a, b))): the FP64 difference rounded to
-// nearest is moved down one ulp when its TwoSum error is negative, then the
-// FP32 conversion rounded to nearest is moved down when it lies above.
-static float sub_rd_f32(double a, double b) {
-  const double c = -b, s = a + c, bb = s - a;
-  const double e = (a - (s - bb)) + (c - bb);
-  const double sd = e < 0.0 ? std::nextafter(s, -INFINITY) : s;
-  float f = (float)sd;
-  if ((double)f > sd) f = std::nextafterf(f, -INFINITY);
-  return f;
-}
-
-// Dominance level thresholds for the tables' radius: t[0] = 0 and t[l] for
-// l >= 1 the value at quantile (l - 1/2) / (kDomLevels - 1) of the sorted
-// growths of H over one lattice step (x steps for a >= 1, y steps for
-// d >= 1), each as the FP32 lower bound the device's pair records hold.
-static void dom_levels(Tables &t) {
-  std::vector<float> g;
-  for (int d = 0; d <= t.Dy; ++d)
-    for (int a = 0; a <= t.Dx[d]; ++a) {
-      const double h = t.H[(size_t)d * t.W + a];
-      if (a >= 1) g.push_back(sub_rd_f32(t.H[(size_t)d * t.W + a - 1], h));
-      if (d >= 1) g.push_back(sub_rd_f32(t.H[(size_t)(d - 1) * t.W + a], h));
-    }
-  std::sort(g.begin(), g.end());
-  t.dom.t[0] = 0.f;
-  for (int l = 1; l < kDomLevels; ++l) {
-    float v = 0.f;
-    if (!g.empty()) {
-      const double q = ((double)l - 0.5) / (double)(kDomLevels - 1);
-      v = g[(size_t)std::floor(q * (double)(g.size() - 1) + 0.5)];
-    }
-    t.dom.t[l] = v > 0.f ? v : 0.f;
-  }
-}
-
 // Host tables with the reference's expressions (compiled with
 // -ffp-contract=off so a*b - c*d is never fused):
 //   pass-1 radius (Voronoi2D.cpp:704-712): r = d==0 ? R : sqrt(R*R - dd*dd), dd = min(d, R)
@@ -96,12 +59,14 @@ int build_tables(double R, int kmax, Tables &t) {
   }
   t.W = t.Dx[0] + 1;
   t.H.assign((size_t)(Dy + 1) * t.W, NAN);
-  t.Hf.assign(t.H.size(), NAN);
+  const int n = t.W + kPatchX + 2;
+  t.hs = n + ((8 - n % 16) + 16) % 16;
+  t.Hp.assign((size_t)(Dy + 2 * kPatchY) * t.hs, -INFINITY);
   for (int d = 0; d <= Dy; ++d)
     for (int dx = 0; dx <= t.Dx[d]; ++dx) {
       const double r = t.r1[d], x = (double)dx;
       t.H[(size_t)d * t.W + dx] = std::sqrt(r * r - x * x);
-      t.Hf[(size_t)d * t.W + dx] = (float)t.H[(size_t)d * t.W + dx];
+      t.Hp[(size_t)d * t.hs + dx] = (float)t.H[(size_t)d * t.W + dx];
     }
   t.HB.assign((size_t)(Dy + 1) * (Dy + 1), NAN);
   for (int dy = 0; dy <= Dy; ++dy)
@@ -109,7 +74,6 @@ int build_tables(double R, int kmax, Tables &t) {
       const double fx = (double)dx * dx, fy = (double)dy * dy;
       if (fx + fy <= R * R) t.HB[(size_t)dy * (Dy + 1) + dx] = std::sqrt(R * R - fx - fy);
     }
-  dom_levels(t);
   return VO_OK;
 }
 
@@ -136,38 +100,31 @@ int get_tables(vo_ctx *ctx, double R, int kmax, const DeviceTables **out) {
   d->kmax = kmax;
   d->host = h;
   cudaError_t e = cudaMalloc(&d->H, sizeof(double) * h.H.size());
-  if (e == cudaSuccess) e = cudaMalloc(&d->Hf, sizeof(float) * h.Hf.size());
+  if (e == cudaSuccess) e = cudaMalloc(&d->Hp, sizeof(float) * h.Hp.size());
   if (e == cudaSuccess) e = cudaMalloc(&d->Dx, sizeof(int) * h.Dx.size());
   if (e == cudaSuccess) e = cudaMalloc(&d->HB, sizeof(double) * h.HB.size());
-  if (e == cudaSuccess) e = cudaMalloc(&d->dH, sizeof(float) * 2 * h.H.size());
   if (e == cudaSuccess)
     e = cudaMemcpy(d->H, h.H.data(), sizeof(double) * h.H.size(), cudaMemcpyHostToDevice);
   if (e == cudaSuccess)
-    e = cudaMemcpy(d->Hf, h.Hf.data(), sizeof(float) * h.Hf.size(), cudaMemcpyHostToDevice);
+    e = cudaMemcpy(d->Hp, h.Hp.data(), sizeof(float) * h.Hp.size(), cudaMemcpyHostToDevice);
   if (e == cudaSuccess)
     e = cudaMemcpy(d->Dx, h.Dx.data(), sizeof(int) * h.Dx.size(), cudaMemcpyHostToDevice);
   if (e == cudaSuccess)
     e = cudaMemcpy(d->HB, h.HB.data(), sizeof(double) * h.HB.size(), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) {
-    launch_dh_tables(ctx->stream, h.Dy, h.W, d->H, d->Dx, d->dH);
-    e = cudaStreamSynchronize(ctx->stream);
-  }
   if (e != cudaSuccess) {
     cudaFree(d->H);
-    cudaFree(d->Hf);
+    cudaFree(d->Hp);
     cudaFree(d->Dx);
     cudaFree(d->HB);
-    cudaFree(d->dH);
     delete d;
     return cuda_error(ctx, e, "table upload");
   }
   if (ctx->tables.size() >= 16) {
     DeviceTables *old = ctx->tables.front();
     cudaFree(old->H);
-    cudaFree(old->Hf);
+    cudaFree(old->Hp);
     cudaFree(old->Dx);
     cudaFree(old->HB);
-    cudaFree(old->dH);
     delete old;
     ctx->tables.erase(ctx->tables.begin());
   }
@@ -285,10 +242,9 @@ void vo_destroy(vo_ctx *ctx) {
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   for (DeviceTables *d : ctx->tables) {
     cudaFree(d->H);
-    cudaFree(d->Hf);
+    cudaFree(d->Hp);
     cudaFree(d->Dx);
     cudaFree(d->HB);
-    cudaFree(d->dH);
     delete d;
   }
   for (auto &e : ctx->ev)

@@ -14,18 +14,17 @@
 //     columns gets the capacity the network predicts for its largest union
 //     (plus a margin, at most kUnionCapMid); without one, every column gets
 //     kUnionCap slots; either way a spill region takes the columns that need
-//     more (unions beyond kUnionCap are computed by the second-tier kernel);
+//     more;
 //   * work queue: dilations in decreasing predicted total work (the network's
-//     per-tile candidate counts, or the mean cost per column), the tiles of
+//     per-tile candidate counts, or the mean cost per column), the patches of
 //     each in bands of 512 columns, all rows of a band before the next;
-//   * union capacity of the main kernel (24 or 32; 48 or 64 for dense inputs,
-//     more than 10 segments per column on average), block shape (1, 2 or 4
-//     warps of 8 x 4 columns per block), register budget and launch mode,
-//     chosen by the autotuner below and cached per context.
+//   * lanes per column of the patch kernel (1 or 4) from the round's size, or
+//     from the autotuner below where the size does not decide it (cached per
+//     context).
 // Then the closures are captured into one graph. vo_batch_run replays it and
 // re-runs, through the single-volume path, every volume whose overflow flag
 // is set (a union larger than its slot with the spill region exhausted, or
-// beyond the FP64 third tier's list), so results never depend on the
+// beyond the FP64 tier's list), so results never depend on the
 // predictions.
 #include <algorithm>
 #include <chrono>
@@ -63,27 +62,19 @@ struct DilPlan {
   int vol = 0;
   SlotVol in, out;
   const DeviceTables *T = nullptr;
-  float *zf = nullptr, *E = nullptr;
-  int4 *col = nullptr;
-  float4 *prec = nullptr;
-  unsigned *dmask = nullptr;
-  int mask_bits = 32;
-  unsigned int *maxbits = nullptr;
-  int2 *pairs = nullptr;
-  int *mid_list = nullptr, *mid_count = nullptr;
-  int *big_list = nullptr, *big_count = nullptr;
-  int npairs = 0;
+  FastArgs A{};
+  PackOut pk;
+  unsigned long long *mm = nullptr;
+  int *big_list = nullptr;
+  int *counters = nullptr;  // spill used, third-tier columns (zeroed before every replay)
   int32_t *tcap = nullptr, *toff = nullptr;
   int tiles32_x = 0, tiles32 = 0;
   std::vector<float> tile_work;  // predicted candidates per column of each sizing tile
   int spill_base = 0, spill_cap = 0;
-  int *spill_used = nullptr;
   double cost = 0;  // mean candidates per column (no sizer)
+  double mean_segs = 0;
   int64_t slot_entries = 0;
 };
-
-constexpr int kTuneShapes[] = {1, 2, 4};
-constexpr int kTuneRegs[] = {64, 80};
 
 }  // namespace
 
@@ -100,7 +91,9 @@ struct vo_batch {
   std::vector<SlotVol> owned;
   std::vector<SlotVol> finals;
   int *d_flags = nullptr;  // [v]: overflow flags of volume v, [n]: complement slot overflow
-  double2 *big_scratch = nullptr;  // working lists of the FP64 third tier
+  double2 *big_scratch = nullptr;  // working lists of the FP64 tier
+  unsigned char *scratch[2] = {nullptr, nullptr};  // working memory of the patch kernel's tiers
+  size_t scratch_bytes[2] = {0, 0};
   struct Spill {
     int *used;
     int cap, round;
@@ -195,7 +188,6 @@ int size_output(vo_ctx *ctx, vo_batch *b, DilPlan &d, double radius) {
     if (entries > 2147483647LL) return set_error(ctx, VO_ERANGE, "batch: slot layout exceeds int32 offsets");
     rc = plan_alloc(ctx, b, &d.tcap, (size_t)d.tiles32);
     if (!rc) rc = plan_alloc(ctx, b, &d.toff, (size_t)d.tiles32);
-    if (!rc) rc = plan_alloc(ctx, b, &d.spill_used, 1);
     if (rc) return rc;
     cudaMemcpyAsync(d.tcap, cap.data(), sizeof(int32_t) * cap.size(), cudaMemcpyHostToDevice, ctx->stream);
     cudaMemcpyAsync(d.toff, off.data(), sizeof(int32_t) * off.size(), cudaMemcpyHostToDevice, ctx->stream);
@@ -206,8 +198,6 @@ int size_output(vo_ctx *ctx, vo_batch *b, DilPlan &d, double radius) {
     d.spill_cap = (int)std::max<int64_t>(4096, entries / 8);
     entries += d.spill_cap;
     if (entries > 2147483647LL) return set_error(ctx, VO_ERANGE, "batch: slot layout exceeds int32 offsets");
-    rc = plan_alloc(ctx, b, &d.spill_used, 1);
-    if (rc) return rc;
   }
   d.slot_entries = entries;
   d.out = SlotVol();
@@ -223,9 +213,8 @@ int size_output(vo_ctx *ctx, vo_batch *b, DilPlan &d, double radius) {
 
 BatchVol batch_vol(const DilPlan &d, int *ovf) {
   BatchVol v;
-  const vo_grid &g = d.in.grid;
-  v.A = FastArgs{g.nx, g.ny, d.T->host.W, d.in.beg, d.in.end, (const double *)d.in.z, d.zf, d.T->Hf, d.T->H,
-                 d.pairs, d.npairs, d.E, d.col, d.prec, d.dmask, d.mask_bits};
+  std::memset(&v, 0, sizeof v);
+  v.A = d.A;
   v.obeg = d.out.beg;
   v.oend = d.out.end;
   v.oz = d.out.z;
@@ -233,56 +222,26 @@ BatchVol batch_vol(const DilPlan &d, int *ovf) {
   v.toff = d.toff;
   v.cap = kUnionCap;
   v.tiles32_x = d.tiles32_x;
-  v.spill_base = d.spill_base;
-  v.spill_cap = d.spill_cap;
-  v.spill_used = d.spill_used;
-  v.mid_list = d.mid_list;
-  v.mid_count = d.mid_count;
+  v.spill_base = (unsigned)d.spill_base;
+  v.spill_cap = (unsigned)d.spill_cap;
+  v.spill_used = reinterpret_cast<unsigned *>(d.counters);
   v.big_list = d.big_list;
-  v.big_count = d.big_count;
+  v.big_count = d.counters + 1;
   v.ovf = ovf;
   return v;
 }
 
-// Work queue for blocks of kFastCols x fby columns: dilations in decreasing
-// estimated total work (longest first, for the balance of the persistent
-// grid), each dilation's tiles in bands of 512 columns, all rows of a band
-// before the next, so that the tiles running at the same time cover a compact
-// region and share their source columns in L1 / L2 (2048^2 r = 32: 7.0 GB of
-// DRAM traffic per launch in full-width rows, 4.1 GB in bands, same time).
-std::vector<int2> build_queue(const std::vector<DilPlan> &dils, int fby) {
-  std::vector<std::pair<double, int>> order;
-  for (size_t i = 0; i < dils.size(); ++i) {
-    const DilPlan &d = dils[i];
-    const vo_grid &g = d.in.grid;
-    double w = 0;
-    if (!d.tile_work.empty()) {
-      for (int t = 0; t < d.tiles32; ++t) {
-        const int tx = t % d.tiles32_x, ty = t / d.tiles32_x;
-        w += (double)d.tile_work[t] * std::min(kSizerTile, g.nx - tx * kSizerTile) *
-             std::min(kSizerTile, g.ny - ty * kSizerTile);
-      }
-    } else {
-      w = d.cost * g.nx * (double)g.ny;
-    }
-    order.push_back({w, (int)i});
+// Estimated total work of a dilation (candidates).
+double total_work(const DilPlan &d) {
+  const vo_grid &g = d.in.grid;
+  if (d.tile_work.empty()) return d.cost * g.nx * (double)g.ny;
+  double w = 0;
+  for (int t = 0; t < d.tiles32; ++t) {
+    const int tx = t % d.tiles32_x, ty = t / d.tiles32_x;
+    w += (double)d.tile_work[t] * std::min(kSizerTile, g.nx - tx * kSizerTile) *
+         std::min(kSizerTile, g.ny - ty * kSizerTile);
   }
-  std::stable_sort(order.begin(), order.end(), [](const std::pair<double, int> &a, const std::pair<double, int> &b) {
-    return a.first > b.first;
-  });
-  std::vector<int2> q;
-  for (const auto &o : order) {
-    const vo_grid &g = dils[o.second].in.grid;
-    const int bw = kPatchX * fby;  // a block's columns: bw x kPatchY
-    // tiles in bands of 512 columns, rows within a band in order: the blocks in flight then cover a
-    // compact region, whose source columns stay in L2 while they are re-read
-    const int tx_n = (g.nx + bw - 1) / bw, ty_n = (g.ny + kPatchY - 1) / kPatchY;
-    const int band = std::max(1, 512 / bw);
-    for (int b0 = 0; b0 < tx_n; b0 += band)
-      for (int ty = 0; ty < ty_n; ++ty)
-        for (int tx = b0; tx < std::min(tx_n, b0 + band); ++tx) q.push_back(make_int2(o.second, ty * tx_n + tx));
-  }
-  return q;
+  return w;
 }
 
 int sm_count() {
@@ -292,220 +251,166 @@ int sm_count() {
   return sms > 0 ? sms : 1;
 }
 
-// Autotuner: times every (union capacity, register budget, block shape,
-// persistent or one block per item) on a sample of the round's queue (four evenly spaced
-// contiguous runs, about 1/16 of it but two to four waves of resident blocks, at least 512 items), the second tier
-// included, and keeps the fastest per column. Results are cached in the
-// context per (one dilation or several, log2 columns, radius bucket, dense or
-// not, learned or not).
-// Tuning launches write into the round's output slots, which the real launch
-// overwrites.
-int tune_shape(vo_ctx *ctx, vo_batch *b, const std::vector<DilPlan> &dils, const BatchVol *dvols,
-               const FastArgs *single, int ka_hint, int *ka_out, int *fby_out, int *persistent_out,
-               int *regs_out) {
-  int64_t cols = 0;
-  double rmax = 0;
+// Autotuner: rounds of kTuneFrom to kTuneTo patches per SM lie where one lane
+// per column (throughput) and four (the longest patch's latency) cross, at a
+// point that depends on the input (8 dexels: 0.19 against 0.27 ms at 200^2,
+// 0.33 against 0.31 ms at 276^2 with four and one). Such a round times both
+// once, and the context keeps the choice per shape (one dilation or several,
+// log2 of the patches, radius / 8, segments per column, learned or not).
+// Smaller and larger rounds follow patch_split.
+constexpr int kTuneFrom = 5, kTuneTo = 24;
+
+int tune_split(vo_ctx *ctx, vo_batch *b, const std::vector<DilPlan> &dils, int64_t patches,
+               const std::function<int(int, float *)> &time, int *split) {
+  double rmax = 0, segs = 0;
   for (const DilPlan &d : dils) {
-    cols += (int64_t)d.in.grid.nx * d.in.grid.ny;
     rmax = std::max(rmax, b->radii[d.vol]);
+    segs = std::max(segs, d.mean_segs);
   }
-  const long long key = (single ? 1LL << 40 : 0) | ((long long)std::ilogb((double)std::max<int64_t>(cols, 1)) << 16) |
-                        ((long long)(rmax / 8) << 2) | (ka_hint == 64 ? 2 : 0) | (ctx->sizer ? 1 : 0);
+  const long long key = (dils.size() == 1 ? 1LL << 40 : 0) | ((long long)std::ilogb((double)patches) << 16) |
+                        ((long long)(rmax / 8) << 8) | ((long long)std::min(segs / 4, 60.0) << 2) | (ctx->sizer ? 1 : 0);
   for (const auto &kv : ctx->tune_cache)
     if (kv.first == key) {
-      *ka_out = (kv.second >> 8) & 255;
-      *fby_out = kv.second & 255;
-      *persistent_out = (kv.second >> 16) & 1;
-      *regs_out = (kv.second >> 17) & 1 ? 80 : 64;
+      *split = kv.second;
       return VO_OK;
     }
-  // union capacities to try: 48 and 64 for dense inputs, else 24 and 32
-  std::vector<int> kas = ka_hint == 64 ? std::vector<int>{48, 64} : std::vector<int>{24, 32};
-  int best_ka = kas.back(), best_pers = 1, best_regs = 64;
-  const int sms = sm_count();
-  int best = 4;
-  double best_t = 1e300;
-  int *dnext = nullptr;
-  int2 *dq = nullptr;
-  int rc = dalloc(ctx, &dnext, 1);
-  size_t qcap = 0;
-  const int gmid = sms * 16;
-  for (int ka : kas)
-  for (int regs : kTuneRegs)
-  for (int fby : kTuneShapes)
-  for (int pers = 1; pers >= 0; --pers) {
-    if (rc) break;
-    const int per_sm = fast_batched_blocks_per_sm(ka, fby, single != nullptr, regs);
-    if (per_sm <= 0) continue;
-    // four contiguous runs of the queue, evenly spaced: neighbouring tiles run
-    // together as in the real launch, so the sample sees its cache reuse
-    const std::vector<int2> full = build_queue(dils, fby);
-    // at least two waves of resident blocks: a sample smaller than a wave
-    // times the tail of a partly idle GPU, not the throughput of a full one;
-    // at most four (or 1/16 of the queue when that is less), so that tuning a
-    // large dense round (4096^2 cylinders: 48 samples) stays a fraction of a second per sample
-    const size_t waves = (size_t)2 * sms * per_sm;
-    const size_t want = std::min(full.size(), std::max<size_t>({512, std::min(full.size() / 16, 2 * waves), waves}));
-    std::vector<int2> sample;
-    for (int r = 0; r < 4; ++r) {
-      const size_t len = want / 4 + (r < (int)(want % 4) ? 1 : 0);
-      const size_t at = std::min(full.size() - len, (full.size() * (2 * r + 1)) / 8);
-      sample.insert(sample.end(), full.begin() + at, full.begin() + at + len);
-    }
-    if (sample.size() > qcap) {
-      dfree(ctx, dq);
-      qcap = sample.size();
-      rc = dalloc(ctx, &dq, qcap);
-      if (rc) break;
-    }
-    cudaMemcpyAsync(dq, sample.data(), sizeof(int2) * sample.size(), cudaMemcpyHostToDevice, ctx->stream);
-    // persistent: one wave of blocks pulling items; otherwise one block per item
-    const int grid = pers ? std::max(1, std::min<int>((int)sample.size(), sms * per_sm)) : (int)sample.size();
-    float ms = 0;
-    for (int rep = 0; rep < 2; ++rep) {  // the first run warms caches and clocks
-      cudaMemsetAsync(dnext, 0, sizeof(int), ctx->stream);
-      for (const DilPlan &d : dils) {
-        cudaMemsetAsync(d.spill_used, 0, sizeof(int), ctx->stream);
-        cudaMemsetAsync(d.mid_count, 0, sizeof(int), ctx->stream);
-        cudaMemsetAsync(d.big_count, 0, sizeof(int), ctx->stream);
-      }
-      cudaEventRecord(ctx->ev[2], ctx->stream);
-      fast_batched_launch(ka, fby, regs, grid, ctx->stream, dvols, dq, (int)sample.size(), dnext, single);
-      fast_batched_mid_launch(ctx->stream, dvols, (int)dils.size(), gmid);  // unions beyond ka count too
-      cudaEventRecord(ctx->ev[3], ctx->stream);
-      cudaError_t e = cudaStreamSynchronize(ctx->stream);
-      if (e != cudaSuccess) {
-        rc = cuda_error(ctx, e, "autotune");
-        break;
-      }
-      cudaEventElapsedTime(&ms, ctx->ev[2], ctx->ev[3]);
-    }
-    if (rc) break;
-    const double per_col = ms / ((double)sample.size() * kFastCols * fby);
-    if (ka == kas.back() && pers && regs == 64) b->stats.tune_ms[fby == 1 ? 0 : fby == 2 ? 1 : 2] = ms;
-    if (per_col < best_t) {
-      best_t = per_col;
-      best = fby;
-      best_ka = ka;
-      best_pers = pers;
-      best_regs = regs;
-    }
-  }
-  dfree(ctx, dnext);
-  dfree(ctx, dq);
+  float ms[2] = {0, 0};
+  int rc = time(1, &ms[0]);
+  if (!rc) rc = time(4, &ms[1]);
   if (rc) return rc;
-  ctx->tune_cache.push_back({key, ((best_regs == 80) << 17) | (best_pers << 16) | (best_ka << 8) | best});
-  *ka_out = best_ka;
-  *fby_out = best;
-  *persistent_out = best_pers;
-  *regs_out = best_regs;
+  b->stats.tune_ms[0] = ms[0];
+  b->stats.tune_ms[2] = ms[1];
+  *split = ms[1] < ms[0] ? 4 : 1;
+  ctx->tune_cache.push_back({key, *split});
   return VO_OK;
 }
 
 int plan_dilation_round(vo_ctx *ctx, vo_batch *b, std::vector<DilPlan> &dils, bool later_rounds) {
-  const int sms = sm_count();
   int rc = VO_OK;
   for (DilPlan &d : dils) {
     const vo_grid &g = d.in.grid;
     const int ncols = g.nx * g.ny;
-    const std::vector<int2> pairs = fast_pairs(d.T->host);
-    d.npairs = (int)pairs.size();
-    rc = plan_alloc(ctx, b, &d.zf, 2 * (size_t)std::max<int64_t>(d.in.entries, 1));
-    if (!rc) rc = plan_alloc(ctx, b, &d.E, 1);
-    if (!rc) rc = plan_alloc(ctx, b, &d.col, (size_t)ncols);
-    // mean segments per column of the input, exact for CSR inputs, the capacity's half for slots
-    const double mean_in = d.in.cap > 0 && d.in.owns ? d.in.cap * 0.5 : (double)d.in.entries / std::max(ncols, 1);
-    d.mask_bits = mask_bits_for(mean_in);
-    if (!rc) rc = plan_alloc(ctx, b, &d.dmask, mask_words((size_t)ncols, d.mask_bits));
-    if (!rc) rc = plan_alloc(ctx, b, &d.prec, pairs.size());
-    if (!rc) rc = plan_alloc(ctx, b, &d.mid_list, (size_t)ncols);
-    if (!rc) rc = plan_alloc(ctx, b, &d.mid_count, 1);
+    const size_t entries = (size_t)std::max<int64_t>(d.in.entries, 1);
+    rc = plan_alloc(ctx, b, &d.pk.zf, entries);
+    if (!rc) rc = plan_alloc(ctx, b, &d.pk.code, entries);
+    if (!rc) rc = plan_alloc(ctx, b, &d.pk.zx, entries);
+    if (!rc) rc = plan_alloc(ctx, b, &d.pk.cl, entries);
+    if (!rc) rc = plan_alloc(ctx, b, &d.pk.coff, pack_offsets(g));
+    if (!rc) rc = plan_alloc(ctx, b, &d.pk.par, 1);
+    if (!rc) rc = plan_alloc(ctx, b, &d.mm, 3);
     if (!rc) rc = plan_alloc(ctx, b, &d.big_list, (size_t)ncols);
-    if (!rc) rc = plan_alloc(ctx, b, &d.big_count, 1);
-    if (!rc) rc = plan_alloc(ctx, b, &d.maxbits, 1);
-    if (!rc) rc = plan_alloc(ctx, b, &d.pairs, pairs.size());
     if (rc) return rc;
-    cudaMemcpyAsync(d.pairs, pairs.data(), sizeof(int2) * pairs.size(), cudaMemcpyHostToDevice, ctx->stream);
-    fast_pair_records(ctx->stream, d.pairs, d.npairs, *d.T, d.prec);  // static: built once, not replayed
-    VO_CK(ctx, cudaStreamSynchronize(ctx->stream));
-    const SlotVol in = d.in;
-    float *zf = d.zf, *E = d.E;
-    int4 *col = d.col;
-    unsigned *dmask = d.dmask;
-    const int mbits = d.mask_bits;
-    unsigned int *mb = d.maxbits;
+    d.A = fast_args(g.nx, g.ny, *d.T, d.in.beg, d.in.end, d.in.z, d.pk);
+    // mean segments per column of the input, exact for CSR inputs, the capacity's half for slots
+    d.mean_segs = d.in.owns ? d.in.cap * 0.5 : (double)d.in.entries / std::max(ncols, 1);
+    const DilPlan c = d;
     const float R = (float)b->radii[d.vol];
-    const DomLevels L = d.T->host.dom;
-    record(b, 3, [in, zf, E, mb, R, col, dmask, mbits, L](cudaStream_t st) {
-      fast_prepare(st, in.grid.nx, in.grid.ny, in.beg, in.end, in.z, zf, mb, R, E, col, dmask, mbits, L);
-    });
-    // candidates per column ~ 4 x pairs x mean segments of the input (no sizer)
-    const double segs = d.in.cap > 0 && d.in.owns ? d.in.cap * 0.5 : (double)d.in.entries / std::max(ncols, 1);
-    d.cost = (double)d.npairs * 4.0 * (segs + 0.5);
+    record(b, 2, [c, R](cudaStream_t st) { fast_prepare(st, c.A, R, c.mean_segs, c.mm, c.pk); });
+    // candidates per column: lattice points of the disc x mean segments of the input (no sizer)
+    d.cost = 3.14159 * (R + 0.5) * (R + 0.5) * (d.mean_segs + 0.5);
   }
   if (ctx->sizer) run_pending(ctx, b);  // features need the dilation inputs
-  for (DilPlan &d : dils) {
+  int *counters = nullptr;
+  rc = plan_alloc(ctx, b, &counters, 4 + 2 * dils.size());
+  if (rc) return rc;
+  for (size_t i = 0; i < dils.size(); ++i) {
+    DilPlan &d = dils[i];
+    d.counters = counters + 4 + 2 * i;
     rc = size_output(ctx, b, d, b->radii[d.vol]);
     if (rc) return rc;
     b->stats.slot_bytes += d.slot_entries * (int64_t)sizeof(double2);
   }
-  std::vector<BatchVol> hv;
-  for (DilPlan &d : dils) hv.push_back(batch_vol(d, b->d_flags + d.vol));
-  BatchVol *dvols = nullptr;
-  int *dnext = nullptr;
-  rc = plan_alloc(ctx, b, &dvols, hv.size());
-  if (!rc) rc = plan_alloc(ctx, b, &dnext, 1);
-  if (rc) return rc;
-  cudaMemcpyAsync(dvols, hv.data(), sizeof(BatchVol) * hv.size(), cudaMemcpyHostToDevice, ctx->stream);
-  VO_CK(ctx, cudaStreamSynchronize(ctx->stream));
-  // union capacity of the round: 64 when its inputs average more than 10 segments per column
-  double segs = 0, cols = 0;
-  for (const DilPlan &d : dils) {
-    const double nc = (double)d.in.grid.nx * d.in.grid.ny;
-    segs += d.in.owns ? 0.5 * d.in.cap * nc : (double)d.in.entries;
-    cols += nc;
-  }
-  int ka = fast_union_cap(segs / std::max(cols, 1.0)), fby = 4, persistent = 1, regs = 64;
-  run_pending(ctx, b);  // tuning reads the dilation inputs
-  // a round of one dilation passes its arguments as a kernel parameter
-  const bool one = hv.size() == 1;
-  const FastArgs a1 = hv[0].A;
-  rc = tune_shape(ctx, b, dils, dvols, one ? &a1 : nullptr, ka, &ka, &fby, &persistent, &regs);
-  if (rc) return rc;
-  const std::vector<int2> q = build_queue(dils, fby);
-  int2 *dq = nullptr;
-  rc = plan_alloc(ctx, b, &dq, q.size());
-  if (rc) return rc;
-  cudaMemcpyAsync(dq, q.data(), sizeof(int2) * q.size(), cudaMemcpyHostToDevice, ctx->stream);
-  VO_CK(ctx, cudaStreamSynchronize(ctx->stream));
-  const int per_sm = std::max(1, fast_batched_blocks_per_sm(ka, fby, one, regs));
-  const int grid = persistent ? std::max(1, std::min<int>((int)q.size(), sms * per_sm)) : std::max(1, (int)q.size());
-  std::vector<int *> counters;  // reset before every replay
-  for (DilPlan &d : dils) {
-    counters.push_back(d.spill_used);
-    counters.push_back(d.mid_count);
-    counters.push_back(d.big_count);
-  }
-  if (!b->big_scratch) {
-    rc = plan_alloc(ctx, b, &b->big_scratch, fast_batched_big_scratch_elems(sms));
-    if (rc) return rc;
-  }
-  double2 *big_scratch = b->big_scratch;
-  const int nq = (int)q.size(), nv = (int)dils.size(), gmid = sms * 16;
-  record(b, 3, [=](cudaStream_t st) {
-    cudaMemsetAsync(dnext, 0, sizeof(int), st);
-    for (int *s : counters) cudaMemsetAsync(s, 0, sizeof(int), st);
-    fast_batched_launch(ka, fby, regs, grid, st, dvols, dq, nq, dnext, one ? &a1 : nullptr);
-    fast_batched_mid_launch(st, dvols, nv, gmid);
-    fast_batched_big_launch(st, dvols, nv, sms, big_scratch);
+  // the queue: dilations in decreasing estimated total work (longest first, for the balance of the
+  // persistent grid), each one's patches in the order of the kernel
+  std::vector<std::pair<double, int>> order;
+  for (size_t i = 0; i < dils.size(); ++i) order.push_back({total_work(dils[i]), (int)i});
+  std::stable_sort(order.begin(), order.end(), [](const std::pair<double, int> &x, const std::pair<double, int> &y) {
+    return x.first > y.first;
   });
-  for (const DilPlan &d : dils) b->spills.push_back({d.spill_used, d.spill_cap, b->rounds});
+  if (!b->big_scratch) rc = plan_alloc(ctx, b, &b->big_scratch, big_scratch_elems());
+  if (rc) return rc;
+  const size_t counter_bytes = sizeof(int) * (4 + 2 * dils.size());
+  double2 *big_scratch = b->big_scratch;
+  const int nv = (int)dils.size();
+  // the round's launch with `split` lanes per column
+  struct RoundLaunch {
+    PatchPlan P;
+    BatchVol *dvols = nullptr;
+  };
+  auto prepare = [&](int split, RoundLaunch &L) -> int {
+    std::vector<BatchVol> hv;
+    int64_t items = 0;
+    int hs = 0;
+    for (const auto &o : order) {
+      const DilPlan &d = dils[o.second];
+      BatchVol v = batch_vol(d, b->d_flags + d.vol);
+      v.item0 = (int)items;
+      items += patch_count(d.in.grid, split);
+      if (items > 2147483647LL) return set_error(ctx, VO_ERANGE, "batch: too many columns");
+      v.item1 = (int)items;
+      hv.push_back(v);
+      hs = std::max(hs, d.T->host.hs);
+    }
+    int r = patch_plan(ctx, (int)items, split, hs, L.P);
+    int *list = nullptr;
+    if (!r) r = plan_alloc(ctx, b, &L.dvols, hv.size());
+    if (!r) r = plan_alloc(ctx, b, &list, (size_t)items);
+    // the rounds run one after the other: they share the largest working memory of each tier
+    for (int t = 0; t < 2 && !r; ++t) {
+      const size_t bytes = patch_scratch_bytes(L.P, t);
+      if (bytes > b->scratch_bytes[t]) {
+        r = plan_alloc(ctx, b, &b->scratch[t], bytes);
+        b->scratch_bytes[t] = bytes;
+      }
+      if (!r) patch_scratch_set(L.P, t, b->scratch[t]);
+    }
+    if (r) return r;
+    L.P.Q = PatchQueue{counters, list};
+    cudaMemcpyAsync(L.dvols, hv.data(), sizeof(BatchVol) * hv.size(), cudaMemcpyHostToDevice, ctx->stream);
+    VO_CK(ctx, cudaStreamSynchronize(ctx->stream));
+    return VO_OK;
+  };
+  auto launch = [counters, counter_bytes, nv, big_scratch](const RoundLaunch &L, cudaStream_t st) {
+    cudaMemsetAsync(counters, 0, counter_bytes, st);
+    patch_launch(false, L.P, st, L.dvols);
+    patch_launch(true, L.P, st, L.dvols);
+    big_launch(st, L.dvols, nv, big_scratch);
+  };
+  std::vector<const vo_grid *> grids;
+  for (const DilPlan &d : dils) grids.push_back(&d.in.grid);
+  int split = patch_split(grids.data(), (int)grids.size());
+  RoundLaunch L;
+  const int64_t patches = patch_total(grids.data(), (int)grids.size());
+  const int sms = sm_count();
+  if (patches < kTuneFrom * sms || patches > kTuneTo * sms) {
+    rc = prepare(split, L);
+  } else {
+    rc = tune_split(ctx, b, dils, patches, [&](int sp, float *ms) -> int {
+      RoundLaunch T;
+      int r = prepare(sp, T);
+      if (r) return r;
+      run_pending(ctx, b);  // tuning reads the dilation inputs; its outputs are written again by the real launch
+      for (int k = 0; k < 2; ++k) {  // the first run warms caches and clocks
+        cudaEventRecord(ctx->ev[2], ctx->stream);
+        launch(T, ctx->stream);
+        cudaEventRecord(ctx->ev[3], ctx->stream);
+      }
+      cudaError_t e = cudaStreamSynchronize(ctx->stream);
+      if (e != cudaSuccess) return cuda_error(ctx, e, "autotune");
+      cudaEventElapsedTime(ms, ctx->ev[2], ctx->ev[3]);
+      return VO_OK;
+    }, &split);
+    if (!rc) rc = prepare(split, L);
+  }
+  if (rc) return rc;
+  record(b, 3, [launch, L](cudaStream_t st) { launch(L, st); });
+  for (const DilPlan &d : dils) b->spills.push_back({d.counters, d.spill_cap, b->rounds});
   ++b->rounds;
-  b->stats.tile_rows = fby;
-  b->stats.union_cap = ka;
-  b->stats.persistent = persistent;
-  b->stats.regs = regs;
-  b->stats.tiles += nq;
+  b->stats.tile_rows = split;
+  b->stats.union_cap = kUnionCapMid / 2;
+  b->stats.persistent = 1;
+  b->stats.regs = 96;
+  b->stats.tiles += L.P.nitems;
   if (later_rounds) run_pending(ctx, b);
   return VO_OK;
 }
@@ -523,7 +428,7 @@ void plan_free(vo_ctx *ctx, vo_batch *b) {
   delete b;
 }
 
-// Plan-owned copy of the tables of radius R (H, Hf and dH on the device, the
+// Plan-owned copy of the tables of radius R (H, Hp and Dx on the device, the
 // host tables), shared by the plan's volumes of the same radius. The cached
 // context entry is copied before any other table lookup can evict it.
 int plan_tables(vo_ctx *ctx, vo_batch *b, double R, int kmax, const DeviceTables **out) {
@@ -540,14 +445,14 @@ int plan_tables(vo_ctx *ctx, vo_batch *b, double R, int kmax, const DeviceTables
   own->R = T->R;
   own->kmax = T->kmax;
   own->host = T->host;
-  const size_t nh = T->host.H.size();
+  const size_t nh = T->host.H.size(), np = T->host.Hp.size(), nd = T->host.Dx.size();
   rc = plan_alloc(ctx, b, &own->H, nh);
-  if (!rc) rc = plan_alloc(ctx, b, &own->Hf, nh);
-  if (!rc) rc = plan_alloc(ctx, b, &own->dH, 2 * nh);
+  if (!rc) rc = plan_alloc(ctx, b, &own->Hp, np);
+  if (!rc) rc = plan_alloc(ctx, b, &own->Dx, nd);
   if (rc) return rc;
   cudaMemcpyAsync(own->H, T->H, sizeof(double) * nh, cudaMemcpyDeviceToDevice, ctx->stream);
-  cudaMemcpyAsync(own->Hf, T->Hf, sizeof(float) * nh, cudaMemcpyDeviceToDevice, ctx->stream);
-  cudaMemcpyAsync(own->dH, T->dH, sizeof(float) * 2 * nh, cudaMemcpyDeviceToDevice, ctx->stream);
+  cudaMemcpyAsync(own->Hp, T->Hp, sizeof(float) * np, cudaMemcpyDeviceToDevice, ctx->stream);
+  cudaMemcpyAsync(own->Dx, T->Dx, sizeof(int) * nd, cudaMemcpyDeviceToDevice, ctx->stream);
   VO_CK(ctx, cudaStreamSynchronize(ctx->stream));
   *out = own.get();
   b->tables.push_back(std::move(own));

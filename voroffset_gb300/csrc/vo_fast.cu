@@ -1,4 +1,4 @@
-// Exact separable dilation with FP32 envelope arithmetic and an FP64 guard
+// Exact separable dilation with FP32 arithmetic and an FP64 guard
 // (VO_METHOD_FAST, and the engine of batch plans).
 //
 // The separable scheme of the reference (VoronoiVorPower.cpp:24-96: a y-pass
@@ -11,421 +11,1171 @@
 // own FP64 value (pass-1 pieces are sub-intervals of these segments whose
 // candidates tile them, so both unions are the same set, bit for bit).
 //
-// One thread per output column walks the (|dx|, |dy|) pairs in decreasing H
-// and merges each source column's dilated segments into a small sorted union
-// (FP32 values in shared memory, endpoint identities in local memory).
-// Candidate endpoints are formed in FP32 (FP32 copies of the inputs and of H);
-// every comparison is decided in FP32 when the values differ by more than a
-// guard band E bounding the FP32 error, and otherwise re-evaluated exactly in
-// FP64 from the candidate's identity (input value index, d, a). Output
+// One warp computes an 8 x 4 patch of output columns (one per lane) in two
+// sweeps over the clusters of source segments within reach, one per lane:
+//
+// 1. Cover. H at the patch column farthest from the source bounds H from
+//    below for all 32 columns, so [z1 - Hmin, z2 + Hmin] is covered in every
+//    one of them. The union of these intervals (the cover) is taken without
+//    sorting: bins of the lower end hold the smallest lower and the largest
+//    upper end of their intervals; intervals of at least a bin's width overlap
+//    every other one of their bin, so a component ends exactly where the
+//    running maximum of the upper ends stops short of the next bin's smallest
+//    lower end. This sweep takes clusters whole: their segments' union is one
+//    interval, and so it stays when every segment is widened by Hmin.
+// 2. Filter and merge. A cluster, and then a segment, whose interval at the
+//    nearest column (Hmax) lies inside one component of the cover cannot
+//    change any of the 32 unions and is dropped (2048^2 spheres + cylinders,
+//    r = 32, modelled: 2,083 clusters of 22,266 segments in reach of a patch;
+//    393 clusters of 4,511 segments pass the first test, 3,001 segments the
+//    second). The others are queued in shared memory, and each is merged by
+//    all lanes at once, one column each: the lane looks up the bin of its
+//    lower end and, only when the interval reaches beyond what its entry for
+//    that bin holds, updates it. Entries (smallest lower and largest upper
+//    end, per lane) exist only for bins that some queued segment can fall
+//    into; bins wholly inside a component of the cover share one entry that
+//    starts at the component's end.
+//
+// The segments are packed beforehand by 4 x 4 tiles of columns into clusters
+// of up to 16 overlapping segments (k_pack), a surface patch typically: the
+// sweeps then load contiguous records, one per lane, and no lane idles over
+// columns of uneven counts.
+//
+// A last pass over the entries in bin order yields the union's intervals.
+// Intervals shorter than a bin (near the rim of the disc) that their entry
+// does not hold are kept aside and inserted into the finished union.
+//
+// Exactness: candidates are formed in FP32 (copies of the inputs relative to
+// a base below them, and of H). E bounds the FP32 error of a comparison: the
+// filter drops a segment only when it is inside by more than E, and every
+// comparison of the merge within E is re-evaluated in FP64 from the
+// candidates' identities (value index, d, a), kept beside each entry. Output
 // endpoints are always recomputed in FP64 from their identities, so results
-// are bit-identical to the FP64 oracle.
+// are bit-identical to the FP64 oracle. Nothing in the cover enters a result:
+// the segments that reach a component's ends are never dropped, and being long
+// they overlap the stretch that its shared entry stands for.
 //
-// Dominance: a source column whose segments all lie in segments of its
-// neighbour one lattice step toward the output column, widened by at most the
-// growth dH of H over that step, adds nothing that neighbour's candidates do
-// not cover, and is skipped. Both bounds are computed with directed rounding,
-// so skipping never changes the union.
+// What bounds it: issue slots (see the figures at k_patch). The bins' width is
+// a power of two, so that binning is exact (one fused multiply-add that
+// rounds to an integer).
 //
-// Capacities: the main kernels keep KA union slots per column (KA in
-// {24, 32, 48, 64}, chosen per input density or by the batch autotuner; one
-// slot holds the sentinel, so KA - 1 intervals); columns that need more are
-// re-run by the same code with kUnionCapMid (128) slots (count, then fill),
-// and beyond that by an FP64 kernel with a large working list in global
-// scratch.
+// Capacities: a patch that needs more entries, kept-aside intervals or union
+// intervals than the launch has re-runs with larger lists (second tier), and a
+// column that outgrows those too goes to an FP64 kernel with an 8,192-interval
+// list.
 #include <algorithm>
-#include <chrono>
 #include <cmath>
 #include <cstring>
 #include <vector>
-
-#include <cuda_fp16.h>
 
 #include "vo_internal.cuh"
 
 namespace vo {
 namespace {
 
-constexpr int kKM = kUnionCapMid;  // union capacity of the second tier
-// Block shape of k_fast: one warp (one patch of columns), at most 64
-// registers so that 32 warps fit an SM; measured faster than four-warp blocks
-// at 80 registers (305 vs 340 ms on the 2048^2 r=32 dilation).
-constexpr int kFB = kFastCols, kFBY = 1;
-constexpr int kBigCap = 8192;    // FP64 fallback working list (intervals)
+constexpr unsigned kFull = 0xffffffffu;
+constexpr int kBins = 1024;       // bins of lower ends (a power of two; indexes are masked into range)
+constexpr int kCoverBins = 512;   // bins of the cover: the same, or two in one for inputs that use more
+constexpr int kTile = 4;          // side of a source tile (columns), equal to the patch's height
+constexpr int kGroup = 16;        // most segments of a cluster (half a warp)
+constexpr int kPackSort = 4096;   // segments that a packing block sorts at a time (its warps share them evenly)
+constexpr int kPairs = 3;         // pairs of clusters expanded at a time
+constexpr int kQueue = 32 + 32 * kPairs;  // queued segments of a patch: flushed above 32
+constexpr int kSplit = 4;         // lanes per column of the split form
+constexpr int kPad = 4 * kSplit;  // padding of the queue
+constexpr int kClusters = 96;     // clusters of a tile row to expand: expanded above 32
+constexpr int kEntries = 512;     // entries of a patch (bins and components of the cover together)
+constexpr int kComps = 63;        // components of the cover that are used
+constexpr int kUnion = 64;        // union intervals per column, plus one
+constexpr int kShort = 1024;      // kept-aside segments of a patch
+constexpr int kEntriesBig = 1600; // the same for the second tier
+constexpr int kUnionBig = 1024;
+constexpr int kShortBig = 8192;
+constexpr int kBigCap = 8192;     // last tier (FP64): intervals of a column's working list
 constexpr int kBigThreads = 32;
-constexpr int kMidThreads = 32;
+constexpr int kBigBlocks = 16;      // last tier: blocks
+constexpr int kPatchBigBlocks = 76; // second tier: warps
+static_assert(kTile == kPatchY && kPatchX % kTile == 0, "tiles and patches are aligned to each other");
 
-// Identities of union endpoints, kept in local memory and read only when an
-// FP32 comparison falls inside the guard band or the output is written.
-template <int KA>
-struct UnionIds {
-  // (input value index, d | a << 8) of the lower / upper endpoint
-  int2 lo[KA], hi[KA];
-};
+// ------------------------------------------------------------ preparation
 
-__device__ __forceinline__ double exact_val(const FastArgs &A, int idx, int da, bool plus) {
-  const double h = A.H64[(da & 255) * A.W + (da >> 8)];
-  const double z = A.zd[idx];
-  return plus ? __dadd_rn(z, h) : __dsub_rn(z, h);
+// Doubles as unsigned integers of the same order (zero: below every one).
+__device__ __forceinline__ unsigned long long order_of(double v) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+  return b >> 63 ? ~b : b | 0x8000000000000000ull;
+}
+__device__ __forceinline__ double value_of(unsigned long long o) {
+  return __longlong_as_double((long long)(o >> 63 ? o & 0x7fffffffffffffffull : ~o));
 }
 
-// Exact comparisons, out of line: identities are loaded only here.
-// Union endpoint (j, hi?) < candidate endpoint (idx, da, plus)?
-template <int KA>
-__device__ __noinline__ bool ex_u_lt_c(const FastArgs &A, const UnionIds<KA> &U, int j, bool jhi, int idx, int da,
-                                       bool plus) {
-  const double u = jhi ? exact_val(A, U.hi[j].x, U.hi[j].y, true) : exact_val(A, U.lo[j].x, U.lo[j].y, false);
-  return u < exact_val(A, idx, da, plus);
-}
-// Candidate endpoint < union endpoint?
-template <int KA>
-__device__ __noinline__ bool ex_c_lt_u(const FastArgs &A, const UnionIds<KA> &U, int idx, int da, bool plus, int j,
-                                       bool jhi) {
-  const double u = jhi ? exact_val(A, U.hi[j].x, U.hi[j].y, true) : exact_val(A, U.lo[j].x, U.lo[j].y, false);
-  return exact_val(A, idx, da, plus) < u;
-}
-// Union endpoint (i, ihi) < union endpoint (j, jhi)?
-template <int KA>
-__device__ __noinline__ bool ex_u_lt_u(const FastArgs &A, const UnionIds<KA> &U, int i, bool ihi, int j, bool jhi) {
-  const double a = ihi ? exact_val(A, U.hi[i].x, U.hi[i].y, true) : exact_val(A, U.lo[i].x, U.lo[i].y, false);
-  const double b = jhi ? exact_val(A, U.hi[j].x, U.hi[j].y, true) : exact_val(A, U.lo[j].x, U.lo[j].y, false);
-  return a < b;
+// Range of the values and, by the last block to finish, the scalars of the
+// dilation (FastPar). mm (zeroed before): orders of the largest value and of
+// the largest negated value, then the blocks that are done.
+// Guard band: with U bounding the magnitude of every FP32 value (relative to
+// the base), each candidate endpoint is within 1.5 ulp32(U) of its FP64 value
+// (rounding of z, of H and of the sum) and a difference of two adds one more
+// ulp32(U): at most 4 ulp32(U) = 2^-21 U. E = 2^-20 U leaves a factor of two;
+// the rounding of the FP64 endpoints themselves is below 2^-50 times the
+// largest magnitude.
+__global__ void k_range(int ncols, const int32_t *__restrict__ beg, const int32_t *__restrict__ end,
+                        const double2 *__restrict__ z, float R, unsigned long long *mm, FastPar *par) {
+  double hi = -INFINITY, lo = -INFINITY;
+  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < ncols; c += gridDim.x * blockDim.x)
+    for (int k = beg[c]; k < end[c]; ++k) {
+      const double2 s = z[k];
+      hi = fmax(hi, fmax(s.x, s.y));
+      lo = fmax(lo, -fmin(s.x, s.y));
+    }
+  for (int o = 16; o > 0; o >>= 1) {
+    hi = fmax(hi, __shfl_xor_sync(kFull, hi, o));
+    lo = fmax(lo, __shfl_xor_sync(kFull, lo, o));
+  }
+  if ((threadIdx.x & 31) == 0 && hi > -INFINITY) {
+    atomicMax(&mm[0], order_of(hi));
+    atomicMax(&mm[1], order_of(lo));
+  }
+  __syncthreads();
+  if (threadIdx.x) return;
+  __threadfence();
+  if (atomicAdd(&mm[2], 1ull) + 1 != gridDim.x) return;
+  __threadfence();
+  const unsigned long long a = atomicMax(&mm[0], 0ull), b = atomicMax(&mm[1], 0ull);
+  const double zmax = a ? value_of(a) : 0.0, zmin = b ? -value_of(b) : 0.0;
+  FastPar p;
+  p.base = floor(zmin - R - 3.0);
+  const float U = (float)(zmax - p.base + R + 3.0);
+  p.E = U * 9.5367431640625e-07f + (float)(fmax(fabs(zmax), fabs(zmin)) * 8.8817841970012523e-16);
+  // bin width: the power of two at or above a quarter of the radius, wide
+  // enough for the range and far above the guard band
+  const float w0 = fmaxf(fmaxf(U / (float)(kBins - 8), 0.25f * R), fmaxf(64.f * p.E, 1e-20f));
+  int e;
+  const float m = frexpf(fminf(w0, 1e30f), &e);
+  if (m == 0.5f) --e;
+  const float w = ldexpf(1.f, e);
+  p.inv_w = ldexpf(1.f, -e);
+  p.thr = w + 4.f * p.E;
+  p.nbins = (int)fminf((float)kBins, U * p.inv_w + 3.f);
+  *par = p;
 }
 
-// The FP16 in the low (lo != 0) or high half of v.
-__device__ __forceinline__ __half half_of(unsigned v, int lo) {
-  return __ushort_as_half((unsigned short)(lo ? (v & 0xffffu) : (v >> 16)));
+// Packs the segments by 4 x 4 tiles of columns into clusters: runs of at most
+// kGroup segments, in order of their lower ends, whose union is one interval
+// (each starts at or below the largest upper end so far). A block per row of
+// tiles, a warp per tile. Tile row T's clusters and segments start at
+// beg[first column of its first row], which leaves room for all of them in
+// CSR and slot layouts alike. Written per cluster: (union's ends, first
+// segment, count | tile << 5); per segment: FP32 values relative to the base,
+// its column in the tile, and its FP64 values.
+// A warp sorts up to kPackSort / WARPS segments, by counting for each those
+// before it (a few dozen per tile); a tile of more keeps every segment a
+// cluster. More warps for sparse inputs: a block's steps are chains of
+// dependent loads, and what bounds it is how many tiles it has in flight.
+template <int WARPS>
+__global__ void __launch_bounds__(32 * WARPS) k_pack(int nx, int ny, const int32_t *__restrict__ beg,
+                                                     const int32_t *__restrict__ end, const double2 *__restrict__ z,
+                                                     const FastPar *__restrict__ par, float2 *__restrict__ zf,
+                                                     unsigned char *__restrict__ code, double2 *__restrict__ zx,
+                                                     float4 *__restrict__ cl, int32_t *__restrict__ coff) {
+  constexpr int CAP = kPackSort / WARPS;
+  __shared__ __align__(16) int s_key[WARPS][CAP];  // bit patterns of the lower ends: a total order, also of NaNs
+  __shared__ float s_hi[WARPS][CAP];
+  __shared__ unsigned short s_ord[WARPS][CAP];  // segment of rank r
+  __shared__ unsigned char s_col[WARPS][CAP];
+  __shared__ int s_src[WARPS][16];  // per column: its segments' index in z minus their position here
+  __shared__ int s_ns[WARPS], s_nc[WARPS];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tiles_x = (nx + kTile - 1) / kTile, T = blockIdx.x;
+  const double base = par->base;
+  int seg0 = beg[T * kTile * nx], cl0 = seg0;  // next free segment and cluster of the tile row
+  for (int t0 = 0; t0 < tiles_x; t0 += WARPS) {
+    const int tx = t0 + warp;
+    // two lanes per column: its segments alternate between them
+    const int c4 = lane >> 1, x = tx * kTile + (c4 & 3), y = T * kTile + (c4 >> 2);
+    int k0 = 0, n = 0;
+    if (tx < tiles_x && x < nx && y < ny) {
+      k0 = beg[x + nx * y];
+      n = end[x + nx * y] - k0;
+    }
+    int pre = lane & 1 ? 0 : n;  // exclusive prefix over the columns
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(kFull, pre, o);
+      if (lane >= o) pre += v;
+    }
+    const int m = __shfl_sync(kFull, pre, 31);
+    pre -= n;  // both lanes of a column: the segments before it
+    if (lane == 0) s_ns[warp] = m;
+    const bool sort = m <= CAP;
+    int nc = m;
+    unsigned starts[CAP / 32];  // per 32 ranks: where the clusters start
+    if (sort) {
+      if ((lane & 1) == 0) s_src[warp][c4] = k0 - pre;
+      for (int i = lane & 1; i < n; i += 2) {
+        const double2 v = z[k0 + i];
+        s_key[warp][pre + i] = __float_as_int(__double2float_rn(__dsub_rn(v.x, base)));
+        s_hi[warp][pre + i] = __double2float_rn(__dsub_rn(v.y, base));
+        s_col[warp][pre + i] = (unsigned char)c4;
+      }
+      // padding up to the next 32: after every segment
+      const int full = (m + 31) & ~31;
+      if (m + lane < full) s_key[warp][m + lane] = 0x7fffffff;
+      __syncwarp();
+      for (int i0 = 0; i0 < m; i0 += 32) {
+        const int v = i0 + lane < m ? s_key[warp][i0 + lane] : 0;
+        int r = 0;
+        for (int j0 = 0; j0 < full; j0 += 32) {
+          // equal ends keep their order: earlier blocks count them, later ones do not
+          if (j0 == i0) {
+            for (int j = 0; j < 32; ++j) {
+              const int u = s_key[warp][j0 + j];
+              r += u < v || (u == v && j < lane) ? 1 : 0;
+            }
+          } else if (j0 < i0) {
+#pragma unroll
+            for (int j = 0; j < 32; j += 4) {
+              const int4 u = *reinterpret_cast<const int4 *>(&s_key[warp][j0 + j]);
+              r += (u.x <= v) + (u.y <= v) + (u.z <= v) + (u.w <= v);
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; j += 4) {
+              const int4 u = *reinterpret_cast<const int4 *>(&s_key[warp][j0 + j]);
+              r += (u.x < v) + (u.y < v) + (u.z < v) + (u.w < v);
+            }
+          }
+        }
+        if (i0 + lane < m) s_ord[warp][r] = (unsigned short)(i0 + lane);
+      }
+      __syncwarp();
+      // where the clusters break: one step per segment, the same in every lane
+      nc = 0;
+      float hi = 0.f;
+      int cnt = kGroup;
+#pragma unroll
+      for (int b = 0; b < CAP / 32; ++b) {
+        starts[b] = 0;
+        if (32 * b >= m) continue;
+        const int i = s_ord[warp][min(32 * b + lane, m - 1)];
+        const float va = __int_as_float(s_key[warp][i]), vb = s_hi[warp][i];
+        const int e = min(32, m - 32 * b);
+        for (int j = 0; j < e; ++j) {
+          const float lo = __shfl_sync(kFull, va, j), up = __shfl_sync(kFull, vb, j);
+          if (cnt == kGroup || !(lo <= hi)) {
+            starts[b] |= 1u << j;
+            cnt = 0;
+            hi = up;
+          }
+          ++cnt;
+          hi = fmaxf(hi, up);
+        }
+        nc += __popc(starts[b]);
+      }
+    }
+    if (lane == 0) s_nc[warp] = nc;
+    __syncthreads();
+    int sb = seg0, seg_all = 0, cb = cl0, cl_all = 0;
+    {
+      int a = lane < WARPS ? s_ns[lane] : 0, c = lane < WARPS ? s_nc[lane] : 0;
+      sb += __reduce_add_sync(kFull, lane < warp ? a : 0);
+      cb += __reduce_add_sync(kFull, lane < warp ? c : 0);
+      seg_all = __reduce_add_sync(kFull, a);
+      cl_all = __reduce_add_sync(kFull, c);
+    }
+    if (tx < tiles_x && lane == 0) coff[(size_t)T * (tiles_x + 1) + tx] = cb;
+    if (sort) {
+      int g = cb;  // clusters before this block of ranks
+#pragma unroll
+      for (int b = 0; b < CAP / 32; ++b) {
+        if (32 * b >= m) continue;
+        const int r = 32 * b + lane;
+        if (r < m) {
+          const int i = s_ord[warp][r], col = s_col[warp][i];
+          const float a = __int_as_float(s_key[warp][i]);
+          zf[sb + r] = make_float2(a, s_hi[warp][i]);
+          code[sb + r] = (unsigned char)col;
+          zx[sb + r] = z[s_src[warp][col] + i];
+          if (starts[b] >> lane & 1) {
+            // the cluster's end: the next start, in this block of ranks or the next one
+            const unsigned after = lane < 31 ? starts[b] >> (lane + 1) : 0u;
+            int e = after ? r + __ffs(after) : 32 * (b + 1);
+            if (!after && b + 1 < CAP / 32) e += starts[b + 1 < CAP / 32 ? b + 1 : b] ? __ffs(starts[b + 1 < CAP / 32 ? b + 1 : b]) - 1 : 32;
+            e = min(e, m);
+            float top = 0.f;
+            for (int q = r; q < e; ++q) top = fmaxf(top, s_hi[warp][s_ord[warp][q]]);
+            cl[g + __popc(starts[b] & ((1u << lane) - 1u))] =
+                make_float4(a, top, __int_as_float(sb + r), __int_as_float((e - r) | (tx << 5)));
+          }
+        }
+        g += __popc(starts[b]);
+      }
+    } else {
+      for (int i = lane & 1; i < n; i += 2) {
+        const double2 v = z[k0 + i];
+        const float2 f = make_float2(__double2float_rn(__dsub_rn(v.x, base)), __double2float_rn(__dsub_rn(v.y, base)));
+        const int r = pre + i;
+        zf[sb + r] = f;
+        code[sb + r] = (unsigned char)c4;
+        zx[sb + r] = v;
+        cl[cb + r] = make_float4(f.x, f.y, __int_as_float(sb + r), __int_as_float(1 | (tx << 5)));
+      }
+    }
+    seg0 += seg_all;
+    cl0 += cl_all;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) coff[(size_t)T * (tiles_x + 1) + tiles_x] = cl0;
 }
 
-// FP32 difference t = y - x decides x < y outside the guard band [-E, E].
+// ------------------------------------------------------------ exact comparisons
+
+// An endpoint's identity: (value index, d | a << 8), index < 0 for none.
+__device__ __forceinline__ double exact_val(const double *H, int W, const double *z, int2 id, bool plus) {
+  const double h = H[(id.y & 255) * W + (id.y >> 8)];
+  const double v = z[max(id.x, 0)];
+  return plus ? __dadd_rn(v, h) : __dsub_rn(v, h);
+}
+__device__ __noinline__ bool exact_less(const double *H, int W, const double *z, int2 a, bool ap, int2 b, bool bp) {
+  return exact_val(H, W, z, a, ap) < exact_val(H, W, z, b, bp);
+}
+
+// x < y for FP32 values with t = y - x, decided exactly inside the guard band
 #define GUARD(t, E, exact) ((t) > (E) ? true : ((t) < -(E) ? false : (exact)))
 
-// Returns the number of intervals of the union (identities in U), or -1 when
-// more than KA - 1 are needed (the last of the KA slots holds the sentinel).
-//
-// `mask` holds the lanes of the warp running this function together. For each
-// (|dx|, |dy|) pair the four source columns' segments form one list per lane;
-// every lane of the warp iterates to the warp's longest list with a predicate,
-// and the loop body has no early exits, so the lanes reconverge after every
-// candidate instead of drifting apart over the source transitions.
-template <int KA>
-__device__ int fast_column(const FastArgs &A, float E, int x, int y, float2 *sv, int stride, UnionIds<KA> &U,
-                           unsigned mask) {
-  int n = 0;
-  bool overflow = false;
-#define SV(k) sv[(k) * stride]
-  // SV(n) holds a sentinel above every value, so the cursor walk stops at
-  // the end of the union without a bounds test; the union holds up to KA - 1
-  // intervals.
-  const float2 kTop = make_float2(INFINITY, INFINITY);
-  SV(0) = kTop;
-  // Per pair: its four source columns' records and their segment dominance
-  // masks at the pair's levels, loaded when the pair starts (only the pair's
-  // own table entry is loaded one pair ahead: holding the source records
-  // across the merge loop cost more in register spills than their load
-  // latency, which the other resident warps hide).
-  // Source S: x + a if S & 1 (its neighbour toward the output is at x - 1,
-  // direction "x-" = 0), else x - a ("x+" = 1); likewise y with S & 2
-  // ("y-" = 2, "y+" = 3).
-  const int ncols = A.nx * A.ny;
-  const int mbits = A.mask_bits;
-#define MASK(DIR, LV, C)                                                                                \
-  ((LV) < kDomLevels ? (mbits == 16 ? (unsigned)static_cast<const unsigned short *>(A.dmask)[((DIR) * kDomLevels + (LV)) * ncols + (C)] \
-                                    : static_cast<const unsigned *>(A.dmask)[((DIR) * kDomLevels + (LV)) * ncols + (C)])        \
-                     : 0u)
-#define LOAD_ONE(OK, XS, YS, S, R, D)                                                                   \
-  {                                                                                                     \
-    const int c_ = (OK) ? (XS) + A.nx * (YS) : 0;                                                       \
-    R = (OK) ? reinterpret_cast<const int2 *>(A.col)[2 * c_] : make_int2(0, 0);                          \
-    D = (OK) ? (MASK((S) & 1 ? 0 : 1, lx_, c_) | MASK((S) & 2 ? 2 : 3, ly_, c_)) : 0u;                  \
+// ------------------------------------------------------------ one patch
+
+// The working memory of one warp. Entry e of column c is at [COLS * e + c]. The
+// entries are read once per queued segment and column; they sit in global
+// memory, where L1 holds them: in shared memory they took 256 bytes each for
+// the most that a patch may need (2048^2, r = 32: 36 on average, 65 at most;
+// r = 16: 86 and 146), and 10 warps per SM instead of 16 ran (81 against 63 ms
+// at r = 32, 244 against 91 ms at r = 16).
+struct PatchMem {
+  float2 *sv;             // entries: smallest lower end + E, largest upper end - E
+  float2 *ml;             // bins of the cover
+  unsigned short *cmap;   // entry of each bin (0: none)
+  float2 *bnd;            // entries 1 .. S.nbnd - 1: the component of the cover that their bins' segments may lie in
+  float *hrow1;           // first sweep: H for the current tile row, at the farthest row of the patch
+  float *hrow;            // second sweep: H for the current tile row, 7 rows (see hrow_row)
+  float4 *queue;          // queued segments (z1, z2, x - X0, row of the tile), and their indices
+  int *qk;
+  int2 *clist;            // clusters to expand (first segment, count | tile << 5)
+  float4 *shorts;         // kept-aside segments (z1, z2, index, x - X0 and y - Y0)
+  int2 *idl, *idh;        // identities of the entries' ends
+  float2 *cv;             // finished intervals and the identities of their ends
+  int2 *cl, *ch;
+  int ne, nunion, nshort; // capacities
+};
+
+// How a warp's lanes are spread: G segments at a time for the kPatchX / G x
+// kPatchY columns of its patch; lane l takes column l % COLS (cell), segment
+// l / COLS of the group.
+template <int G>
+struct Shape {
+  static constexpr int PX = kPatchX / G, COLS = PX * kPatchY;
+};
+
+struct PatchState {
+  int X0, Y0, lx, ly, lane, col, g;
+  int nent;               // entries in use, the dummy entry 0 included
+  int nbnd;               // entries with a component of the cover, entry 0 included
+  int ns;                 // kept-aside segments
+  int qn, cn;             // queued segments, clusters to expand
+  float E, inv_w, thr;
+  int cshift;             // cover bins: bins >> cshift
+  float cthr;             // least length of an interval of the cover
+};
+
+// Bin of a lower end: rounds lo / w to an integer (exact scaling, one
+// rounding), masked so that no value can index out of range.
+__device__ __forceinline__ unsigned bin_of(float lo, float inv_w) {
+  return __float_as_uint(__fmaf_rn(lo, inv_w, 8388608.f)) & (kBins - 1);
+}
+
+// New entry for bin b (uniform). False when the entries are used up.
+template <int G>
+__device__ __forceinline__ bool new_entry(const PatchMem &M, PatchState &S, int b) {
+  const int e = S.nent;
+  if (e >= M.ne) return false;
+  ++S.nent;
+  if (S.lane == 0) M.cmap[b] = (unsigned short)e;
+  if (S.g == 0) {
+    const int a = Shape<G>::COLS * e + S.col;
+    M.sv[a] = make_float2(INFINITY, -INFINITY);
+    M.idl[a] = make_int2(-1, 0);
+    M.idh[a] = make_int2(-1, 0);
   }
-#define LOAD_SOURCES(PR)                                                                                \
-  {                                                                                                     \
-    const int ad_ = __float_as_int((PR).x), a_ = ad_ & 0xff, d_ = (ad_ >> 8) & 0xff;                    \
-    const int lx_ = (ad_ >> 16) & 0xf, ly_ = (ad_ >> 20) & 0xf;                                         \
-    const bool xm = x - a_ >= 0, xp = a_ > 0 && x + a_ < A.nx;                                          \
-    const bool ym = y - d_ >= 0, yp = d_ > 0 && y + d_ < A.ny;                                          \
-    LOAD_ONE(xm && ym, x - a_, y - d_, 0, c0, d0)                                                       \
-    LOAD_ONE(xp && ym, x + a_, y - d_, 1, c1, d1)                                                       \
-    LOAD_ONE(xm && yp, x - a_, y + d_, 2, c2, d2)                                                       \
-    LOAD_ONE(xp && yp, x + a_, y + d_, 3, c3, d3)                                                       \
+  __syncwarp();
+  return true;
+}
+
+// The component of the cover that an interval with lower end lo may lie in.
+__device__ __forceinline__ float2 component_of(const PatchMem &M, const PatchState &S, float lo) {
+  const int e = M.cmap[bin_of(lo, S.inv_w)];
+  return M.bnd[e < S.nbnd ? e : 0];
+}
+
+// Row of hrow for |dy| between row sy of the tile row k (relative to the
+// patch's) and row ly of the patch: the rows hold 4 |k| - 3 .. 4 |k| + 3 for
+// k != 0, and 3, 2, 1, 0, 1, 2, 3 for k = 0.
+__device__ __forceinline__ int hrow_row(int k, int sy, int ly) {
+  return k < 0 ? kTile - 1 + ly - sy : kTile - 1 + sy - ly;
+}
+// distances of a column t = x - X0 to the nearest and the farthest column of the patch
+template <int G>
+__device__ __forceinline__ int near_dx(int t) {
+  return max(0, max(-t, t - (Shape<G>::PX - 1)));
+}
+template <int G>
+__device__ __forceinline__ int far_dx(int t) {
+  return max(t, Shape<G>::PX - 1 - t);
+}
+
+// Merges the segments of `todo` (bits 0 .. 3: queue positions G apart) into
+// this lane's column with every comparison inside the guard band decided in FP64.
+// Closings bring such ties in numbers: every column under one ball of the
+// first dilation gives the second one the same end up to rounding. All loads
+// of a segment go out together (identities and candidate, then the entry's
+// values). Not inlined: the merge loop has to stay in the instruction cache.
+template <int G>
+__device__ __noinline__ void merge_exact(const double *__restrict__ H, int W, const double2 *__restrict__ zx,
+                                         const float4 *queue, const int *qk, const float *hl, int step,
+                                         const unsigned short *cmap, float2 *sv, int2 *idl, int2 *idh, int lx, int dy0,
+                                         float E, float inv_w, unsigned todo) {
+  const double *z = reinterpret_cast<const double *>(zx);
+  for (; todo; todo &= todo - 1) {
+    const int i = __ffs(todo) - 1;
+    const float4 u = queue[G * i];
+    const int key = qk[G * i], sy = __float_as_int(u.w), dx = abs(__float_as_int(u.z) - lx), dy = abs(dy0 + sy);
+    const float g = hl[sy * step + dx];
+    const float l = u.x - g, r = u.y + g;
+    const int en = Shape<G>::COLS * cmap[bin_of(l, inv_w)];
+    const int2 il = idl[en], ih = idh[en];
+    float2 w = sv[en];
+    const double2 zc = zx[key];
+    const double hc = H[dy * W + dx];
+    const double zl = z[max(il.x, 0)], zh = z[max(ih.x, 0)];
+    const double hl64 = H[(il.y & 255) * W + (il.y >> 8)], hh64 = H[(ih.y & 255) * W + (ih.y >> 8)];
+    const int da = dy | (dx << 8);
+    const float tl = (w.x - E) - l, th = r - (w.y + E);
+    if (GUARD(tl, E, il.x < 0 || __dsub_rn(zc.x, hc) < __dsub_rn(zl, hl64))) {
+      w.x = l + E;
+      idl[en] = make_int2(2 * key, da);
+    }
+    if (GUARD(th, E, ih.x < 0 || __dadd_rn(zh, hh64) < __dadd_rn(zc.y, hc))) {
+      w.y = r - E;
+      idh[en] = make_int2(2 * key + 1, da);
+    }
+    sv[en] = w;
   }
-  float4 pr = A.prec[0];
-  for (int p = 0; p < A.npairs; ++p) {
-    const float4 pc = pr;
-    if (p + 1 < A.npairs) pr = A.prec[p + 1];
-    int2 c0, c1, c2, c3;  // (beg, end) of each source column
-    unsigned d0, d1, d2, d3;
-    LOAD_SOURCES(pc)
-    const int ad = __float_as_int(pc.x), a = ad & 0xff, d = (ad >> 8) & 0xff;
-    const float h = pc.y;
-    const int da = d | (a << 8);
-    // growth of H over one step toward the output column (x step, y step),
-    // against which the sources' dominance widths are tested
-    const float dhx = pc.z, dhy = pc.w;
-    // FP16 bounds of the pair's growths (rounded down) for the source tests
-    const __half dhx_h = __float2half_rd(dhx), dhy_h = __float2half_rd(dhy);
-    // Per source: [kb, ke) and the mask of its kept segments (bit j: segment
-    // kb + j); a source of more than mbits segments keeps all (m = 0, dense).
-    // A source of up to mbits segments that is dominated whole has an empty kept
-    // mask; a source of more segments (no masks) is tested with its column
-    // widths.
-#define SRC(S, XS, YS, C, DM, KB, KE, M)                                                                \
-  {                                                                                                     \
-    KB = (C).x;                                                                                         \
-    KE = (C).y;                                                                                         \
-    const int ns_ = KE - KB;                                                                            \
-    if (ns_ > mbits) {                                                                                  \
-      const int4 cr_ = A.col[(XS) + A.nx * (YS)];                                                       \
-      if (__hle(half_of((unsigned)cr_.z, (S) & 1), dhx_h) || __hle(half_of((unsigned)cr_.w, (S) & 2), dhy_h)) \
-        KE = KB;                                                                                        \
-    }                                                                                                   \
-    M = ns_ <= mbits ? ~(DM) & (ns_ == 32 ? 0xffffffffu : ((1u << ns_) - 1u)) : 0u;                    \
+}
+
+// Merges the queued segments of tile row k (relative to the patch's) into
+// every column's entries. Returns false when a capacity is exceeded.
+template <int G>
+__device__ __forceinline__ bool flush_queue(const FastArgs &A, const PatchMem &M, PatchState &S, int k) {
+  const int lane = S.lane, qn = S.qn, hs = A.hs;
+  const float E = S.E, inv_w = S.inv_w;
+  constexpr int COLS = Shape<G>::COLS;
+  if (lane < 4 * G) M.queue[qn + lane] = make_float4(INFINITY, -INFINITY, 0.f, 0.f);  // padding: no candidate
+  __syncwarp();
+  // entries for every bin that a queued segment's lower end can fall into in some column
+  for (int q0 = 0; q0 < qn; q0 += 32) {
+    int b = 1, b1 = 0;
+    if (q0 + lane < qn) {
+      const float4 c = M.queue[q0 + lane];
+      const int t = __float_as_int(c.z), sy = __float_as_int(c.w);
+      const int near = k > 0 ? kPatchY - 1 : k < 0 ? 0 : sy;
+      const int far = k > 0 || (k == 0 && sy >= kPatchY / 2) ? 0 : kPatchY - 1;
+      b = (int)bin_of(c.x - M.hrow[hrow_row(k, sy, near) * hs + near_dx<G>(t)], inv_w);
+      b1 = (int)bin_of(c.x - fmaxf(M.hrow[hrow_row(k, sy, far) * hs + far_dx<G>(t)], 0.f), inv_w);
+    }
+    for (;;) {
+      while (b <= b1 && M.cmap[b] != 0) ++b;
+      const unsigned w = __ballot_sync(kFull, b <= b1);
+      if (!w) break;
+      if (!new_entry<G>(M, S, __shfl_sync(kFull, b, __ffs(w) - 1))) return false;
+    }
   }
-    int kb0, ke0, kb1, ke1, kb2, ke2, kb3, ke3;
-    unsigned m0, m1, m2, m3;
-    SRC(0, x - a, y - d, c0, d0, kb0, ke0, m0)
-    SRC(1, x + a, y - d, c1, d1, kb1, ke1, m1)
-    SRC(2, x - a, y + d, c2, d2, kb2, ke2, m2)
-    SRC(3, x + a, y + d, c3, d3, kb3, ke3, m3)
-#undef SRC
-#define KEPT(KB, KE, M) ((KE) - (KB) > mbits ? (KE) - (KB) : __popc(M))
-    const int t0 = KEPT(kb0, ke0, m0), t1 = KEPT(kb1, ke1, m1), t2 = KEPT(kb2, ke2, m2), t3 = KEPT(kb3, ke3, m3);
-#undef KEPT
-    const int total = t0 + t1 + t2 + t3;
-    const int iters = __reduce_max_sync(mask, total);
-    // Walk state: the sources still to visit that keep candidates (bit s),
-    // the current source s, its remaining mask ms (sparse) or next index kc
-    // (dense); NEXT yields the next kept candidate (KN, SN), or KN = -1. A
-    // source is entered only when it keeps a candidate, so NEXT takes at most
-    // one source switch and no loop.
-    unsigned srcs = (t0 > 0 ? 1u : 0u) | (t1 > 0 ? 2u : 0u) | (t2 > 0 ? 4u : 0u) | (t3 > 0 ? 8u : 0u);
-    int s = -1, kc = 0, kend = 0, kbs = 0;
-    unsigned ms = 0;
-    bool dense = false;
-#define NEXT(KN, SN)                                                                                    \
-  {                                                                                                     \
-    if ((dense ? kc >= kend : ms == 0u) && srcs) {                                                      \
-      s = __ffs(srcs) - 1;                                                                              \
-      srcs &= srcs - 1;                                                                                 \
-      kbs = s == 0 ? kb0 : s == 1 ? kb1 : s == 2 ? kb2 : kb3;                                           \
-      kend = s == 0 ? ke0 : s == 1 ? ke1 : s == 2 ? ke2 : ke3;                                          \
-      ms = s == 0 ? m0 : s == 1 ? m1 : s == 2 ? m2 : m3;                                                \
-      dense = kend - kbs > mbits;                                                                       \
-      kc = kbs;                                                                                         \
-    }                                                                                                   \
-    KN = -1;                                                                                            \
-    if (dense) {                                                                                        \
-      if (kc < kend) KN = kc++;                                                                         \
-    } else if (ms) {                                                                                    \
-      KN = kbs + __ffs(ms) - 1;                                                                         \
-      ms &= ms - 1;                                                                                     \
-    }                                                                                                   \
-    SN = s;                                                                                             \
-  }
-    int cur = 0, cur_src = -1;
-    float2 cv = make_float2(0.f, 0.f);
-    int kn, sn;
-    NEXT(kn, sn)
-    float2 znext = kn >= 0 ? *reinterpret_cast<const float2 *>(A.zf + 2 * kn) : make_float2(0.f, 0.f);
-    for (int it = 0; it < iters; ++it) {
-      if (it < total && !overflow) {
-        const int k = kn, src = sn;
-        const float2 zf = znext;
-        NEXT(kn, sn)
-        if (kn >= 0) znext = *reinterpret_cast<const float2 *>(A.zf + 2 * kn);
-        if (src != cur_src) {  // first candidate of a new source column: restart the cursor
-          cur_src = src;
-          cur = 0;
-          cv = SV(0);
+  // row sy of the tile row: hl[sy * step]
+  const float *hl = M.hrow + hrow_row(k, 0, S.ly) * hs;
+  const int step = k < 0 ? -hs : hs;
+  float2 *const sv = M.sv + S.col;
+  int2 *const idl = M.idl + S.col, *const idh = M.idh + S.col;
+  const float E2 = 2.f * E;
+  for (int q = 0; q < qn; q += 4 * G) {
+    // Four segments per lane at a time in stages, so that their dependent loads (segment, H, bin, entry)
+    // overlap: one after the other they took 462 cycles each, staged 210 (2048^2, r = 32).
+    unsigned need = 0;
+    float4 c[4];
+    float h[4], lo[4], hi[4];
+    int e[4];
+    float2 v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) c[i] = M.queue[q + G * i + S.g];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) h[i] = hl[__float_as_int(c[i].w) * step + abs(__float_as_int(c[i].z) - S.lx)];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      lo[i] = c[i].x - h[i];
+      hi[i] = c[i].y + h[i];
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) e[i] = COLS * M.cmap[bin_of(lo[i], inv_w)];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = sv[e[i]];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) need |= lo[i] < v[i].x || hi[i] > v[i].y ? 1u << i : 0u;
+    // segments with which some column's union may grow: the entry is updated where the comparison is
+    // clear of the guard band; short intervals are kept aside, the others left to the exact merge
+    const unsigned any = __ballot_sync(kFull, need != 0);
+    if (!any) continue;
+    unsigned unclear = 0, shorts = 0;
+#pragma unroll
+    for (int s = 0; s < G; ++s) {  // one lane of a column after the other
+      if (G == 1 || (any >> (COLS * s) & (0xffffffffu >> (32 - COLS)))) {
+        if (G == 1 || (S.g == s && need)) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            if (G > 1) {
+              v[i] = sv[e[i]];
+            } else {
+#pragma unroll
+              for (int j = 0; j < i; ++j)
+                if (e[j] == e[i]) v[i] = v[j];  // as the segments before left it
+            }
+            const bool gl = lo[i] < v[i].x, gh = hi[i] > v[i].y;
+            const bool cl = lo[i] < v[i].x - E2, ch = hi[i] > v[i].y + E2;
+            const bool grow = gl || gh, brief = hi[i] - lo[i] < S.thr, clear = gl == cl && gh == ch;
+            if (grow && brief) shorts |= 1u << (G * i + S.g);
+            if (grow && !brief && !clear) unclear |= 1u << i;
+            if (grow && !brief && clear) {
+              const int key = M.qk[q + G * i + S.g];
+              const int da = abs(kTile * k - S.ly + __float_as_int(c[i].w)) | (abs(__float_as_int(c[i].z) - S.lx) << 8);
+              if (cl) {
+                v[i].x = lo[i] + E;
+                idl[e[i]] = make_int2(2 * key, da);
+              }
+              if (ch) {
+                v[i].y = hi[i] - E;
+                idh[e[i]] = make_int2(2 * key + 1, da);
+              }
+              sv[e[i]] = v[i];
+            }
+          }
         }
-        {
-          const float lo = zf.x - h, hi = zf.y + h;
-          const int il = 2 * k, ih = 2 * k + 1;
-          // skip union intervals that end strictly below the candidate: U.hi[cur] < lo
-          // (the next interval's values are loaded one step ahead)
-          if (lo - cv.y > E) {  // two intervals per step: cur < n here, so cur + 1 <= n
-            float2 c1 = SV(cur + 1), c2 = SV(min(cur + 2, n));
-            for (;;) {
-              if (!(lo - c1.y > E)) {
-                cur += 1;
-                cv = c1;
-                break;
-              }
-              if (!(lo - c2.y > E)) {
-                cur += 2;
-                cv = c2;
-                break;
-              }
-              cur += 2;
-              c1 = SV(cur + 1);
-              c2 = SV(min(cur + 2, n));
+        if (G > 1) __syncwarp();
+      }
+    }
+    for (unsigned todo = __reduce_or_sync(kFull, shorts); todo; todo &= todo - 1) {
+      const int i = __ffs(todo) - 1;
+      if (S.ns >= M.nshort) return false;
+      if (lane == 0) {
+        const float4 u = M.queue[q + i];
+        const int at = (__float_as_int(u.z) + 1024) | ((kTile * k + __float_as_int(u.w) + 1024) << 16);
+        M.shorts[S.ns] = make_float4(u.x, u.y, __int_as_float(M.qk[q + i]), __int_as_float(at));
+      }
+      ++S.ns;
+    }
+    if (__any_sync(kFull, unclear != 0)) {
+      for (int s = 0; s < G; ++s) {
+        if (S.g == s && unclear)
+          merge_exact<G>(A.H64, A.W, reinterpret_cast<const double2 *>(A.zx), M.queue + q + S.g, M.qk + q + S.g, hl,
+                         step, M.cmap, sv, idl, idh, S.lx, kTile * k - S.ly, E, inv_w, unclear);
+        __syncwarp();
+      }
+    }
+  }
+  S.qn = 0;
+  __syncwarp();
+  return true;
+}
+
+// Expands the listed clusters of tile row k: their segments that no component
+// of the cover holds are queued (half a warp per cluster, kPairs pairs at a
+// time so that their loads overlap), and the queue is flushed when it fills
+// up and, with `last`, at the end of the tile row.
+template <int G>
+__device__ __forceinline__ bool expand_clusters(const FastArgs &A, const PatchMem &M, PatchState &S, int k,
+                                                bool last) {
+  const int lane = S.lane, hs = A.hs, cn = S.cn;
+  __syncwarp();
+  for (int q = 0;; q += 2 * kPairs) {
+    float2 z[kPairs];
+    int key[kPairs], t[kPairs], col[kPairs];
+    bool ok[kPairs];
+#pragma unroll
+    for (int i = 0; i < kPairs; ++i) {
+      const int p = q + 2 * i + (lane >> 4);
+      const int2 c = p < cn ? M.clist[p] : make_int2(0, 0);
+      ok[i] = (lane & 15) < (c.y & 31);
+      key[i] = c.x + (lane & 15);
+      t[i] = (c.y >> 5) * kTile - S.X0;
+      z[i] = ok[i] ? __ldcg(A.zf + key[i]) : make_float2(0.f, 0.f);
+      col[i] = ok[i] ? __ldcg(A.code + key[i]) : 0;
+    }
+#pragma unroll
+    for (int i = 0; i < kPairs; ++i) {
+      t[i] += col[i] & 3;
+      const int sy = col[i] >> 2;
+      const int row = hrow_row(k, sy, k > 0 ? kPatchY - 1 : k < 0 ? 0 : sy);
+      const float h = M.hrow[row * hs + (ok[i] ? near_dx<G>(t[i]) : 0)];
+      const float lo = z[i].x - h, hi = z[i].y + h;
+      const float2 b = component_of(M, S, lo);
+      const bool keep = ok[i] && !(b.x <= lo && hi <= b.y);
+      const unsigned w = __ballot_sync(kFull, keep);
+      if (keep) {
+        const int p = S.qn + __popc(w & ((1u << lane) - 1u));
+        M.queue[p] = make_float4(z[i].x, z[i].y, __int_as_float(t[i]), __int_as_float(sy));
+        M.qk[p] = key[i];
+      }
+      S.qn += __popc(w);
+    }
+    const bool end = q + 2 * kPairs >= cn;
+    if (S.qn > (end && last ? 0 : 32))
+      if (!flush_queue<G>(A, M, S, k)) return false;
+    if (end) break;
+  }
+  S.cn = 0;
+  __syncwarp();
+  return true;
+}
+
+// One sweep over the tile rows within reach: PASS 1 builds the cover's bins
+// from the clusters, PASS 2 filters the clusters and merges what is left.
+template <int PASS, int G>
+__device__ __forceinline__ bool sweep(const FastArgs &A, const PatchMem &M, PatchState &S) {
+  const int lane = S.lane, X0 = S.X0, T0 = S.Y0 / kTile, hs = A.hs;
+  constexpr int PX = Shape<G>::PX;
+  const int tiles_x = (A.nx + kTile - 1) / kTile, tiles_y = (A.ny + kTile - 1) / kTile;
+  const int reach = (A.Dy + kTile - 1) / kTile, nrows = 2 * reach + 1;
+  const float inv_w = S.inv_w;
+  for (int jb = 0; jb < nrows; jb += 32) {
+    // the lanes look up the cluster ranges of 32 tile rows, the patch's own first, then outwards
+    int r0 = 0, r1 = 0, rm = 0;
+    {
+      const int j = jb + lane, kk = (j + 1) >> 1, k = j & 1 ? kk : -kk;
+      const int T = T0 + k;
+      const int d = PASS == 1 ? kTile * kk + kTile - 1 : max(0, kTile * kk - (kTile - 1));
+      if (j < nrows && T >= 0 && T < tiles_y && d <= A.Dy) {
+        const int a = A.Dx[d];
+        int ta, tb;
+        if (PASS == 1) {  // every column of the patch within reach of every column of the tile
+          ta = max(0, (X0 + PX - 1 - a + kTile - 1) >> 2);
+          tb = min(tiles_x - 1, (X0 + a - (kTile - 1)) >> 2);
+        } else {
+          ta = max(0, X0 - a) / kTile;
+          tb = min(A.nx - 1, X0 + PX - 1 + a) / kTile;
+        }
+        if (ta <= tb) {
+          const int32_t *o = A.coff + (size_t)T * (tiles_x + 1);
+          r0 = o[ta];
+          r1 = o[tb + 1];
+          rm = o[X0 / kTile];
+        }
+      }
+    }
+    for (unsigned rows = __ballot_sync(kFull, r1 > r0); rows; rows &= rows - 1) {
+      const int jj = __ffs(rows) - 1;
+      const int cb = __shfl_sync(kFull, r0, jj), ce = __shfl_sync(kFull, r1, jj);
+      const int kk = (jb + jj + 1) >> 1, k = (jb + jj) & 1 ? kk : -kk;
+      // In the second sweep from the patch's own columns to the right, then to the left: the nearest
+      // segments come first, and those that reach less far than they change nothing (a plane of equal
+      // ends would otherwise be approached step by step, with ties at each).
+      const int cm = __shfl_sync(kFull, rm, jj), right = ce - cm;
+      auto load = [&](int p) {
+        if (p >= ce - cb) return make_float4(INFINITY, -INFINITY, 0.f, 0.f);
+        return __ldcg(A.cl + (PASS == 1 ? cb + p : p < right ? cm + p : cm - 1 - (p - right)));
+      };
+      float4 cn[2];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) cn[i] = load(32 * i + lane);
+      __syncwarp();
+      if (PASS == 1) {
+        const float *src = A.Hp + (kTile * kk + kTile - 1) * hs;
+        for (int i = lane; i < hs; i += 32) M.hrow1[i] = src[i];
+      } else if (k == 0) {
+        for (int r = 0; r < 2 * kTile - 1; ++r) {
+          const float *src = A.Hp + abs(r - (kTile - 1)) * hs;
+          for (int i = lane; i < hs; i += 32) M.hrow[r * hs + i] = src[i];
+        }
+      } else {
+        const float4 *src = reinterpret_cast<const float4 *>(A.Hp + (kTile * kk - (kTile - 1)) * hs);
+        for (int i = lane; i < (2 * kTile - 1) * hs / 4; i += 32) reinterpret_cast<float4 *>(M.hrow)[i] = src[i];
+      }
+      __syncwarp();
+      // second sweep: the nearest rows
+      const float *hM = M.hrow + (k == 0 ? (kTile - 1) * hs : 0);
+      const int n = ce - cb;
+      for (int c0 = 0; c0 < n; c0 += 64) {
+        float4 c[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) c[i] = cn[i];
+        if (c0 + 64 < n) {
+#pragma unroll
+          for (int i = 0; i < 2; ++i) cn[i] = load(c0 + 64 + 32 * i + lane);
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          if (c0 + 32 * i >= n) break;
+          const int info = __float_as_int(c[i].w), t = (info >> 5) * kTile - X0;
+          const bool in = c0 + 32 * i + lane < n;
+          if (PASS == 1) {
+            const float h = in ? M.hrow1[max(t + kTile - 1, PX - 1 - t)] : -1.f;
+            const float lo = c[i].x - h, hi = c[i].y + h;
+            if (2.f * h >= S.cthr) {  // every segment of the cluster gives a long interval
+              float2 *bin = M.ml + (bin_of(lo, inv_w) >> S.cshift);
+              // values are positive: their bit patterns are ordered like them
+              if (lo < bin->x) atomicMin(reinterpret_cast<int *>(&bin->x), __float_as_int(lo));
+              if (hi > bin->y) atomicMax(reinterpret_cast<int *>(&bin->y), __float_as_int(hi));
             }
+          } else {
+            const float h = in ? hM[max(0, max(-t - (kTile - 1), t - (PX - 1)))] : 0.f;
+            const float lo = c[i].x - h, hi = c[i].y + h;
+            const float2 b = component_of(M, S, lo);
+            const bool keep = in && !(b.x <= lo && hi <= b.y);
+            const unsigned w = __ballot_sync(kFull, keep);
+            if (keep)
+              M.clist[S.cn + __popc(w & ((1u << lane) - 1u))] = make_int2(__float_as_int(c[i].z), info);
+            S.cn += __popc(w);
           }
-          while (cur < n && GUARD(lo - cv.y, E, ex_u_lt_c(A, U, cur, true, il, da, false))) {
-            ++cur;
-            cv = SV(cur);
-          }
-          // covered: inside U[cur]; else ext_lo / ext_hi: the candidate reaches
-          // below / above U[cur] (both decided once, used again to extend it)
-          bool covered = false, ext_lo = false, ext_hi = false;
-          if (cur < n) {
-            if (lo - cv.x > E && cv.y - hi > E) {
-              covered = true;  // inside U[cur] by more than the guard band
-            } else {
-              ext_lo = GUARD(cv.x - lo, E, ex_c_lt_u(A, U, il, da, false, cur, false));
-              ext_hi = GUARD(hi - cv.y, E, ex_u_lt_c(A, U, cur, true, ih, da, true));
-              covered = !ext_lo && !ext_hi;
-            }
-          }
-          if (!covered) {
-            if (cur == n || GUARD(cv.x - hi, E, ex_c_lt_u(A, U, ih, da, true, cur, false))) {
-              // disjoint: insert before cur
-              if (n >= KA - 1) {
-                overflow = true;
-              } else {
-                for (int j = n; j > cur; --j) {
-                  SV(j) = SV(j - 1);
-                  U.lo[j] = U.lo[j - 1];
-                  U.hi[j] = U.hi[j - 1];
-                }
-                cv = make_float2(lo, hi);
-                SV(cur) = cv;
-                U.lo[cur] = make_int2(il, da);
-                U.hi[cur] = make_int2(ih, da);
-                ++n;
-                SV(n) = kTop;
-              }
-            } else {
-              // overlapping or touching U[cur]: extend it
-              if (ext_lo) {
-                cv.x = lo;
-                U.lo[cur] = make_int2(il, da);
-              }
-              if (ext_hi) {
-                cv.y = hi;
-                U.hi[cur] = make_int2(ih, da);
-                // absorb following intervals that now start at or below the new end
-                int j = cur + 1;
-                while (j < n) {
-                  const float2 nv = SV(j);
-                  if (GUARD(nv.x - cv.y, E, ex_u_lt_u(A, U, cur, true, j, false))) break;  // U.hi[cur] < U.lo[j]
-                  if (GUARD(nv.y - cv.y, E, ex_u_lt_u(A, U, cur, true, j, true))) {       // U.hi[cur] < U.hi[j]
-                    cv.y = nv.y;
-                    U.hi[cur] = U.hi[j];
-                  }
-                  ++j;
-                }
-                const int gone = j - cur - 1;
-                if (gone > 0) {
-                  for (int m = cur + 1; m + gone < n; ++m) {
-                    SV(m) = SV(m + gone);
-                    U.lo[m] = U.lo[m + gone];
-                    U.hi[m] = U.hi[m + gone];
-                  }
-                  n -= gone;
-                  SV(n) = kTop;
-                }
-              }
-              SV(cur) = cv;
-            }
-          }
+        }
+        if (PASS == 2) {
+          const bool last = c0 + 64 >= n;
+          if (S.cn > (last ? 0 : 32) || (last && S.qn > 0))
+            if (!expand_clusters<G>(A, M, S, k, last)) return false;
         }
       }
     }
   }
-#undef SV
-#undef LOAD_SOURCES
-#undef LOAD_ONE
-#undef MASK
-#undef NEXT
-  return overflow ? -1 : n;
+  return true;
 }
 
-// Writes the exact FP64 union held by U (n intervals) to out[0..n).
-template <int KA>
-__device__ __forceinline__ void write_union(const FastArgs &A, const UnionIds<KA> &U, int n, double2 *out) {
-  for (int k = 0; k < n; ++k)
-    out[k] = make_double2(exact_val(A, U.lo[k].x, U.lo[k].y, false), exact_val(A, U.hi[k].x, U.hi[k].y, true));
-}
-
-// One pass: the exact union of every output column goes to its fixed-capacity
-// staging slot (KA entries, at most KA - 1 used) with its count; columns that need more are
-// listed for the second tier. A compaction pass then packs the slots.
-template <int KA>
-__global__ void __launch_bounds__(kFB *kFBY, 1024 / (kFB * kFBY)) k_fast(FastArgs A, int32_t *counts,
-                                                                          double2 *staging,
-                                                    int *ovf_count, int *ovf_cols) {
-  extern __shared__ float2 sv_dyn[];
-  const int tid = threadIdx.x + kFB * threadIdx.y;
-  // blocks (patches) in bands of 512 columns, all rows of a band before the next: the blocks running
-  // together cover a compact region, whose source columns stay in L2
-  constexpr int kBand = 512 / kPatchX;
-  const int tiles_x = (A.nx + kPatchX - 1) / kPatchX, tiles_y = (A.ny + kPatchY - 1) / kPatchY;
-  const int band = (int)blockIdx.x / (kBand * tiles_y);
-  const int rb = (int)blockIdx.x - band * kBand * tiles_y;
-  const int bw = min(kBand, tiles_x - band * kBand);
-  const int x = (band * kBand + rb % bw) * kPatchX + threadIdx.x % kPatchX;
-  const int y = (rb / bw) * kPatchY + threadIdx.x / kPatchX;
-  if (x >= A.nx || y >= A.ny) return;
-  const int c = x + A.nx * y;
-  const float E = *A.E;
-  UnionIds<KA> U;
-  const unsigned mask = __activemask();
-  const int n = fast_column<KA>(A, E, x, y, sv_dyn + tid, kFB * kFBY, U, mask);
-  if (n > 0) write_union(A, U, n, staging + (size_t)c * KA);
-  if (n < 0) {
-    ovf_cols[atomicAdd(ovf_count, 1)] = c;
-    counts[c] = 0;
-  } else {
-    counts[c] = n;
+// Components of the cover from its bins, and the entries that come with them.
+template <int G>
+__device__ __forceinline__ bool cover_entries(const PatchMem &M, PatchState &S, int nbins) {  // nbins: of the cover
+  const int lane = S.lane;
+  const float E = S.E;
+  int m = 0;
+  float carry = -INFINITY;
+  for (int b0 = 0; b0 < nbins; b0 += 32) {
+    const int b = b0 + lane;
+    const float2 v = b < nbins ? M.ml[b] : make_float2(INFINITY, -INFINITY);
+    const bool full = v.y > -INFINITY;
+    if (!__any_sync(kFull, full)) continue;
+    float mx = v.y;
+    for (int o = 1; o < 32; o <<= 1) {
+      const float y = __shfl_up_sync(kFull, mx, o);
+      if (lane >= o) mx = fmaxf(mx, y);
+    }
+    float before = __shfl_up_sync(kFull, mx, 1);  // largest upper end of the earlier bins
+    before = fmaxf(carry, lane ? before : -INFINITY);
+    const bool start = full && !(v.x <= before - E);
+    const unsigned w = __ballot_sync(kFull, start);
+    const int c = m + __popc(w & ((1u << lane) - 1u));  // component starting here
+    if (start) {
+      if (c < kComps) M.bnd[c + 1].x = v.x;
+      if (c > 0 && c <= kComps) M.bnd[c].y = before;
+    }
+    m += __popc(w);
+    carry = fmaxf(carry, __shfl_sync(kFull, mx, 31));
   }
-}
-
-// Packs the staging slots (ka intervals each) of the columns that fit into
-// the CSR output.
-__global__ void k_compact(int ncols, int ka, const int32_t *__restrict__ counts,
-                          const double2 *__restrict__ staging, const int32_t *__restrict__ ooffs,
-                          double2 *__restrict__ oz) {
-  // one warp per column, lanes over intervals
-  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (w >= ncols) return;
-  const int n = ooffs[w + 1] - ooffs[w];
-  if (n > ka) return;  // written by the second tier
-  for (int k = lane; k < n; k += 32) oz[ooffs[w] + k] = staging[(size_t)w * ka + k];
-}
-
-// Second tier over the columns listed by k_fast (grid-stride): the same
-// computation with kKM slots (kKM - 1 intervals). Count pass: counts[c], or the
-// column goes to the FP64 list when even that is exceeded. Fill pass: writes the union at its
-// CSR offset (columns of the FP64 list are left to it).
-template <bool FILL>
-__global__ void __launch_bounds__(kMidThreads) k_fast_mid(FastArgs A, int32_t *counts, const int32_t *ooffs,
-                                                          double2 *oz, const int *list_count, const int *list,
-                                                          int *big_count, int *big_list) {
-  __shared__ float2 sv[kKM * kMidThreads];
-  const float E = *A.E;
-  const int m = *list_count;
-  const int nth = gridDim.x * kMidThreads;
-  for (int i = blockIdx.x * kMidThreads + threadIdx.x; i < m; i += nth) {
-    const int c = list[i];
-    const int x = c % A.nx, y = c / A.nx;
-    UnionIds<kKM> U;
-    const unsigned mask = __activemask();
-    const int n = fast_column<kKM>(A, E, x, y, sv + threadIdx.x, kMidThreads, U, mask);
-    if (FILL) {
-      if (n >= 0) write_union(A, U, n, oz + ooffs[c]);
-    } else if (n < 0) {
-      big_list[atomicAdd(big_count, 1)] = c;
-      counts[c] = 0;
-    } else {
-      counts[c] = n;
+  if (lane == 0) {
+    if (m > 0 && m <= kComps) M.bnd[m].y = carry;
+    M.bnd[0] = make_float2(INFINITY, -INFINITY);
+  }
+  m = min(m, kComps);  // any part of the cover may be left out
+  __syncwarp();
+  constexpr int COLS = Shape<G>::COLS;
+  if (S.g == 0) M.sv[S.col] = make_float2(-INFINITY, INFINITY);  // entry 0: bins without an entry, never updated
+  S.nent = m + 1;
+  // Entry k + 1: the bins wholly inside component k. Their intervals attach to
+  // the component, so only upper ends matter; the entry starts just short of
+  // the component's end, which a segment of every column reaches.
+  for (int k = 0; k < m; ++k) {
+    const float2 c = M.bnd[k + 1];
+    const int bf = (int)ceilf((c.x + 2.f * E) * S.inv_w + 0.5f), bl = (int)floorf((c.y - 2.f * E) * S.inv_w - 0.5f);
+    for (int b = max(bf, 0) + lane; b <= min(bl, kBins - 1); b += 32) M.cmap[b] = (unsigned short)(k + 1);
+    if (S.g == 0) {
+      const int a = COLS * (k + 1) + S.col;
+      M.sv[a] = make_float2(-INFINITY, c.y - 3.f * E);
+      M.idl[a] = make_int2(-1, 0);
+      M.idh[a] = make_int2(-1, 0);
     }
   }
+  __syncwarp();
+  // bins in which a component starts: segments there may lie in it. bnd holds the components shrunk by
+  // the guard band from here on.
+  for (int k = 0; k < m; ++k) {
+    const float2 c = M.bnd[k + 1], in = make_float2(c.x + E, c.y - E);
+    const int b = (int)bin_of(c.x, S.inv_w);
+    __syncwarp();
+    if (lane == 0) M.bnd[k + 1] = in;
+    if (M.cmap[b] == 0) {
+      if (lane == 0) M.bnd[S.nent] = in;
+      if (!new_entry<G>(M, S, b)) return false;
+    }
+  }
+  S.nbnd = S.nent;
+  __syncwarp();
+  return true;
 }
 
-// FP64 re-run of columns whose union outgrew kKM: same candidate set, exact
-// arithmetic, insertion into a large sorted list in global scratch.
+// Inserts a kept-aside interval into a column's finished union (n intervals);
+// returns the new count, or -1 beyond the capacity.
+template <int COLS>
+__device__ __noinline__ int insert_short(const FastArgs &A, float2 *cv, int2 *cl, int2 *ch, int n, int cap, float E,
+                                         float lo, float hi, int k, int da) {
+  const int2 il = make_int2(2 * k, da), ih = make_int2(2 * k + 1, da);
+  int j = 0;
+  while (j < n) {
+    const float t = lo - cv[COLS * j].y;
+    if (!GUARD(t, E, exact_less(A.H64, A.W, A.zx, ch[COLS * j], true, il, false))) break;
+    ++j;
+  }
+  if (j == n || GUARD(cv[COLS * j].x - hi, E, exact_less(A.H64, A.W, A.zx, ih, true, cl[COLS * j], false))) {
+    if (n >= cap) return -1;
+    for (int i = n; i > j; --i) {
+      cv[COLS * i] = cv[COLS * (i - 1)];
+      cl[COLS * i] = cl[COLS * (i - 1)];
+      ch[COLS * i] = ch[COLS * (i - 1)];
+    }
+    cv[COLS * j] = make_float2(lo, hi);
+    cl[COLS * j] = il;
+    ch[COLS * j] = ih;
+    return n + 1;
+  }
+  if (GUARD(cv[COLS * j].x - lo, E, exact_less(A.H64, A.W, A.zx, il, false, cl[COLS * j], false))) {
+    cv[COLS * j].x = lo;
+    cl[COLS * j] = il;
+  }
+  if (GUARD(hi - cv[COLS * j].y, E, exact_less(A.H64, A.W, A.zx, ch[COLS * j], true, ih, true))) {
+    cv[COLS * j].y = hi;
+    ch[COLS * j] = ih;
+    int i = j + 1;  // absorb the intervals that it now reaches
+    while (i < n) {
+      if (GUARD(cv[COLS * i].x - cv[COLS * j].y, E, exact_less(A.H64, A.W, A.zx, ch[COLS * j], true, cl[COLS * i], false)))
+        break;
+      if (GUARD(cv[COLS * i].y - cv[COLS * j].y, E, exact_less(A.H64, A.W, A.zx, ch[COLS * j], true, ch[COLS * i], true))) {
+        cv[COLS * j].y = cv[COLS * i].y;
+        ch[COLS * j] = ch[COLS * i];
+      }
+      ++i;
+    }
+    const int gone = i - j - 1;
+    if (gone > 0) {
+      for (; i < n; ++i) {
+        cv[COLS * (i - gone)] = cv[COLS * i];
+        cl[COLS * (i - gone)] = cl[COLS * i];
+        ch[COLS * (i - gone)] = ch[COLS * i];
+      }
+      n -= gone;
+    }
+  }
+  return n;
+}
+
+// The union of this lane's column, in M.cv / cl / ch: its interval count; -1
+// beyond a capacity (of any lane or of the patch); -2 when an end of this
+// lane's union has no identity (never for finite inputs).
+template <int G>
+__device__ __forceinline__ int patch_union(const FastArgs &A, const PatchMem &M, PatchState &S, int nbins) {
+  const int lane = S.lane;
+  const float E = S.E;
+  S.cshift = nbins > kCoverBins ? 1 : 0;
+  S.cthr = S.cshift ? 2.f * S.thr : S.thr;
+  const int cbins = (nbins + S.cshift) >> S.cshift;
+  for (int b = lane; b < cbins; b += 32) M.ml[b] = make_float2(INFINITY, -INFINITY);
+  for (int b = lane; b < kBins / 2; b += 32) reinterpret_cast<unsigned *>(M.cmap)[b] = 0u;
+  __syncwarp();
+  sweep<1, G>(A, M, S);
+  __syncwarp();
+  if (!cover_entries<G>(M, S, cbins)) return -1;
+  if (!sweep<2, G>(A, M, S)) return -1;
+  // the entries in bin order (bins inside one component share an entry), listed in the memory of the
+  // queue and loaded two ahead
+  unsigned short *const list = reinterpret_cast<unsigned short *>(M.ml);
+  int ne = 0;
+  for (int b0 = 0, last = 0; b0 < nbins; b0 += 32) {
+    const int e = M.cmap[b0 + lane];
+    int prev = __shfl_up_sync(kFull, e, 1);
+    if (lane == 0) prev = last;
+    last = __shfl_sync(kFull, e, 31);
+    const bool first = e != 0 && e != prev;
+    const unsigned w = __ballot_sync(kFull, first);
+    if (first) list[ne + __popc(w & ((1u << lane) - 1u))] = (unsigned short)e;
+    ne += __popc(w);
+  }
+  __syncwarp();
+  constexpr int COLS = Shape<G>::COLS;
+  int2 *const cl = M.cl + S.col, *const ch = M.ch + S.col;
+  float2 *const cv = M.cv + S.col;
+  if (S.g > 0) ne = 0;  // one lane per column
+  int n = 0;
+  bool open = false, full = false, bad = false;
+  float2 cur = make_float2(0.f, 0.f);
+  int2 il = make_int2(-1, 0), ih = make_int2(-1, 0);
+  constexpr int kAhead = 3;
+  float2 pv[kAhead];
+  int2 pl[kAhead], ph[kAhead];
+#pragma unroll
+  for (int i = 0; i < kAhead; ++i) {
+    const int e = COLS * (i < ne ? list[i] : 0) + S.col;
+    pv[i] = M.sv[e];
+    pl[i] = M.idl[e];
+    ph[i] = M.idh[e];
+  }
+  for (int j0 = 0; j0 < ne; j0 += kAhead) {
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i) {
+      const int j = j0 + i;
+      if (j >= ne) break;
+      float2 v = pv[i];
+      const int2 vl = pl[i], vh = ph[i];
+      {
+        const int e = COLS * (j + kAhead < ne ? list[j + kAhead] : 0) + S.col;
+        pv[i] = M.sv[e];
+        pl[i] = M.idl[e];
+        ph[i] = M.idh[e];
+      }
+      if (!(v.y > -INFINITY)) continue;
+      v.x -= E;
+      v.y += E;
+      if (open) {
+        const float t = v.x - cur.y;
+        if (!GUARD(t, E, vl.x >= 0 && ih.x >= 0 && exact_less(A.H64, A.W, A.zx, ih, true, vl, false))) {
+          // overlapping or touching: extend the open interval
+          const float tl = cur.x - v.x;
+          if (vl.x >= 0 && il.x >= 0 && GUARD(tl, E, exact_less(A.H64, A.W, A.zx, vl, false, il, false))) {
+            cur.x = v.x;  // a tie across a bin's edge
+            il = vl;
+            if (n > 0 && !GUARD(cur.x - cv[COLS * (n - 1)].y, E,
+                                exact_less(A.H64, A.W, A.zx, ch[COLS * (n - 1)], true, il, false))) {
+              --n;  // it reaches the interval before
+              cur.x = cv[COLS * n].x;
+              il = cl[COLS * n];
+              if (ih.x < 0 || GUARD(cv[COLS * n].y - cur.y, E, exact_less(A.H64, A.W, A.zx, ih, true, ch[COLS * n], true))) {
+                cur.y = cv[COLS * n].y;
+                ih = ch[COLS * n];
+              }
+            }
+          }
+          const float th = v.y - cur.y;
+          if (GUARD(th, E, ih.x < 0 || (vh.x >= 0 && exact_less(A.H64, A.W, A.zx, ih, true, vh, true)))) {
+            cur.y = v.y;
+            ih = vh;
+          }
+          continue;
+        }
+        if (n < M.nunion - 1) {
+          cv[COLS * n] = cur;
+          cl[COLS * n] = il;
+          ch[COLS * n] = ih;
+          bad |= il.x < 0 || ih.x < 0;
+          ++n;
+        } else {
+          full = true;
+        }
+      }
+      open = true;
+      cur = v;
+      il = vl;
+      ih = vh;
+    }
+  }
+  if (open) {
+    if (n < M.nunion - 1) {
+      cv[COLS * n] = cur;
+      cl[COLS * n] = il;
+      ch[COLS * n] = ih;
+      bad |= il.x < 0 || ih.x < 0;
+      ++n;
+    } else {
+      full = true;
+    }
+  }
+  // kept-aside segments
+  for (int s = 0; s < (S.g == 0 ? S.ns : 0); s += 4) {
+    // four at a time, so that their loads overlap
+    float lo[4], hi[4];
+    int key[4], da[4];
+    unsigned need = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float4 c = M.shorts[min(s + i, S.ns - 1)];
+      const int at = __float_as_int(c.w);
+      const int dx = abs((at & 0xffff) - 1024 - S.lx), dy = abs((at >> 16) - 1024 - S.ly);
+      const float h = A.Hp[dy * A.hs + dx];
+      lo[i] = c.x - h;
+      hi[i] = c.y + h;
+      key[i] = __float_as_int(c.z);
+      da[i] = dy | (dx << 8);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 v = M.sv[COLS * M.cmap[bin_of(lo[i], S.inv_w)] + S.col];
+      // intervals that are long in this column have been merged
+      if (s + i < S.ns && hi[i] >= lo[i] && hi[i] - lo[i] < S.thr && (lo[i] < v.x || hi[i] > v.y)) need |= 1u << i;
+    }
+    if (full || bad) need = 0;
+    for (; need; need &= need - 1) {
+      const int i = __ffs(need) - 1;
+      const float l = i == 0 ? lo[0] : i == 1 ? lo[1] : i == 2 ? lo[2] : lo[3];
+      const float u = i == 0 ? hi[0] : i == 1 ? hi[1] : i == 2 ? hi[2] : hi[3];
+      const int ks = i == 0 ? key[0] : i == 1 ? key[1] : i == 2 ? key[2] : key[3];
+      const int ds = i == 0 ? da[0] : i == 1 ? da[1] : i == 2 ? da[2] : da[3];
+      const int r = insert_short<COLS>(A, cv, cl, ch, n, M.nunion - 1, E, l, u, ks, ds);
+      if (r < 0) {
+        full = true;
+        need = 0;
+        break;
+      }
+      n = r;
+    }
+  }
+  if (__any_sync(kFull, full)) return -1;
+  return bad ? -2 : n;
+}
+
+// Output slot of column (x, y) for an n-interval union: the column's own slot
+// when its capacity allows, else spill space, else false (the dilation's
+// overflow flag is then set). Slot indices are unsigned 32-bit.
+__device__ __forceinline__ bool place_union(const BatchVol &V, int x, int y, int n, unsigned &dst) {
+  const int nx = V.A.nx;
+  int cap = V.cap;
+  if (V.tcap) {
+    const int tx = x / kSizerTile, ty = y / kSizerTile, t = tx + V.tiles32_x * ty;
+    const int w = min(kSizerTile, nx - tx * kSizerTile);
+    cap = V.tcap[t];
+    dst = (unsigned)V.toff[t] + (unsigned)(((x - tx * kSizerTile) + w * (y - ty * kSizerTile)) * cap);
+  } else {
+    dst = (unsigned)(x + nx * y) * (unsigned)cap;
+  }
+  if (n > cap) {
+    const unsigned off = atomicAdd(V.spill_used, (unsigned)n);
+    if (off + (unsigned)n <= V.spill_cap) {
+      dst = V.spill_base + off;
+      return true;
+    }
+    atomicOr(V.ovf, 4);  // spill region exhausted
+    return false;
+  }
+  return true;
+}
+
+// Persistent: a warp per block takes patches of the launch's dilations from a
+// queue (dilations in the order of vols; each one's patches in bands of 512
+// columns, all rows of a band before the next, so that the patches in flight
+// share their source rows in L2). BIG: the second tier, over the patches that
+// the first one listed, with larger working lists.
+template <bool BIG, int G>
+__global__ void __launch_bounds__(32, 20) k_patch(const BatchVol *__restrict__ vols, int nitems, PatchQueue Q,
+                                                  int hs_max, PatchScratch scratch) {
+  constexpr int ne = BIG ? kEntriesBig : kEntries, PX = Shape<G>::PX, COLS = Shape<G>::COLS;
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ BatchVol V;
+  PatchMem M;
+  M.ne = ne;
+  M.nunion = BIG ? kUnionBig : kUnion;
+  M.nshort = BIG ? kShortBig : kShort;
+  const size_t wb = blockIdx.x;
+  // shared memory: what lasts for the whole patch, then the bins of the cover, whose memory the queue,
+  // the cluster list and the rows of H take over in the second sweep
+  unsigned char *p = smem;
+  M.bnd = reinterpret_cast<float2 *>(p);
+  p += sizeof(float2) * (2 * kComps + 2);
+  M.cmap = reinterpret_cast<unsigned short *>(p);
+  p += sizeof(unsigned short) * kBins;
+  M.hrow1 = reinterpret_cast<float *>(p);
+  p += sizeof(float) * hs_max;
+  M.ml = reinterpret_cast<float2 *>(p);
+  M.hrow = reinterpret_cast<float *>(p);
+  p += sizeof(float) * (2 * kTile - 1) * hs_max;
+  M.queue = reinterpret_cast<float4 *>(p);
+  p += sizeof(float4) * (kQueue + kPad);
+  M.clist = reinterpret_cast<int2 *>(p);
+  p += sizeof(int2) * kClusters;
+  M.qk = reinterpret_cast<int *>(p);
+  M.sv = scratch.sv + wb * COLS * ne;
+  M.shorts = scratch.shorts + wb * M.nshort;
+  M.idl = scratch.ids + wb * 2 * COLS * ne;
+  M.idh = M.idl + COLS * ne;
+  M.cv = scratch.cv + wb * COLS * M.nunion;
+  M.cl = scratch.cids + wb * 2 * COLS * M.nunion;
+  M.ch = M.cl + COLS * M.nunion;
+  PatchState S;
+  S.lane = threadIdx.x;
+  S.col = threadIdx.x % COLS;
+  S.g = threadIdx.x / COLS;
+  S.lx = S.col % PX;
+  S.ly = S.col / PX;
+  int cur = -1;
+  const int todo = BIG ? min(Q.count[1], nitems) : nitems;
+  for (;;) {
+    int item = 0;
+    if (S.lane == 0) item = atomicAdd(&Q.count[BIG ? 2 : 0], 1);
+    item = __shfl_sync(kFull, item, 0);
+    if (item >= todo) return;
+    if (BIG) item = Q.list[item];
+    int v = max(cur, 0);
+    if (BIG)
+      while (item < vols[v].item0) --v;
+    while (item >= vols[v].item1) ++v;
+    if (v != cur) {
+      __syncwarp();
+      for (int i = S.lane; i < (int)(sizeof(BatchVol) / sizeof(int)); i += 32)
+        reinterpret_cast<int *>(&V)[i] = reinterpret_cast<const int *>(&vols[v])[i];
+      cur = v;
+      __syncwarp();
+    }
+    constexpr int kBand = 512 / PX;
+    const int nx = V.A.nx, ny = V.A.ny;
+    const int tiles_x = (nx + PX - 1) / PX, tiles_y = (ny + kPatchY - 1) / kPatchY;
+    const int rel = item - V.item0, band = rel / (kBand * tiles_y), rb = rel - band * kBand * tiles_y;
+    const int bw = min(kBand, tiles_x - band * kBand);
+    S.X0 = (band * kBand + rb % bw) * PX;
+    S.Y0 = (rb / bw) * kPatchY;
+    S.nent = 1;
+    S.ns = S.qn = S.cn = 0;
+    const FastPar *par = V.A.par;
+    S.E = par->E;
+    S.inv_w = par->inv_w;
+    S.thr = par->thr;
+    const int n = patch_union<G>(V.A, M, S, par->nbins);
+    const int x = S.X0 + S.lx, y = S.Y0 + S.ly;
+    const bool in = S.g == 0 && x < nx && y < ny;
+    const bool over = __any_sync(kFull, n == -1);
+    if (over && !BIG) {  // the whole patch goes to the next tier
+      const int cols = __popc(__ballot_sync(kFull, in));
+      if (S.lane == 0) {
+        Q.list[atomicAdd(&Q.count[1], 1)] = item;
+        atomicAdd(&Q.count[3], cols);
+      }
+      if (in) V.obeg[x + nx * y] = V.oend[x + nx * y] = 0;
+    } else if (in) {
+      const int c = x + nx * y;
+      unsigned dst = 0;
+      int m = n;
+      if (over || n < 0) {
+        V.big_list[atomicAdd(V.big_count, 1)] = c;  // the FP64 tier
+        m = 0;
+      } else if (!place_union(V, x, y, n, dst)) {
+        m = 0;
+        dst = 0;
+      } else {
+        double2 *o = V.oz + dst;
+        for (int k = 0; k < n; ++k)
+          o[k] = make_double2(exact_val(V.A.H64, V.A.W, V.A.zx, M.cl[COLS * k + S.col], false),
+                              exact_val(V.A.H64, V.A.W, V.A.zx, M.ch[COLS * k + S.col], true));
+      }
+      V.obeg[c] = (int32_t)dst;
+      V.oend[c] = (int32_t)(dst + (unsigned)m);
+    }
+    __syncwarp();
+  }
+}
+
+// ------------------------------------------------------------ last tier
+
+// Inserts [lo, hi] into the sorted list L of n disjoint closed intervals.
 __device__ bool big_insert(double2 *L, int &n, int cap, double lo, double hi) {
   int l = 0, r = n;
   while (l < r) {
@@ -454,307 +1204,10 @@ __device__ bool big_insert(double2 *L, int &n, int cap, double lo, double hi) {
   return true;
 }
 
-template <bool FILL>
-__global__ void __launch_bounds__(kBigThreads) k_fast_big(FastArgs A, int32_t *counts, const int32_t *ooffs,
-                                                         double2 *oz, const int *ovf_count, const int *ovf_cols,
-                                                         double2 *scratch, int *fatal) {
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
-  double2 *L = scratch + (size_t)tid * kBigCap;
-  for (int i = tid; i < *ovf_count; i += nth) {
-    const int c = ovf_cols[i];
-    const int x = c % A.nx, y = c / A.nx;
-    int n = 0;
-    bool ok = true;
-    for (int p = 0; p < A.npairs && ok; ++p) {
-      const int2 ad = A.pairs[p];
-      const int a = ad.x, d = ad.y;
-      const double h = A.H64[d * A.W + a];
-      for (int s = 0; s < 4 && ok; ++s) {
-        const int xs = (s & 1) ? x + a : x - a;
-        const int ys = (s & 2) ? y + d : y - d;
-        if ((s & 1) && a == 0) continue;
-        if ((s & 2) && d == 0) continue;
-        if (xs < 0 || xs >= A.nx || ys < 0 || ys >= A.ny) continue;
-        const int cs = xs + A.nx * ys;
-        for (int k = A.beg[cs]; k < A.end[cs] && ok; ++k)
-          ok = big_insert(L, n, kBigCap, __dsub_rn(A.zd[2 * k], h), __dadd_rn(A.zd[2 * k + 1], h));
-      }
-    }
-    if (!ok) {
-      *fatal = 1;
-      n = 0;
-    }
-    if (FILL) {
-      double2 *o = oz + ooffs[c];
-      for (int k = 0; k < n; ++k) o[k] = L[k];
-    } else {
-      counts[c] = n;
-    }
-  }
-}
-
-// ---------------------------------------------------------------- helpers
-
-// FP32 copies of the values of columns [beg, end) (slot layouts leave unused
-// slots, which are skipped) and max |z| for the guard band.
-__global__ void k_to_f32_cols(int ncols, const int32_t *beg, const int32_t *end, const double *zd, float *zf,
-                              unsigned int *maxabs_bits) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  unsigned int m = 0;
-  if (c < ncols)
-    for (int k = 2 * beg[c]; k < 2 * end[c]; ++k) {
-      const float f = __double2float_rn(zd[k]);
-      zf[k] = f;
-      const unsigned int b = __float_as_uint(fabsf(f));
-      m = b > m ? b : m;
-    }
-  for (int o = 16; o > 0; o >>= 1) {
-    const unsigned int t = __shfl_xor_sync(0xffffffffu, m, o);
-    m = t > m ? t : m;
-  }
-  if ((threadIdx.x & 31) == 0) atomicMax(maxabs_bits, m);
-}
-
-// Guard band: E bounds the error of an FP32 comparison t = y - x of two
-// candidate endpoints (each within 1.5 ulp of its FP64 value: rounding of z,
-// of H and of the sum), plus the rounding of t itself: 4 ulp32(U) for
-// magnitudes up to U; E = 2^-20 * U leaves a factor two of margin.
-__global__ void k_guard(const unsigned int *maxabs_bits, float R, float *E) {
-  const float U = __uint_as_float(*maxabs_bits) + R + 1.0f;
-  *E = U * 9.5367431640625e-07f;  // 2^-20
-}
-
-// Lower bounds of the growth of H per lattice step toward the centre.
-__global__ void k_dh_tables(int Dy, int W, const double *__restrict__ H, const int *__restrict__ Dx,
-                            float *__restrict__ dH) {
-  const int n = (Dy + 1) * W;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int d = i / W, a = i % W;
-  float fx = -INFINITY, fy = -INFINITY;
-  if (a <= Dx[d]) {
-    if (a >= 1) fx = __double2float_rd(__dsub_rd(H[d * W + a - 1], H[i]));
-    if (d >= 1) fy = __double2float_rd(__dsub_rd(H[(d - 1) * W + a], H[i]));
-  }
-  dH[i] = fx;
-  dH[n + i] = fy;
-}
-
-// Dominance widths, one thread per column. For segment i and direction k
-// (neighbour (x-1, y), (x+1, y), (x, y-1), (x, y+1)):
-//   w_i = min over the neighbour's segments j of max(z1_j - z1_i, z2_i - z2_j),
-// evaluated in FP32 on bounds of the FP64 values with every difference
-// rounded up, so w bounds the exact value from above (+inf outside the grid
-// or without a neighbour segment). The scan stops after the
-// first neighbour segment starting above segment i: every later neighbour
-// segment gives a larger value. The column's width per direction is the max
-// over its segments (-inf for an empty column), stored as FP16 rounded up in
-// the column record col[c] = (beg, end, x- | x+ << 16, y- | y+ << 16).
-__global__ void k_dominance(int nx, int ny, const int32_t *__restrict__ beg, const int32_t *__restrict__ end,
-                            const float2 *__restrict__ zf, int4 *__restrict__ col, void *__restrict__ dmask,
-                            int mask_bits, const DomLevels L) {
-  const int ncols = nx * ny;
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ncols) return;
-  const int x = c % nx, y = c / nx;
-  const int k0 = beg[c], k1 = end[c];
-  int nb0[4], nb1[4];
-  for (int k = 0; k < 4; ++k) {
-    const int xn = x + (k == 0 ? -1 : k == 1 ? 1 : 0), yn = y + (k == 2 ? -1 : k == 3 ? 1 : 0);
-    const bool in = xn >= 0 && xn < nx && yn >= 0 && yn < ny;
-    const int cn = in ? xn + nx * yn : 0;
-    nb0[k] = in ? beg[cn] : 0;
-    nb1[k] = in ? end[cn] : 0;
-  }
-  float cmax[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-  unsigned bits[4][kDomLevels];
-  for (int k = 0; k < 4; ++k)
-    for (int l = 0; l < kDomLevels; ++l) bits[k][l] = 0u;
-  const bool masked = k1 - k0 <= mask_bits;
-  for (int i = k0; i < k1; ++i) {
-    // bounds of the exact values: an FP32 copy is within half an ulp of its
-    // FP64 value, so the neighbouring floats enclose it
-    const float2 fi = zf[i];
-    const float i1 = nextafterf(fi.x, -INFINITY), i2 = nextafterf(fi.y, INFINITY);
-    for (int k = 0; k < 4; ++k) {
-      float best = INFINITY;
-      for (int j = nb0[k]; j < nb1[k]; ++j) {
-        const float2 fj = zf[j];
-        const float lo = __fsub_ru(nextafterf(fj.x, INFINITY), i1);
-        const float hi = __fsub_ru(i2, nextafterf(fj.y, -INFINITY));
-        const float m = lo > hi ? lo : hi;
-        best = m < best ? m : best;
-        if (fj.x > fi.y) break;  // any early stop only leaves the bound larger
-      }
-      cmax[k] = best > cmax[k] ? best : cmax[k];
-      if (masked)
-        for (int l = 0; l < kDomLevels; ++l)
-          if (best <= L.t[l]) bits[k][l] |= 1u << (i - k0);
-    }
-  }
-  if (dmask)
-    for (int k = 0; k < 4; ++k)
-      for (int l = 0; l < kDomLevels; ++l) {
-        const size_t idx = (size_t)(k * kDomLevels + l) * ncols + c;
-        if (mask_bits == 16) static_cast<unsigned short *>(dmask)[idx] = (unsigned short)bits[k][l];
-        else static_cast<unsigned *>(dmask)[idx] = bits[k][l];
-      }
-  unsigned h[4];
-  for (int k = 0; k < 4; ++k) h[k] = __half_as_ushort(__float2half_ru(cmax[k]));
-  col[c] = make_int4(k0, k1, (int)(h[0] | (h[1] << 16)), (int)(h[2] | (h[3] << 16)));
-}
-
-static_assert(kDomLevels <= 15, "pair records hold a level in 4 bits, 15 meaning none");
-
-// Largest dominance level whose threshold is <= dh (15: none).
-__device__ __forceinline__ int dom_level_of(float dh, const DomLevels &L) {
-  int lv = 15;
-  for (int l = 0; l < kDomLevels; ++l)
-    if (L.t[l] <= dh) lv = l;
-  return lv;
-}
-
-// Pair records: (a | d << 8 | x-step level << 16 | y-step level << 20 as
-// float bits, H in FP32, dH x step, dH y step).
-__global__ void k_pair_records(const int2 *__restrict__ pairs, int npairs, const float *__restrict__ Hf,
-                               const float *__restrict__ dH, int W, int dHy, float4 *__restrict__ prec,
-                               const DomLevels L) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= npairs) return;
-  const int a = pairs[p].x, d = pairs[p].y;
-  const float dx = dH[d * W + a], dy = dH[dHy + d * W + a];
-  const int code = a | (d << 8) | (dom_level_of(dx, L) << 16) | (dom_level_of(dy, L) << 20);
-  prec[p] = make_float4(__int_as_float(code), Hf[d * W + a], dx, dy);
-}
-
-// ---------------------------------------------------------------- batches
-
-static_assert(sizeof(BatchVol) % sizeof(int) == 0, "BatchVol is copied as ints");
-
-// Output slot of column (x, y) of a batch dilation for an n-interval union:
-// the column's own slot when its tile capacity allows, else spill space, else
-// -1 (the dilation's overflow flag is then set).
-__device__ __forceinline__ int place_union(const BatchVol &V, int x, int y, int n) {
-  const int nx = V.A.nx;
-  int cap = V.cap, dst;
-  if (V.tcap) {
-    const int tx = x / kSizerTile, ty = y / kSizerTile, t = tx + V.tiles32_x * ty;
-    const int w = min(kSizerTile, nx - tx * kSizerTile);
-    cap = V.tcap[t];
-    dst = V.toff[t] + ((x - tx * kSizerTile) + w * (y - ty * kSizerTile)) * cap;
-  } else {
-    dst = (x + nx * y) * cap;
-  }
-  if (n > cap) {
-    const int off = atomicAdd(V.spill_used, n);
-    if (off + n <= V.spill_cap) return V.spill_base + off;
-    atomicOr(V.ovf, 4);  // spill region exhausted
-    return -1;
-  }
-  return dst;
-}
-
-// Persistent kernel over the tiles (FBY patches of 8 x 4 output columns) of every
-// dilation of a batch: blocks pull (dilation, tile) items from a queue ordered
-// by decreasing estimated work, so uneven volumes balance across the SMs.
-// Each column's union goes to its slot (place_union); a union of more than
-// KA - 1 intervals is listed for k_fast_batched_mid.
-// SINGLE: the round has one dilation, whose arguments come as the kernel
-// parameter A1 (constant bank) instead of from memory.
-// LBN / (kFB * FBY) blocks per SM bound the registers: LBN = 1024 gives 64
-// per thread (32 warps per SM, some spills), 768 gives 85 (24 warps); the
-// autotuner picks per round (the first wins on the 2048^2 r=32 dilation).
-template <int KA, int FBY, bool SINGLE, int LBN>
-__global__ void __launch_bounds__(kFB *FBY, LBN / (kFB * FBY)) k_fast_batched(const BatchVol *vols,
-                                                                               const int2 *queue, int nq, int *next,
-                                                                               const FastArgs A1) {
-  extern __shared__ float2 sv_dyn[];
-  __shared__ int s_item;
-  __shared__ BatchVol s_vol;  // the item's arguments, read by every thread in the hot loop
-  const int tid = threadIdx.x + kFB * threadIdx.y;
-  int cur_vol = -1;
-  for (;;) {
-    if (tid == 0) s_item = atomicAdd(next, 1);
-    __syncthreads();
-    const int item = s_item;
-    if (item >= nq) return;
-    const int2 q = queue[item];
-    if (q.x != cur_vol) {
-      for (int i = tid; i < (int)(sizeof(BatchVol) / sizeof(int)); i += kFB * FBY)
-        reinterpret_cast<int *>(&s_vol)[i] = reinterpret_cast<const int *>(&vols[q.x])[i];
-      cur_vol = q.x;
-    }
-    __syncthreads();
-    const BatchVol &V = s_vol;
-    const int nx = V.A.nx, ny = V.A.ny;
-    const int bw = kPatchX * FBY;  // the item's columns: bw x kPatchY, warp w at x offset w * kPatchX
-    const int tiles_x = (nx + bw - 1) / bw;
-    const int x = (q.y % tiles_x) * bw + threadIdx.y * kPatchX + threadIdx.x % kPatchX;
-    const int y = (q.y / tiles_x) * kPatchY + threadIdx.x / kPatchX;
-    if (x < nx && y < ny) {
-      const int c = x + nx * y;
-      UnionIds<KA> U;
-      const unsigned mask = __activemask();
-      const FastArgs &A = SINGLE ? A1 : V.A;
-      int n = fast_column<KA>(A, *A.E, x, y, sv_dyn + tid, kFB * FBY, U, mask);
-      int dst = 0;
-      if (n < 0) {
-        V.mid_list[atomicAdd(V.mid_count, 1)] = c;
-        n = 0;
-      } else {
-        dst = place_union(V, x, y, n);
-        if (dst < 0) {
-          dst = 0;
-          n = 0;
-        } else {
-          write_union(A, U, n, V.oz + dst);
-        }
-      }
-      V.obeg[c] = dst;
-      V.oend[c] = dst + n;
-    }
-  }
-}
-
-// Second tier of a batch round: the listed columns of every dilation with
-// kKM slots, placed like the first tier; a union of more than kKM - 1
-// intervals sets the dilation's overflow flag.
-__global__ void __launch_bounds__(kMidThreads) k_fast_batched_mid(const BatchVol *vols, int nv) {
-  __shared__ float2 sv[kKM * kMidThreads];
-  const int nth = gridDim.x * kMidThreads;
-  for (int v = 0; v < nv; ++v) {
-    const BatchVol &V = vols[v];
-    const int m = *V.mid_count;
-    for (int i = blockIdx.x * kMidThreads + threadIdx.x; i < m; i += nth) {
-      const int c = V.mid_list[i];
-      const int x = c % V.A.nx, y = c / V.A.nx;
-      UnionIds<kKM> U;
-      const unsigned mask = __activemask();
-      int n = fast_column<kKM>(V.A, *V.A.E, x, y, sv + threadIdx.x, kMidThreads, U, mask);
-      int dst = -1;
-      if (n < 0) {
-        V.big_list[atomicAdd(V.big_count, 1)] = c;  // third tier
-        n = 0;
-        dst = 0;
-      } else {
-        dst = place_union(V, x, y, n);
-      }
-      if (dst < 0) {
-        dst = 0;
-        n = 0;
-      } else if (n > 0) {
-        write_union(V.A, U, n, V.oz + dst);
-      }
-      V.obeg[c] = dst;
-      V.oend[c] = dst + n;
-    }
-  }
-}
-
-// Third tier of a batch round (FP64, grid-stride): the columns whose union
-// exceeds kKM, each built in a kBigCap-interval list in global scratch and
-// placed like the other tiers; a union beyond kBigCap sets the overflow flag.
-__global__ void __launch_bounds__(kBigThreads) k_fast_batched_big(const BatchVol *vols, int nv, double2 *scratch) {
+// The listed columns of every dilation in FP64 (grid-stride), each built in a
+// kBigCap-interval list in global scratch and placed like the other tiers; a
+// union beyond kBigCap sets the overflow flag.
+__global__ void __launch_bounds__(kBigThreads) k_big(const BatchVol *vols, int nv, double2 *scratch) {
   const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
   double2 *L = scratch + (size_t)tid * kBigCap;
   for (int v = 0; v < nv; ++v) {
@@ -766,37 +1219,31 @@ __global__ void __launch_bounds__(kBigThreads) k_fast_batched_big(const BatchVol
       const int x = c % A.nx, y = c / A.nx;
       int n = 0;
       bool ok = true;
-      for (int p = 0; p < A.npairs && ok; ++p) {
-        const int2 ad = A.pairs[p];
-        const int a = ad.x, d = ad.y;
-        const double h = A.H64[d * A.W + a];
-        for (int s = 0; s < 4 && ok; ++s) {
-          const int xs = (s & 1) ? x + a : x - a;
-          const int ys = (s & 2) ? y + d : y - d;
-          if ((s & 1) && a == 0) continue;
-          if ((s & 2) && d == 0) continue;
-          if (xs < 0 || xs >= A.nx || ys < 0 || ys >= A.ny) continue;
+      for (int ys = max(0, y - A.Dy); ys <= min(A.ny - 1, y + A.Dy) && ok; ++ys) {
+        const int d = abs(ys - y), reach = A.Dx[d];
+        for (int xs = max(0, x - reach); xs <= min(A.nx - 1, x + reach) && ok; ++xs) {
+          const double h = A.H64[d * A.W + abs(xs - x)];
           const int cs = xs + A.nx * ys;
           for (int k = A.beg[cs]; k < A.end[cs] && ok; ++k)
             ok = big_insert(L, n, kBigCap, __dsub_rn(A.zd[2 * k], h), __dadd_rn(A.zd[2 * k + 1], h));
         }
       }
-      int dst = -1;
-      if (!ok)
+      unsigned dst = 0;
+      if (!ok) {
         atomicOr(V.ovf, 1);
-      else
-        dst = place_union(V, x, y, n);
-      if (dst < 0) {
-        dst = 0;
         n = 0;
-      } else {
-        for (int k = 0; k < n; ++k) V.oz[dst + k] = L[k];
+      } else if (!place_union(V, x, y, n, dst)) {
+        n = 0;
+        dst = 0;
       }
-      V.obeg[c] = dst;
-      V.oend[c] = dst + n;
+      for (int k = 0; k < n; ++k) V.oz[dst + k] = L[k];
+      V.obeg[c] = (int32_t)dst;
+      V.oend[c] = (int32_t)(dst + (unsigned)n);
     }
   }
 }
+
+static_assert(sizeof(BatchVol) % sizeof(int) == 0, "BatchVol is copied as ints");
 
 }  // namespace
 
@@ -811,7 +1258,124 @@ int sm_count_fast() {
   return sms > 0 ? sms : 148;
 }
 
+size_t patch_smem(int hs_max) {
+  const size_t kept = sizeof(float2) * (2 * kComps + 2) + sizeof(unsigned short) * kBins + sizeof(float) * hs_max;
+  const size_t second = sizeof(float) * (2 * kTile - 1) * hs_max + (sizeof(float4) + sizeof(int)) * (kQueue + kPad) +
+                        sizeof(int2) * kClusters;
+  return kept + std::max(second, sizeof(float2) * kCoverBins);
+}
+
 }  // namespace
+
+int patch_count(const vo_grid &g, int split) {
+  const int px = kPatchX / split;
+  return ((g.nx + px - 1) / px) * ((g.ny + kPatchY - 1) / kPatchY);
+}
+
+// Lanes per column for a launch over the given columns. A launch of few
+// patches is bound by the longest one's chain of dependent steps, not by
+// throughput: with four lanes per column a warp merges four segments at a
+// time into 2 x 4 columns, at the cost of sweeping the same clusters four
+// times as often.
+int64_t patch_total(const vo_grid *const *grids, int n) {
+  int64_t patches = 0;
+  for (int i = 0; i < n; ++i) patches += patch_count(*grids[i], 1);
+  return patches;
+}
+int patch_split(const vo_grid *const *grids, int n) {
+  const int64_t patches = patch_total(grids, n);
+  return patches <= 9 * (int64_t)sm_count_fast() ? kSplit : 1;
+}
+
+namespace {
+using PatchFn = void (*)(const BatchVol *, int, PatchQueue, int, PatchScratch);
+PatchFn patch_fn(bool big, int split) {
+  return split == 1 ? (big ? &k_patch<true, 1> : &k_patch<false, 1>)
+                    : (big ? &k_patch<true, kSplit> : &k_patch<false, kSplit>);
+}
+}  // namespace
+
+void patch_launch(bool big, const PatchPlan &P, cudaStream_t st, const BatchVol *vols) {
+  patch_fn(big, P.split)<<<P.grid[big], 32, patch_smem(P.hs_max), st>>>(vols, P.nitems, P.Q, P.hs_max, P.scratch[big]);
+}
+
+int patch_plan(vo_ctx *ctx, int nitems, int split, int hs_max, PatchPlan &P) {
+  P = PatchPlan();
+  P.nitems = nitems;
+  P.split = split;
+  P.hs_max = hs_max;
+  int per_sm = 0;
+  cudaError_t e =
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, patch_fn(false, split), 32, patch_smem(hs_max));
+  if (e != cudaSuccess) return cuda_error(ctx, e, "k_patch");
+  P.grid[0] = std::max(1, std::min(nitems, std::max(1, per_sm) * sm_count_fast()));
+  P.grid[1] = std::max(1, std::min(nitems, kPatchBigBlocks));
+  return VO_OK;
+}
+
+namespace {
+size_t tier_entries(bool big) { return big ? kEntriesBig : kEntries; }
+size_t tier_unions(bool big) { return big ? kUnionBig : kUnion; }
+size_t tier_shorts(bool big) { return big ? kShortBig : kShort; }
+}  // namespace
+
+size_t patch_scratch_bytes(const PatchPlan &P, bool big) {
+  const size_t cols = 32 / P.split;
+  return P.grid[big] * (cols * (tier_entries(big) + tier_unions(big)) * (sizeof(float2) + 2 * sizeof(int2)) +
+                        tier_shorts(big) * sizeof(float4));
+}
+
+void patch_scratch_set(PatchPlan &P, bool big, void *mem) {
+  const size_t w = P.grid[big], ne = tier_entries(big), nu = tier_unions(big), cols = 32 / P.split;
+  PatchScratch &S = P.scratch[big];
+  unsigned char *p = static_cast<unsigned char *>(mem);
+  S.shorts = reinterpret_cast<float4 *>(p);
+  p += w * tier_shorts(big) * sizeof(float4);
+  S.sv = reinterpret_cast<float2 *>(p);
+  p += w * cols * ne * sizeof(float2);
+  S.ids = reinterpret_cast<int2 *>(p);
+  p += w * 2 * cols * ne * sizeof(int2);
+  S.cv = reinterpret_cast<float2 *>(p);
+  p += w * cols * nu * sizeof(float2);
+  S.cids = reinterpret_cast<int2 *>(p);
+}
+
+size_t big_scratch_elems() { return (size_t)kBigBlocks * kBigThreads * kBigCap; }
+
+void big_launch(cudaStream_t st, const BatchVol *vols, int nv, double2 *scratch) {
+  k_big<<<kBigBlocks, kBigThreads, 0, st>>>(vols, nv, scratch);
+}
+
+size_t pack_offsets(const vo_grid &g) {
+  return (size_t)((g.ny + kTile - 1) / kTile) * ((g.nx + kTile - 1) / kTile + 1);
+}
+
+void fast_prepare(cudaStream_t st, const FastArgs &A, float R, double mean_segs, unsigned long long *mm,
+                  const PackOut &out) {
+  const int ncols = A.nx * A.ny;
+  const double2 *z = reinterpret_cast<const double2 *>(A.zd);
+  cudaMemsetAsync(mm, 0, 3 * sizeof(unsigned long long), st);
+  const int grid = std::max(1, std::min((ncols + 255) / 256, 8 * sm_count_fast()));
+  k_range<<<grid, 256, 0, st>>>(ncols, A.beg, A.end, z, R, mm, out.par);
+  // warps per block by the segments of a tile: twice the mean should fit a warp's share of the sort
+  const double most = 2.2 * mean_segs * kTile * std::min(kTile, A.ny);
+  const int warps = most <= kPackSort / 32 ? 32 : most <= kPackSort / 16 ? 16 : 8;
+  auto *pack = warps == 32 ? &k_pack<32> : warps == 16 ? &k_pack<16> : &k_pack<8>;
+  pack<<<(A.ny + kTile - 1) / kTile, 32 * warps, 0, st>>>(A.nx, A.ny, A.beg, A.end, z, out.par, out.zf, out.code, out.zx,
+                                                          out.cl, out.coff);
+}
+
+FastArgs fast_args(int nx, int ny, const DeviceTables &T, const int32_t *beg, const int32_t *end, const double2 *z,
+                   const PackOut &out) {
+  return FastArgs{nx,  ny,  T.host.W, T.host.Dy, T.host.hs, beg, end, (const double *)z, out.zf, out.code,
+                  (const double *)out.zx, out.cl, out.coff, T.Hp, T.H, T.Dx, out.par};
+}
+
+// Slots per column of a single dilation's output (the rest goes to the spill
+// region), from the input's mean segment count per column.
+static int slot_cap(double mean_segs) {
+  return mean_segs > 24.0 ? 64 : mean_segs > 10.0 ? 48 : mean_segs > 6.0 ? 32 : 24;
+}
 
 int dilate_fast(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out, vo_timings *tm) {
   const vo_grid g = in->grid;
@@ -819,247 +1383,129 @@ int dilate_fast(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out, vo_
   const DeviceTables *T = nullptr;
   int rc = get_tables(ctx, R, std::max(nx, ny), &T);
   if (rc) return rc;
-  const Tables &h = T->host;
-  const std::vector<int2> pairs = fast_pairs(h);
-  float *zf = nullptr, *dE = nullptr;
-  int4 *col = nullptr;
-  float4 *prec = nullptr;
-  unsigned *dmask = nullptr;
-  unsigned int *dmax = nullptr;
-  int2 *dpairs = nullptr;
-  int32_t *counts = nullptr;
-  int *ovf_cols = nullptr, *big_cols = nullptr;
-  double2 *big = nullptr;
-  vo_volume *res = nullptr;
-  long long total = 0;
-  const int sms = sm_count_fast();
-  const int gbig = sms, gmid = sms * 16;
-  rc = dalloc(ctx, &zf, (size_t)std::max<int64_t>(2 * in->nseg, 2));
-  if (!rc) rc = dalloc(ctx, &dE, 1);
-  if (!rc) rc = dalloc(ctx, &col, (size_t)ncols);
-  const int mbits = mask_bits_for((double)in->nseg / std::max(ncols, 1));
-  if (!rc) rc = dalloc(ctx, &dmask, mask_words((size_t)ncols, mbits));
-  if (!rc) rc = dalloc(ctx, &prec, pairs.size());
-  if (!rc) rc = dalloc(ctx, &dmax, 1);
-  if (!rc) rc = dalloc(ctx, &dpairs, pairs.size());
-  if (!rc) rc = dalloc(ctx, &counts, (size_t)ncols);
-  if (!rc) rc = dalloc(ctx, &ovf_cols, (size_t)ncols);
-  if (!rc) rc = dalloc(ctx, &big_cols, (size_t)ncols);
-  if (!rc) rc = dalloc(ctx, &big, (size_t)gbig * kBigThreads * kBigCap);
-  if (!rc) {
-    cudaMemcpyAsync(dpairs, pairs.data(), sizeof(int2) * pairs.size(), cudaMemcpyHostToDevice, ctx->stream);
-    cudaMemsetAsync(ctx->d_flags, 0, 3 * sizeof(int), ctx->stream);  // [0] tier-2 list, [1] fatal, [2] FP64 list
-    cudaEventRecord(ctx->ev[0], ctx->stream);
-    fast_prepare(ctx->stream, nx, ny, in->offs, in->offs + 1, in->z, zf, dmax, (float)R, dE, col, dmask, mbits,
-                 T->host.dom);
-    fast_pair_records(ctx->stream, dpairs, (int)pairs.size(), *T, prec);
-    ctx->launches += 4;
-    cudaEventRecord(ctx->ev[1], ctx->stream);
-  }
-  FastArgs A{nx, ny, h.W, in->offs, in->offs + 1, (const double *)in->z, zf, T->Hf, T->H, dpairs,
-             (int)pairs.size(), dE, col, prec, dmask, mbits};
-  const dim3 blk(kFB, kFBY), grd(((nx + kPatchX - 1) / kPatchX) * ((ny + kPatchY - 1) / kPatchY));
-  // union capacity from the input's mean segment count per column (24, 32,
-  // 48 or 64; dense inputs take 48 up to 24 segments per column, which keeps
-  // more warps per SM than 64, the rest going to the second tier)
   const double mean_segs = (double)in->nseg / std::max(ncols, 1);
-  const int ka = fast_union_cap(mean_segs) == 64 ? (mean_segs > 24.0 ? 64 : 48) : fast_union_cap(mean_segs);
-  const size_t smem = sizeof(float2) * ka * kFB * kFBY;
-  double2 *staging = nullptr;
-  if (!rc) rc = dalloc(ctx, &staging, (size_t)ncols * ka);
-  if (!rc && ka == 64 &&
-      cudaFuncSetAttribute(reinterpret_cast<const void *>(&k_fast<64>), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem) != cudaSuccess)
-    rc = cuda_error(ctx, cudaGetLastError(), "k_fast shared memory");
-  if (!rc) {
+  PatchPlan P;
+  const vo_grid *const gp = &g;
+  const int split = patch_split(&gp, 1);
+  rc = patch_plan(ctx, patch_count(g, split), split, T->host.hs, P);
+  if (rc) return rc;
+  // slot indices are unsigned 32-bit: columns and spill together below 2^32
+  const int64_t most = 4294967295LL;
+  int cap = slot_cap(mean_segs);
+  cap = (int)std::max<int64_t>(1, std::min<int64_t>(cap, most / 9 * 8 / std::max(ncols, 1)));
+  int64_t spill = std::max<int64_t>(4096, (int64_t)ncols * cap / 8);
+  const size_t nseg = (size_t)std::max<int64_t>(in->nseg, 1);
+  PackOut pk;
+  int32_t *obeg = nullptr, *big_list = nullptr;
+  int *list = nullptr;
+  unsigned char *misc = nullptr, *scratch[2] = {nullptr, nullptr};
+  double2 *oz = nullptr, *big = nullptr;
+  BatchVol *dv = nullptr;
+  // misc: range orders (3 x 8 bytes), FastPar at 64, counters at 128 (4 of the queue, FP64-tier columns,
+  // spill used, overflow flags)
+  rc = dalloc(ctx, &misc, 256);
+  if (!rc) rc = dalloc(ctx, &dv, 1);
+  if (!rc) rc = dalloc(ctx, &pk.zf, nseg);
+  if (!rc) rc = dalloc(ctx, &pk.code, nseg);
+  if (!rc) rc = dalloc(ctx, &pk.zx, nseg);
+  if (!rc) rc = dalloc(ctx, &pk.cl, nseg);
+  if (!rc) rc = dalloc(ctx, &pk.coff, pack_offsets(g));
+  if (!rc) rc = dalloc(ctx, &obeg, 2 * (size_t)ncols);
+  if (!rc) rc = dalloc(ctx, &list, (size_t)P.nitems);
+  if (!rc) rc = dalloc(ctx, &big_list, (size_t)ncols);
+  if (!rc) rc = dalloc(ctx, &scratch[0], patch_scratch_bytes(P, false));
+  if (!rc) patch_scratch_set(P, false, scratch[0]);
+  unsigned long long *mm = reinterpret_cast<unsigned long long *>(misc);
+  pk.par = reinterpret_cast<FastPar *>(misc + 64);
+  int *cnt = reinterpret_cast<int *>(misc + 128);
+  P.Q = PatchQueue{cnt, list};
+  vo_volume *res = nullptr;
+  int cols2 = 0;
+  for (int attempt = 0; !rc; ++attempt) {
+    rc = dalloc(ctx, &oz, (size_t)ncols * cap + (size_t)spill);
+    if (rc) break;
+    BatchVol V;
+    std::memset(&V, 0, sizeof V);
+    V.A = fast_args(nx, ny, *T, in->offs, in->offs + 1, in->z, pk);
+    V.obeg = obeg;
+    V.oend = obeg + ncols;
+    V.oz = oz;
+    V.cap = cap;
+    V.item1 = P.nitems;
+    V.spill_base = (unsigned)((int64_t)ncols * cap);
+    V.spill_cap = (unsigned)spill;
+    V.big_list = big_list;
+    V.big_count = cnt + 4;
+    V.spill_used = reinterpret_cast<unsigned *>(cnt + 5);
+    V.ovf = cnt + 6;
+    cudaMemcpyAsync(dv, &V, sizeof V, cudaMemcpyHostToDevice, ctx->stream);
+    cudaMemsetAsync(cnt, 0, 7 * sizeof(int), ctx->stream);
+    cudaEventRecord(ctx->ev[0], ctx->stream);
+    fast_prepare(ctx->stream, V.A, (float)R, mean_segs, mm, pk);
+    cudaEventRecord(ctx->ev[1], ctx->stream);
     cudaEventRecord(ctx->ev[4], ctx->stream);
-    if (ka == 64)
-      k_fast<64><<<grd, blk, smem, ctx->stream>>>(A, counts, staging, ctx->d_flags, ovf_cols);
-    else if (ka == 48)
-      k_fast<48><<<grd, blk, smem, ctx->stream>>>(A, counts, staging, ctx->d_flags, ovf_cols);
-    else if (ka == 32)
-      k_fast<32><<<grd, blk, smem, ctx->stream>>>(A, counts, staging, ctx->d_flags, ovf_cols);
-    else
-      k_fast<24><<<grd, blk, smem, ctx->stream>>>(A, counts, staging, ctx->d_flags, ovf_cols);
-    k_fast_mid<false><<<gmid, kMidThreads, 0, ctx->stream>>>(A, counts, nullptr, nullptr, ctx->d_flags, ovf_cols,
-                                                               ctx->d_flags + 2, big_cols);
-    k_fast_big<false><<<gbig, kBigThreads, 0, ctx->stream>>>(A, counts, nullptr, nullptr, ctx->d_flags + 2,
-                                                             big_cols, big, ctx->d_flags + 1);
-    ctx->launches += 3;
+    patch_launch(false, P, ctx->stream, dv);
     cudaEventRecord(ctx->ev[5], ctx->stream);
-    rc = volume_alloc(ctx, g, 0, &res);
-  }
-  if (!rc) rc = scan_counts(ctx, counts, res->offs, ncols, &total);
-  if (!rc) {
-    res->nseg = total;
-    rc = dalloc(ctx, &res->z, (size_t)total);
-  }
-  if (!rc) {
-    cudaEventRecord(ctx->ev[6], ctx->stream);
-    k_compact<<<(int)(((int64_t)ncols * 32 + 255) / 256), 256, 0, ctx->stream>>>(ncols, ka, counts, staging,
-                                                                                 res->offs, res->z);
-    k_fast_mid<true><<<gmid, kMidThreads, 0, ctx->stream>>>(A, nullptr, res->offs, res->z, ctx->d_flags, ovf_cols,
-                                                              nullptr, nullptr);
-    k_fast_big<true><<<gbig, kBigThreads, 0, ctx->stream>>>(A, nullptr, res->offs, res->z, ctx->d_flags + 2,
-                                                            big_cols, big, ctx->d_flags + 1);
     ctx->launches += 3;
-    cudaEventRecord(ctx->ev[7], ctx->stream);
-    int hf[3] = {0, 0, 0};
-    cudaMemcpyAsync(hf, ctx->d_flags, sizeof(hf), cudaMemcpyDeviceToHost, ctx->stream);
-    cudaError_t e = cudaStreamSynchronize(ctx->stream);
-    if (e != cudaSuccess)
-      rc = cuda_error(ctx, e, "dilate_fast");
-    else if (hf[1])
+    SlotVol sv;
+    sv.grid = g;
+    sv.cap = cap;
+    sv.beg = obeg;
+    sv.end = obeg + ncols;
+    sv.z = oz;
+    int hc[7] = {0};
+    rc = slot_to_volume(ctx, sv, &res, cnt, hc, 7);
+    if (!rc && hc[1] + hc[4] > 0) {  // patches and columns for the last tiers
+      vo_volume_free(ctx, res);
+      res = nullptr;
+      if (!scratch[1]) rc = dalloc(ctx, &scratch[1], patch_scratch_bytes(P, true));
+      if (!rc && !big) rc = dalloc(ctx, &big, big_scratch_elems());
+      if (!rc) {
+        patch_scratch_set(P, true, scratch[1]);
+        patch_launch(true, P, ctx->stream, dv);
+        big_launch(ctx->stream, dv, 1, big);
+        ctx->launches += 2;
+        rc = slot_to_volume(ctx, sv, &res, cnt, hc, 7);
+      }
+    }
+    if (rc) break;
+    cols2 = hc[3] + (hc[3] == 0 ? hc[4] : 0);
+    if (hc[6] & 1) {
       rc = set_error(ctx, VO_EINTERNAL, "a column exceeds the fallback union capacity");
-    else
-      ctx->ovf_cols += hf[0];
+    } else if (hc[6] & 4) {  // the spill region was too small: its counter says what it takes
+      vo_volume_free(ctx, res);
+      res = nullptr;
+      dfree(ctx, oz);
+      oz = nullptr;
+      spill = (int64_t)(unsigned)hc[5] + 4096;
+      if (attempt >= 2 || (int64_t)ncols * cap + spill > most)
+        rc = set_error(ctx, VO_ERANGE, "dilation: the result exceeds the slot range");
+      continue;
+    }
+    break;
   }
-  dfree(ctx, staging);
-  if (!rc && tm) {
-    float e0 = 0, e1 = 0, e2 = 0;
-    cudaEventElapsedTime(&e0, ctx->ev[0], ctx->ev[1]);
-    cudaEventElapsedTime(&e1, ctx->ev[4], ctx->ev[5]);
-    cudaEventElapsedTime(&e2, ctx->ev[6], ctx->ev[7]);
-    tm->pass1_ms += e0;
-    tm->pass2_ms += e1 + e2;
-    tm->kernel_ms[0] += e0;
-    tm->kernel_ms[2] += e1;
-    tm->kernel_ms[3] += e2;
+  if (!rc) {
+    ctx->ovf_cols += cols2;
+    if (tm) {
+      float e0 = 0, e1 = 0;
+      cudaEventElapsedTime(&e0, ctx->ev[0], ctx->ev[1]);
+      cudaEventElapsedTime(&e1, ctx->ev[4], ctx->ev[5]);
+      tm->pass1_ms += e0;
+      tm->pass2_ms += e1;
+      tm->kernel_ms[0] += e0;
+      tm->kernel_ms[2] += e1;
+    }
   }
-  dfree(ctx, zf);
-  dfree(ctx, dE);
-  dfree(ctx, col);
-  dfree(ctx, dmask);
-  dfree(ctx, prec);
-  dfree(ctx, dmax);
-  dfree(ctx, dpairs);
-  dfree(ctx, counts);
-  dfree(ctx, ovf_cols);
-  dfree(ctx, big_cols);
-  dfree(ctx, big);
+  for (void *p : {(void *)misc, (void *)dv, (void *)pk.zf, (void *)pk.code, (void *)pk.zx, (void *)pk.cl,
+                  (void *)pk.coff, (void *)obeg, (void *)list, (void *)big_list, (void *)scratch[0],
+                  (void *)scratch[1], (void *)oz, (void *)big})
+    dfree(ctx, p);
   if (rc) {
     if (res) vo_volume_free(ctx, res);
     return rc;
   }
   *out = res;
   return VO_OK;
-}
-
-// ================================================================ batch launch helpers
-
-std::vector<int2> fast_pairs(const Tables &h) {
-  std::vector<int2> pairs;
-  for (int d = 0; d <= h.Dy; ++d)
-    for (int a = 0; a <= h.Dx[d]; ++a) pairs.push_back(make_int2(a, d));
-  std::stable_sort(pairs.begin(), pairs.end(), [&](const int2 &p, const int2 &q) {
-    return h.H[(size_t)p.y * h.W + p.x] > h.H[(size_t)q.y * h.W + q.x];
-  });
-  return pairs;
-}
-
-void fast_prepare(cudaStream_t st, int nx, int ny, const int32_t *beg, const int32_t *end, const double2 *z,
-                  float *zf, unsigned int *maxbits, float R, float *E, int4 *col, void *dmask, int mask_bits,
-                  const DomLevels &L) {
-  const int ncols = nx * ny;
-  cudaMemsetAsync(maxbits, 0, sizeof(unsigned int), st);
-  k_to_f32_cols<<<(ncols + 255) / 256, 256, 0, st>>>(ncols, beg, end, (const double *)z, zf, maxbits);
-  k_guard<<<1, 1, 0, st>>>(maxbits, R, E);
-  k_dominance<<<(ncols + 127) / 128, 128, 0, st>>>(nx, ny, beg, end, reinterpret_cast<const float2 *>(zf), col,
-                                                    dmask, mask_bits, L);
-}
-
-void fast_pair_records(cudaStream_t st, const int2 *pairs, int npairs, const DeviceTables &T, float4 *prec) {
-  const int W = T.host.W;
-  k_pair_records<<<(npairs + 127) / 128, 128, 0, st>>>(pairs, npairs, T.Hf, T.dH, W, (T.host.Dy + 1) * W, prec,
-                                                       T.host.dom);
-}
-
-void launch_dh_tables(cudaStream_t st, int Dy, int W, const double *H, const int *Dx, float *dH) {
-  const int n = (Dy + 1) * W;
-  k_dh_tables<<<(n + 127) / 128, 128, 0, st>>>(Dy, W, H, Dx, dH);
-}
-
-int fast_union_cap(double mean_segments_per_column) {
-  return mean_segments_per_column > 10.0 ? 64 : mean_segments_per_column > 6.0 ? 32 : 24;
-}
-
-namespace {
-using BatchedFn = void (*)(const BatchVol *, const int2 *, int, int *, const FastArgs);
-
-template <int KA, int FBY, bool SINGLE>
-BatchedFn batched_fn_regs(int regs) {
-  return regs == 64 ? &k_fast_batched<KA, FBY, SINGLE, 1024> : &k_fast_batched<KA, FBY, SINGLE, 768>;
-}
-template <int KA, int FBY>
-BatchedFn batched_fn_single(bool single, int regs) {
-  return single ? batched_fn_regs<KA, FBY, true>(regs) : batched_fn_regs<KA, FBY, false>(regs);
-}
-template <int KA>
-BatchedFn batched_fn_fby(int fby, bool single, int regs) {
-  switch (fby) {
-    case 1:
-      return batched_fn_single<KA, 1>(single, regs);
-    case 2:
-      return batched_fn_single<KA, 2>(single, regs);
-    case 4:
-      return batched_fn_single<KA, 4>(single, regs);
-  }
-  return nullptr;
-}
-BatchedFn batched_fn(int ka, int fby, bool single, int regs) {
-  if (regs != 64 && regs != 80) return nullptr;
-  switch (ka) {
-    case 24:
-      return batched_fn_fby<24>(fby, single, regs);
-    case 32:
-      return batched_fn_fby<32>(fby, single, regs);
-    case 48:
-      return batched_fn_fby<48>(fby, single, regs);
-    case 64:
-      return batched_fn_fby<64>(fby, single, regs);
-  }
-  return nullptr;
-}
-}  // namespace
-
-int fast_batched_blocks_per_sm(int ka, int fby, bool single, int regs) {
-  const BatchedFn f = batched_fn(ka, fby, single, regs);
-  if (!f) return 0;
-  const size_t smem = sizeof(float2) * ka * kFB * fby;
-  if (smem > 227 * 1024 ||
-      cudaFuncSetAttribute(reinterpret_cast<const void *>(f), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, reinterpret_cast<const void *>(f), kFB * fby, smem) !=
-      cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
-  return per_sm;
-}
-
-int fast_batched_launch(int ka, int fby, int regs, int grid, cudaStream_t st, const BatchVol *vols,
-                        const int2 *queue, int nq, int *next, const FastArgs *single) {
-  const BatchedFn f = batched_fn(ka, fby, single != nullptr, regs);
-  if (!f) return VO_EINVAL;
-  const size_t smem = sizeof(float2) * ka * kFB * fby;
-  FastArgs none;
-  std::memset(&none, 0, sizeof none);
-  f<<<grid, dim3(kFB, fby), smem, st>>>(vols, queue, nq, next, single ? *single : none);
-  return VO_OK;
-}
-
-void fast_batched_mid_launch(cudaStream_t st, const BatchVol *vols, int nv, int grid) {
-  k_fast_batched_mid<<<grid, kMidThreads, 0, st>>>(vols, nv);
-}
-
-size_t fast_batched_big_scratch_elems(int grid) { return (size_t)grid * kBigThreads * kBigCap; }
-
-void fast_batched_big_launch(cudaStream_t st, const BatchVol *vols, int nv, int grid, double2 *scratch) {
-  k_fast_batched_big<<<grid, kBigThreads, 0, st>>>(vols, nv, scratch);
 }
 
 }  // namespace vo

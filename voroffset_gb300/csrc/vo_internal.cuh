@@ -17,27 +17,6 @@ namespace vo {
 constexpr int kCapSmall = 32;    // pass-1 touching-merged piece list / pass-2 union
 constexpr int kCapLarge = 2048;  // overflow re-run capacity per column
 
-// Dominance levels of the FP32 kernels: a segment is dominated at level l
-// in a direction when its width there is <= t[l]; a pair uses the largest
-// level whose threshold is <= its FP32 lower bound of the growth of H. Any
-// thresholds keep the pruning exact; t[0] = 0 and the others are quantiles of
-// the pairs' growths for the radius, so that levels fall where pairs are.
-constexpr int kDomLevels = 11;  // 15 in a pair record means "no level"
-// Segment dominance masks hold one bit per segment of columns with at most
-// mask_bits segments (16 or 32 per dilation: 16 when the input averages at
-// most kMask16MeanSegs segments per column — 0.02 % of the 2048^2 workload's
-// columns have more than 16 — else 32); a column with more takes the dense
-// path: every segment, with the whole-column width test.
-constexpr double kMask16MeanSegs = 8.0;
-inline int mask_bits_for(double mean_segments_per_column) {
-  return mean_segments_per_column <= kMask16MeanSegs ? 16 : 32;
-}
-// 32-bit words of the mask planes [4 directions][kDomLevels][ncols]
-inline size_t mask_words(size_t ncols, int bits) { return (4 * (size_t)kDomLevels * ncols * bits + 31) / 32; }
-struct DomLevels {
-  float t[kDomLevels];
-};
-
 // Radius tables, computed on the host with the reference's own FP64
 // expressions (so device results match bit for bit) and uploaded once per
 // (radius, grid extent).
@@ -48,16 +27,20 @@ struct Tables {
   std::vector<double> r1;     // [Dy+1] pass-1 radius per label
   std::vector<int> Dx;        // [Dy+1] max |dx| per label
   std::vector<double> H;      // [(Dy+1)*W] sqrt(r1*r1 - dx*dx), NaN beyond Dx
-  std::vector<float> Hf;      // FP32 rounding of H
+  // FP32 rounding of H for patches of columns: rows 0 .. Dy + 2 kPatchY - 1 of
+  // stride hs >= W + kPatchX + 2, -inf beyond the disc (the distances between
+  // the columns of a patch and of a 4 x 4 tile within its reach). hs is 8 or 24 modulo 32,
+  // so that the 4 rows of 8 consecutive entries that a warp reads fall into 32
+  // different banks.
+  int hs = 0;
+  std::vector<float> Hp;
   std::vector<double> HB;     // [(Dy+1)^2] brute force sqrt(R*R - dx^2 - dy^2), NaN outside
-  DomLevels dom{};            // dominance level thresholds for this radius
 };
 
 // Device view of the tables (kernel argument by value).
 struct DevTables {
   int Dy, W;
   const double *H;
-  const float *Hf;
   const int *Dx;
   const double *HB;
 };
@@ -70,16 +53,11 @@ struct DeviceTables {
   double R = -1;
   int kmax = 0;
   double *H = nullptr;
-  float *Hf = nullptr;
+  float *Hp = nullptr;
   int *Dx = nullptr;
   double *HB = nullptr;
-  // FP32 lower bounds of the growth of H one lattice step toward the centre:
-  // dH[d*W + a] <= H[d][a-1] - H[d][a] (x step, a >= 1) and
-  // dH[(Dy+1)*W + d*W + a] <= H[d-1][a] - H[d][a] (y step, d >= 1); -inf where
-  // no step exists (used by the dominance test of the FP32 kernels).
-  float *dH = nullptr;
   Tables host;
-  DevTables view() const { return DevTables{host.Dy, host.W, H, Hf, Dx, HB}; }
+  DevTables view() const { return DevTables{host.Dy, host.W, H, Dx, HB}; }
 };
 
 }  // namespace vo
@@ -115,7 +93,7 @@ struct vo_ctx {
   long long *h_total = nullptr;  // pinned
   vo_sizer *sizer = nullptr;     // learned sizing for the batched executor (not owned)
   int64_t dexel_odd_columns = -1;  // odd-hit columns of the last vo_dexelize (-1: none yet)
-  std::vector<std::pair<long long, int>> tune_cache;  // batch autotuner: shape key -> rows per block
+  std::vector<std::pair<long long, int>> tune_cache;  // batch autotuner: shape key -> lanes per column
 };
 
 namespace vo {
@@ -150,9 +128,10 @@ int get_tables(vo_ctx *ctx, double R, int kmax, const DeviceTables **out);
 
 // Exclusive scan of int32 counts into int32 offsets (n+1 entries); the total
 // is returned through ctx->h_total (synchronising read). Returns VO_ERANGE if
-// the total exceeds INT32_MAX.
-int scan_counts(vo_ctx *ctx, const int32_t *counts, int32_t *offs, int n, long long *total);
-
+// the total exceeds INT32_MAX. With extra_n > 0 that many ints at extra_dev are
+// read back by the same synchronisation.
+int scan_counts(vo_ctx *ctx, const int32_t *counts, int32_t *offs, int n, long long *total,
+                const int *extra_dev = nullptr, int *extra_host = nullptr, int extra_n = 0);
 // The separable scheme in its sweeping envelope form, FP64 (vo_env.cu).
 // Returns VO_OK, an error, or 1 when the volume exceeds the kernels' working
 // capacities and must take the painter form (VO_METHOD_SEPARABLE).
@@ -195,38 +174,46 @@ void slot_normalize_launch(cudaStream_t st, const SlotVol &in, const SlotVol &ou
 void slot_negate_inv_launch(cudaStream_t st, const SlotVol &in, const vo_grid &g, const SlotVol &out,
                             int *overflow);
 int slot_max_count(vo_ctx *ctx, const SlotVol &v, int *d_max);
-int slot_to_volume(vo_ctx *ctx, const SlotVol &v, vo_volume **out);
+// CSR volume of a slot volume; extra_*: see scan_counts.
+int slot_to_volume(vo_ctx *ctx, const SlotVol &v, vo_volume **out, const int *extra_dev = nullptr,
+                   int *extra_host = nullptr, int extra_n = 0);
+
+// Scalars of a dilation's FP32 arithmetic, from the range of its input
+// (k_range in vo_fast.cu): FP32 values are relative to base, E is the guard
+// band, 1 / inv_w the bin width, thr the least length of a long interval.
+struct FastPar {
+  double base;
+  float E, inv_w, thr;
+  int nbins;
+};
+
+// Columns of a warp of the FP32 kernel: a kPatchX x kPatchY patch, lane l at
+// (l % kPatchX, l / kPatchX).
+constexpr int kPatchX = 8, kPatchY = 4;
 
 // Arguments of the FP32-guarded dilation of one volume (vo_fast.cu).
 struct FastArgs {
-  int nx, ny, W;
-  // Column c's segments are [beg[c], end[c]); for CSR input beg = offs and
-  // end = offs + 1, for a slot layout beg / end are the slot arrays.
-  const int32_t *beg, *end;
-  const double *zd;     // FP64 values, 2 per segment
-  const float *zf;      // FP32 copies
-  const float *Hf;      // [(Dy+1) * W]
-  const double *H64;    // [(Dy+1) * W]
-  const int2 *pairs;    // (a, d) sorted by decreasing H
-  int npairs;
-  const float *E;       // guard band (device scalar)
-  // Column records (beg, end, dominance widths x- | x+ << 16, y- | y+ << 16 as
-  // FP16) and pair records (a | d << 16 as float bits, H in FP32, dH of an x
-  // step, dH of a y step), both built by the fast_* helpers below.
-  const int4 *col;
-  const float4 *prec;
-  // Segment dominance masks [4 directions][kDomLevels][ncols] of mask_bits
-  // (16 or 32) bits: bit j of a column with at most mask_bits segments is set
-  // when its segment j lies in a neighbour segment widened by the level's
-  // threshold.
-  const void *dmask;
-  int mask_bits;
+  int nx, ny, W, Dy, hs;
+  const int32_t *beg, *end;  // segments [beg[c], end[c]) of column c as given (CSR or slots)
+  const double *zd;          // FP64 values as given
+  // Packed by 4 x 4 tiles of columns (k_pack in vo_fast.cu): FP32 values
+  // relative to FastPar::base, column in the tile, FP64 values; the clusters
+  // and their offsets [tile rows][tiles per row + 1].
+  const float2 *zf;
+  const unsigned char *code;
+  const double *zx;
+  const float4 *cl;
+  const int32_t *coff;
+  const float *Hp;      // [(Dy + 2 kPatchY)][hs], -inf beyond the disc
+  const double *H64;    // [(Dy + 1) * W]
+  const int *Dx;        // [Dy + 1]
+  const FastPar *par;
 };
 
-// One dilation of a batch (device array element of the persistent kernel).
-constexpr int kSizerTile = 32;  // side of a sizing tile (columns)
-constexpr int kUnionCap = 32;      // union capacity of the main FP32 kernels
-constexpr int kUnionCapMid = 128;  // union capacity of their second tier
+constexpr int kSizerTile = 32;     // side of a sizing tile (columns)
+constexpr int kUnionCap = 32;      // output slots per column of a batch dilation without a sizer
+constexpr int kUnionCapMid = 128;  // most output slots per column of a sized tile
+// One dilation of a launch (device array element).
 struct BatchVol {
   FastArgs A;
   int32_t *obeg, *oend;  // output slot arrays, written for every column
@@ -235,50 +222,62 @@ struct BatchVol {
   const int32_t *toff;   // per sizing tile offset into oz
   int cap;
   int tiles32_x;
-  int spill_base, spill_cap;
-  int *spill_used;
-  int *mid_list, *mid_count;  // columns whose union exceeds the main capacity (second tier)
-  int *big_list, *big_count;  // columns whose union exceeds kUnionCapMid (third tier, FP64)
+  int item0, item1;      // its patches in the launch's queue
+  unsigned spill_base, spill_cap;
+  unsigned *spill_used;
+  int *big_list, *big_count;  // columns for the third tier (FP64)
   int *ovf;  // flags: 1 a union beyond the FP64 list, 4 spill region exhausted
 };
 
-// Fills DeviceTables::dH from H on the device (directed rounding).
-void launch_dh_tables(cudaStream_t st, int Dy, int W, const double *H, const int *Dx, float *dH);
-
-// (a, d) pairs with a <= Dx[d], sorted by decreasing H (the candidate order of
-// the FP32 kernels).
-std::vector<int2> fast_pairs(const Tables &h);
-// FP32 copies of the values of a slot volume, the guard band scalar, the
-// column records (ncols int4) and the dominance masks (4 * kDomLevels * ncols).
-void fast_prepare(cudaStream_t st, int nx, int ny, const int32_t *beg, const int32_t *end, const double2 *z,
-                  float *zf, unsigned int *maxbits, float R, float *E, int4 *col, void *dmask, int mask_bits,
-                  const DomLevels &L);
-// Pair records (npairs float4) from the device tables of radius T.
-void fast_pair_records(cudaStream_t st, const int2 *pairs, int npairs, const DeviceTables &T, float4 *prec);
-// Union capacity (24, 32 or 64) of the main FP32 kernels for inputs with the
-// given mean segment count per column.
-int fast_union_cap(double mean_segments_per_column);
-// Launch of the batch kernel with union capacity ka (24, 32 or 64), `fby`
-// rows of kFastCols columns per block (1, 2 or 4) and a register budget of
-// regs (64 or 80) per thread; fast_batched_blocks_per_sm is the occupancy of
-// that variant (0: unusable). single: the round's one dilation's arguments
-// (passed as a kernel parameter), or nullptr for a round of several.
-int fast_batched_launch(int ka, int fby, int regs, int grid, cudaStream_t st, const BatchVol *vols,
-                        const int2 *queue, int nq, int *next, const FastArgs *single);
-int fast_batched_blocks_per_sm(int ka, int fby, bool single, int regs);
-// Second tier of a batch round over the dilations vols[0..nv) (grid-stride).
-void fast_batched_mid_launch(cudaStream_t st, const BatchVol *vols, int nv, int grid);
-// Third tier (FP64) of a batch round; scratch holds
-// fast_batched_big_scratch_elems(grid) intervals.
-size_t fast_batched_big_scratch_elems(int grid);
-void fast_batched_big_launch(cudaStream_t st, const BatchVol *vols, int nv, int grid, double2 *scratch);
-// Columns of a warp of the FP32 kernels: a kPatchX x kPatchY patch, lane l at
-// (l % kPatchX, l / kPatchX). Lanes iterate to the warp's longest candidate
-// list, and a compact patch keeps their lists closer in length than a row of
-// 32 (2048^2 r=32 dilation: 217 vs 243 ms). A block of FBY warps covers FBY
-// patches side by side in x.
-constexpr int kPatchX = 8, kPatchY = 4;
-constexpr int kFastCols = kPatchX * kPatchY;  // columns per warp
+// Queue of a launch. count: the first tier's next item, the items it listed
+// for the second tier, that tier's next one, columns of the listed items.
+struct PatchQueue {
+  int *count = nullptr, *list = nullptr;
+};
+// Global working memory of a tier's warps.
+struct PatchScratch {
+  float2 *sv = nullptr;
+  int2 *ids = nullptr;
+  float2 *cv = nullptr;
+  int2 *cids = nullptr;
+  float4 *shorts = nullptr;
+};
+// A launch and its second tier (index 1).
+struct PatchPlan {
+  int nitems = 0, split = 1, hs_max = 0, grid[2] = {0, 0};
+  PatchQueue Q;
+  PatchScratch scratch[2];
+};
+// Lanes per column for a launch over the given grids (1, or more for small
+// ones), and the patches of a grid with that many.
+int patch_split(const vo_grid *const *grids, int n);
+int64_t patch_total(const vo_grid *const *grids, int n);  // with one lane per column
+int patch_count(const vo_grid &g, int split);
+// Grids of a launch over nitems patches; the working memory of each tier is
+// given by patch_scratch_bytes / patch_scratch_set.
+int patch_plan(vo_ctx *ctx, int nitems, int split, int hs_max, PatchPlan &P);
+size_t patch_scratch_bytes(const PatchPlan &P, bool big);
+void patch_scratch_set(PatchPlan &P, bool big, void *mem);
+void patch_launch(bool big, const PatchPlan &P, cudaStream_t st, const BatchVol *vols);
+// Last tier (FP64) over the dilations vols[0..nv); scratch holds big_scratch_elems() intervals.
+size_t big_scratch_elems();
+void big_launch(cudaStream_t st, const BatchVol *vols, int nv, double2 *scratch);
+// Outputs of the packing step, each as long as the input's segment array
+// (with its unused slots), coff pack_offsets(grid).
+struct PackOut {
+  float2 *zf = nullptr;
+  unsigned char *code = nullptr;
+  double2 *zx = nullptr;
+  float4 *cl = nullptr;
+  int32_t *coff = nullptr;
+  FastPar *par = nullptr;
+};
+size_t pack_offsets(const vo_grid &g);
+FastArgs fast_args(int nx, int ny, const DeviceTables &T, const int32_t *beg, const int32_t *end, const double2 *z,
+                   const PackOut &out);
+// Packs the input of a dilation (CSR or slots in column order). mm: three words of scratch.
+void fast_prepare(cudaStream_t st, const FastArgs &A, float R, double mean_segs, unsigned long long *mm,
+                  const PackOut &out);
 
 // Batch plans (vo_batch.cu).
 int morph_batched_fast(vo_ctx *ctx, int n, const int *ops, const double *radii, const vo_volume *const *ins,

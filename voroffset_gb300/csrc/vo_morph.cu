@@ -870,7 +870,7 @@ __global__ void k_slot_counts(int ncols, const int32_t *beg, const int32_t *end,
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   int n = 0;
   if (c < ncols) {
-    n = end[c] - beg[c];
+    n = (int)((uint32_t)end[c] - (uint32_t)beg[c]);
     if (counts) counts[c] = n;
   }
   if (maxc) {
@@ -884,14 +884,16 @@ __global__ void k_slot_compact(int ncols, const int32_t *__restrict__ beg, const
   const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (w >= ncols) return;
   const int n = ooffs[w + 1] - ooffs[w];
-  for (int k = lane; k < n; k += 32) oz[ooffs[w] + k] = z[beg[w] + k];
+  const uint32_t b = (uint32_t)beg[w];  // slot indices are unsigned
+  for (int k = lane; k < n; k += 32) oz[ooffs[w] + k] = z[(size_t)b + k];
 }
 
 }  // namespace
 
 // ================================================================ host side
 
-int scan_counts(vo_ctx *ctx, const int32_t *counts, int32_t *offs, int n, long long *total) {
+int scan_counts(vo_ctx *ctx, const int32_t *counts, int32_t *offs, int n, long long *total, const int *extra_dev,
+                int *extra_host, int extra_n) {
   const int ntiles = (n + kScanTile - 1) / kScanTile;
   if (ntiles > kScanTile) return set_error(ctx, VO_ERANGE, "scan: too many columns");
   long long *tmp = nullptr, *sums = nullptr;
@@ -911,6 +913,8 @@ int scan_counts(vo_ctx *ctx, const int32_t *counts, int32_t *offs, int n, long l
   k_scan_finish<<<(n + 1 + 255) / 256, 256, 0, ctx->stream>>>(tmp, sums, n, ctx->d_total, offs);
   ctx->launches += n > 0 ? 3 : 1;
   cudaMemcpyAsync(ctx->h_total, ctx->d_total, sizeof(long long), cudaMemcpyDeviceToHost, ctx->stream);
+  if (extra_n > 0)
+    cudaMemcpyAsync(extra_host, extra_dev, sizeof(int) * extra_n, cudaMemcpyDeviceToHost, ctx->stream);
   dfree(ctx, tmp);
   dfree(ctx, sums);
   VO_CK(ctx, cudaStreamSynchronize(ctx->stream));
@@ -1327,7 +1331,8 @@ int slot_max_count(vo_ctx *ctx, const SlotVol &v, int *d_max) {
   return VO_OK;
 }
 
-int slot_to_volume(vo_ctx *ctx, const SlotVol &v, vo_volume **out) {
+int slot_to_volume(vo_ctx *ctx, const SlotVol &v, vo_volume **out, const int *extra_dev, int *extra_host,
+                   int extra_n) {
   const int ncols = v.grid.nx * v.grid.ny;
   int32_t *counts = nullptr;
   int rc = dalloc(ctx, &counts, (size_t)ncols);
@@ -1337,7 +1342,7 @@ int slot_to_volume(vo_ctx *ctx, const SlotVol &v, vo_volume **out) {
   k_slot_counts<<<nblocks(ncols, 256), 256, 0, ctx->stream>>>(ncols, v.beg, v.end, counts, nullptr);
   ctx->launches += 1;
   rc = volume_alloc(ctx, v.grid, 0, &res);
-  if (!rc) rc = scan_counts(ctx, counts, res->offs, ncols, &total);
+  if (!rc) rc = scan_counts(ctx, counts, res->offs, ncols, &total, extra_dev, extra_host, extra_n);
   if (!rc) {
     res->nseg = total;
     rc = dalloc(ctx, &res->z, (size_t)total);
