@@ -15,10 +15,15 @@
 //   full extra row before the first and after the last row (voronoi_half_erode,
 //   Voronoi.h:126-150, then negate, CompressedImage.cpp:366-397).
 //
-// One block per output row: each candidate span adds +1 / -1 at its ends in a
-// shared-memory difference array, a block prefix sum gives the coverage, and a
-// block scan of the coverage changes places the output events. A count launch
-// sizes the CSR output, a fill launch writes it.
+// One block per output row, a warp per source row within reach: each candidate
+// span adds +1 / -1 at its ends in a shared-memory difference array, a block
+// prefix sum gives the coverage, and a block scan of the coverage changes
+// places the output events. They go to a staging buffer in the order in which
+// the rows finish, and a gather packs them once their counts are scanned; a
+// result larger than the buffer is written by a second pass instead. The reach
+// of every row distance is tabulated once: computed per thread and source row,
+// its FP64 square root took most of the time (2048 x 1536 pixels, r = 24: 418
+// us per pass, four passes per closing).
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -30,6 +35,7 @@ namespace {
 
 constexpr int kImgThreads = 256;
 constexpr int kImgMaxWidth = 50000;  // the difference array lives in shared memory
+constexpr int kImgSmem = (kImgMaxWidth + 1) * 4;
 
 __device__ __forceinline__ void img_add(int32_t *diff, int w, long long lo, long long hi) {
   if (lo < 0) lo = 0;
@@ -39,33 +45,44 @@ __device__ __forceinline__ void img_add(int32_t *diff, int w, long long lo, long
   atomicAdd(&diff[hi], -1);
 }
 
+// reach[t] = floor(sqrt(r*r - t*t)) for t <= n
+__global__ void k_image_reach(int n, double r, int32_t *__restrict__ reach) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t <= n) reach[t] = (int32_t)floor(sqrt(r * r - (double)((long long)t * t)));
+}
+
+// FILL: the events go to their CSR places (ooffs); else to the staging buffer
+// (slot[i] is row i's place there, -1 when it does not fit) with their counts.
 template <bool FILL>
 __global__ void __launch_bounds__(kImgThreads) k_image(int w, int h, const int32_t *__restrict__ offs,
-                                                       const int32_t *__restrict__ ev, double r, int D, int erode,
+                                                       const int32_t *__restrict__ ev,
+                                                       const int32_t *__restrict__ reach, int D, int erode,
                                                        int32_t *__restrict__ counts, const int32_t *__restrict__ ooffs,
-                                                       int32_t *__restrict__ oev) {
+                                                       int32_t *__restrict__ oev, long long *__restrict__ slot,
+                                                       unsigned long long *used, long long capacity) {
   extern __shared__ int32_t diff[];  // [w + 1]
   __shared__ int wsum[kImgThreads / 32];
+  __shared__ long long s_at;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int i = blockIdx.x; i < h; i += gridDim.x) {
     for (int p = tid; p <= w; p += kImgThreads) diff[p] = 0;
     __syncthreads();
     // rows beyond the image and its two border rows contribute nothing
-    for (int i0 = max(i - D, -1); i0 <= min(i + D, h); ++i0) {
+    for (int i0 = max(i - D, -1) + warp; i0 <= min(i + D, h); i0 += kImgThreads / 32) {
       const int t = i0 < i ? i - i0 : i0 - i;
       if (erode && (i0 == -1 || i0 == h)) {  // the extra full row
-        if (tid == 0) img_add(diff, w, 0, w);
+        if (lane == 0) img_add(diff, w, 0, w);
         continue;
       }
       if (i0 < 0 || i0 >= h) continue;
-      const long long dy = (long long)floor(sqrt(r * r - (double)((long long)t * t)));
+      const long long dy = reach[t];
       const int32_t *e = ev + offs[i0];
       const int n = offs[i0 + 1] - offs[i0];
       if (!erode) {
-        for (int k = 2 * tid; k + 1 < n; k += 2 * kImgThreads) img_add(diff, w, e[k] - dy, e[k + 1] + dy);
+        for (int k = 2 * lane; k + 1 < n; k += 64) img_add(diff, w, e[k] - dy, e[k + 1] + dy);
       } else {
         // complement spans [-1, a0 - 1], [b0, a1 - 1], ..., [b_last, w] (inclusive), widened
-        for (int q = tid; q <= n / 2; q += kImgThreads) {
+        for (int q = lane; q <= n / 2; q += 32) {
           const long long y1 = q == 0 ? -1 : e[2 * q - 1];
           const long long y2e = q == n / 2 ? (long long)w + 1 : e[2 * q];  // one past the span's last pixel
           img_add(diff, w, y1 - dy, y2e + dy);
@@ -117,9 +134,18 @@ __global__ void __launch_bounds__(kImgThreads) k_image(int w, int h, const int32
     }
     base += y - nev;
     if (!FILL) {
-      if (tid == 0) counts[i] = total;
-    } else {
-      int c2 = cov, pf = prevf, o = ooffs[i] + base;
+      if (tid == 0) {
+        counts[i] = total;
+        const long long at = (long long)atomicAdd(used, (unsigned long long)total);
+        s_at = at + total <= capacity ? at : -1;
+        slot[i] = s_at;
+      }
+      __syncthreads();
+    }
+    const long long at = FILL ? (long long)ooffs[i] : s_at;
+    if (at >= 0) {
+      int c2 = cov, pf = prevf;
+      long long o = at + base;
       for (int p = p0; p < p1; ++p) {
         c2 += diff[p];
         const int f = flag(p, c2);
@@ -131,30 +157,60 @@ __global__ void __launch_bounds__(kImgThreads) k_image(int w, int h, const int32
   }
 }
 
-int image_op(vo_ctx *ctx, int erode, double r, int w, int h, const int32_t *offs, const int32_t *ev, int32_t **ooffs,
+// Packs the staged rows: one warp per row.
+__global__ void k_image_gather(int h, const int32_t *__restrict__ ooffs, const long long *__restrict__ slot,
+                               const int32_t *__restrict__ staged, int32_t *__restrict__ oev) {
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (i >= h) return;
+  const int o = ooffs[i], n = ooffs[i + 1] - o;
+  for (int k = lane; k < n; k += 32) oev[o + k] = staged[slot[i] + k];
+}
+
+int image_op(vo_ctx *ctx, int erode, double r, int w, int h, const int32_t *offs, const int32_t *ev, long long nev,
+             int32_t **ooffs,
              int32_t **oev, long long *total) {
   const int D = (int)std::floor(r);
-  int32_t *counts = nullptr;
+  const int far = std::min(D, h + 1);  // the farthest row distance that occurs
+  // staging buffer: a dilated or eroded image rarely has more events than its input and a few per row
+  const long long capacity = 2 * nev + 8LL * h + 1024;
+  int32_t *counts = nullptr, *reach = nullptr, *staged = nullptr;
+  long long *slot = nullptr;
+  unsigned long long *used = nullptr;
   *ooffs = nullptr;
   *oev = nullptr;
   int rc = dalloc(ctx, &counts, (size_t)h + 1);
+  if (!rc) rc = dalloc(ctx, &reach, (size_t)far + 1);
+  if (!rc) rc = dalloc(ctx, &staged, (size_t)capacity);
+  if (!rc) rc = dalloc(ctx, &slot, (size_t)h + 1);
+  if (!rc) rc = dalloc(ctx, &used, 1);
   if (!rc) rc = dalloc(ctx, ooffs, (size_t)h + 1);
   const size_t sh = sizeof(int32_t) * ((size_t)w + 1);
   const int grid = std::min(h, 152 * 8);
   if (!rc) {
-    cudaFuncSetAttribute(k_image<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
-    cudaFuncSetAttribute(k_image<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
+    cudaFuncSetAttribute(k_image<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kImgSmem);
+    cudaFuncSetAttribute(k_image<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kImgSmem);
+    k_image_reach<<<far / 256 + 1, 256, 0, ctx->stream>>>(far, r, reach);
+    cudaMemsetAsync(used, 0, sizeof *used, ctx->stream);
     if (h > 0)
-      k_image<false><<<grid, kImgThreads, sh, ctx->stream>>>(w, h, offs, ev, r, D, erode, counts, nullptr, nullptr);
-    ctx->launches += 1;
+      k_image<false><<<grid, kImgThreads, sh, ctx->stream>>>(w, h, offs, ev, reach, D, erode, counts, nullptr, staged,
+                                                             slot, used, capacity);
+    ctx->launches += 2;
     rc = scan_counts(ctx, counts, *ooffs, h, total);
   }
   if (!rc) rc = dalloc(ctx, oev, (size_t)std::max<long long>(*total, 1));
   if (!rc && h > 0) {
-    k_image<true><<<grid, kImgThreads, sh, ctx->stream>>>(w, h, offs, ev, r, D, erode, nullptr, *ooffs, *oev);
+    if (*total <= capacity)
+      k_image_gather<<<(h + 7) / 8, 256, 0, ctx->stream>>>(h, *ooffs, slot, staged, *oev);
+    else
+      k_image<true><<<grid, kImgThreads, sh, ctx->stream>>>(w, h, offs, ev, reach, D, erode, nullptr, *ooffs, *oev,
+                                                            nullptr, nullptr, 0);
     ctx->launches += 1;
   }
   dfree(ctx, counts);
+  dfree(ctx, reach);
+  dfree(ctx, staged);
+  dfree(ctx, slot);
+  dfree(ctx, used);
   if (!rc) {
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) rc = cuda_error(ctx, e, "image kernels");
@@ -218,7 +274,7 @@ extern "C" int vo_image_morph(vo_ctx *ctx, int op, double radius, int width, int
   long long total = nev;
   for (size_t s = 0; !rc && s < steps.size(); ++s) {
     int32_t *o2 = nullptr, *e2 = nullptr;
-    rc = image_op(ctx, steps[s], radius, width, height, d_offs, d_ev, &o2, &e2, &total);
+    rc = image_op(ctx, steps[s], radius, width, height, d_offs, d_ev, total, &o2, &e2, &total);
     dfree(ctx, d_offs);
     dfree(ctx, d_ev);
     d_offs = o2;
