@@ -2,7 +2,7 @@
 // the plain GPU method, two sweeping kernels.
 //
 // Pass 1 (k_env1, VoronoiMorpho2D along y, Voronoi2D.cpp:591-723): one warp
-// per x-line sweeps the line's columns forward and backward. Its state is the
+// per x-line, or segment of one, sweeps its columns forward and backward. Its state is the
 // half-space Voronoi envelope of the segments seen so far: for every z, the
 // most recent row that covers it (disjoint labelled pieces, sorted by z), the
 // lower envelope of the distance to the sweep line from one side. A step
@@ -18,7 +18,7 @@
 // VoronoiVorPower.cpp:24-66: each piece dilates by r(d) = sqrt(R^2 - d^2)).
 //
 // Pass 2 (k_env2, SeparatePowerMorpho2D along x, SeparatePower2D.cpp:228-541):
-// one block per row sweeps the row's columns forward, then backward. Its state
+// one block per row, or segment of one, sweeps its columns forward, then backward. Its state
 // is the set of live stadiums, the pass-1 pieces of the columns within reach
 // (a piece of column x0 with label d reaches |x - x0| <= Dx[d], the
 // reference's floor(x_s + r) + 1 expiry, SeparatePower2D.cpp:258-293), kept
@@ -38,11 +38,23 @@
 // holds for the rest of their lives (covers_for_life): exact, and the state
 // shrinks about threefold.
 //
-// Capacities: pass 1's first launch keeps each line's state in shared memory,
-// and lines whose state outgrows it re-run with it in global memory. Pass 2
-// does the same for bands of few rows; bands of at least two rows per SM, or
-// whose state is estimated beyond shared memory, sweep with global-memory
-// state from the start (five rows per SM against one). A column whose union
+// Segments: a line or row is a chain of dependent steps, so where there are few
+// of them they are swept in segments, each after the columns before it (behind
+// it, backward) that can still reach into it. Both kernels compare and select
+// ends as integers of the same order and do only a chord's additions in FP64:
+// with FP64 comparisons that unit was the bound (512^2 spheres + cylinders,
+// r = 16: pass 1 5.3 + 4.9 ms and pass 2 55 ms; with integers 4.2 + 3.9 and
+// 29 ms; in segments 2.0 + 1.8 and 21.7 ms). What bounds pass 2 now are its
+// barriers and the latency of its global-memory state (per issued instruction
+// 5.8 and 4.3 cycles of stall out of 16.8; the FP64 unit is 4 % busy). Blocks of
+// 128 or 64 threads, with fewer threads per barrier, sweep more slowly (28 and
+// 40 ms).
+//
+// Capacities: pass 1's first launch keeps each segment's state in shared memory,
+// and those whose state outgrows it re-run with it in global memory. Pass 2
+// does the same where there are few row segments; with at least two per SM, or
+// a state estimated beyond shared memory, it sweeps with global-memory
+// state from the start (five segments per SM against one). A column whose union
 // outgrows its output slot, or a state beyond the global capacity, sends the
 // whole volume to the painter form of the method (VO_METHOD_SEPARABLE), which
 // has no such limits.
@@ -61,7 +73,7 @@ constexpr int kE1Warps = 4;          // lines (one warp each) per pass-1 block
 constexpr int kE1Stage = 128;        // staged segments per column (more: read from global memory)
 constexpr int kE1Cap = 448;          // shared-memory envelope capacity per line (pieces)
 constexpr int kE1CapBig = 16384;     // global-memory capacity of the re-run
-constexpr int kE2Threads = 256;      // threads of a pass-2 block (one row)
+constexpr int kE2Threads = 256;      // threads of a pass-2 block (one row segment)
 constexpr int kE2Stage = 768;        // staged pieces per column
 constexpr int kE2CapSmall = 4864;    // shared-memory stadium capacity of the first launch (227 KB in all)
 constexpr int kE2CapBig = 65536;     // global-memory stadium capacity of the re-run
@@ -110,15 +122,49 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
   return false;
 }
 
+// ------------------------------------------------------------ ordered keys
+
+// Both passes compare and select values far more often than they add them, and
+// an FP64 comparison occupies the SM for as long as sixteen integer ones. So
+// pieces and stadiums hold their ends as signed integers of the same order (the
+// bit pattern, its lower 63 bits flipped for negative values, -0 as 0), and
+// only a chord's two additions go through FP64.
+using Key = long long;
+using Key2 = longlong2;
+constexpr Key kKeyMin = -0x7fffffffffffffffll - 1, kKeyMax = 0x7fffffffffffffffll;
+
+__device__ __forceinline__ Key key_of(double v) {
+  const Key b = __double_as_longlong(v);
+  const Key k = b ^ ((b >> 63) & 0x7fffffffffffffffll);
+  return k == -1 ? 0 : k;  // -0
+}
+__device__ __forceinline__ double value_of(Key k) {
+  return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffll));
+}
+__device__ __forceinline__ Key2 key2_of(double2 v) { return make_longlong2(key_of(v.x), key_of(v.y)); }
+// The value as FP32, rounded towards zero (NaN beyond its range): integer
+// operations only, within 2^-23 of the magnitude for normal values, 0 for
+// smaller ones.
+__device__ __forceinline__ float trunc32(Key k) {
+  const Key b = k ^ ((k >> 63) & 0x7fffffffffffffffll);
+  const unsigned hi = (unsigned)(b >> 32), lo = (unsigned)b, e = hi & 0x7fffffffu;
+  unsigned f = e < 0x38100000u ? 0u : ((e - 0x38000000u) << 3) | (lo >> 29);
+  if (e >= 0x47f00000u) f = 0x7fc00000u;
+  return __uint_as_float((hi & 0x80000000u) | f);
+}
+__device__ __forceinline__ Key kmax(Key a, Key b) { return a > b ? a : b; }
+__device__ __forceinline__ Key kmin(Key a, Key b) { return a < b ? a : b; }
+
 // ------------------------------------------------------------ small searches
 
 // Pieces and stadiums are ordered by (start, end): a zero-length piece [s, s]
 // precedes [s, b]. Ordered by start alone, splitting [s, b] could move its
 // later part past the point piece; with ends breaking ties the order survives
 // every split, since a point piece only ever sits at another piece's end.
-__device__ __forceinline__ bool lex_less(double2 a, double2 b) { return a.x < b.x || (a.x == b.x && a.y < b.y); }
+__device__ __forceinline__ bool lex_less(Key2 a, Key2 b) { return a.x < b.x || (a.x == b.x && a.y < b.y); }
 // number of entries of v[0..n) (sorted by (start, end)) before / not after key
-__device__ __forceinline__ int count_lex_less(const double2 *v, int n, double2 key) {
+template <typename V>
+__device__ __forceinline__ int count_lex_less(const V &v, int n, Key2 key) {
   int l = 0, r = n;
   while (l < r) {
     const int m = (l + r) >> 1;
@@ -126,7 +172,8 @@ __device__ __forceinline__ int count_lex_less(const double2 *v, int n, double2 k
   }
   return l;
 }
-__device__ __forceinline__ int count_lex_leq(const double2 *v, int n, double2 key) {
+template <typename V>
+__device__ __forceinline__ int count_lex_leq(const V &v, int n, Key2 key) {
   int l = 0, r = n;
   while (l < r) {
     const int m = (l + r) >> 1;
@@ -135,7 +182,7 @@ __device__ __forceinline__ int count_lex_leq(const double2 *v, int n, double2 ke
   return l;
 }
 // number of entries of v[0..n) (sorted by .x) with .x < key / <= key
-__device__ __forceinline__ int count_less(const double2 *v, int n, double key) {
+__device__ __forceinline__ int count_less(const Key2 *v, int n, Key key) {
   int l = 0, r = n;
   while (l < r) {
     const int m = (l + r) >> 1;
@@ -143,7 +190,7 @@ __device__ __forceinline__ int count_less(const double2 *v, int n, double key) {
   }
   return l;
 }
-__device__ __forceinline__ int count_leq(const double2 *v, int n, double key) {
+__device__ __forceinline__ int count_leq(const Key2 *v, int n, Key key) {
   int l = 0, r = n;
   while (l < r) {
     const int m = (l + r) >> 1;
@@ -152,7 +199,8 @@ __device__ __forceinline__ int count_leq(const double2 *v, int n, double key) {
   return l;
 }
 // first entry of v[0..n) (sorted, disjoint) whose end .y is >= key
-__device__ __forceinline__ int first_ending_at_or_after(const double2 *v, int n, double key) {
+template <typename V>
+__device__ __forceinline__ int first_ending_at_or_after(const V &v, int n, Key key) {
   int l = 0, r = n;
   while (l < r) {
     const int m = (l + r) >> 1;
@@ -168,25 +216,33 @@ __device__ __forceinline__ int first_ending_at_or_after(const double2 *v, int n,
 // where a segment starts, a part [s2, b] starts where one ends (closed
 // intervals: a shared endpoint is covered by the segment, whose own label is
 // nearer); a point piece covered by a segment has no part.
-template <bool WRITE>
-__device__ __forceinline__ int piece_parts(double a, double b, const double2 *N, int m, int j, double2 *out) {
+template <bool WRITE, typename V>
+__device__ __forceinline__ int piece_parts(Key a, Key b, const V &N, int m, int j, Key2 *out) {
   int k = 0;
   while (a <= b) {
-    if (j >= m || N[j].x > b) {
-      if (WRITE) out[k] = make_double2(a, b);
+    const Key2 s = j < m ? N[j] : make_longlong2(kKeyMax, kKeyMax);
+    if (j >= m || s.x > b) {
+      if (WRITE) out[k] = make_longlong2(a, b);
       ++k;
       break;
     }
-    if (N[j].x > a) {
-      if (WRITE) out[k] = make_double2(a, N[j].x);
+    if (s.x > a) {
+      if (WRITE) out[k] = make_longlong2(a, s.x);
       ++k;
     }
-    a = N[j].y;
+    a = s.y;
     if (a >= b) break;
     ++j;
   }
   return k;
 }
+
+// A column's segments as keys: staged (converted in shared memory) or read from the input.
+struct Column {
+  const Key2 *staged;
+  const double2 *raw;
+  __device__ __forceinline__ Key2 operator[](int j) const { return staged ? staged[j] : key2_of(raw[j]); }
+};
 
 __device__ __forceinline__ int warp_excl_sum(int v, int lane, int &total) {
   int x = v;
@@ -200,21 +256,25 @@ __device__ __forceinline__ int warp_excl_sum(int v, int lane, int &total) {
 
 struct E1Args {
   int nx, ny, yb0, yb1, Dy;
+  int rows, segs;             // rows per segment of a line, segments per line
   const int32_t *offs;
   const double2 *z;
   int32_t *nF, *nB;           // COUNT: forward / backward (d >= 1) pieces per column
   const int32_t *poff;        // FILL: piece offsets of the band's columns (index c - yb0 * nx)
-  double2 *pz;                // FILL: piece cores
+  Key2 *pz;                   // FILL: piece cores
   uint8_t *pd;                // FILL: piece labels d
   int *flags;
-  int *list;                  // lines whose envelope outgrew the shared capacity (first launch)
-  double2 *gz;                // re-run: global envelope storage, 2 * kE1CapBig pieces per warp
+  int *list;                  // line segments whose envelope outgrew the shared capacity (first launch)
+  Key2 *gz;                   // re-run: global envelope storage, 2 * kE1CapBig pieces per warp
   int *gl;                    // re-run: labels, 2 * kE1CapBig per warp
+  int nlist;                  // re-run: listed line segments
 };
 
-// One warp per x-line (first launch: x = global warp index; re-run: the
-// listed lines). FILL writes the pieces of the band's rows [yb0, yb1); COUNT
-// counts them for every row of [yb0, yb1).
+// One warp per segment of an x-line (first launch: by global warp index;
+// re-run: the listed ones): its rows [ylo, yhi) of the band, after the Dy rows
+// before them (behind them in the backward sweep) have built the envelope.
+// Segments instead of whole lines keep every SM supplied with warps: a line is
+// a chain of dependent steps. FILL writes the pieces, COUNT counts them.
 template <bool FILL, bool BIG>
 __global__ void __launch_bounds__(32 * kE1Warps) k_env1(E1Args A) {
   extern __shared__ __align__(16) unsigned char e1_smem[];
@@ -225,7 +285,7 @@ __global__ void __launch_bounds__(32 * kE1Warps) k_env1(E1Args A) {
   unsigned char *base = e1_smem + warp * per_warp;
   double2 *stage = reinterpret_cast<double2 *>(base);
   uint64_t *bar = reinterpret_cast<uint64_t *>(base + 2 * kE1Stage * sizeof(double2));
-  double2 *Az, *Tz;
+  Key2 *Az, *Tz;
   int *Al, *Tl;
   const int gw = blockIdx.x * kE1Warps + warp;
   if (BIG) {
@@ -235,19 +295,20 @@ __global__ void __launch_bounds__(32 * kE1Warps) k_env1(E1Args A) {
     Tl = Al + kE1CapBig;
   } else {
     unsigned char *e = base + 2 * kE1Stage * sizeof(double2) + 16;
-    Az = reinterpret_cast<double2 *>(e);
+    Az = reinterpret_cast<Key2 *>(e);
     Tz = Az + kE1Cap;
     Al = reinterpret_cast<int *>(Tz + kE1Cap);
     Tl = Al + kE1Cap;
   }
-  int x;
+  int id = gw;
   if (BIG) {
-    if (gw >= A.flags[kFlagListed]) return;
-    x = A.list[gw];
-  } else {
-    x = gw;
-    if (x >= A.nx) return;
+    if (gw >= A.nlist) return;
+    id = A.list[gw];
+  } else if (gw >= A.nx * A.segs) {
+    return;
   }
+  const int x = id % A.nx, ylo = A.yb0 + id / A.nx * A.rows, yhi = min(A.yb1, ylo + A.rows);
+  if (ylo >= yhi) return;
   if (lane == 0) {
     mbar_init(&bar[0]);
     mbar_init(&bar[1]);
@@ -256,9 +317,9 @@ __global__ void __launch_bounds__(32 * kE1Warps) k_env1(E1Args A) {
   uint32_t phase[2] = {0u, 0u};
   const int nx = A.nx;
   for (int dir = 0; dir < 2; ++dir) {
-    // forward: rows from yb0 - Dy (to build the envelope) to yb1 - 1; backward: from yb1 - 1 + Dy down to yb0
-    const int ys = dir == 0 ? max(0, A.yb0 - A.Dy) : min(A.ny - 1, A.yb1 - 1 + A.Dy);
-    const int ye = dir == 0 ? A.yb1 : A.yb0 - 1;
+    // forward: rows from ylo - Dy (to build the envelope) to yhi - 1; backward: from yhi - 1 + Dy down to ylo
+    const int ys = dir == 0 ? max(0, ylo - A.Dy) : min(A.ny - 1, yhi - 1 + A.Dy);
+    const int ye = dir == 0 ? yhi : ylo - 1;
     const int step = dir == 0 ? 1 : -1;
     int n = 0;  // envelope size (in Az, Al)
     // stage the first column
@@ -274,7 +335,7 @@ __global__ void __launch_bounds__(32 * kE1Warps) k_env1(E1Args A) {
     for (int y = ys; y != ye; y += step) {
       const int c = x + nx * y;
       const int kb = A.offs[c], m = A.offs[c + 1] - kb;
-      const double2 *N = A.z + kb;
+      Column N{nullptr, A.z + kb};
       if (staged_cur) {
         if (!mbar_wait(&bar[buf], phase[buf])) {
           if (lane == 0) {
@@ -285,7 +346,11 @@ __global__ void __launch_bounds__(32 * kE1Warps) k_env1(E1Args A) {
           return;
         }
         phase[buf] ^= 1u;
-        N = stage + buf * kE1Stage;
+        // to keys, in place
+        double2 *raw = stage + buf * kE1Stage;
+        for (int j = lane; j < m; j += 32) reinterpret_cast<Key2 *>(raw)[j] = key2_of(raw[j]);
+        N.staged = reinterpret_cast<Key2 *>(raw);
+        __syncwarp();
       }
       // prefetch the next column into the other buffer (its last reader finished at the previous step)
       const int yn = y + step;
@@ -297,7 +362,7 @@ __global__ void __launch_bounds__(32 * kE1Warps) k_env1(E1Args A) {
       for (int i0 = 0; i0 < n; i0 += 32) {
         const int i = i0 + lane;
         int cnt = 0, j0 = 0;
-        double pa = 0, pb = 0;
+        Key pa = 0, pb = 0;
         if (i < n) {
           const int age = dir == 0 ? y - Al[i] : Al[i] - y;
           if (age <= A.Dy) {
@@ -325,7 +390,7 @@ __global__ void __launch_bounds__(32 * kE1Warps) k_env1(E1Args A) {
           if (BIG) {
             atomicExch(&A.flags[kFlagFatal], 1);
           } else {
-            A.list[atomicAdd(&A.flags[kFlagListed], 1)] = x;
+            A.list[atomicAdd(&A.flags[kFlagListed], 1)] = id;
           }
         }
         // leave the line: drain the copy in flight, if any, before the block's shared memory is released
@@ -341,7 +406,7 @@ __global__ void __launch_bounds__(32 * kE1Warps) k_env1(E1Args A) {
         Al[pos] = Tl[k];
       }
       for (int j = lane; j < m; j += 32) {
-        const double2 s = N[j];
+        const Key2 s = N[j];
         const int pos = j + count_lex_leq(Tz, r, s);
         Az[pos] = s;
         Al[pos] = y;
@@ -349,7 +414,7 @@ __global__ void __launch_bounds__(32 * kE1Warps) k_env1(E1Args A) {
       n = r + m;
       __syncwarp();
       // 3. emit the envelope's pieces for this column (backward: without the column's own segments)
-      if (y >= A.yb0 && y < A.yb1) {
+      if (y >= ylo && y < yhi) {
         if (!FILL) {
           if (lane == 0) {
             if (dir == 0) A.nF[c] = n;
@@ -384,19 +449,21 @@ __global__ void __launch_bounds__(32 * kE1Warps) k_env1(E1Args A) {
 
 struct E2Args {
   int nx, yb0, Dy, W;
+  int cols, segs;        // columns per segment of a row, segments per row
+  const float *Hf;       // FP32 rounding of H, rows of stride hs
+  int hs;
   const double *H;       // [(Dy + 1) * W], NaN beyond Dx
   const int *Dx;         // [Dy + 1]
   const int32_t *poff;   // piece offsets of the band's columns (index c - yb0 * nx)
   const int32_t *nF;     // forward pieces per column (the first ones of its run)
-  const double2 *pz;
+  const Key2 *pz;
   const uint8_t *pd;
-  double2 *slots;        // kE2Out intervals per column (index c)
+  double2 *slots;        // kE2Out intervals per column (index c); keys between the two sweeps
   int32_t *counts;       // intervals per column
   int *flags;
-  int *list;             // rows (band-relative) whose stadium set outgrew the shared capacity
-  double2 *gz;           // re-run: 2 * kE2CapBig per block
+  int *list;             // row segments whose stadium set outgrew the shared capacity
+  Key2 *gz;              // re-run: 2 * kE2CapBig per block
   uint32_t *gk;          // re-run: keys, 2 * kE2CapBig per block
-  double prune_eps;      // margin of the dominance test (a bound on the H tables' rounding)
   int cap_small;         // stadium capacity of the first launch (<= kE2CapSmall)
   int *ghist;            // placement counts of columns with more than kE2Stage pieces (per block)
   int ghist_stride;      // ints per block of ghist (the band's most pieces per column + 2)
@@ -426,24 +493,28 @@ __device__ __forceinline__ bool live(uint32_t k, int x, int dir, const E2Args &A
 // M the larger of the core overhangs a_p - a_v, b_v - b_p (at least 0) and
 // M' = M + 4 table errors, the tables' chords at every later column satisfy
 // [a_v - H_v, b_v + H_v] inside [a_p - H_p, b_p + H_p] in exact arithmetic on
-// the FP64 values, hence also after each endpoint's rounding. The test takes M
-// rounded up, the table difference rounded down and prune_eps >= 2^-50 * R.
-__device__ __forceinline__ bool covers_for_life(double2 p, int dp, double2 v, uint32_t k, int x, int dir,
-                                                const E2Args &A) {
-  const int di = (int)(k >> 24), xi = (int)(k & 0xffffffu);
-  const int li = __ldg(&A.Dx[di]), lj = __ldg(&A.Dx[dp]);
-  if (dir == 0 ? x + lj < xi + li : x - lj > xi - li) return false;  // the piece expires first
-  const int age = dir == 0 ? x - xi : xi - x;
-  const double hv = __ldg(&A.H[di * A.W + age]), hp = __ldg(&A.H[dp * A.W]);
-  const double m = fmax(fmax(__dsub_ru(p.x, v.x), __dsub_ru(v.y, p.y)), 0.0);
-  return __dsub_rd(hp, hv) >= __dadd_ru(m, A.prune_eps);
+// the FP64 values, hence also after each endpoint's rounding. The test runs in
+// FP32 on values within 2^-23 of theirs (trunc32) and tables within 2^-24; eps
+// bounds those errors, the roundings of the differences and the table errors
+// four times over.
+__device__ __forceinline__ bool covers_for_life(Key2 pk, int dp, float vx, float vy, uint32_t k, float hv, int reach,
+                                                int x, int dir, const E2Args &A) {
+  const int xi = (int)(k & 0xffffffu);
+  const int lj = __ldg(&A.Dx[dp]);
+  if (dir == 0 ? x + lj < xi + reach : x - lj > xi - reach) return false;  // the piece expires first
+  const float hp = __ldg(&A.Hf[dp * A.hs]);
+  if (!(hp > hv)) return false;
+  const float px = trunc32(pk.x), py = trunc32(pk.y);
+  const float m = fmaxf(fmaxf(px - vx, vy - py), 0.f);
+  const float eps = 4.76837158203125e-7f * (fabsf(px) + fabsf(vx) + fabsf(py) + fabsf(vy) + hp + hv);
+  return hp - hv - m >= eps;
 }
 
 // Block scans over kE2Threads threads (8 warps): exclusive sum, and the
 // exclusive prefix maximum with the exclusive suffix minimum.
 struct BlockScratch {
   int isum[kE2Threads / 32];
-  double dmax[kE2Threads / 32], dmin[kE2Threads / 32];
+  Key dmax[kE2Threads / 32], dmin[kE2Threads / 32];
   int tot;
 };
 
@@ -468,80 +539,78 @@ __device__ __forceinline__ int block_excl_sum(int v, BlockScratch &s, int &total
 
 // Exclusive prefix maximum of vmax (thread order) and exclusive suffix
 // minimum of vmin (reverse order), with one pair of barriers.
-__device__ __forceinline__ void block_excl_max_min(double vmax, double vmin, BlockScratch &s, double &pmax,
-                                                   double &smin) {
+__device__ __forceinline__ void block_excl_max_min(Key vmax, Key vmin, BlockScratch &s, Key &pmax, Key &smin) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  double x = vmax, y = vmin;
+  Key x = vmax, y = vmin;
   for (int o = 1; o < 32; o <<= 1) {
-    const double a = __shfl_up_sync(0xffffffffu, x, o);
-    const double b = __shfl_down_sync(0xffffffffu, y, o);
-    if (lane >= o) x = fmax(x, a);
-    if (lane + o < 32) y = fmin(y, b);
+    const Key a = __shfl_up_sync(0xffffffffu, x, o);
+    const Key b = __shfl_down_sync(0xffffffffu, y, o);
+    if (lane >= o) x = kmax(x, a);
+    if (lane + o < 32) y = kmin(y, b);
   }
   if (lane == 31) s.dmax[w] = x;
   if (lane == 0) s.dmin[w] = y;
-  double ex = __shfl_up_sync(0xffffffffu, x, 1), ey = __shfl_down_sync(0xffffffffu, y, 1);
-  if (lane == 0) ex = -INFINITY;
-  if (lane == 31) ey = INFINITY;
+  Key ex = __shfl_up_sync(0xffffffffu, x, 1), ey = __shfl_down_sync(0xffffffffu, y, 1);
+  if (lane == 0) ex = kKeyMin;
+  if (lane == 31) ey = kKeyMax;
   __syncthreads();
-  double pre = -INFINITY, suf = INFINITY;
-  for (int k = 0; k < w; ++k) pre = fmax(pre, s.dmax[k]);
-  for (int k = w + 1; k < kE2Threads / 32; ++k) suf = fmin(suf, s.dmin[k]);
+  Key pre = kKeyMin, suf = kKeyMax;
+  for (int k = 0; k < w; ++k) pre = kmax(pre, s.dmax[k]);
+  for (int k = w + 1; k < kE2Threads / 32; ++k) suf = kmin(suf, s.dmin[k]);
   __syncthreads();
-  pmax = fmax(pre, ex);
-  smin = fmin(suf, ey);
+  pmax = kmax(pre, ex);
+  smin = kmin(suf, ey);
 }
 
 // Union of the sorted (by lower end) interval lists U1[0..n1) and U2[0..n2)
 // into out[0..), touching intervals merged; one warp; returns the count or -1
 // beyond `cap`. M is scratch for n1 + n2 entries.
-__device__ int warp_union_two(const double2 *U1, int n1, const double2 *U2, int n2, double2 *M, double2 *out,
-                              int cap) {
+__device__ int warp_union_two(const Key2 *U1, int n1, const Key2 *U2, int n2, Key2 *M, double2 *out, int cap) {
   const int lane = threadIdx.x & 31;
   for (int i = lane; i < n1; i += 32) M[i + count_less(U2, n2, U1[i].x)] = U1[i];
   for (int j = lane; j < n2; j += 32) M[j + count_leq(U1, n1, U2[j].x)] = U2[j];
   __syncwarp();
   const int n = n1 + n2;
   // sorted by lower end: a gap follows item i exactly when max(hi[0..i]) < lo[i + 1]
-  double carry = -INFINITY;
+  Key carry = kKeyMin;
   int outn = 0;
-  double start = n > 0 ? M[0].x : 0.0;
+  const Key start = n > 0 ? M[0].x : 0;
   for (int i0 = 0; i0 < n; i0 += 32) {
     const int i = i0 + lane;
-    double h = i < n ? M[i].y : -INFINITY;
+    Key h = i < n ? M[i].y : kKeyMin;
     for (int o = 1; o < 32; o <<= 1) {
-      const double y = __shfl_up_sync(0xffffffffu, h, o);
-      if (lane >= o) h = fmax(h, y);
+      const Key y = __shfl_up_sync(0xffffffffu, h, o);
+      if (lane >= o) h = kmax(h, y);
     }
-    h = fmax(h, carry);
-    const double nlo = i + 1 < n ? M[i + 1].x : INFINITY;
+    h = kmax(h, carry);
+    const Key nlo = i + 1 < n ? M[i + 1].x : kKeyMax;
     const bool gap = i < n && h < nlo;
     const unsigned bal = __ballot_sync(0xffffffffu, gap);
     // interval k ends at the k-th gap: [lo after the previous gap, h]
     const int k = outn + __popc(bal & ((1u << lane) - 1u));
-    if (gap && k < cap) out[k].y = h;
-    if (gap && k + 1 < cap && i + 1 < n) out[k + 1].x = nlo;
+    if (gap && k < cap) out[k].y = value_of(h);
+    if (gap && k + 1 < cap && i + 1 < n) out[k + 1].x = value_of(nlo);
     outn += __popc(bal);
     carry = __shfl_sync(0xffffffffu, h, 31);
   }
   __syncwarp();
-  if (lane == 0 && n > 0 && cap > 0) out[0].x = start;
+  if (lane == 0 && n > 0 && cap > 0) out[0].x = value_of(start);
   __syncwarp();
   return outn > cap ? -1 : outn;
 }
 
 template <bool BIG>
-__global__ void __launch_bounds__(kE2Threads, BIG ? 5 : 1) k_env2(E2Args A, int nrows_or_list) {
+__global__ void __launch_bounds__(kE2Threads, BIG ? 5 : 1) k_env2(E2Args A, int nitems) {
   extern __shared__ __align__(16) unsigned char e2_smem[];
   __shared__ uint64_t bar[2];
   __shared__ BlockScratch bs;
-  __shared__ double2 U[kE2Out], U1[kE2Out], Mrg[2 * kE2Out];
+  __shared__ Key2 U[kE2Out], U1[kE2Out], Mrg[2 * kE2Out];
   __shared__ int s_hist[2 * kE2Stage + 2];
   const int tid = threadIdx.x;
   const int cap = BIG ? kE2CapBig : A.cap_small;
   // shared layout: staging (2 buffers), then (first launch) stadiums S and T
-  double2 *stage = reinterpret_cast<double2 *>(e2_smem);
-  double2 *Sz, *Tz;
+  Key2 *stage = reinterpret_cast<Key2 *>(e2_smem);
+  Key2 *Sz, *Tz;
   uint32_t *Sk, *Tk;
   if (BIG) {
     Sz = A.gz + (size_t)blockIdx.x * 2 * kE2CapBig;
@@ -550,20 +619,17 @@ __global__ void __launch_bounds__(kE2Threads, BIG ? 5 : 1) k_env2(E2Args A, int 
     Tk = Sk + kE2CapBig;
   } else {
     unsigned char *p = e2_smem + 2 * kE2Stage * sizeof(double2);
-    Sz = reinterpret_cast<double2 *>(p);
+    Sz = reinterpret_cast<Key2 *>(p);
     Tz = Sz + A.cap_small;
     Sk = reinterpret_cast<uint32_t *>(Tz + A.cap_small);
     Tk = Sk + A.cap_small;
   }
-  int yrel;
-  if (BIG) {
-    if ((int)blockIdx.x >= nrows_or_list) return;
-    yrel = A.list[blockIdx.x];
-  } else {
-    yrel = blockIdx.x;
-    if (yrel >= nrows_or_list) return;
-  }
-  const int nx = A.nx, y = A.yb0 + yrel;
+  if ((int)blockIdx.x >= nitems) return;
+  const int id = BIG ? A.list[blockIdx.x] : (int)blockIdx.x;  // row segment
+  const int nx = A.nx, yrel = id / A.segs, y = A.yb0 + yrel;
+  // its columns, and how far stadiums reach into it from its sides
+  const int xlo = id % A.segs * A.cols, xhi = min(nx, xlo + A.cols), halo = A.W - 1;
+  if (xlo >= xhi) return;
   if (tid == 0) {
     mbar_init(&bar[0]);
     mbar_init(&bar[1]);
@@ -571,7 +637,8 @@ __global__ void __launch_bounds__(kE2Threads, BIG ? 5 : 1) k_env2(E2Args A, int 
   __syncthreads();
   uint32_t phase[2] = {0u, 0u};
   for (int dir = 0; dir < 2; ++dir) {
-    const int xs = dir == 0 ? 0 : nx - 1, xe = dir == 0 ? nx : -1, step = dir == 0 ? 1 : -1;
+    const int xs = dir == 0 ? max(0, xlo - halo) : min(nx - 1, xhi - 1 + halo), xe = dir == 0 ? xhi : xlo - 1;
+    const int step = dir == 0 ? 1 : -1;
     int n = 0;
     auto issue = [&](int x, int b) -> bool {
       const int bc = x + nx * yrel;
@@ -586,7 +653,7 @@ __global__ void __launch_bounds__(kE2Threads, BIG ? 5 : 1) k_env2(E2Args A, int 
     for (int x = xs; x != xe; x += step) {
       const int c = x + nx * y, bc = x + nx * yrel;
       const int kb = A.poff[bc], m = A.poff[bc + 1] - kb, f = A.nF[c], b = m - f;
-      const double2 *P = A.pz + kb;
+      const Key2 *P = A.pz + kb;
       if (staged_cur) {
         if (!mbar_wait(&bar[buf], phase[buf])) {
           if (tid == 0) {
@@ -601,7 +668,7 @@ __global__ void __launch_bounds__(kE2Threads, BIG ? 5 : 1) k_env2(E2Args A, int 
       const int xn = x + step;
       bool staged_next = false;
       if (xn != xe) staged_next = issue(xn, buf ^ 1);
-      const double2 *F = P, *B = P + f;  // the column's forward and backward pieces, each sorted
+      const Key2 *F = P, *B = P + f;  // the column's forward and backward pieces, each sorted
       const uint8_t *Fd = A.pd + kb, *Bd = A.pd + kb + f;
       // placement counts: bin c of F (0 <= c <= f) and bin f + 1 + c of B
       const int nbins = f + b + 2;
@@ -621,7 +688,7 @@ __global__ void __launch_bounds__(kE2Threads, BIG ? 5 : 1) k_env2(E2Args A, int 
       if (nn > cap) {
         if (tid == 0) {
           if (BIG) atomicExch(&A.flags[kFlagFatal], 1);
-          else A.list[atomicAdd(&A.flags[kFlagListed], 1)] = yrel;
+          else A.list[atomicAdd(&A.flags[kFlagListed], 1)] = id;
         }
         if (staged_next && tid == 0) mbar_wait(&bar[buf ^ 1], phase[buf ^ 1]);
         return;
@@ -642,7 +709,7 @@ __global__ void __launch_bounds__(kE2Threads, BIG ? 5 : 1) k_env2(E2Args A, int 
         for (int i = r0; i < r1; ++i) {
           const uint32_t k = Sk[i];
           if (live(k, x, dir, A)) {
-            const double2 v = Sz[i];
+            const Key2 v = Sz[i];
             if (cF < 0) {
               cF = count_lex_less(F, f, v);
               cB = count_lex_less(B, b, v);
@@ -656,10 +723,14 @@ __global__ void __launch_bounds__(kE2Threads, BIG ? 5 : 1) k_env2(E2Args A, int 
             // column, 3.34 s every other one, 3.41 s every fourth; two candidates instead of four: 3.55 s)
             bool dom = false;
             if ((x & 1) == 0) {
-              dom = cF > 0 && covers_for_life(F[cF - 1], Fd[cF - 1], v, k, x, dir, A);
-              dom = dom || (cF < f && covers_for_life(F[cF], Fd[cF], v, k, x, dir, A));
-              dom = dom || (cB > 0 && covers_for_life(B[cB - 1], Bd[cB - 1], v, k, x, dir, A));
-              dom = dom || (cB < b && covers_for_life(B[cB], Bd[cB], v, k, x, dir, A));
+              const float vx = trunc32(v.x), vy = trunc32(v.y);
+              const int di = (int)(k >> 24), xi = (int)(k & 0xffffffu);
+              const float hv = __ldg(&A.Hf[di * A.hs + (dir == 0 ? x - xi : xi - x)]);
+              const int reach = __ldg(&A.Dx[di]);
+              dom = cF > 0 && covers_for_life(F[cF - 1], Fd[cF - 1], vx, vy, k, hv, reach, x, dir, A);
+              dom = dom || (cF < f && covers_for_life(F[cF], Fd[cF], vx, vy, k, hv, reach, x, dir, A));
+              dom = dom || (cB > 0 && covers_for_life(B[cB - 1], Bd[cB - 1], vx, vy, k, hv, reach, x, dir, A));
+              dom = dom || (cB < b && covers_for_life(B[cB], Bd[cB], vx, vy, k, hv, reach, x, dir, A));
             }
             Tz[pos] = v;
             Tk[pos] = dom ? kDeadKey : k;
@@ -685,7 +756,7 @@ __global__ void __launch_bounds__(kE2Threads, BIG ? 5 : 1) k_env2(E2Args A, int 
       for (int j = tid; j < m; j += kE2Threads) {
         const bool isF = j < f;
         const int jj = isF ? j : j - f;
-        const double2 p = isF ? F[jj] : B[jj];
+        const Key2 p = isF ? F[jj] : B[jj];
         const int d = isF ? Fd[jj] : Bd[jj];
         const int before = isF ? hist[jj] : hist[f + 1 + jj] - hist[f];  // survivors before the piece
         const int pos = jj + before + (isF ? count_lex_less(B, b, p) : count_lex_leq(F, f, p));
@@ -694,7 +765,7 @@ __global__ void __launch_bounds__(kE2Threads, BIG ? 5 : 1) k_env2(E2Args A, int 
       }
       __syncthreads();
       {
-        double2 *t = Sz;
+        Key2 *t = Sz;
         Sz = Tz;
         Tz = t;
         uint32_t *u = Sk;
@@ -708,13 +779,21 @@ __global__ void __launch_bounds__(kE2Threads, BIG ? 5 : 1) k_env2(E2Args A, int 
       // its survivor counts from here)
       const int L2 = (n + kE2Threads - 1) / kE2Threads;
       const int q0 = min(n, tid * L2), q1 = min(n, q0 + L2);
-      double run_max = -INFINITY, run_min = INFINITY;
+      if (x < xlo || x >= xhi) {  // beside the segment: its state only
+        keep = 0;
+        for (int i = q0; i < q1; ++i) keep += live(Sk[i], x + step, dir, A) ? 1 : 0;
+        __syncthreads();
+        staged_cur = staged_next;
+        buf ^= 1;
+        continue;
+      }
+      Key run_max = kKeyMin, run_min = kKeyMax;
       keep = 0;
       for (int i = q0; i < q1; ++i) {
         const uint32_t k = Sk[i];
         keep += live(k, x + step, dir, A) ? 1 : 0;
         if (k == kDeadKey) {  // held by a new piece's chord: no chord of its own
-          Tz[i] = make_double2(INFINITY, -INFINITY);
+          Tz[i] = make_longlong2(kKeyMax, kKeyMin);
           continue;
         }
         // every other item here is live (d <= Dy, 0 <= age <= Dx[d] < W); the clamps only keep the
@@ -722,21 +801,21 @@ __global__ void __launch_bounds__(kE2Threads, BIG ? 5 : 1) k_env2(E2Args A, int 
         const int d = min((int)(k >> 24), A.Dy);
         const int age = max(0, min(A.W - 1, dir == 0 ? x - (int)(k & 0xffffffu) : (int)(k & 0xffffffu) - x));
         const double h = __ldg(&A.H[d * A.W + age]);
-        const double2 zz = Sz[i];
-        const double lo = __dsub_rn(zz.x, h), hi = __dadd_rn(zz.y, h);
-        Tz[i] = make_double2(lo, hi);
-        run_max = fmax(run_max, hi);
-        run_min = fmin(run_min, lo);
+        const Key2 zz = Sz[i];
+        const Key lo = key_of(__dsub_rn(value_of(zz.x), h)), hi = key_of(__dadd_rn(value_of(zz.y), h));
+        Tz[i] = make_longlong2(lo, hi);
+        run_max = kmax(run_max, hi);
+        run_min = kmin(run_min, lo);
       }
-      double pmax0, smin_after;
+      Key pmax0, smin_after;
       block_excl_max_min(run_max, run_min, bs, pmax0, smin_after);
-      double start0 = INFINITY;
+      Key start0 = kKeyMax;
       {
-        double sm = smin_after;
+        Key sm = smin_after;
         for (int i = q1 - 1; i >= q0; --i) {
-          const double lo = Tz[i].x;
+          const Key lo = Tz[i].x;
           Tz[i].x = sm;  // min lo over items i + 1 .. n - 1
-          sm = fmin(sm, lo);
+          sm = kmin(sm, lo);
         }
         if (q0 == 0 && q1 > 0) start0 = sm;  // min lo over all items
       }
@@ -744,11 +823,11 @@ __global__ void __launch_bounds__(kE2Threads, BIG ? 5 : 1) k_env2(E2Args A, int 
       // and the live items after which only dead ones follow (no later start) have none
       int gaps = 0;
       {
-        double pm = pmax0;
+        Key pm = pmax0;
         for (int i = q0; i < q1; ++i) {
-          const double2 t = Tz[i];
-          pm = fmax(pm, t.y);
-          if (i + 1 < n && t.y != -INFINITY && t.x != INFINITY && pm < t.x) ++gaps;
+          const Key2 t = Tz[i];
+          pm = kmax(pm, t.y);
+          if (i + 1 < n && t.y != kKeyMin && t.x != kKeyMax && pm < t.x) ++gaps;
         }
       }
       int G;
@@ -760,13 +839,13 @@ __global__ void __launch_bounds__(kE2Threads, BIG ? 5 : 1) k_env2(E2Args A, int 
         return;
       }
       {
-        double pm = pmax0;
+        Key pm = pmax0;
         int g = gbase;
         if (q0 == 0 && q1 > 0) U[0].x = start0;
         for (int i = q0; i < q1; ++i) {
-          const double2 t = Tz[i];
-          pm = fmax(pm, t.y);
-          if (i + 1 < n && t.y != -INFINITY && t.x != INFINITY && pm < t.x) {
+          const Key2 t = Tz[i];
+          pm = kmax(pm, t.y);
+          if (i + 1 < n && t.y != kKeyMin && t.x != kKeyMax && pm < t.x) {
             U[g].y = pm;
             U[g + 1].x = t.x;
             ++g;
@@ -778,11 +857,11 @@ __global__ void __launch_bounds__(kE2Threads, BIG ? 5 : 1) k_env2(E2Args A, int 
       // ---- 4. output: the forward half-union to the column's slot; backward: merged with it
       double2 *slot = A.slots + (size_t)c * kE2Out;
       if (dir == 0) {
-        for (int k = tid; k < nu; k += kE2Threads) slot[k] = U[k];
+        for (int k = tid; k < nu; k += kE2Threads) reinterpret_cast<Key2 *>(slot)[k] = U[k];
         if (tid == 0) A.counts[c] = nu;
       } else if (tid < 32) {
         const int n1 = A.counts[c];
-        for (int k = tid; k < n1; k += 32) U1[k] = slot[k];
+        for (int k = tid; k < n1; k += 32) U1[k] = reinterpret_cast<const Key2 *>(slot)[k];
         __syncwarp();
         const int nf = warp_union_two(U1, n1, U, nu, Mrg, slot, kE2Out);
         if (tid == 0) {
@@ -815,7 +894,7 @@ __global__ void k_row_pieces(int nx, int ny, const int32_t *nF, const int32_t *n
   rows[y] = s;
 }
 
-// Lists every row of a band for the global-memory sweep.
+// Lists every row segment of a band for the global-memory sweep.
 __global__ void k_list_rows(int n, int *list, int *flags) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) list[i] = i;
@@ -868,19 +947,29 @@ int dilate_envelope(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out,
   int32_t *nF = nullptr, *nB = nullptr, *counts = nullptr, *bcnt = nullptr, *list = nullptr;
   long long *rowp = nullptr;
   double2 *slots = nullptr;
+  // Segments of the lines (pass 1) and rows (pass 2): enough to give every SM `per` of them (the warps of
+  // six pass-1 blocks, three times the pass-2 blocks it holds), with at least eight times the halo that
+  // each one sweeps beside its own part, so that this costs at most an eighth more steps. Whole lines
+  // remain where there are that many: 512^2, r = 16 gains (see above), 2048^2 has the lines.
+  int sms = 0;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+  auto segments = [sms](int length, int lines, int halo, int per) {
+    const int want = (per * std::max(sms, 1) + lines - 1) / std::max(lines, 1);
+    return std::max(1, std::min(want, length / std::max(32, 8 * halo)));
+  };
   rc = dalloc(ctx, &nF, (size_t)ncols);
   if (!rc) rc = dalloc(ctx, &nB, (size_t)ncols);
   if (!rc) rc = dalloc(ctx, &counts, (size_t)ncols + 1);
   if (!rc) rc = dalloc(ctx, &bcnt, (size_t)ncols + 1);
-  if (!rc) rc = dalloc(ctx, &list, (size_t)std::max(nx, ny));
+  if (!rc) rc = dalloc(ctx, &list, (size_t)std::max(nx, ny) * (size_t)std::max(1, std::max(nx, ny) / 32 + 1));
   if (!rc) rc = dalloc(ctx, &rowp, (size_t)ny);
   if (!rc) rc = dalloc(ctx, &slots, (size_t)ncols * kE2Out);
-  double2 *gz1 = nullptr, *gz2 = nullptr;
-  int gz1_lines = 0;
+  Key2 *gz1 = nullptr, *gz2 = nullptr;
+  int gz1_lines = 0, big1_most = 0;
   int *gl1 = nullptr, *ghist = nullptr;
   uint32_t *gk2 = nullptr;
   int32_t *poff = nullptr;
-  double2 *pz = nullptr;
+  Key2 *pz = nullptr;
   uint8_t *pd = nullptr;
   vo_volume *res = nullptr;
   int fallback = 0;
@@ -890,14 +979,20 @@ int dilate_envelope(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out,
     VO_CK(ctx, cudaStreamSynchronize(ctx->stream));
     return VO_OK;
   };
-  E1Args a1{nx, ny, 0, ny, Dy, in->offs, in->z, nF, nB, nullptr, nullptr, nullptr, ctx->d_flags, list, nullptr,
-            nullptr};
-  const int e1_blocks = (nx + kE1Warps - 1) / kE1Warps;
+  E1Args a1{nx, ny, 0, ny, Dy, 0, 0, in->offs, in->z, nF, nB, nullptr, nullptr, nullptr, ctx->d_flags, list, nullptr,
+            nullptr, 0};
+  auto segment_lines = [&](E1Args &a) {
+    const int rows = a.yb1 - a.yb0, segs = segments(rows, nx, Dy, 24);
+    a.rows = (rows + segs - 1) / segs;
+    a.segs = segs;
+    return (nx * segs + kE1Warps - 1) / kE1Warps;
+  };
   float ms1 = 0, ms2 = 0;
   // ---- pass 1, count (every row)
   if (!rc) {
     cudaMemsetAsync(ctx->d_flags, 0, 3 * sizeof(int), ctx->stream);
     cudaEventRecord(ctx->ev[0], ctx->stream);
+    const int e1_blocks = segment_lines(a1);
     k_env1<false, false><<<e1_blocks, 32 * kE1Warps, e1_smem_bytes(false), ctx->stream>>>(a1);
     ctx->launches += 1;
     rc = flags_now();
@@ -907,22 +1002,31 @@ int dilate_envelope(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out,
     const int nl = hflags[kFlagListed];
     if (nl == 0 || hflags[kFlagFatal]) return VO_OK;
     if (!a.pz) ctx->ovf_cols += nl;  // counted once, in the count pass
-    if (nl > gz1_lines) {
+    if (gz1_lines == 0 || (nl > gz1_lines && gz1_lines < big1_most)) {
+      // as many at a time as fit a quarter of the free device memory
       dfree(ctx, gz1);
       dfree(ctx, gl1);
       gz1 = nullptr;
       gl1 = nullptr;
-      int r2 = dalloc(ctx, &gz1, (size_t)2 * kE1CapBig * nl);
-      if (!r2) r2 = dalloc(ctx, &gl1, (size_t)2 * kE1CapBig * nl);
+      size_t freeb = 0, totb = 0;
+      cudaMemGetInfo(&freeb, &totb);
+      big1_most = (int)std::max<size_t>(1, std::min<size_t>(1 << 20, freeb / 4 / (2 * kE1CapBig * (sizeof(Key2) + sizeof(int)))));
+      gz1_lines = std::min(nl, big1_most);
+      int r2 = dalloc(ctx, &gz1, (size_t)2 * kE1CapBig * gz1_lines);
+      if (!r2) r2 = dalloc(ctx, &gl1, (size_t)2 * kE1CapBig * gz1_lines);
       if (r2) return r2;
-      gz1_lines = nl;
     }
     a.gz = gz1;
     a.gl = gl1;
-    const int blocks = (nl + kE1Warps - 1) / kE1Warps;
-    if (a.pz) k_env1<true, true><<<blocks, 32 * kE1Warps, e1_smem_bytes(true), ctx->stream>>>(a);
-    else k_env1<false, true><<<blocks, 32 * kE1Warps, e1_smem_bytes(true), ctx->stream>>>(a);
-    ctx->launches += 1;
+    int *const listed = a.list;
+    for (int l0 = 0; l0 < nl; l0 += gz1_lines) {
+      a.list = listed + l0;
+      a.nlist = std::min(gz1_lines, nl - l0);
+      const int blocks = (a.nlist + kE1Warps - 1) / kE1Warps;
+      if (a.pz) k_env1<true, true><<<blocks, 32 * kE1Warps, e1_smem_bytes(true), ctx->stream>>>(a);
+      else k_env1<false, true><<<blocks, 32 * kE1Warps, e1_smem_bytes(true), ctx->stream>>>(a);
+      ctx->launches += 1;
+    }
     return flags_now();
   };
   if (!rc) rc = run_big1(a1);
@@ -979,7 +1083,9 @@ int dilate_envelope(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out,
     // placement counts of columns beyond the staging buffer live in global memory, one range per block
     const int max_pieces = hflags[3];
     const int hstride = max_pieces > kE2Stage ? max_pieces + 2 : 0;
-    if (!rc && hstride > 0) rc = dalloc(ctx, &ghist, (size_t)hstride * (yb1 - yb0));
+    // (whole rows then: one range per row, however large a column)
+    const int rows2 = yb1 - yb0, segs2 = hstride > 0 ? 1 : segments(nx, rows2, W - 1, 16), items2 = rows2 * segs2;
+    if (!rc && hstride > 0) rc = dalloc(ctx, &ghist, (size_t)hstride * items2);
     if (!rc) rc = dalloc(ctx, &pz, (size_t)ptotal);
     if (!rc) rc = dalloc(ctx, &pd, (size_t)ptotal);
     if (rc) break;
@@ -996,6 +1102,7 @@ int dilate_envelope(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out,
     cudaEventCreate(&e2);
     cudaMemsetAsync(ctx->d_flags, 0, 3 * sizeof(int), ctx->stream);
     cudaEventRecord(e0, ctx->stream);
+    const int e1_blocks = segment_lines(f1);
     k_env1<true, false><<<e1_blocks, 32 * kE1Warps, e1_smem_bytes(false), ctx->stream>>>(f1);
     ctx->launches += 1;
     rc = flags_now();
@@ -1003,21 +1110,19 @@ int dilate_envelope(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out,
     if (!rc && hflags[kFlagFatal]) fallback = 1;
     cudaEventRecord(e1, ctx->stream);
     if (!rc && !fallback) {
-      E2Args a2{nx,    yb0,    Dy,      W,  T->H, T->Dx, poff, nF, pz, pd, slots, counts, ctx->d_flags, list,
-                nullptr, nullptr, std::ldexp(std::max(R, 1.0), -46), cap2, ghist, hstride};
+      E2Args a2{nx, yb0, Dy, W, (nx + segs2 - 1) / segs2, segs2, T->Hp, T->host.hs, T->H, T->Dx, poff, nF, pz, pd,
+                slots, counts, ctx->d_flags, list, nullptr, nullptr, cap2, ghist, hstride};
       cudaMemsetAsync(ctx->d_flags, 0, 3 * sizeof(int), ctx->stream);
-      // The global-memory sweep runs five rows per SM against one in shared memory (227 KB per
-      // block); with at least two rows per SM to run it is the faster one (1024^2 spheres, r = 16:
+      // The global-memory sweep runs five row segments per SM against one in shared memory (227 KB per
+      // block); with at least two per SM to run it is the faster one (1024^2 spheres, r = 16, whole rows:
       // 389 against 467 ms), and so it is for rows whose live-stadium state would mostly outgrow
       // shared memory, estimated as a third of the pieces of the floor(R) + 1 columns within reach
       // (what the pruning leaves on the 2048^2 and 1024^2 sphere workloads at r = 32).
       const double mean_pieces = bcols > 0 ? (double)ptotal / bcols : 0.0;
-      int sms = 0;
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
-      if (yb1 - yb0 >= 2 * std::max(sms, 1) || mean_pieces * (Dy + 1) / 3.0 > 0.6 * cap2) {
-        k_list_rows<<<(yb1 - yb0 + 255) / 256, 256, 0, ctx->stream>>>(yb1 - yb0, list, ctx->d_flags);
+      if (items2 >= 2 * std::max(sms, 1) || mean_pieces * (Dy + 1) / 3.0 > 0.6 * cap2) {
+        k_list_rows<<<(items2 + 255) / 256, 256, 0, ctx->stream>>>(items2, list, ctx->d_flags);
       } else {
-        k_env2<false><<<yb1 - yb0, kE2Threads, e2_smem_bytes(false), ctx->stream>>>(a2, yb1 - yb0);
+        k_env2<false><<<items2, kE2Threads, e2_smem_bytes(false), ctx->stream>>>(a2, items2);
       }
       ctx->launches += 1;
       rc = flags_now();
