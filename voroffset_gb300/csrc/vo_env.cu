@@ -124,24 +124,8 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
 
 // ------------------------------------------------------------ ordered keys
 
-// Both passes compare and select values far more often than they add them, and
-// an FP64 comparison occupies the SM for as long as sixteen integer ones. So
-// pieces and stadiums hold their ends as signed integers of the same order (the
-// bit pattern, its lower 63 bits flipped for negative values, -0 as 0), and
-// only a chord's two additions go through FP64.
-using Key = long long;
-using Key2 = longlong2;
-constexpr Key kKeyMin = -0x7fffffffffffffffll - 1, kKeyMax = 0x7fffffffffffffffll;
-
-__device__ __forceinline__ Key key_of(double v) {
-  const Key b = __double_as_longlong(v);
-  const Key k = b ^ ((b >> 63) & 0x7fffffffffffffffll);
-  return k == -1 ? 0 : k;  // -0
-}
-__device__ __forceinline__ double value_of(Key k) {
-  return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffll));
-}
-__device__ __forceinline__ Key2 key2_of(double2 v) { return make_longlong2(key_of(v.x), key_of(v.y)); }
+// Pieces and stadiums hold their ends as ordered integers (Key); only a chord's
+// two additions go through FP64.
 // The value as FP32, rounded towards zero (NaN beyond its range): integer
 // operations only, within 2^-23 of the magnitude for normal values, 0 for
 // smaller ones.
@@ -152,8 +136,6 @@ __device__ __forceinline__ float trunc32(Key k) {
   if (e >= 0x47f00000u) f = 0x7fc00000u;
   return __uint_as_float((hi & 0x80000000u) | f);
 }
-__device__ __forceinline__ Key kmax(Key a, Key b) { return a > b ? a : b; }
-__device__ __forceinline__ Key kmin(Key a, Key b) { return a < b ? a : b; }
 
 // ------------------------------------------------------------ small searches
 

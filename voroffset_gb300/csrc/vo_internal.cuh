@@ -291,4 +291,26 @@ int sizer_predict_device(vo_ctx *ctx, const vo_sizer *s, const float *feats, int
 // Volume allocation (vo_api.cu).
 int volume_alloc(vo_ctx *ctx, const vo_grid &g, int64_t nseg, vo_volume **out);
 
+#ifdef __CUDACC__
+// The FP64 methods compare and select values far more often than they add them,
+// and an FP64 comparison occupies the SM for as long as sixteen integer ones.
+// So they hold ends as signed integers of the same order: the bit pattern, its
+// lower 63 bits flipped for negative values, -0 as 0.
+using Key = long long;
+using Key2 = longlong2;
+constexpr Key kKeyMin = -0x7fffffffffffffffll - 1, kKeyMax = 0x7fffffffffffffffll;
+
+__device__ __forceinline__ Key key_of(double v) {
+  const Key b = __double_as_longlong(v);
+  const Key k = b ^ ((b >> 63) & 0x7fffffffffffffffll);
+  return k == -1 ? 0 : k;  // -0
+}
+__device__ __forceinline__ double value_of(Key k) {
+  return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffll));
+}
+__device__ __forceinline__ Key2 key2_of(double2 v) { return make_longlong2(key_of(v.x), key_of(v.y)); }
+__device__ __forceinline__ Key kmax(Key a, Key b) { return a > b ? a : b; }
+__device__ __forceinline__ Key kmin(Key a, Key b) { return a < b ? a : b; }
+#endif
+
 }  // namespace vo

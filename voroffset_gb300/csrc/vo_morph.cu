@@ -1,7 +1,8 @@
 // Dexel morphology kernels for sm_103a and their host drivers.
 //
 // Separable dilation ("ours", src/vor3d/VoronoiVorPower.cpp:24-96) runs as
-// two passes, each count -> scan -> fill, one thread per output column:
+// two passes, one thread or a few per output column; pass 1 counts, then fills,
+// pass 2 keeps what it finds until the offsets are known:
 //
 //   pass 1 (replaces the y-sweeps of Voronoi2D.cpp + the radius-aware
 //   appendSegment/unionSegs of MorphologyOperators.cpp:37-95, .hpp:74-127):
@@ -36,6 +37,9 @@ namespace vo {
 namespace {
 
 constexpr int kBX = 32, kBY = 4;  // 2D thread block: x-major, 128 threads
+constexpr int kPass2Lanes = 4;    // threads that share a column's union where that is the faster way
+constexpr long long kPass2SplitCols = 16384;  // up to this many columns, times W^2, share (k_pass2)
+constexpr int kUnionSlots = 16;   // intervals of a column's union kept until the offsets are known
 constexpr int kBigThreads = 32;   // threads per block of the overflow re-run kernels
 
 __device__ __forceinline__ double dsub(double a, double b) { return __dsub_rn(a, b); }
@@ -49,42 +53,43 @@ __device__ __forceinline__ double dadd(double a, double b) { return __dadd_rn(a,
 struct MergeStream {
   const double2 *z;
   int ia, ea, ib, eb;
-  __device__ bool next(double &ma, double &mb) {
+  Key2 ha, hb;  // the next segment of each list
+  __device__ __forceinline__ void start(const double2 *zz, int a0, int a1, int b0, int b1) {
+    z = zz, ia = a0, ea = a1, ib = b0, eb = b1;
+    ha = hb = make_longlong2(kKeyMax, kKeyMax);
+    if (ia < ea) ha = key2_of(z[ia]);
+    if (ib < eb) hb = key2_of(z[ib]);
+  }
+  __device__ __forceinline__ bool from_b() const { return ib < eb && (ia >= ea || hb.x <= ha.x); }
+  __device__ __forceinline__ Key2 take() {
+    Key2 s;
+    if (from_b()) {
+      s = hb;
+      if (++ib < eb) hb = key2_of(z[ib]);
+    } else {
+      s = ha;
+      if (++ia < ea) ha = key2_of(z[ia]);
+    }
+    return s;
+  }
+  __device__ __forceinline__ bool next(Key &ma, Key &mb) {
     if (ia >= ea && ib >= eb) return false;
-    double2 s;
-    if (ib < eb && (ia >= ea || z[ib].x <= z[ia].x))
-      s = z[ib++];
-    else
-      s = z[ia++];
+    Key2 s = take();
     ma = s.x;
     mb = s.y;
-    for (;;) {
-      double nx;
-      bool fromb;
-      if (ib < eb && (ia >= ea || z[ib].x <= z[ia].x)) {
-        nx = z[ib].x;
-        fromb = true;
-      } else if (ia < ea) {
-        nx = z[ia].x;
-        fromb = false;
-      } else {
-        break;
-      }
-      if (!(nx <= mb)) break;
-      double ny = fromb ? z[ib++].y : z[ia++].y;
-      if (ny > mb) mb = ny;
-    }
+    while ((ia < ea || ib < eb) && (from_b() ? hb.x : ha.x) <= mb) mb = kmax(mb, take().y);
     return true;
   }
 };
 
-__device__ __forceinline__ bool list_append(double2 *Q, int &nQ, int cap, double lo, double hi) {
-  if (nQ > 0 && Q[nQ - 1].y == lo) {
-    Q[nQ - 1].y = hi;
+__device__ __forceinline__ bool list_append(Key2 *Q, int &nQ, int cap, Key &last, Key lo, Key hi) {
+  if (nQ > 0 && last == lo) {
+    Q[nQ - 1].y = last = hi;
     return true;
   }
   if (nQ >= cap) return false;
-  Q[nQ++] = make_double2(lo, hi);
+  Q[nQ++] = make_longlong2(lo, hi);
+  last = hi;
   return true;
 }
 
@@ -93,48 +98,50 @@ __device__ __forceinline__ bool list_append(double2 *Q, int &nQ, int cap, double
 // (by label, then z).
 template <bool FILL>
 __device__ int pass1_column(int x, int y, int nx, int ny, const int32_t *__restrict__ offs,
-                            const double2 *__restrict__ z, int Dy, double2 *P, double2 *Q,
+                            const double2 *__restrict__ z, int Dy, Key2 *P, Key2 *Q,
                             int cap, double2 *outz, uint8_t *outd) {
+  const Key none_below = key_of(-INFINITY), none_above = key_of(INFINITY);
   int nP = 0, np = 0;
   for (int d = 0; d <= Dy; ++d) {
-    MergeStream ms;
-    ms.z = z;
-    ms.ia = ms.ea = ms.ib = ms.eb = 0;
+    int a0 = 0, a1 = 0, b0 = 0, b1 = 0;
     const int ya = y - d, yb = y + d;
     if (ya >= 0) {
       const int c = x + nx * ya;
-      ms.ia = offs[c];
-      ms.ea = offs[c + 1];
+      a0 = offs[c];
+      a1 = offs[c + 1];
     }
     if (d > 0 && yb < ny) {
       const int c = x + nx * yb;
-      ms.ib = offs[c];
-      ms.eb = offs[c + 1];
+      b0 = offs[c];
+      b1 = offs[c + 1];
     }
-    if (ms.ia == ms.ea && ms.ib == ms.eb) continue;
-    double ma = 0, mb = 0;
+    if (a0 == a1 && b0 == b1) continue;
+    MergeStream ms;
+    ms.start(z, a0, a1, b0, b1);
+    Key ma = 0, mb = 0, last = 0;
     bool mv = ms.next(ma, mb);
     int nQ = 0;
+    Key2 below = make_longlong2(none_below, none_below);
     for (int k = 0; k <= nP; ++k) {
-      if (k > 0 && !list_append(Q, nQ, cap, P[k - 1].x, P[k - 1].y)) return -1;
-      const double g1 = k == 0 ? -INFINITY : P[k - 1].y;
-      const double g2 = k == nP ? INFINITY : P[k].x;
+      if (k > 0 && !list_append(Q, nQ, cap, last, below.x, below.y)) return -1;
+      const Key2 above = k == nP ? make_longlong2(none_above, none_above) : P[k];
+      const Key g1 = below.y, g2 = above.x;
+      below = above;
       if (!(g1 < g2)) continue;
       while (mv && mb <= g1) mv = ms.next(ma, mb);
       while (mv && ma < g2) {
-        const double lo = ma > g1 ? ma : g1;
-        const double hi = mb < g2 ? mb : g2;
+        const Key lo = kmax(ma, g1), hi = kmin(mb, g2);
         if (FILL) {
-          outz[np] = make_double2(lo, hi);
+          outz[np] = make_double2(value_of(lo), value_of(hi));
           outd[np] = (uint8_t)d;
         }
         ++np;
-        if (!list_append(Q, nQ, cap, lo, hi)) return -1;
+        if (!list_append(Q, nQ, cap, last, lo, hi)) return -1;
         if (mb >= g2) break;
         mv = ms.next(ma, mb);
       }
     }
-    double2 *t = P;
+    Key2 *t = P;
     P = Q;
     Q = t;
     nP = nQ;
@@ -178,48 +185,93 @@ __device__ __forceinline__ bool union_insert(double2 *A, int &n, int cap, double
 
 // ---------------------------------------------------------------- pass 2
 
-template <bool FILL>
+// The same on ordered integers, as one function: pass 2 calls it from several
+// places, and copies of it would crowd the instruction cache. Returns the
+// position of the interval that now holds [lo, hi], or -1 beyond `cap`.
+__device__ __noinline__ int2 union_insert_keys(Key2 *A, int n, int cap, Key lo, Key hi) {
+  int l = 0, r = n;
+  while (l < r) {
+    const int m = (l + r) >> 1;
+    if (A[m].y >= lo)
+      r = m;
+    else
+      l = m + 1;
+  }
+  if (l == n || A[l].x > hi) {
+    if (n >= cap) return make_int2(-1, n);
+    for (int k = n; k > l; --k) A[k] = A[k - 1];
+    A[l] = make_longlong2(lo, hi);
+    return make_int2(l, n + 1);
+  }
+  int j = l;
+  while (j + 1 < n && A[j + 1].x <= hi) ++j;
+  A[l] = make_longlong2(kmin(A[l].x, lo), kmax(A[j].y, hi));
+  if (j > l) {
+    const int sh = j - l;
+    for (int k = l + 1; k + sh < n; ++k) A[k] = A[k + sh];
+    n -= sh;
+  }
+  return make_int2(l, n);
+}
+
+// The union of column (x, y)'s chords into A; returns their count or -1 beyond
+// `cap`. Most chords lie inside an interval that is there already: the one the
+// last insertion made is kept in registers, and a chord inside it is passed
+// over. Pieces are loaded four at a time so that their latencies overlap.
 __device__ int pass2_column(int x, int y, int nx, const int32_t *__restrict__ poffs,
                             const double2 *__restrict__ pz, const uint8_t *__restrict__ pd,
                             const DevTables t, const double *__restrict__ sH,
-                            const int *__restrict__ sDx, double2 *A, int cap, double2 *outz) {
+                            const int *__restrict__ sDx, Key2 *A, int cap, int first = 0, int stride = 1) {
+  constexpr int kStep = 4;
   int nA = 0;
+  Key2 hot = make_longlong2(kKeyMax, kKeyMin);
   const int W = t.W;
-  for (int adx = 0; adx < W; ++adx) {
-    for (int s = 0; s < 2; ++s) {
-      if (adx == 0 && s == 1) break;
-      const int xs = s == 0 ? x - adx : x + adx;
-      if (xs < 0 || xs >= nx) continue;
-      const int c = xs + nx * y;
-      const int b = poffs[c], e = poffs[c + 1];
-      bool open = false;
-      double glo = 0, ghi = 0;
-      for (int k = b; k < e; ++k) {
-        const int d = pd[k];
-        if (adx > sDx[d]) continue;
-        const double h = sH[d * W + adx];
-        const double2 p = pz[k];
-        if (p.x > p.y) {
-          if (!union_insert(A, nA, cap, dsub(p.x, h), dadd(p.x, h))) return -1;
-          if (!union_insert(A, nA, cap, dsub(p.y, h), dadd(p.y, h))) return -1;
-          continue;
+  auto insert = [&](Key lo, Key hi) {
+    const int2 at = union_insert_keys(A, nA, cap, lo, hi);
+    nA = at.y;
+    if (at.x >= 0) hot = A[at.x];
+    return at.x >= 0;
+  };
+  for (int side = first; side < 2 * W - 1; side += stride) {
+    const int adx = (side + 1) >> 1;
+    const int xs = (side & 1) ? x - adx : x + adx;
+    if (xs < 0 || xs >= nx) continue;
+    const int c = xs + nx * y;
+    const int b = poffs[c], e = poffs[c + 1];
+    bool open = false;
+    Key glo = 0, ghi = 0;
+    for (int k0 = b; k0 < e; k0 += kStep) {
+      double2 p[kStep];
+      int d[kStep];
+#pragma unroll
+      for (int j = 0; j < kStep; ++j) {
+        const int k = min(k0 + j, e - 1);
+        p[j] = pz[k];
+        d[j] = pd[k];
+      }
+#pragma unroll
+      for (int j = 0; j < kStep; ++j) {
+        if (k0 + j >= e || adx > sDx[d[j]]) continue;
+        const double h = sH[d[j] * W + adx];
+        Key lo = key_of(dsub(p[j].x, h)), hi = key_of(dadd(p[j].y, h));
+        if (key_of(p[j].x) > key_of(p[j].y)) {
+          if (!insert(lo, key_of(dadd(p[j].x, h)))) return -1;
+          lo = key_of(dsub(p[j].y, h));
         }
-        const double lo = dsub(p.x, h), hi = dadd(p.y, h);
+        if (lo >= hot.x && hi <= hot.y) continue;
         if (open && lo <= ghi && hi >= glo) {
-          if (lo < glo) glo = lo;
-          if (hi > ghi) ghi = hi;
+          glo = kmin(glo, lo);
+          ghi = kmax(ghi, hi);
         } else {
-          if (open && !union_insert(A, nA, cap, glo, ghi)) return -1;
+          if (open && !insert(glo, ghi)) return -1;
           open = true;
           glo = lo;
           ghi = hi;
         }
       }
-      if (open && !union_insert(A, nA, cap, glo, ghi)) return -1;
     }
+    if (open && !insert(glo, ghi)) return -1;
   }
-  if (FILL)
-    for (int k = 0; k < nA; ++k) outz[k] = A[k];
   return nA;
 }
 
@@ -287,7 +339,7 @@ __global__ void __launch_bounds__(kBX *kBY) k_pass1(int nx, int ny, const int32_
   const int y = blockIdx.y * kBY + threadIdx.y;
   if (x >= nx || y >= ny) return;
   const int c = x + nx * y;
-  double2 P[kCapSmall], Q[kCapSmall];
+  Key2 P[kCapSmall], Q[kCapSmall];
   double2 *oz = FILL ? pz + poffs[c] : nullptr;
   uint8_t *od = FILL ? pd + poffs[c] : nullptr;
   const int n = pass1_column<FILL>(x, y, nx, ny, offs, z, Dy, P, Q, kCapSmall, oz, od);
@@ -311,8 +363,8 @@ __global__ void __launch_bounds__(kBigThreads) k_pass1_big(int nx, int ny, const
                                                           double2 *scratch) {
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   const int nthreads = gridDim.x * blockDim.x;
-  double2 *P = scratch + (size_t)tid * 2 * kCapLarge;
-  double2 *Q = P + kCapLarge;
+  Key2 *P = reinterpret_cast<Key2 *>(scratch) + (size_t)tid * 2 * kCapLarge;
+  Key2 *Q = P + kCapLarge;
   const int n_ovf = *ovf.count;
   for (int i = tid; i < n_ovf; i += nthreads) {
     const int c = ovf.cols[i];
@@ -329,33 +381,84 @@ __global__ void __launch_bounds__(kBigThreads) k_pass1_big(int nx, int ny, const
   }
 }
 
-template <bool FILL>
+// A column's union is found once: up to `nslots` of its intervals wait in its
+// slots (interval i of column c at slots[i * ncols + c]) until the offsets are
+// known, and k_pass2_place moves them. Only a larger union is found again there.
+//
+// What bounds it is latency: a column is a chain of dependent insertions. With
+// LANES = 4 each of four threads takes every fourth source column, and the first
+// one then inserts the others' unions into its own. That pays while there are
+// few columns for the chip or many source columns for a thread (ms with one and
+// with four threads; W = 3, 9 and 21 are radii 2, 8 and 20):
+//   256^2   0.059 / 0.049   0.52 / 0.22   1.99 / 0.85
+//   512^2   0.083 / 0.108   0.86 / 0.60   4.81 / 2.94
+//   1024^2  0.21 / 0.35     2.24 / 2.04   14.4 / 10.8
+//   2048^2  0.66 / 1.31     7.36 / 7.57   50.0 / 41.1
+// Hence the rule: columns <= 16384 W^2. Two threads are in between, eight are
+// better by up to a third below 512^2 and worse by as much above. A pass over
+// FP64 ends without the interval in registers, run to count and again to fill,
+// took 2 x 0.90 (256^2, r = 8) and 2 x 22 ms (2048^2, r = 8).
+template <int LANES>
 __global__ void __launch_bounds__(kBX *kBY) k_pass2(int nx, int ny, const int32_t *__restrict__ poffs,
                                                     const double2 *__restrict__ pz,
                                                     const uint8_t *__restrict__ pd, DevTables t,
-                                                    int32_t *__restrict__ counts,
-                                                    const int32_t *__restrict__ ooffs,
-                                                    double2 *__restrict__ oz, OvfList ovf) {
+                                                    int32_t *__restrict__ counts, double2 *__restrict__ slots,
+                                                    int nslots, OvfList ovf) {
   extern __shared__ double smem[];
   const int nH = (t.Dy + 1) * t.W;
   double *sH = smem;
   int *sDx = (int *)(smem + nH);
   SmemTables::load(t, sH, sDx, nH);
   __syncthreads();
+  constexpr int kCols = kBX / LANES;
+  const int part = threadIdx.x / kCols, lane = threadIdx.x % kCols;
+  const int x = blockIdx.x * kCols + lane;
+  const int y = blockIdx.y * kBY + threadIdx.y;
+  const bool inside = x < nx && y < ny;
+  const int c = x + nx * y;
+  Key2 A[kCapSmall];
+  int n = inside ? pass2_column(x, y, nx, poffs, pz, pd, t, sH, sDx, A, kCapSmall, part, LANES) : 0;
+  // the other lanes' unions into the first one's
+#pragma unroll 1
+  for (int p = 1; p < LANES; ++p) {
+    const int from = lane + p * kCols, m = __shfl_sync(0xffffffffu, n, from);
+    if (part == 0 && m < 0) n = -1;
+    const int most = __reduce_max_sync(0xffffffffu, m);
+#pragma unroll 1
+    for (int i = 0; i < most; ++i) {
+      const Key2 s = A[min(i, kCapSmall - 1)];
+      const Key lo = __shfl_sync(0xffffffffu, s.x, from), hi = __shfl_sync(0xffffffffu, s.y, from);
+      if (part == 0 && n >= 0 && i < m) {
+        const int2 at = union_insert_keys(A, n, kCapSmall, lo, hi);
+        n = at.x < 0 ? -1 : at.y;
+      }
+    }
+  }
+  if (part != 0 || !inside) return;
+  if (n < 0) record_overflow(ovf, c);
+  counts[c] = max(n, 0);
+  if (n <= nslots)
+    for (int k = 0; k < n; ++k) slots[(size_t)k * nx * ny + c] = make_double2(value_of(A[k].x), value_of(A[k].y));
+}
+
+__global__ void __launch_bounds__(kBX *kBY) k_pass2_place(int nx, int ny, const int32_t *__restrict__ poffs,
+                                                          const double2 *__restrict__ pz,
+                                                          const uint8_t *__restrict__ pd, DevTables t,
+                                                          const int32_t *__restrict__ counts,
+                                                          const double2 *__restrict__ slots, int nslots,
+                                                          const int32_t *__restrict__ ooffs,
+                                                          double2 *__restrict__ oz) {
   const int x = blockIdx.x * kBX + threadIdx.x;
   const int y = blockIdx.y * kBY + threadIdx.y;
   if (x >= nx || y >= ny) return;
-  const int c = x + nx * y;
-  double2 A[kCapSmall];
-  const int n = pass2_column<FILL>(x, y, nx, poffs, pz, pd, t, sH, sDx, A, kCapSmall,
-                                   FILL ? oz + ooffs[c] : nullptr);
-  if (!FILL) {
-    if (n < 0) {
-      record_overflow(ovf, c);
-      counts[c] = 0;
-    } else {
-      counts[c] = n;
-    }
+  const int c = x + nx * y, n = counts[c];
+  double2 *out = oz + ooffs[c];
+  if (n <= nslots) {
+    for (int k = 0; k < n; ++k) out[k] = slots[(size_t)k * nx * ny + c];
+  } else if (n <= kCapSmall) {
+    Key2 A[kCapSmall];
+    const int m = pass2_column(x, y, nx, poffs, pz, pd, t, t.H, t.Dx, A, kCapSmall);
+    for (int k = 0; k < m; ++k) out[k] = make_double2(value_of(A[k].x), value_of(A[k].y));
   }
 }
 
@@ -369,18 +472,19 @@ __global__ void __launch_bounds__(kBigThreads) k_pass2_big(int nx, int ny, const
                                                           double2 *scratch) {
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   const int nthreads = gridDim.x * blockDim.x;
-  double2 *A = scratch + (size_t)tid * 2 * kCapLarge;
+  Key2 *A = reinterpret_cast<Key2 *>(scratch) + (size_t)tid * 2 * kCapLarge;
   const int n_ovf = *ovf.count;
   for (int i = tid; i < n_ovf; i += nthreads) {
     const int c = ovf.cols[i];
     const int x = c % nx, y = c / nx;
-    const int n = pass2_column<FILL>(x, y, nx, poffs, pz, pd, t, t.H, t.Dx, A, 2 * kCapLarge,
-                                     FILL ? oz + ooffs[c] : nullptr);
+    const int n = pass2_column(x, y, nx, poffs, pz, pd, t, t.H, t.Dx, A, 2 * kCapLarge);
     if (n < 0) {
       *ovf.fatal = 1;
       if (!FILL) counts[c] = 0;
     } else if (!FILL) {
       counts[c] = n;
+    } else {
+      for (int k = 0; k < n; ++k) oz[ooffs[c] + k] = make_double2(value_of(A[k].x), value_of(A[k].y));
     }
   }
 }
@@ -1121,6 +1225,7 @@ int dilate(vo_ctx *ctx, int method, double R, const vo_volume *in_user, vo_volum
     int32_t *poffs = nullptr;
     double2 *pz = nullptr;
     uint8_t *pd = nullptr;
+    double2 *slots = nullptr;
     long long ptotal = 0;
     rc = dalloc(ctx, &poffs, (size_t)ncols + 1);
     if (!rc) rc = scan_counts(ctx, s.counts, poffs, ncols, &ptotal);
@@ -1139,15 +1244,27 @@ int dilate(vo_ctx *ctx, int method, double R, const vo_volume *in_user, vo_volum
     // ---- pass 2
     if (!rc) {
       const size_t sh = sizeof(double) * (size_t)(t.Dy + 1) * t.W + sizeof(int) * (t.Dy + 1);
+      // slots for as many intervals per column as fit 1 GB (all of them up to 2048^2 columns)
+      const int nslots = (int)std::min<long long>(kUnionSlots, (1LL << 30) / (16LL * ncols));
+      // (the rule is explained at k_pass2)
+      const bool split = (long long)ncols <= kPass2SplitCols * t.W * t.W;
       if (sh > 200 * 1024) {
         rc = set_error(ctx, VO_EINVAL, "radius too large for the pass-2 table");
       } else {
-        cudaFuncSetAttribute(k_pass2<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
-        cudaFuncSetAttribute(k_pass2<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
+        const void *const pass2 = split ? (const void *)k_pass2<kPass2Lanes> : (const void *)k_pass2<1>;
+        cudaFuncSetAttribute(pass2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
+        rc = dalloc(ctx, &slots, (size_t)nslots * ncols);
+      }
+      if (!rc) {
         cudaMemsetAsync(ctx->d_flags, 0, 2 * sizeof(int), ctx->stream);
         cudaEventRecord(ctx->ev[4], ctx->stream);
-        k_pass2<false><<<grd, blk, sh, ctx->stream>>>(nx, ny, poffs, pz, pd, t, s.counts, nullptr,
-                                                      nullptr, ovf);
+        if (split) {
+          const int cols = kBX / kPass2Lanes;
+          k_pass2<kPass2Lanes><<<dim3((nx + cols - 1) / cols, grd.y), blk, sh, ctx->stream>>>(
+              nx, ny, poffs, pz, pd, t, s.counts, slots, nslots, ovf);
+        } else {
+          k_pass2<1><<<grd, blk, sh, ctx->stream>>>(nx, ny, poffs, pz, pd, t, s.counts, slots, nslots, ovf);
+        }
         k_pass2_big<false><<<gbig, kBigThreads, 0, ctx->stream>>>(nx, ny, poffs, pz, pd, t, s.counts,
                                                                  nullptr, nullptr, ovf, s.big);
         ctx->launches += 2;
@@ -1160,8 +1277,8 @@ int dilate(vo_ctx *ctx, int method, double R, const vo_volume *in_user, vo_volum
         }
         if (!rc) {
           cudaEventRecord(ctx->ev[6], ctx->stream);
-          k_pass2<true><<<grd, blk, sh, ctx->stream>>>(nx, ny, poffs, pz, pd, t, nullptr, res->offs,
-                                                       res->z, ovf);
+          k_pass2_place<<<grd, blk, 0, ctx->stream>>>(nx, ny, poffs, pz, pd, t, s.counts, slots, nslots, res->offs,
+                                                      res->z);
           k_pass2_big<true><<<gbig, kBigThreads, 0, ctx->stream>>>(nx, ny, poffs, pz, pd, t, nullptr,
                                                                   res->offs, res->z, ovf, s.big);
           ctx->launches += 2;
@@ -1183,6 +1300,7 @@ int dilate(vo_ctx *ctx, int method, double R, const vo_volume *in_user, vo_volum
     dfree(ctx, poffs);
     dfree(ctx, pz);
     dfree(ctx, pd);
+    dfree(ctx, slots);
   }
   free_scratch(ctx, s);
   if (norm) vo_volume_free(ctx, norm);
