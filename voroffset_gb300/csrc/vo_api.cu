@@ -68,6 +68,21 @@ int build_tables(double R, int kmax, Tables &t) {
       t.H[(size_t)d * t.W + dx] = std::sqrt(r * r - x * x);
       t.Hp[(size_t)d * t.hs + dx] = (float)t.H[(size_t)d * t.W + dx];
     }
+  // growth of H over one step inwards, along x and along y
+  auto floor16 = [](double v) -> int {  // bits of the largest FP16 not above v >= 0
+    if (v >= 65504.0) return 0x7bff;
+    const int e = v > 0 ? std::max(std::ilogb(v), -14) : -14;
+    return ((e + 14) << 10) + (int)std::floor(std::ldexp(v, 10 - e));
+  };
+  t.Dx.resize((size_t)(Dy + 1) * (t.W + 1), -1);
+  for (int d = 0; d <= Dy; ++d)
+    for (int dx = 0; dx <= t.Dx[d]; ++dx) {
+      const double h = t.H[(size_t)d * t.W + dx];
+      const double gx = dx ? std::nextafter(t.H[(size_t)d * t.W + dx - 1] - h, -1.0) : -1.0;
+      const double gy = d ? std::nextafter(t.H[(size_t)(d - 1) * t.W + dx] - h, -1.0) : -1.0;
+      t.Dx[Dy + 1 + (size_t)d * t.W + dx] =
+          (int)((unsigned)(gx < 0 ? 0xffff : floor16(gx)) | (unsigned)(gy < 0 ? 0xffff : floor16(gy)) << 16);
+    }
   t.HB.assign((size_t)(Dy + 1) * (Dy + 1), NAN);
   for (int dy = 0; dy <= Dy; ++dy)
     for (int dx = 0; dx <= Dy; ++dx) {

@@ -73,6 +73,7 @@ struct DilPlan {
   int spill_base = 0, spill_cap = 0;
   double cost = 0;  // mean candidates per column (no sizer)
   double mean_segs = 0;
+  bool direct = false;  // small radius, small columns: k_direct
   int64_t slot_entries = 0;
 };
 
@@ -251,6 +252,10 @@ int sm_count() {
   return sms > 0 ? sms : 1;
 }
 
+// Largest column of an input up to which its dilation may go column by column:
+// a union beyond that kernel's list re-runs the volume at every replay.
+constexpr int kDirectColumn = 16;
+
 // Autotuner: rounds of kTuneFrom to kTuneTo patches per SM lie where one lane
 // per column (throughput) and four (the longest patch's latency) cross, at a
 // point that depends on the input (8 dexels: 0.19 against 0.27 ms at 200^2,
@@ -291,6 +296,22 @@ int plan_dilation_round(vo_ctx *ctx, vo_batch *b, std::vector<DilPlan> &dils, bo
     const vo_grid &g = d.in.grid;
     const int ncols = g.nx * g.ny;
     const size_t entries = (size_t)std::max<int64_t>(d.in.entries, 1);
+    // mean segments per column of the input, exact for CSR inputs, the capacity's half for slots
+    d.mean_segs = d.in.owns ? d.in.cap * 0.5 : (double)d.in.entries / std::max(ncols, 1);
+    const float R = (float)b->radii[d.vol];
+    // candidates per column: lattice points of the disc x mean segments of the input (no sizer)
+    d.cost = 3.14159 * (R + 0.5) * (R + 0.5) * (d.mean_segs + 0.5);
+    d.direct = (d.in.owns || d.in.end == d.in.beg + 1) && d.in.cap <= kDirectColumn && direct_choice(g, *d.T, d.mean_segs);
+    if (d.direct) {
+      rc = plan_alloc(ctx, b, &d.pk.rec, entries);
+      if (!rc && d.in.owns) rc = plan_alloc(ctx, b, &d.pk.zx, entries);
+      if (!rc && d.in.owns) rc = plan_alloc(ctx, b, &d.pk.rbeg, 2 * (size_t)ncols);
+      if (rc) return rc;
+      d.A = fast_args(g.nx, g.ny, *d.T, d.in.beg, d.in.end, d.in.z, d.pk);
+      const DilPlan c = d;
+      record(b, 1, [c](cudaStream_t st) { direct_prepare(st, c.A, c.pk); });
+      continue;
+    }
     rc = plan_alloc(ctx, b, &d.pk.zf, entries);
     if (!rc) rc = plan_alloc(ctx, b, &d.pk.code, entries);
     if (!rc) rc = plan_alloc(ctx, b, &d.pk.zx, entries);
@@ -301,13 +322,8 @@ int plan_dilation_round(vo_ctx *ctx, vo_batch *b, std::vector<DilPlan> &dils, bo
     if (!rc) rc = plan_alloc(ctx, b, &d.big_list, (size_t)ncols);
     if (rc) return rc;
     d.A = fast_args(g.nx, g.ny, *d.T, d.in.beg, d.in.end, d.in.z, d.pk);
-    // mean segments per column of the input, exact for CSR inputs, the capacity's half for slots
-    d.mean_segs = d.in.owns ? d.in.cap * 0.5 : (double)d.in.entries / std::max(ncols, 1);
     const DilPlan c = d;
-    const float R = (float)b->radii[d.vol];
     record(b, 2, [c, R](cudaStream_t st) { fast_prepare(st, c.A, R, c.mean_segs, c.mm, c.pk); });
-    // candidates per column: lattice points of the disc x mean segments of the input (no sizer)
-    d.cost = 3.14159 * (R + 0.5) * (R + 0.5) * (d.mean_segs + 0.5);
   }
   if (ctx->sizer) run_pending(ctx, b);  // features need the dilation inputs
   int *counters = nullptr;
@@ -327,15 +343,26 @@ int plan_dilation_round(vo_ctx *ctx, vo_batch *b, std::vector<DilPlan> &dils, bo
   std::stable_sort(order.begin(), order.end(), [](const std::pair<double, int> &x, const std::pair<double, int> &y) {
     return x.first > y.first;
   });
-  if (!b->big_scratch) rc = plan_alloc(ctx, b, &b->big_scratch, big_scratch_elems());
+  // those by patches first
+  std::stable_partition(order.begin(), order.end(), [&](const std::pair<double, int> &x) { return !dils[x.second].direct; });
+  int np = 0;
+  int64_t direct_cols = 0;
+  size_t direct_shared = 0;
+  for (const DilPlan &d : dils) {
+    np += !d.direct;
+    if (d.direct) direct_cols += (int64_t)d.in.grid.nx * d.in.grid.ny;
+    if (d.direct) direct_shared = std::max(direct_shared, direct_smem(d.A));
+  }
+  const int nd = (int)dils.size() - np;
+  if (np > 0 && !b->big_scratch) rc = plan_alloc(ctx, b, &b->big_scratch, big_scratch_elems());
   if (rc) return rc;
   const size_t counter_bytes = sizeof(int) * (4 + 2 * dils.size());
   double2 *big_scratch = b->big_scratch;
-  const int nv = (int)dils.size();
   // the round's launch with `split` lanes per column
   struct RoundLaunch {
     PatchPlan P;
-    BatchVol *dvols = nullptr;
+    BatchVol *dvols = nullptr;  // those by patches, then the direct ones
+    int direct_items = 0;
   };
   auto prepare = [&](int split, RoundLaunch &L) -> int {
     std::vector<BatchVol> hv;
@@ -344,6 +371,13 @@ int plan_dilation_round(vo_ctx *ctx, vo_batch *b, std::vector<DilPlan> &dils, bo
     for (const auto &o : order) {
       const DilPlan &d = dils[o.second];
       BatchVol v = batch_vol(d, b->d_flags + d.vol);
+      if (d.direct) {
+        v.item0 = L.direct_items;
+        L.direct_items += direct_blocks(d.in.grid, direct_cols);
+        v.item1 = L.direct_items;
+        hv.push_back(v);
+        continue;
+      }
       v.item0 = (int)items;
       items += patch_count(d.in.grid, split);
       if (items > 2147483647LL) return set_error(ctx, VO_ERANGE, "batch: too many columns");
@@ -351,12 +385,12 @@ int plan_dilation_round(vo_ctx *ctx, vo_batch *b, std::vector<DilPlan> &dils, bo
       hv.push_back(v);
       hs = std::max(hs, d.T->host.hs);
     }
-    int r = patch_plan(ctx, (int)items, split, hs, L.P);
+    int r = plan_alloc(ctx, b, &L.dvols, hv.size());
     int *list = nullptr;
-    if (!r) r = plan_alloc(ctx, b, &L.dvols, hv.size());
-    if (!r) r = plan_alloc(ctx, b, &list, (size_t)items);
+    if (!r && np > 0) r = patch_plan(ctx, (int)items, split, hs, L.P);
+    if (!r && np > 0) r = plan_alloc(ctx, b, &list, (size_t)items);
     // the rounds run one after the other: they share the largest working memory of each tier
-    for (int t = 0; t < 2 && !r; ++t) {
+    for (int t = 0; t < 2 && !r && np > 0; ++t) {
       const size_t bytes = patch_scratch_bytes(L.P, t);
       if (bytes > b->scratch_bytes[t]) {
         r = plan_alloc(ctx, b, &b->scratch[t], bytes);
@@ -370,19 +404,24 @@ int plan_dilation_round(vo_ctx *ctx, vo_batch *b, std::vector<DilPlan> &dils, bo
     VO_CK(ctx, cudaStreamSynchronize(ctx->stream));
     return VO_OK;
   };
-  auto launch = [counters, counter_bytes, nv, big_scratch](const RoundLaunch &L, cudaStream_t st) {
+  auto launch = [counters, counter_bytes, np, nd, direct_cols, direct_shared, big_scratch](const RoundLaunch &L,
+                                                                                           cudaStream_t st) {
     cudaMemsetAsync(counters, 0, counter_bytes, st);
-    patch_launch(false, L.P, st, L.dvols);
-    patch_launch(true, L.P, st, L.dvols);
-    big_launch(st, L.dvols, nv, big_scratch);
+    if (np > 0) {
+      patch_launch(false, L.P, st, L.dvols);
+      patch_launch(true, L.P, st, L.dvols);
+      big_launch(st, L.dvols, np, big_scratch);
+    }
+    if (nd > 0) direct_launch(st, L.dvols + np, nd, L.direct_items, direct_cols, direct_shared);
   };
   std::vector<const vo_grid *> grids;
-  for (const DilPlan &d : dils) grids.push_back(&d.in.grid);
+  for (const DilPlan &d : dils)
+    if (!d.direct) grids.push_back(&d.in.grid);
   int split = patch_split(grids.data(), (int)grids.size());
   RoundLaunch L;
   const int64_t patches = patch_total(grids.data(), (int)grids.size());
   const int sms = sm_count();
-  if (patches < kTuneFrom * sms || patches > kTuneTo * sms) {
+  if (np == 0 || patches < kTuneFrom * sms || patches > kTuneTo * sms) {
     rc = prepare(split, L);
   } else {
     rc = tune_split(ctx, b, dils, patches, [&](int sp, float *ms) -> int {
@@ -403,14 +442,14 @@ int plan_dilation_round(vo_ctx *ctx, vo_batch *b, std::vector<DilPlan> &dils, bo
     if (!rc) rc = prepare(split, L);
   }
   if (rc) return rc;
-  record(b, 3, [launch, L](cudaStream_t st) { launch(L, st); });
+  record(b, (np > 0 ? 3 : 0) + (nd > 0 ? 1 : 0), [launch, L](cudaStream_t st) { launch(L, st); });
   for (const DilPlan &d : dils) b->spills.push_back({d.counters, d.spill_cap, b->rounds});
   ++b->rounds;
   b->stats.tile_rows = split;
   b->stats.union_cap = kUnionCapMid / 2;
   b->stats.persistent = 1;
   b->stats.regs = 96;
-  b->stats.tiles += L.P.nitems;
+  b->stats.tiles += L.P.nitems + L.direct_items;
   if (later_rounds) run_pending(ctx, b);
   return VO_OK;
 }

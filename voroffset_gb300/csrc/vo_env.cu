@@ -126,16 +126,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
 
 // Pieces and stadiums hold their ends as ordered integers (Key); only a chord's
 // two additions go through FP64.
-// The value as FP32, rounded towards zero (NaN beyond its range): integer
-// operations only, within 2^-23 of the magnitude for normal values, 0 for
-// smaller ones.
-__device__ __forceinline__ float trunc32(Key k) {
-  const Key b = k ^ ((k >> 63) & 0x7fffffffffffffffll);
-  const unsigned hi = (unsigned)(b >> 32), lo = (unsigned)b, e = hi & 0x7fffffffu;
-  unsigned f = e < 0x38100000u ? 0u : ((e - 0x38000000u) << 3) | (lo >> 29);
-  if (e >= 0x47f00000u) f = 0x7fc00000u;
-  return __uint_as_float((hi & 0x80000000u) | f);
-}
 
 // ------------------------------------------------------------ small searches
 
@@ -858,13 +848,10 @@ __global__ void __launch_bounds__(kE2Threads, BIG ? 5 : 1) k_env2(E2Args A, int 
   }
 }
 
-// Compaction of the slots into the CSR output: one warp per column.
+// Compaction of the slots into the CSR output.
 __global__ void k_env_compact(int ncols, const double2 *__restrict__ slots, const int32_t *__restrict__ ooffs,
                               double2 *__restrict__ oz) {
-  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (w >= ncols) return;
-  const int n = ooffs[w + 1] - ooffs[w];
-  for (int k = lane; k < n; k += 32) oz[ooffs[w] + k] = slots[(size_t)w * kE2Out + k];
+  compact_columns(ncols, ooffs, oz, [=](int c) { return slots + (size_t)c * kE2Out; });
 }
 
 // Pieces per row of the band (for the band split): one thread per row.
@@ -1169,7 +1156,7 @@ int dilate_envelope(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out,
       rc = dalloc(ctx, &res->z, (size_t)total);
     }
     if (!rc) {
-      k_env_compact<<<(ncols + 7) / 8, 256, 0, ctx->stream>>>(ncols, slots, res->offs, res->z);
+      k_env_compact<<<(ncols + 255) / 256, 256, 0, ctx->stream>>>(ncols, slots, res->offs, res->z);
       ctx->launches += 1;
       VO_CK(ctx, cudaGetLastError());
     }

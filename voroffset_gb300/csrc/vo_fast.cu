@@ -59,6 +59,8 @@
 // a power of two, so that binning is exact (one fused multiply-add that
 // rounds to an integer).
 //
+// Small radii take another way (k_direct).
+//
 // Capacities: a patch that needs more entries, kept-aside intervals or union
 // intervals than the launch has re-runs with larger lists (second tier), and a
 // column that outgrows those too goes to an FP64 kernel with an 8,192-interval
@@ -67,6 +69,8 @@
 #include <cmath>
 #include <cstring>
 #include <vector>
+
+#include <cuda_fp16.h>
 
 #include "vo_internal.cuh"
 
@@ -91,6 +95,13 @@ constexpr int kShort = 1024;      // kept-aside segments of a patch
 constexpr int kEntriesBig = 1600; // the same for the second tier
 constexpr int kUnionBig = 1024;
 constexpr int kShortBig = 8192;
+constexpr double kDirectWork = 600;            // candidates per column up to which k_direct takes a dilation
+constexpr int64_t kDirectSplitCols = 1 << 16;  // columns of a launch up to which kSplit threads share one there
+constexpr int kStep = 8;          // segments that k_direct loads at a time
+constexpr int kPrepThreads = 256;
+constexpr int kList = 16;         // intervals that it keeps at hand, unordered
+constexpr int kHot = 2;           // intervals that each candidate is compared with at once
+constexpr int kDirectCap = 48;    // union intervals per column there
 constexpr int kBigCap = 8192;     // last tier (FP64): intervals of a column's working list
 constexpr int kBigThreads = 32;
 constexpr int kBigBlocks = 16;      // last tier: blocks
@@ -104,7 +115,7 @@ __device__ __forceinline__ unsigned long long order_of(double v) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(v);
   return b >> 63 ? ~b : b | 0x8000000000000000ull;
 }
-__device__ __forceinline__ double value_of(unsigned long long o) {
+__device__ __forceinline__ double order_value(unsigned long long o) {
   return __longlong_as_double((long long)(o >> 63 ? o & 0x7fffffffffffffffull : ~o));
 }
 
@@ -140,7 +151,7 @@ __global__ void k_range(int ncols, const int32_t *__restrict__ beg, const int32_
   if (atomicAdd(&mm[2], 1ull) + 1 != gridDim.x) return;
   __threadfence();
   const unsigned long long a = atomicMax(&mm[0], 0ull), b = atomicMax(&mm[1], 0ull);
-  const double zmax = a ? value_of(a) : 0.0, zmin = b ? -value_of(b) : 0.0;
+  const double zmax = a ? order_value(a) : 0.0, zmin = b ? -order_value(b) : 0.0;
   FastPar p;
   p.base = floor(zmin - R - 3.0);
   const float U = (float)(zmax - p.base + R + 3.0);
@@ -1173,6 +1184,266 @@ __global__ void __launch_bounds__(32, 20) k_patch(const BatchVol *__restrict__ v
   }
 }
 
+// ------------------------------------------------------------ small radii
+
+// What k_direct needs of a segment: its ends as FP32, its column and, for each
+// of its four neighbour columns, by how much at most it reaches beyond one of
+// their segments (FP16 bits, rounded up to 12). Where H grows by at least as
+// much over the step to that neighbour, the neighbour's candidate holds the
+// segment's, in exact arithmetic and so after rounding, and the segment is
+// passed over for all columns on that side. A block per row; the segments of a
+// row become contiguous (CSR inputs are already so: slots == false).
+template <bool SLOTS>
+__global__ void __launch_bounds__(kPrepThreads) k_direct_prep(int nx, int ny, const int32_t *__restrict__ beg,
+                                                              const int32_t *__restrict__ end,
+                                                              const longlong2 *__restrict__ z, uint4 *__restrict__ rec,
+                                                              longlong2 *__restrict__ rz, int32_t *__restrict__ rbeg,
+                                                              int32_t *__restrict__ rend) {
+  __shared__ int s_sum[kPrepThreads / 32];
+  const int y = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int base = SLOTS ? beg[nx * y] : 0;
+  for (int x0 = 0; x0 < nx; x0 += kPrepThreads) {
+    const int x = x0 + threadIdx.x, c = x + nx * y;
+    const int k0 = x < nx ? beg[c] : 0, n = x < nx ? end[c] - k0 : 0;
+    int out = k0;
+    if (SLOTS) {
+      int upto = n;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(kFull, upto, o);
+        if (lane >= o) upto += v;
+      }
+      __syncthreads();
+      if (lane == 31) s_sum[warp] = upto;
+      __syncthreads();
+      int before = 0, all = 0;
+      for (int w = 0; w < kPrepThreads / 32; ++w) {
+        before += w < warp ? s_sum[w] : 0;
+        all += s_sum[w];
+      }
+      out = base + before + upto - n;
+      base += all;
+      if (x < nx) {
+        rbeg[c] = out;
+        rend[c] = out + n;
+      }
+    }
+    if (n <= 0) continue;
+    int nb[4], ne[4];
+#pragma unroll
+    for (int d = 0; d < 4; ++d) {
+      const bool ok = d == 0 ? x > 0 : d == 1 ? x + 1 < nx : d == 2 ? y > 0 : y + 1 < ny;
+      const int cn = ok ? c + (d == 0 ? -1 : d == 1 ? 1 : d == 2 ? -nx : nx) : c;
+      nb[d] = beg[cn];
+      ne[d] = ok ? end[cn] : nb[d];
+    }
+    for (int k = 0; k < n; ++k) {
+      const longlong2 v = z[k0 + k];
+      const float lo = trunc32_bits(v.x), hi = trunc32_bits(v.y);
+      unsigned w[4];
+#pragma unroll
+      for (int d = 0; d < 4; ++d) {
+        float best = INFINITY;
+        // of the neighbour's segments the first two that reach this one (any other choice is safe too)
+        int j = nb[d];
+        longlong2 u = make_longlong2(0, 0);
+        for (; j < ne[d]; ++j) {
+          u = z[j];
+          if (!(trunc32_bits(u.y) < lo)) break;
+        }
+        nb[d] = j;
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          if (j + q < ne[d]) {
+            if (q) u = z[j + q];
+            const float a = trunc32_bits(u.x), b = trunc32_bits(u.y);
+            const float e = 4.76837158203125e-7f * (fabsf(a) + fabsf(b) + fabsf(lo) + fabsf(hi)) + 1e-30f;
+            best = fminf(best, fmaxf(fmaxf(a - lo, hi - b), 0.f) + e);
+          }
+        }
+        w[d] = min(0xfffu, (__half_as_ushort(__float2half_ru(best)) + 7u) >> 3);
+      }
+      rec[out + k] = make_uint4(__float_as_uint(lo), __float_as_uint(hi), w[0] | w[1] << 12 | (unsigned)(x & 0xff) << 24,
+                                w[2] | w[3] << 12 | (unsigned)(x >> 8) << 24);
+      if (SLOTS) rz[out + k] = v;
+    }
+  }
+}
+
+// Dilations by small radii, one thread per column: few columns are in reach, so
+// that the candidates are met one by one, without clusters, cover or bins. A
+// candidate that its neighbour's holds (k_direct_prep), or that lies, in FP32
+// and by more than its error, inside one of the first kHot intervals found, is
+// passed over. What is left each lane takes from a list of its own, so that the
+// lanes do not wait for one another's: it is compared with all intervals found,
+// extends one that it is certain to meet, in FP64, or else begins another. Ends
+// are compared as integers (Key). Intervals that have come to meet are merged at
+// the end; more than kList of them are inserted into a sorted list at once.
+//
+// What bounds it: instructions (1024^2, 1.5 segments per column, radius 6: 70 of
+// them per candidate and warp, 2.3 per cycle), in inputs of many segments the
+// latency of the lists in local memory, and in small volumes that of a thread's
+// chain. There G = 4 threads share a column, each taking every fourth row, and
+// the first one inserts the others' unions into its own: with four threads 64^2
+// takes 0.027 instead of 0.051 ms at radius 4, 276^2 0.054 instead of 0.043 and
+// 0.146 instead of 0.153 at 2.75 and 6, 512^2 0.23 instead of 0.17 at 4. Hence
+// the line at 2^16 columns.
+//
+// Against patches, packing included (ms; segments per column; radius 4, 6, 8):
+//   276^2   1.5   0.10 / 0.29   0.15 / 0.36   0.21 / 0.33
+//   1024^2  1.5   0.39 / 1.45   0.68 / 2.14   1.01 / 1.95
+//   2048^2  5.1   11.2 / 18.9   21.9 / 28.1   40   / 36.7
+// A patch's candidates are those of the whole patch's reach, at radius 4 four
+// times a column's, and its steps take some ten thousand cycles however few they
+// are; but their number grows more slowly. Both take the same at about 600
+// candidates per column: the line of direct_choice. (In FP64 throughout, without
+// the neighbours' test, 1024^2 took 0.53, 1.1 and 1.9 ms.)
+template <int G>
+__global__ void __launch_bounds__(128) k_direct(const BatchVol *__restrict__ vols, int nv) {
+  __shared__ BatchVol V;
+  extern __shared__ float2 s_tab[];
+  int v = 0;
+  for (int r = nv - 1; v < r;) {
+    const int m = (v + r) >> 1;
+    if ((int)blockIdx.x < vols[m].item1) r = m; else v = m + 1;
+  }
+  for (int i = threadIdx.x; i < (int)(sizeof(BatchVol) / sizeof(int)); i += 128)
+    reinterpret_cast<int *>(&V)[i] = reinterpret_cast<const int *>(&vols[v])[i];
+  __syncthreads();
+  constexpr int COLS = 32 / G;
+  const int nx = V.A.nx, ny = V.A.ny, W = V.A.W, tw = min(W, nx);
+  // H in FP32 and its growth inwards, for the distances that occur
+  for (int i = threadIdx.x; i < tw * (min(V.A.Dy, ny - 1) + 1); i += 128) {
+    const int d = i / tw, a = i - d * tw;
+    s_tab[i] = make_float2(V.A.Hp[d * V.A.hs + a], __int_as_float(V.A.Dx[V.A.Dy + 1 + d * W + a]));
+  }
+  __syncthreads();
+  const int blocks_x = (nx + COLS - 1) / COLS, blk = (int)blockIdx.x - V.item0;
+  const int lane = threadIdx.x & 31, part = lane / COLS;
+  const int x = blk % blocks_x * COLS + lane % COLS, y = blk / blocks_x * 4 + (threadIdx.x >> 5);
+  const bool inside = x < nx && y < ny;
+  Key2 A[kDirectCap];
+  Key2 found[kList];  // intervals found so far; those that have come to meet are merged at the end
+  float2 sure[kHot];  // of the first ones, inside which an FP32 candidate is certain to lie in them
+#pragma unroll
+  for (int i = 0; i < kHot; ++i) sure[i] = make_float2(INFINITY, -INFINITY);
+  float2 *const all = s_tab + tw * (min(V.A.Dy, ny - 1) + 1) + threadIdx.x;  // the same of all, 128 apart
+  int n = 0, m = 0;
+  const float reach = 2.f * V.A.Hp[0];
+  auto insert = [&](Key2 u) {
+    if (n < 0) return;
+    const int2 at = union_insert_keys(A, n, kDirectCap, u.x, u.y);
+    n = at.x < 0 ? -1 : at.y;
+  };
+  auto inner = [&](Key2 u) {
+    const float lo = trunc32(u.x), hi = trunc32(u.y);
+    const float e = 9.5367431640625e-07f * (fabsf(lo) + fabsf(hi) + reach);
+    return make_float2(lo + e, hi - e);
+  };
+  const double2 *z = V.A.rz;
+  const uint4 *rec = V.A.rec;
+  if (inside) {
+    // rows outwards from the column's own one, before them its own segments; the threads of a column take
+    // every G-th row, or every G-th step of a grid of one row
+    const int rows = 2 * min(V.A.Dy, ny - 1);
+    const int row_step = ny > 1 ? G : 1, k_first = ny > 1 ? 0 : kStep * part, k_step = ny > 1 ? kStep : kStep * G;
+    for (int row = part == 0 ? -1 : ny > 1 ? part : 0; row <= rows; row += row < 0 ? 1 : row_step) {
+      const int ady = (row + 1) >> 1, ys = row & 1 ? y - ady : y + ady;
+      const bool own = row < 0;
+      if (!own && (ys < 0 || ys >= ny)) continue;
+      const int reach_x = own ? 0 : V.A.Dx[ady];
+      const int cy = own ? y : ys;
+      const float2 *tab = s_tab + (own ? 0 : ady) * tw;
+      const bool above = cy < y;
+      int k = V.A.rbeg[max(0, x - reach_x) + nx * cy] + (own ? 0 : k_first);
+      const int ke = V.A.rend[min(nx - 1, x + reach_x) + nx * cy];
+      for (; k < ke; k += own ? kStep : k_step) {
+        uint4 v[kStep];
+#pragma unroll
+        for (int i = 0; i < kStep; ++i) v[i] = rec[min(k + i, ke - 1)];
+        unsigned todo = 0;
+#pragma unroll
+        for (int i = 0; i < kStep; ++i) {
+          const int dx = (int)((v[i].z >> 24) | (v[i].w >> 24) << 8) - x;
+          const float2 t = tab[abs(dx)];
+          const int g = __float_as_int(t.y);
+          const int wx = (int)(dx < 0 ? v[i].z >> 12 & 0xfff : v[i].z & 0xfff) << 3;
+          const int wy = (int)(above ? v[i].w >> 12 & 0xfff : v[i].w & 0xfff) << 3;
+          const float lo = __uint_as_float(v[i].x) - t.x, hi = __uint_as_float(v[i].y) + t.x;
+          bool out = wx <= (short)g || wy <= g >> 16 || k + i >= ke;
+#pragma unroll
+          for (int j = 0; j < kHot; ++j) out |= lo >= sure[j].x && hi <= sure[j].y;
+          todo |= out ? 0u : 1u << i;
+        }
+        // what is not certain to change nothing, in FP64: each lane its own next one
+        for (; todo; todo &= todo - 1) {
+          const int i = __ffs(todo) - 1;
+          const uint4 r = rec[k + i];
+          const int a = abs((int)((r.z >> 24) | (r.w >> 24) << 8) - x);
+          const float h = tab[a].x;
+          const float lo = __uint_as_float(r.x) - h, hi = __uint_as_float(r.y) + h;
+          int at = -1;
+          bool in = false;
+          for (int j = 0; j < m; ++j) {
+            const float2 s = all[128 * j];
+            in |= lo >= s.x && hi <= s.y;
+            if (lo <= s.y && hi >= s.x) at = j;  // certain to meet it
+          }
+          if (in) continue;
+          const double2 u = z[k + i];
+          const double d = V.A.H64[(own ? 0 : ady) * W + a];
+          Key2 w = make_longlong2(key_of(__dsub_rn(u.x, d)), key_of(__dadd_rn(u.y, d)));
+          if (at >= 0) {
+            const Key2 q = found[at];
+            w = make_longlong2(kmin(w.x, q.x), kmax(w.y, q.y));
+          } else if (m < kList) {
+            at = m++;
+          } else {
+            insert(w);
+            continue;
+          }
+          found[at] = w;
+          const float2 s = inner(w);
+          all[128 * at] = s;
+#pragma unroll
+          for (int j = 0; j < kHot; ++j)
+            if (j == at) sure[j] = s;
+        }
+      }
+    }
+  }
+#pragma unroll 1
+  for (int i = 0; i < m; ++i) insert(found[i]);
+  // the other lanes' unions into the first one's
+#pragma unroll 1
+  for (int p = 1; p < G; ++p) {
+    const int from = lane % COLS + p * COLS, m = __shfl_sync(kFull, n, from);
+    if (part == 0 && m < 0) n = -1;
+    const int most = __reduce_max_sync(kFull, m);
+#pragma unroll 1
+    for (int i = 0; i < most; ++i) {
+      const Key2 u = A[i];
+      const Key lo = __shfl_sync(kFull, u.x, from), hi = __shfl_sync(kFull, u.y, from);
+      if (part == 0 && n >= 0 && i < m) {
+        const int2 at = union_insert_keys(A, n, kDirectCap, lo, hi);
+        n = at.x < 0 ? -1 : at.y;
+      }
+    }
+  }
+  if (!inside || part != 0) return;
+  const int c = x + nx * y;
+  unsigned dst = 0;
+  if (n < 0) {
+    atomicOr(V.ovf, 8);
+    n = 0;
+  } else if (!place_union(V, x, y, n, dst)) {
+    n = 0;
+    dst = 0;
+  }
+  for (int i = 0; i < n; ++i) V.oz[dst + i] = make_double2(value_of(A[i].x), value_of(A[i].y));
+  V.obeg[c] = (int32_t)dst;
+  V.oend[c] = (int32_t)(dst + (unsigned)n);
+}
+
 // ------------------------------------------------------------ last tier
 
 // Inserts [lo, hi] into the sorted list L of n disjoint closed intervals.
@@ -1368,7 +1639,45 @@ void fast_prepare(cudaStream_t st, const FastArgs &A, float R, double mean_segs,
 FastArgs fast_args(int nx, int ny, const DeviceTables &T, const int32_t *beg, const int32_t *end, const double2 *z,
                    const PackOut &out) {
   return FastArgs{nx,  ny,  T.host.W, T.host.Dy, T.host.hs, beg, end, (const double *)z, out.zf, out.code,
-                  (const double *)out.zx, out.cl, out.coff, T.Hp, T.H, T.Dx, out.par};
+                  (const double *)out.zx, out.cl, out.coff, T.Hp, T.H, T.Dx, out.par, out.rec, out.zx ? out.zx : z,
+                  out.zx ? out.rbeg : beg, out.zx ? out.rbeg + (size_t)nx * ny : end};
+}
+
+// Threads per column: the line is explained at k_direct.
+static int direct_split(int64_t cols) {
+  return cols <= kDirectSplitCols ? kSplit : 1;
+}
+int direct_blocks(const vo_grid &g, int64_t launch_cols) {
+  const int cols = 32 / direct_split(launch_cols);
+  return ((g.nx + cols - 1) / cols) * ((g.ny + 3) / 4);
+}
+void direct_prepare(cudaStream_t st, const FastArgs &A, const PackOut &out) {
+  if (A.ny <= 0) return;
+  const longlong2 *z = reinterpret_cast<const longlong2 *>(A.zd);
+  if (out.zx)
+    k_direct_prep<true><<<A.ny, kPrepThreads, 0, st>>>(A.nx, A.ny, A.beg, A.end, z, out.rec,
+                                                       reinterpret_cast<longlong2 *>(out.zx), out.rbeg,
+                                                       out.rbeg + (size_t)A.nx * A.ny);
+  else
+    k_direct_prep<false><<<A.ny, kPrepThreads, 0, st>>>(A.nx, A.ny, A.beg, A.end, z, out.rec, nullptr, nullptr, nullptr);
+}
+static size_t direct_table(int nx, int ny, int W, int Dy) {
+  return sizeof(float2) * (size_t)std::min(W, nx) * (std::min(Dy, ny - 1) + 1);
+}
+size_t direct_smem(const FastArgs &A) { return direct_table(A.nx, A.ny, A.W, A.Dy); }
+void direct_launch(cudaStream_t st, const BatchVol *vols, int nv, int blocks, int64_t launch_cols, size_t smem) {
+  const int split = direct_split(launch_cols);
+  (split == 1 ? &k_direct<1> : &k_direct<kSplit>)<<<blocks, 128, smem + sizeof(float2) * kList * 128, st>>>(vols, nv);
+}
+
+bool direct_choice(const vo_grid &g, const DeviceTables &T, double mean_segs) {
+  // source columns in reach of a column, on average over the grid
+  double cols = 0;
+  for (int d = 0; d <= std::min(T.host.Dy, g.ny - 1); ++d)
+    cols += (d ? 2.0 : 1.0) * (1.0 - (double)d / g.ny) * std::min(2 * T.host.Dx[d] + 1, g.nx);
+  // patches are four rows high: of a grid of fewer rows they use as much less
+  if (g.nx < 1 || g.ny < 1 || g.nx > 65535 || direct_table(g.nx, g.ny, T.host.W, T.host.Dy) > 32 * 1024) return false;
+  return cols * std::max(mean_segs, 1.0) <= kDirectWork * kPatchY / std::min(g.ny, kPatchY);
 }
 
 // Slots per column of a single dilation's output (the rest goes to the spill
@@ -1384,11 +1693,8 @@ int dilate_fast(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out, vo_
   int rc = get_tables(ctx, R, std::max(nx, ny), &T);
   if (rc) return rc;
   const double mean_segs = (double)in->nseg / std::max(ncols, 1);
+  bool direct = direct_choice(g, *T, mean_segs);
   PatchPlan P;
-  const vo_grid *const gp = &g;
-  const int split = patch_split(&gp, 1);
-  rc = patch_plan(ctx, patch_count(g, split), split, T->host.hs, P);
-  if (rc) return rc;
   // slot indices are unsigned 32-bit: columns and spill together below 2^32
   const int64_t most = 4294967295LL;
   int cap = slot_cap(mean_segs);
@@ -1405,20 +1711,28 @@ int dilate_fast(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out, vo_
   // spill used, overflow flags)
   rc = dalloc(ctx, &misc, 256);
   if (!rc) rc = dalloc(ctx, &dv, 1);
-  if (!rc) rc = dalloc(ctx, &pk.zf, nseg);
-  if (!rc) rc = dalloc(ctx, &pk.code, nseg);
-  if (!rc) rc = dalloc(ctx, &pk.zx, nseg);
-  if (!rc) rc = dalloc(ctx, &pk.cl, nseg);
-  if (!rc) rc = dalloc(ctx, &pk.coff, pack_offsets(g));
   if (!rc) rc = dalloc(ctx, &obeg, 2 * (size_t)ncols);
-  if (!rc) rc = dalloc(ctx, &list, (size_t)P.nitems);
-  if (!rc) rc = dalloc(ctx, &big_list, (size_t)ncols);
-  if (!rc) rc = dalloc(ctx, &scratch[0], patch_scratch_bytes(P, false));
-  if (!rc) patch_scratch_set(P, false, scratch[0]);
   unsigned long long *mm = reinterpret_cast<unsigned long long *>(misc);
   pk.par = reinterpret_cast<FastPar *>(misc + 64);
   int *cnt = reinterpret_cast<int *>(misc + 128);
-  P.Q = PatchQueue{cnt, list};
+  // what the patches need beside that
+  auto patch_memory = [&]() -> int {
+    const vo_grid *const gp = &g;
+    const int split = patch_split(&gp, 1);
+    int r = patch_plan(ctx, patch_count(g, split), split, T->host.hs, P);
+    if (!r) r = dalloc(ctx, &pk.zf, nseg);
+    if (!r) r = dalloc(ctx, &pk.code, nseg);
+    if (!r) r = dalloc(ctx, &pk.zx, nseg);
+    if (!r) r = dalloc(ctx, &pk.cl, nseg);
+    if (!r) r = dalloc(ctx, &pk.coff, pack_offsets(g));
+    if (!r) r = dalloc(ctx, &list, (size_t)P.nitems);
+    if (!r) r = dalloc(ctx, &big_list, (size_t)ncols);
+    if (!r) r = dalloc(ctx, &scratch[0], patch_scratch_bytes(P, false));
+    if (!r) patch_scratch_set(P, false, scratch[0]);
+    P.Q = PatchQueue{cnt, list};
+    return r;
+  };
+  if (!rc) rc = direct ? dalloc(ctx, &pk.rec, nseg) : patch_memory();
   vo_volume *res = nullptr;
   int cols2 = 0;
   for (int attempt = 0; !rc; ++attempt) {
@@ -1431,7 +1745,7 @@ int dilate_fast(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out, vo_
     V.oend = obeg + ncols;
     V.oz = oz;
     V.cap = cap;
-    V.item1 = P.nitems;
+    V.item1 = direct ? direct_blocks(g, ncols) : P.nitems;
     V.spill_base = (unsigned)((int64_t)ncols * cap);
     V.spill_cap = (unsigned)spill;
     V.big_list = big_list;
@@ -1441,12 +1755,18 @@ int dilate_fast(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out, vo_
     cudaMemcpyAsync(dv, &V, sizeof V, cudaMemcpyHostToDevice, ctx->stream);
     cudaMemsetAsync(cnt, 0, 7 * sizeof(int), ctx->stream);
     cudaEventRecord(ctx->ev[0], ctx->stream);
-    fast_prepare(ctx->stream, V.A, (float)R, mean_segs, mm, pk);
+    if (direct)
+      direct_prepare(ctx->stream, V.A, pk);
+    else
+      fast_prepare(ctx->stream, V.A, (float)R, mean_segs, mm, pk);
     cudaEventRecord(ctx->ev[1], ctx->stream);
     cudaEventRecord(ctx->ev[4], ctx->stream);
-    patch_launch(false, P, ctx->stream, dv);
+    if (direct)
+      direct_launch(ctx->stream, dv, 1, V.item1, ncols, direct_smem(V.A));
+    else
+      patch_launch(false, P, ctx->stream, dv);
     cudaEventRecord(ctx->ev[5], ctx->stream);
-    ctx->launches += 3;
+    ctx->launches += direct ? 2 : 3;
     SlotVol sv;
     sv.grid = g;
     sv.cap = cap;
@@ -1469,6 +1789,16 @@ int dilate_fast(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out, vo_
       }
     }
     if (rc) break;
+    if (hc[6] & 8) {  // a union beyond the small list: by patches
+      vo_volume_free(ctx, res);
+      res = nullptr;
+      dfree(ctx, oz);
+      oz = nullptr;
+      direct = false;
+      rc = patch_memory();
+      --attempt;
+      continue;
+    }
     cols2 = hc[3] + (hc[3] == 0 ? hc[4] : 0);
     if (hc[6] & 1) {
       rc = set_error(ctx, VO_EINTERNAL, "a column exceeds the fallback union capacity");
@@ -1496,7 +1826,7 @@ int dilate_fast(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out, vo_
       tm->kernel_ms[2] += e1;
     }
   }
-  for (void *p : {(void *)misc, (void *)dv, (void *)pk.zf, (void *)pk.code, (void *)pk.zx, (void *)pk.cl,
+  for (void *p : {(void *)misc, (void *)dv, (void *)pk.zf, (void *)pk.code, (void *)pk.zx, (void *)pk.cl, (void *)pk.rec,
                   (void *)pk.coff, (void *)obeg, (void *)list, (void *)big_list, (void *)scratch[0],
                   (void *)scratch[1], (void *)oz, (void *)big})
     dfree(ctx, p);

@@ -206,8 +206,13 @@ struct FastArgs {
   const int32_t *coff;
   const float *Hp;      // [(Dy + 2 kPatchY)][hs], -inf beyond the disc
   const double *H64;    // [(Dy + 1) * W]
-  const int *Dx;        // [Dy + 1]
+  const int *Dx;        // [Dy + 1], then the growth of H over a step inwards (Tables::Dx)
   const FastPar *par;
+  // small radii (k_direct_prep): per segment what k_direct needs and its FP64 values, contiguous by rows;
+  // [rbeg[c], rend[c]) of column c
+  const uint4 *rec;
+  const double2 *rz;
+  const int32_t *rbeg, *rend;
 };
 
 constexpr int kSizerTile = 32;     // side of a sizing tile (columns)
@@ -226,7 +231,7 @@ struct BatchVol {
   unsigned spill_base, spill_cap;
   unsigned *spill_used;
   int *big_list, *big_count;  // columns for the third tier (FP64)
-  int *ovf;  // flags: 1 a union beyond the FP64 list, 4 spill region exhausted
+  int *ovf;  // flags: 1 a union beyond the FP64 list, 4 spill region exhausted, 8 a union beyond k_direct's list
 };
 
 // Queue of a launch. count: the first tier's next item, the items it listed
@@ -251,6 +256,13 @@ struct PatchPlan {
 // Lanes per column for a launch over the given grids (1, or more for small
 // ones), and the patches of a grid with that many.
 int patch_split(const vo_grid *const *grids, int n);
+// Small radii: whether a dilation meets its candidates column by column
+// (k_direct; its prepared inputs are not needed then), the launch over the nv
+// dilations vols and its blocks for a grid. launch_cols: columns of all of them.
+bool direct_choice(const vo_grid &g, const DeviceTables &T, double mean_segs);
+int direct_blocks(const vo_grid &g, int64_t launch_cols);
+size_t direct_smem(const FastArgs &A);
+void direct_launch(cudaStream_t st, const BatchVol *vols, int nv, int blocks, int64_t launch_cols, size_t smem);
 int64_t patch_total(const vo_grid *const *grids, int n);  // with one lane per column
 int patch_count(const vo_grid &g, int split);
 // Grids of a launch over nitems patches; the working memory of each tier is
@@ -271,8 +283,12 @@ struct PackOut {
   float4 *cl = nullptr;
   int32_t *coff = nullptr;
   FastPar *par = nullptr;
+  uint4 *rec = nullptr;     // small radii: instead of all the others; for slots zx and rbeg (2 x columns) too
+  int32_t *rbeg = nullptr;
 };
 size_t pack_offsets(const vo_grid &g);
+// Prepares the input of k_direct (pk.rec).
+void direct_prepare(cudaStream_t st, const FastArgs &A, const PackOut &out);
 FastArgs fast_args(int nx, int ny, const DeviceTables &T, const int32_t *beg, const int32_t *end, const double2 *z,
                    const PackOut &out);
 // Packs the input of a dilation (CSR or slots in column order). mm: three words of scratch.
@@ -309,8 +325,72 @@ __device__ __forceinline__ double value_of(Key k) {
   return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffll));
 }
 __device__ __forceinline__ Key2 key2_of(double2 v) { return make_longlong2(key_of(v.x), key_of(v.y)); }
+// A double's bits, or a key's value, as FP32, rounded towards zero (NaN beyond
+// its range): integer operations only, within 2^-23 of the magnitude for normal
+// values, 0 for smaller ones.
+__device__ __forceinline__ float trunc32_bits(Key b) {
+  const unsigned hi = (unsigned)(b >> 32), lo = (unsigned)b, e = hi & 0x7fffffffu;
+  unsigned f = e < 0x38100000u ? 0u : ((e - 0x38000000u) << 3) | (lo >> 29);
+  if (e >= 0x47f00000u) f = 0x7fc00000u;
+  return __uint_as_float((hi & 0x80000000u) | f);
+}
+__device__ __forceinline__ float trunc32(Key k) { return trunc32_bits(k ^ ((k >> 63) & 0x7fffffffffffffffll)); }
 __device__ __forceinline__ Key kmax(Key a, Key b) { return a > b ? a : b; }
 __device__ __forceinline__ Key kmin(Key a, Key b) { return a < b ? a : b; }
+
+// Inserts [lo, hi] into a sorted list of n disjoint closed intervals, merging
+// overlapping or touching ones. One function, not inlined: its callers use it
+// in several places, and copies would crowd the instruction cache. Returns the
+// position of the interval that now holds [lo, hi] (-1 beyond `cap`) and the
+// list's new length.
+static __device__ __noinline__ int2 union_insert_keys(Key2 *A, int n, int cap, Key lo, Key hi) {
+  int l = 0, r = n;
+  while (l < r) {
+    const int m = (l + r) >> 1;
+    if (A[m].y >= lo)
+      r = m;
+    else
+      l = m + 1;
+  }
+  if (l == n || A[l].x > hi) {
+    if (n >= cap) return make_int2(-1, n);
+    for (int k = n; k > l; --k) A[k] = A[k - 1];
+    A[l] = make_longlong2(lo, hi);
+    return make_int2(l, n + 1);
+  }
+  int j = l;
+  while (j + 1 < n && A[j + 1].x <= hi) ++j;
+  A[l] = make_longlong2(kmin(A[l].x, lo), kmax(A[j].y, hi));
+  if (j > l) {
+    const int sh = j - l;
+    for (int k = l + 1; k + sh < n; ++k) A[k] = A[k + sh];
+    n -= sh;
+  }
+  return make_int2(l, n);
+}
+
+// Moves the columns' segments from src(c) to oz[ooffs[c] ..): a warp per 32
+// columns, whose lanes share out the segments, so that few per column leave no
+// lane idle and the writes are contiguous (a warp per column took 0.13 ms for
+// 810,000 columns of 1.6 segments).
+template <typename Src>
+__device__ __forceinline__ void compact_columns(int ncols, const int32_t *__restrict__ ooffs,
+                                                double2 *__restrict__ oz, Src src) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+  if (c - lane >= ncols) return;
+  const int off = ooffs[min(c, ncols)];
+  const long long from = c < ncols ? reinterpret_cast<long long>(src(c)) : 0;
+  const int first = __shfl_sync(0xffffffffu, off, 0), end = ooffs[min(c - lane + 32, ncols)];
+  for (int k0 = first; k0 < end; k0 += 32) {
+    const int k = k0 + lane;
+    int l = 0;  // the last column that starts at or before k (of those that do, the one with segments)
+    for (int o = 16; o > 0; o >>= 1)
+      if (__shfl_sync(0xffffffffu, off, l + o) <= k) l += o;
+    const double2 *p = reinterpret_cast<const double2 *>(__shfl_sync(0xffffffffu, from, l));
+    const int at = k - __shfl_sync(0xffffffffu, off, l);
+    if (k < end) oz[k] = p[at];
+  }
+}
 #endif
 
 }  // namespace vo

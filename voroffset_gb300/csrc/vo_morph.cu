@@ -185,35 +185,6 @@ __device__ __forceinline__ bool union_insert(double2 *A, int &n, int cap, double
 
 // ---------------------------------------------------------------- pass 2
 
-// The same on ordered integers, as one function: pass 2 calls it from several
-// places, and copies of it would crowd the instruction cache. Returns the
-// position of the interval that now holds [lo, hi], or -1 beyond `cap`.
-__device__ __noinline__ int2 union_insert_keys(Key2 *A, int n, int cap, Key lo, Key hi) {
-  int l = 0, r = n;
-  while (l < r) {
-    const int m = (l + r) >> 1;
-    if (A[m].y >= lo)
-      r = m;
-    else
-      l = m + 1;
-  }
-  if (l == n || A[l].x > hi) {
-    if (n >= cap) return make_int2(-1, n);
-    for (int k = n; k > l; --k) A[k] = A[k - 1];
-    A[l] = make_longlong2(lo, hi);
-    return make_int2(l, n + 1);
-  }
-  int j = l;
-  while (j + 1 < n && A[j + 1].x <= hi) ++j;
-  A[l] = make_longlong2(kmin(A[l].x, lo), kmax(A[j].y, hi));
-  if (j > l) {
-    const int sh = j - l;
-    for (int k = l + 1; k + sh < n; ++k) A[k] = A[k + sh];
-    n -= sh;
-  }
-  return make_int2(l, n);
-}
-
 // The union of column (x, y)'s chords into A; returns their count or -1 beyond
 // `cap`. Most chords lie inside an interval that is there already: the one the
 // last insertion made is kept in registers, and a chord inside it is passed
@@ -985,11 +956,7 @@ __global__ void k_slot_counts(int ncols, const int32_t *beg, const int32_t *end,
 
 __global__ void k_slot_compact(int ncols, const int32_t *__restrict__ beg, const double2 *__restrict__ z,
                                const int32_t *__restrict__ ooffs, double2 *__restrict__ oz) {
-  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (w >= ncols) return;
-  const int n = ooffs[w + 1] - ooffs[w];
-  const uint32_t b = (uint32_t)beg[w];  // slot indices are unsigned
-  for (int k = lane; k < n; k += 32) oz[ooffs[w] + k] = z[(size_t)b + k];
+  compact_columns(ncols, ooffs, oz, [=](int c) { return z + (uint32_t)beg[c]; });  // slot indices are unsigned
 }
 
 }  // namespace
@@ -1466,8 +1433,7 @@ int slot_to_volume(vo_ctx *ctx, const SlotVol &v, vo_volume **out, const int *ex
     rc = dalloc(ctx, &res->z, (size_t)total);
   }
   if (!rc) {
-    k_slot_compact<<<nblocks((int64_t)ncols * 32, 256), 256, 0, ctx->stream>>>(ncols, v.beg, v.z, res->offs,
-                                                                               res->z);
+    k_slot_compact<<<nblocks(ncols, 256), 256, 0, ctx->stream>>>(ncols, v.beg, v.z, res->offs, res->z);
     ctx->launches += 1;
   }
   dfree(ctx, counts);
