@@ -241,7 +241,7 @@ int vo_create(vo_ctx **out, int device) {
   }
   if (cudaMalloc(&ctx->d_flags, 16 * sizeof(int)) != cudaSuccess ||
       cudaMalloc(&ctx->d_total, 4 * sizeof(long long)) != cudaSuccess ||
-      cudaMallocHost(&ctx->h_total, 4 * sizeof(long long)) != cudaSuccess) {
+      cudaMallocHost(&ctx->h_total, (1 + kScanExtra / 2) * sizeof(long long)) != cudaSuccess) {
     vo_destroy(ctx);
     return VO_ENOMEM;
   }

@@ -67,6 +67,7 @@
 // list.
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstring>
 #include <vector>
 
@@ -1708,10 +1709,19 @@ int dilate_fast(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out, vo_
   double2 *oz = nullptr, *big = nullptr;
   BatchVol *dv = nullptr;
   // misc: range orders (3 x 8 bytes), FastPar at 64, counters at 128 (4 of the queue, FP64-tier columns,
-  // spill used, overflow flags)
-  rc = dalloc(ctx, &misc, 256);
-  if (!rc) rc = dalloc(ctx, &dv, 1);
-  if (!rc) rc = dalloc(ctx, &obeg, 2 * (size_t)ncols);
+  // spill used, overflow flags), the launch's BatchVol at 256, then the columns' slots; the first two
+  // parts are written by one copy
+  struct Head {
+    unsigned char zeros[256];
+    BatchVol V;
+  } head;
+  static_assert(offsetof(Head, V) == 256, "the counters lie before the launch's description");
+  const size_t head_bytes = (sizeof(Head) + 255) / 256 * 256;
+  rc = dalloc(ctx, &misc, head_bytes + sizeof(int32_t) * 2 * (size_t)ncols);
+  if (!rc) {
+    dv = reinterpret_cast<BatchVol *>(misc + offsetof(Head, V));
+    obeg = reinterpret_cast<int32_t *>(misc + head_bytes);
+  }
   unsigned long long *mm = reinterpret_cast<unsigned long long *>(misc);
   pk.par = reinterpret_cast<FastPar *>(misc + 64);
   int *cnt = reinterpret_cast<int *>(misc + 128);
@@ -1738,8 +1748,8 @@ int dilate_fast(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out, vo_
   for (int attempt = 0; !rc; ++attempt) {
     rc = dalloc(ctx, &oz, (size_t)ncols * cap + (size_t)spill);
     if (rc) break;
-    BatchVol V;
-    std::memset(&V, 0, sizeof V);
+    std::memset(&head, 0, sizeof head);
+    BatchVol &V = head.V;
     V.A = fast_args(nx, ny, *T, in->offs, in->offs + 1, in->z, pk);
     V.obeg = obeg;
     V.oend = obeg + ncols;
@@ -1752,8 +1762,7 @@ int dilate_fast(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out, vo_
     V.big_count = cnt + 4;
     V.spill_used = reinterpret_cast<unsigned *>(cnt + 5);
     V.ovf = cnt + 6;
-    cudaMemcpyAsync(dv, &V, sizeof V, cudaMemcpyHostToDevice, ctx->stream);
-    cudaMemsetAsync(cnt, 0, 7 * sizeof(int), ctx->stream);
+    cudaMemcpyAsync(misc, &head, sizeof head, cudaMemcpyHostToDevice, ctx->stream);
     cudaEventRecord(ctx->ev[0], ctx->stream);
     if (direct)
       direct_prepare(ctx->stream, V.A, pk);
@@ -1826,8 +1835,8 @@ int dilate_fast(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out, vo_
       tm->kernel_ms[2] += e1;
     }
   }
-  for (void *p : {(void *)misc, (void *)dv, (void *)pk.zf, (void *)pk.code, (void *)pk.zx, (void *)pk.cl, (void *)pk.rec,
-                  (void *)pk.coff, (void *)obeg, (void *)list, (void *)big_list, (void *)scratch[0],
+  for (void *p : {(void *)misc, (void *)pk.zf, (void *)pk.code, (void *)pk.zx, (void *)pk.cl, (void *)pk.rec,
+                  (void *)pk.coff, (void *)list, (void *)big_list, (void *)scratch[0],
                   (void *)scratch[1], (void *)oz, (void *)big})
     dfree(ctx, p);
   if (rc) {

@@ -45,6 +45,13 @@ __device__ __forceinline__ void img_add(int32_t *diff, int w, long long lo, long
   atomicAdd(&diff[hi], -1);
 }
 
+// The reach of row distances below kReachArg, passed by value: a kernel and a
+// buffer for a few numbers would be a tenth of a small image's time.
+constexpr int kReachArg = 32;
+struct Reach {
+  int32_t dy[kReachArg];
+};
+
 // reach[t] = floor(sqrt(r*r - t*t)) for t <= n
 __global__ void k_image_reach(int n, double r, int32_t *__restrict__ reach) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -56,7 +63,7 @@ __global__ void k_image_reach(int n, double r, int32_t *__restrict__ reach) {
 template <bool FILL>
 __global__ void __launch_bounds__(kImgThreads) k_image(int w, int h, const int32_t *__restrict__ offs,
                                                        const int32_t *__restrict__ ev,
-                                                       const int32_t *__restrict__ reach, int D, int erode,
+                                                       const int32_t *__restrict__ reach, Reach near, int D, int erode,
                                                        int32_t *__restrict__ counts, const int32_t *__restrict__ ooffs,
                                                        int32_t *__restrict__ oev, long long *__restrict__ slot,
                                                        unsigned long long *used, long long capacity) {
@@ -75,7 +82,7 @@ __global__ void __launch_bounds__(kImgThreads) k_image(int w, int h, const int32
         continue;
       }
       if (i0 < 0 || i0 >= h) continue;
-      const long long dy = reach[t];
+      const long long dy = reach ? reach[t] : near.dy[t];
       const int32_t *e = ev + offs[i0];
       const int n = offs[i0 + 1] - offs[i0];
       if (!erode) {
@@ -173,28 +180,32 @@ int image_op(vo_ctx *ctx, int erode, double r, int w, int h, const int32_t *offs
   const int far = std::min(D, h + 1);  // the farthest row distance that occurs
   // staging buffer: a dilated or eroded image rarely has more events than its input and a few per row
   const long long capacity = 2 * nev + 8LL * h + 1024;
-  int32_t *counts = nullptr, *reach = nullptr, *staged = nullptr;
-  long long *slot = nullptr;
-  unsigned long long *used = nullptr;
   *ooffs = nullptr;
   *oev = nullptr;
-  int rc = dalloc(ctx, &counts, (size_t)h + 1);
-  if (!rc) rc = dalloc(ctx, &reach, (size_t)far + 1);
-  if (!rc) rc = dalloc(ctx, &staged, (size_t)capacity);
-  if (!rc) rc = dalloc(ctx, &slot, (size_t)h + 1);
-  if (!rc) rc = dalloc(ctx, &used, 1);
+  // one buffer: the rows' places, the events staged, their counts, the reach (beyond kReachArg)
+  unsigned char *buf = nullptr;
+  const size_t nslot = sizeof(long long) * ((size_t)h + 2), nstaged = sizeof(int32_t) * (size_t)capacity,
+               ncounts = sizeof(int32_t) * ((size_t)h + 1);
+  int rc = dalloc(ctx, &buf, nslot + nstaged + ncounts + (far < kReachArg ? 0 : sizeof(int32_t) * ((size_t)far + 1)));
   if (!rc) rc = dalloc(ctx, ooffs, (size_t)h + 1);
+  unsigned long long *used = reinterpret_cast<unsigned long long *>(buf);
+  long long *slot = reinterpret_cast<long long *>(buf) + 1;
+  int32_t *staged = reinterpret_cast<int32_t *>(buf + nslot), *counts = staged + capacity,
+          *reach = far < kReachArg ? nullptr : counts + h + 1;
+  Reach near;
+  for (int t = 0; t < kReachArg; ++t)
+    near.dy[t] = t <= far ? (int32_t)std::floor(std::sqrt(r * r - (double)((long long)t * t))) : 0;
   const size_t sh = sizeof(int32_t) * ((size_t)w + 1);
   const int grid = std::min(h, 152 * 8);
   if (!rc) {
     cudaFuncSetAttribute(k_image<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kImgSmem);
     cudaFuncSetAttribute(k_image<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kImgSmem);
-    k_image_reach<<<far / 256 + 1, 256, 0, ctx->stream>>>(far, r, reach);
+    if (reach) k_image_reach<<<far / 256 + 1, 256, 0, ctx->stream>>>(far, r, reach);
     cudaMemsetAsync(used, 0, sizeof *used, ctx->stream);
     if (h > 0)
-      k_image<false><<<grid, kImgThreads, sh, ctx->stream>>>(w, h, offs, ev, reach, D, erode, counts, nullptr, staged,
+      k_image<false><<<grid, kImgThreads, sh, ctx->stream>>>(w, h, offs, ev, reach, near, D, erode, counts, nullptr, staged,
                                                              slot, used, capacity);
-    ctx->launches += 2;
+    ctx->launches += reach ? 2 : 1;
     rc = scan_counts(ctx, counts, *ooffs, h, total);
   }
   if (!rc) rc = dalloc(ctx, oev, (size_t)std::max<long long>(*total, 1));
@@ -202,15 +213,11 @@ int image_op(vo_ctx *ctx, int erode, double r, int w, int h, const int32_t *offs
     if (*total <= capacity)
       k_image_gather<<<(h + 7) / 8, 256, 0, ctx->stream>>>(h, *ooffs, slot, staged, *oev);
     else
-      k_image<true><<<grid, kImgThreads, sh, ctx->stream>>>(w, h, offs, ev, reach, D, erode, nullptr, *ooffs, *oev,
+      k_image<true><<<grid, kImgThreads, sh, ctx->stream>>>(w, h, offs, ev, reach, near, D, erode, nullptr, *ooffs, *oev,
                                                             nullptr, nullptr, 0);
     ctx->launches += 1;
   }
-  dfree(ctx, counts);
-  dfree(ctx, reach);
-  dfree(ctx, staged);
-  dfree(ctx, slot);
-  dfree(ctx, used);
+  dfree(ctx, buf);
   if (!rc) {
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) rc = cuda_error(ctx, e, "image kernels");

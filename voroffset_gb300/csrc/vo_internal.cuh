@@ -15,6 +15,7 @@ namespace vo {
 // column that needs more is flagged and re-run by the large-capacity variant
 // of the same kernel, whose lists live in global scratch.
 constexpr int kCapSmall = 32;    // pass-1 touching-merged piece list / pass-2 union
+constexpr int kScanExtra = 16;   // ints that a scan's synchronisation may read back besides its total
 constexpr int kCapLarge = 2048;  // overflow re-run capacity per column
 
 // Radius tables, computed on the host with the reference's own FP64
@@ -90,7 +91,7 @@ struct vo_ctx {
   // persistent small device scratch
   int *d_flags = nullptr;  // [0]: overflow count, [1..]: misc status
   long long *d_total = nullptr;
-  long long *h_total = nullptr;  // pinned
+  long long *h_total = nullptr;  // pinned, written by the scan's kernels: its total, then up to kScanExtra ints
   vo_sizer *sizer = nullptr;     // learned sizing for the batched executor (not owned)
   int64_t dexel_odd_columns = -1;  // odd-hit columns of the last vo_dexelize (-1: none yet)
   std::vector<std::pair<long long, int>> tune_cache;  // batch autotuner: shape key -> lanes per column
@@ -130,8 +131,10 @@ int get_tables(vo_ctx *ctx, double R, int kmax, const DeviceTables **out);
 // is returned through ctx->h_total (synchronising read). Returns VO_ERANGE if
 // the total exceeds INT32_MAX. With extra_n > 0 that many ints at extra_dev are
 // read back by the same synchronisation.
+// (at most kScanExtra). With `ends` the counts are ends[i] - counts[i].
 int scan_counts(vo_ctx *ctx, const int32_t *counts, int32_t *offs, int n, long long *total,
-                const int *extra_dev = nullptr, int *extra_host = nullptr, int extra_n = 0);
+                const int *extra_dev = nullptr, int *extra_host = nullptr, int extra_n = 0,
+                const int32_t *ends = nullptr);
 // The separable scheme in its sweeping envelope form, FP64 (vo_env.cu).
 // Returns VO_OK, an error, or 1 when the volume exceeds the kernels' working
 // capacities and must take the painter form (VO_METHOD_SEPARABLE).

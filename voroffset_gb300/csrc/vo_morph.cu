@@ -649,6 +649,7 @@ __global__ void k_negate_inv(int nx, int ny, const int32_t *__restrict__ offs,
 // ---------------------------------------------------------------- scan
 
 constexpr int kScanThreads = 1024, kScanItems = 8, kScanTile = kScanThreads * kScanItems;
+constexpr int kScanSmall = 4 * kScanTile;  // counts up to which one block scans them all
 
 __device__ long long block_exclusive_scan(long long v, long long *warp_sums, long long &total) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -677,7 +678,13 @@ __device__ long long block_exclusive_scan(long long v, long long *warp_sums, lon
 }
 
 // Per tile: local exclusive scan into offs (as int64 partials), tile sums out.
-__global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const int32_t *__restrict__ in, int n,
+// A count, or the difference of two (unsigned) positions.
+__device__ __forceinline__ int scan_item(const int32_t *in, const int32_t *ends, int i) {
+  return ends ? (int)((uint32_t)ends[i] - (uint32_t)in[i]) : in[i];
+}
+
+__global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const int32_t *__restrict__ in,
+                                                            const int32_t *__restrict__ ends, int n,
                                                             long long *__restrict__ tmp,
                                                             long long *__restrict__ tile_sums) {
   __shared__ long long ws[33];
@@ -686,7 +693,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const int32_t *__re
   long long s = 0;
 #pragma unroll
   for (int k = 0; k < kScanItems; ++k) {
-    v[k] = (base + k < n) ? in[base + k] : 0;
+    v[k] = base + k < n ? scan_item(in, ends, base + k) : 0;
     s += v[k];
   }
   long long total;
@@ -700,7 +707,8 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const int32_t *__re
 }
 
 __global__ void __launch_bounds__(kScanThreads) k_scan_sums(long long *tile_sums, int ntiles,
-                                                           long long *d_total) {
+                                                           long long *d_total, long long *h_total,
+                                                           const int *extra, int extra_n) {
   __shared__ long long ws[33];
   const int base = threadIdx.x * kScanItems;
   long long v[kScanItems];
@@ -717,7 +725,42 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_sums(long long *tile_sums
     if (base + k < ntiles) tile_sums[base + k] = ex;
     ex += v[k];
   }
-  if (threadIdx.x == 0) *d_total = total;
+  if (threadIdx.x == 0) *d_total = *h_total = total;
+  if (threadIdx.x < extra_n) reinterpret_cast<int *>(h_total + 1)[threadIdx.x] = extra[threadIdx.x];
+}
+
+// All of it in one launch, for few counts: three launches and the copies of the
+// total and of the extra words took 16 us where this takes 5 (4,096 counts).
+__global__ void __launch_bounds__(kScanThreads) k_scan_small(const int32_t *__restrict__ in,
+                                                           const int32_t *__restrict__ ends, int n,
+                                                           int32_t *__restrict__ offs, long long *h_total,
+                                                           const int *extra, int extra_n) {
+  __shared__ long long ws[33];
+  long long before = 0;
+  for (int t0 = 0; t0 < n; t0 += kScanTile) {
+    const int base = t0 + threadIdx.x * kScanItems;
+    int v[kScanItems];
+    long long s = 0;
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) {
+      v[k] = base + k < n ? scan_item(in, ends, base + k) : 0;
+      s += v[k];
+    }
+    long long total;
+    long long ex = before + block_exclusive_scan(s, ws, total);
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) {
+      if (base + k < n) offs[base + k] = (int32_t)ex;  // a total beyond int32 is an error to the caller
+      ex += v[k];
+    }
+    before += total;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    offs[n] = (int32_t)before;
+    *h_total = before;
+  }
+  if (threadIdx.x < extra_n) reinterpret_cast<int *>(h_total + 1)[threadIdx.x] = extra[threadIdx.x];
 }
 
 __global__ void k_scan_finish(const long long *__restrict__ tmp, const long long *__restrict__ tile_sums,
@@ -941,17 +984,11 @@ __global__ void k_negate_inv_slot(int nx, int ny, const int32_t *__restrict__ be
   oend[i] = i * cap + w / 2;
 }
 
-__global__ void k_slot_counts(int ncols, const int32_t *beg, const int32_t *end, int32_t *counts, int *maxc) {
+__global__ void k_slot_counts(int ncols, const int32_t *beg, const int32_t *end, int *maxc) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  int n = 0;
-  if (c < ncols) {
-    n = (int)((uint32_t)end[c] - (uint32_t)beg[c]);
-    if (counts) counts[c] = n;
-  }
-  if (maxc) {
-    for (int o = 16; o > 0; o >>= 1) n = max(n, __shfl_xor_sync(0xffffffffu, n, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(maxc, n);
-  }
+  int n = c < ncols ? scan_item(beg, end, c) : 0;
+  for (int o = 16; o > 0; o >>= 1) n = max(n, __shfl_xor_sync(0xffffffffu, n, o));
+  if ((threadIdx.x & 31) == 0) atomicMax(maxc, n);
 }
 
 __global__ void k_slot_compact(int ncols, const int32_t *__restrict__ beg, const double2 *__restrict__ z,
@@ -964,33 +1001,28 @@ __global__ void k_slot_compact(int ncols, const int32_t *__restrict__ beg, const
 // ================================================================ host side
 
 int scan_counts(vo_ctx *ctx, const int32_t *counts, int32_t *offs, int n, long long *total, const int *extra_dev,
-                int *extra_host, int extra_n) {
+                int *extra_host, int extra_n, const int32_t *ends) {
   const int ntiles = (n + kScanTile - 1) / kScanTile;
   if (ntiles > kScanTile) return set_error(ctx, VO_ERANGE, "scan: too many columns");
-  long long *tmp = nullptr, *sums = nullptr;
-  int rc = dalloc(ctx, &tmp, (size_t)n + 1);
-  if (rc) return rc;
-  rc = dalloc(ctx, &sums, (size_t)ntiles + 1);
-  if (rc) {
-    dfree(ctx, tmp);
-    return rc;
-  }
-  if (n > 0) {
-    k_scan_tiles<<<ntiles, kScanThreads, 0, ctx->stream>>>(counts, n, tmp, sums);
-    k_scan_sums<<<1, kScanThreads, 0, ctx->stream>>>(sums, ntiles, ctx->d_total);
+  if (extra_n > kScanExtra) return set_error(ctx, VO_EINTERNAL, "scan: too many words to read back");
+  if (n <= kScanSmall) {
+    k_scan_small<<<1, kScanThreads, 0, ctx->stream>>>(counts, ends, n, offs, ctx->h_total, extra_dev, extra_n);
+    ctx->launches += 1;
   } else {
-    cudaMemsetAsync(ctx->d_total, 0, sizeof(long long), ctx->stream);
+    long long *tmp = nullptr;  // and the tiles' sums
+    int rc = dalloc(ctx, &tmp, (size_t)n + 1 + (size_t)ntiles + 1);
+    if (rc) return rc;
+    long long *sums = tmp + n + 1;
+    k_scan_tiles<<<ntiles, kScanThreads, 0, ctx->stream>>>(counts, ends, n, tmp, sums);
+    k_scan_sums<<<1, kScanThreads, 0, ctx->stream>>>(sums, ntiles, ctx->d_total, ctx->h_total, extra_dev, extra_n);
+    k_scan_finish<<<(n + 1 + 255) / 256, 256, 0, ctx->stream>>>(tmp, sums, n, ctx->d_total, offs);
+    ctx->launches += 3;
+    dfree(ctx, tmp);
   }
-  k_scan_finish<<<(n + 1 + 255) / 256, 256, 0, ctx->stream>>>(tmp, sums, n, ctx->d_total, offs);
-  ctx->launches += n > 0 ? 3 : 1;
-  cudaMemcpyAsync(ctx->h_total, ctx->d_total, sizeof(long long), cudaMemcpyDeviceToHost, ctx->stream);
-  if (extra_n > 0)
-    cudaMemcpyAsync(extra_host, extra_dev, sizeof(int) * extra_n, cudaMemcpyDeviceToHost, ctx->stream);
-  dfree(ctx, tmp);
-  dfree(ctx, sums);
   VO_CK(ctx, cudaStreamSynchronize(ctx->stream));
   VO_CK(ctx, cudaGetLastError());
   *total = *ctx->h_total;
+  if (extra_n > 0) std::memcpy(extra_host, ctx->h_total + 1, sizeof(int) * extra_n);
   if (*total > 2147483647LL) return set_error(ctx, VO_ERANGE, "result exceeds int32 CSR offsets");
   return VO_OK;
 }
@@ -1411,7 +1443,7 @@ void slot_negate_inv_launch(cudaStream_t st, const SlotVol &in, const vo_grid &g
 
 int slot_max_count(vo_ctx *ctx, const SlotVol &v, int *d_max) {
   const int ncols = v.grid.nx * v.grid.ny;
-  k_slot_counts<<<nblocks(ncols, 256), 256, 0, ctx->stream>>>(ncols, v.beg, v.end, nullptr, d_max);
+  k_slot_counts<<<nblocks(ncols, 256), 256, 0, ctx->stream>>>(ncols, v.beg, v.end, d_max);
   ctx->launches += 1;
   return VO_OK;
 }
@@ -1419,15 +1451,10 @@ int slot_max_count(vo_ctx *ctx, const SlotVol &v, int *d_max) {
 int slot_to_volume(vo_ctx *ctx, const SlotVol &v, vo_volume **out, const int *extra_dev, int *extra_host,
                    int extra_n) {
   const int ncols = v.grid.nx * v.grid.ny;
-  int32_t *counts = nullptr;
-  int rc = dalloc(ctx, &counts, (size_t)ncols);
-  if (rc) return rc;
   vo_volume *res = nullptr;
   long long total = 0;
-  k_slot_counts<<<nblocks(ncols, 256), 256, 0, ctx->stream>>>(ncols, v.beg, v.end, counts, nullptr);
-  ctx->launches += 1;
-  rc = volume_alloc(ctx, v.grid, 0, &res);
-  if (!rc) rc = scan_counts(ctx, counts, res->offs, ncols, &total, extra_dev, extra_host, extra_n);
+  int rc = volume_alloc(ctx, v.grid, 0, &res);
+  if (!rc) rc = scan_counts(ctx, v.beg, res->offs, ncols, &total, extra_dev, extra_host, extra_n, v.end);
   if (!rc) {
     res->nseg = total;
     rc = dalloc(ctx, &res->z, (size_t)total);
@@ -1436,7 +1463,6 @@ int slot_to_volume(vo_ctx *ctx, const SlotVol &v, vo_volume **out, const int *ex
     k_slot_compact<<<nblocks(ncols, 256), 256, 0, ctx->stream>>>(ncols, v.beg, v.z, res->offs, res->z);
     ctx->launches += 1;
   }
-  dfree(ctx, counts);
   if (rc) {
     if (res) vo_volume_free(ctx, res);
     return rc;
