@@ -78,8 +78,10 @@ int build_tables(double R, int kmax, Tables &t) {
   for (int d = 0; d <= Dy; ++d)
     for (int dx = 0; dx <= t.Dx[d]; ++dx) {
       const double h = t.H[(size_t)d * t.W + dx];
-      const double gx = dx ? std::nextafter(t.H[(size_t)d * t.W + dx - 1] - h, -1.0) : -1.0;
-      const double gy = d ? std::nextafter(t.H[(size_t)(d - 1) * t.W + dx] - h, -1.0) : -1.0;
+      // less than it by more than the rounding of H: so it never exceeds the growth at farther distances
+      const double e = 3.6e-15 * (R + 1.0);
+      const double gx = dx ? t.H[(size_t)d * t.W + dx - 1] - h - e : -1.0;
+      const double gy = d ? t.H[(size_t)(d - 1) * t.W + dx] - h - e : -1.0;
       t.Dx[Dy + 1 + (size_t)d * t.W + dx] =
           (int)((unsigned)(gx < 0 ? 0xffff : floor16(gx)) | (unsigned)(gy < 0 ? 0xffff : floor16(gy)) << 16);
     }

@@ -28,7 +28,8 @@
 //    change any of the 32 unions and is dropped (2048^2 spheres + cylinders,
 //    r = 32, modelled: 2,083 clusters of 22,266 segments in reach of a patch;
 //    393 clusters of 4,511 segments pass the first test, 3,001 segments the
-//    second). The others are queued in shared memory, and each is merged by
+//    second). So is one that the candidate of a neighbour between it and the
+//    patch holds in every column (k_widths). The others are queued in shared memory, and each is merged by
 //    all lanes at once, one column each: the lane looks up the bin of its
 //    lower end and, only when the interval reaches beyond what its entry for
 //    that bin holds, updates it. Entries (smallest lower and largest upper
@@ -52,8 +53,9 @@
 // candidates' identities (value index, d, a), kept beside each entry. Output
 // endpoints are always recomputed in FP64 from their identities, so results
 // are bit-identical to the FP64 oracle. Nothing in the cover enters a result:
-// the segments that reach a component's ends are never dropped, and being long
-// they overlap the stretch that its shared entry stands for.
+// a segment that reaches a component's ends is never dropped but for a neighbour
+// whose candidate holds its own, which then reaches them too; and being long they
+// overlap the stretch that its shared entry stands for.
 //
 // What bounds it: issue slots (see the figures at k_patch). The bins' width is
 // a power of two, so that binning is exact (one fused multiply-add that
@@ -96,7 +98,7 @@ constexpr int kShort = 1024;      // kept-aside segments of a patch
 constexpr int kEntriesBig = 1600; // the same for the second tier
 constexpr int kUnionBig = 1024;
 constexpr int kShortBig = 8192;
-constexpr double kDirectWork = 600;            // candidates per column up to which k_direct takes a dilation
+constexpr double kDirectWork = 450;            // candidates per column up to which k_direct takes a dilation
 constexpr int64_t kDirectSplitCols = 1 << 16;  // columns of a launch up to which kSplit threads share one there
 constexpr int kStep = 8;          // segments that k_direct loads at a time
 constexpr int kPrepThreads = 256;
@@ -186,7 +188,8 @@ template <int WARPS>
 __global__ void __launch_bounds__(32 * WARPS) k_pack(int nx, int ny, const int32_t *__restrict__ beg,
                                                      const int32_t *__restrict__ end, const double2 *__restrict__ z,
                                                      const FastPar *__restrict__ par, float2 *__restrict__ zf,
-                                                     unsigned char *__restrict__ code, double2 *__restrict__ zx,
+                                                     const uint2 *__restrict__ wide, uint2 *__restrict__ code,
+                                                     double2 *__restrict__ zx,
                                                      float4 *__restrict__ cl, int32_t *__restrict__ coff) {
   constexpr int CAP = kPackSort / WARPS;
   __shared__ __align__(16) int s_key[WARPS][CAP];  // bit patterns of the lower ends: a total order, also of NaNs
@@ -303,7 +306,8 @@ __global__ void __launch_bounds__(32 * WARPS) k_pack(int nx, int ny, const int32
           const int i = s_ord[warp][r], col = s_col[warp][i];
           const float a = __int_as_float(s_key[warp][i]);
           zf[sb + r] = make_float2(a, s_hi[warp][i]);
-          code[sb + r] = (unsigned char)col;
+          const uint2 w = wide[s_src[warp][col] + i];
+          code[sb + r] = make_uint2(w.x | (unsigned)col << 24, w.y);
           zx[sb + r] = z[s_src[warp][col] + i];
           if (starts[b] >> lane & 1) {
             // the cluster's end: the next start, in this block of ranks or the next one
@@ -325,7 +329,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_pack(int nx, int ny, const int32
         const float2 f = make_float2(__double2float_rn(__dsub_rn(v.x, base)), __double2float_rn(__dsub_rn(v.y, base)));
         const int r = pre + i;
         zf[sb + r] = f;
-        code[sb + r] = (unsigned char)c4;
+        code[sb + r] = make_uint2(wide[k0 + i].x | (unsigned)c4 << 24, wide[k0 + i].y);
         zx[sb + r] = v;
         cl[cb + r] = make_float4(f.x, f.y, __int_as_float(sb + r), __int_as_float(1 | (tx << 5)));
       }
@@ -612,7 +616,8 @@ __device__ __forceinline__ bool expand_clusters(const FastArgs &A, const PatchMe
   __syncwarp();
   for (int q = 0;; q += 2 * kPairs) {
     float2 z[kPairs];
-    int key[kPairs], t[kPairs], col[kPairs];
+    int key[kPairs], t[kPairs];
+    uint2 code[kPairs];
     bool ok[kPairs];
 #pragma unroll
     for (int i = 0; i < kPairs; ++i) {
@@ -622,17 +627,27 @@ __device__ __forceinline__ bool expand_clusters(const FastArgs &A, const PatchMe
       key[i] = c.x + (lane & 15);
       t[i] = (c.y >> 5) * kTile - S.X0;
       z[i] = ok[i] ? __ldcg(A.zf + key[i]) : make_float2(0.f, 0.f);
-      col[i] = ok[i] ? __ldcg(A.code + key[i]) : 0;
+      code[i] = ok[i] ? __ldcg(A.code + key[i]) : make_uint2(0u, 0u);
     }
 #pragma unroll
     for (int i = 0; i < kPairs; ++i) {
-      t[i] += col[i] & 3;
-      const int sy = col[i] >> 2;
-      const int row = hrow_row(k, sy, k > 0 ? kPatchY - 1 : k < 0 ? 0 : sy);
+      const int sy = code[i].x >> 26, near = k > 0 ? kPatchY - 1 : k < 0 ? 0 : sy;
+      t[i] += code[i].x >> 24 & 3;
+      const int row = hrow_row(k, sy, near);
+      // held, for every column of the patch, by the candidate of a neighbour between it and the patch
+      bool held = false;
+      {
+        const int a = near_dx<G>(t[i]), d = abs(kTile * k + sy - near);
+        if (ok[i] && d <= A.Dy && a < A.W) {
+          const int g = A.Dx[A.Dy + 1 + d * A.W + a];
+          const unsigned wx = t[i] < 0 ? code[i].x >> 12 : code[i].x, wy = k < 0 ? code[i].y >> 12 : code[i].y;
+          held = (a > 0 && (int)(wx & 0xfff) << 3 <= (short)g) || (d > 0 && (int)(wy & 0xfff) << 3 <= g >> 16);
+        }
+      }
       const float h = M.hrow[row * hs + (ok[i] ? near_dx<G>(t[i]) : 0)];
       const float lo = z[i].x - h, hi = z[i].y + h;
       const float2 b = component_of(M, S, lo);
-      const bool keep = ok[i] && !(b.x <= lo && hi <= b.y);
+      const bool keep = ok[i] && !held && !(b.x <= lo && hi <= b.y);
       const unsigned w = __ballot_sync(kFull, keep);
       if (keep) {
         const int p = S.qn + __popc(w & ((1u << lane) - 1u));
@@ -1187,19 +1202,23 @@ __global__ void __launch_bounds__(32, 20) k_patch(const BatchVol *__restrict__ v
 
 // ------------------------------------------------------------ small radii
 
-// What k_direct needs of a segment: its ends as FP32, its column and, for each
-// of its four neighbour columns, by how much at most it reaches beyond one of
-// their segments (FP16 bits, rounded up to 12). Where H grows by at least as
-// much over the step to that neighbour, the neighbour's candidate holds the
-// segment's, in exact arithmetic and so after rounding, and the segment is
-// passed over for all columns on that side. A block per row; the segments of a
-// row become contiguous (CSR inputs are already so: slots == false).
-template <bool SLOTS>
-__global__ void __launch_bounds__(kPrepThreads) k_direct_prep(int nx, int ny, const int32_t *__restrict__ beg,
+// By how much at most a segment reaches beyond one of the segments of each of
+// its four neighbour columns (FP16 bits, rounded up to 12). Where H grows by at
+// least as much over the step to that neighbour, the neighbour's candidate holds
+// the segment's, in exact arithmetic and so after rounding, and the segment is
+// passed over for all columns on that side: by patches on their nearest column's
+// growth, which is the least (2048^2, r = 32: 33.0 to 24.7 ms, this kernel
+// included; 1024^2 spheres, r = 32: 5.1 to 4.0), by k_direct on each column's
+// own. For k_direct (RECORDS) with the ends in FP32 and the column, the segments
+// of a row contiguous (CSR inputs are already so: SLOTS false); else the widths
+// alone, in the input's order. A block per row: it loads what it needs of five
+// columns, and is bound by the latency of that (0.7 ms at 2048^2).
+template <bool SLOTS, bool RECORDS>
+__global__ void __launch_bounds__(kPrepThreads) k_widths(int nx, int ny, const int32_t *__restrict__ beg,
                                                               const int32_t *__restrict__ end,
                                                               const longlong2 *__restrict__ z, uint4 *__restrict__ rec,
                                                               longlong2 *__restrict__ rz, int32_t *__restrict__ rbeg,
-                                                              int32_t *__restrict__ rend) {
+                                                              int32_t *__restrict__ rend, uint2 *__restrict__ wide) {
   __shared__ int s_sum[kPrepThreads / 32];
   const int y = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int base = SLOTS ? beg[nx * y] : 0;
@@ -1263,7 +1282,10 @@ __global__ void __launch_bounds__(kPrepThreads) k_direct_prep(int nx, int ny, co
         }
         w[d] = min(0xfffu, (__half_as_ushort(__float2half_ru(best)) + 7u) >> 3);
       }
-      rec[out + k] = make_uint4(__float_as_uint(lo), __float_as_uint(hi), w[0] | w[1] << 12 | (unsigned)(x & 0xff) << 24,
+      if (!RECORDS)
+        wide[out + k] = make_uint2(w[0] | w[1] << 12, w[2] | w[3] << 12);
+      else
+        rec[out + k] = make_uint4(__float_as_uint(lo), __float_as_uint(hi), w[0] | w[1] << 12 | (unsigned)(x & 0xff) << 24,
                                 w[2] | w[3] << 12 | (unsigned)(x >> 8) << 24);
       if (SLOTS) rz[out + k] = v;
     }
@@ -1272,7 +1294,7 @@ __global__ void __launch_bounds__(kPrepThreads) k_direct_prep(int nx, int ny, co
 
 // Dilations by small radii, one thread per column: few columns are in reach, so
 // that the candidates are met one by one, without clusters, cover or bins. A
-// candidate that its neighbour's holds (k_direct_prep), or that lies, in FP32
+// candidate that its neighbour's holds (k_widths), or that lies, in FP32
 // and by more than its error, inside one of the first kHot intervals found, is
 // passed over. What is left each lane takes from a list of its own, so that the
 // lanes do not wait for one another's: it is compared with all intervals found,
@@ -1290,14 +1312,14 @@ __global__ void __launch_bounds__(kPrepThreads) k_direct_prep(int nx, int ny, co
 // the line at 2^16 columns.
 //
 // Against patches, packing included (ms; segments per column; radius 4, 6, 8):
-//   276^2   1.5   0.10 / 0.29   0.15 / 0.36   0.21 / 0.33
-//   1024^2  1.5   0.39 / 1.45   0.68 / 2.14   1.01 / 1.95
-//   2048^2  5.1   11.2 / 18.9   21.9 / 28.1   40   / 36.7
+//   276^2   1.5   0.10 / 0.21   0.15 / 0.21   0.21 / 0.20
+//   1024^2  1.5   0.39 / 1.09   0.68 / 1.36   1.01 / 1.43
+//   2048^2  5.1   11.1 / 16.5   21.9 / 21.4   36.0 / 24.4
 // A patch's candidates are those of the whole patch's reach, at radius 4 four
 // times a column's, and its steps take some ten thousand cycles however few they
-// are; but their number grows more slowly. Both take the same at about 600
-// candidates per column: the line of direct_choice. (In FP64 throughout, without
-// the neighbours' test, 1024^2 took 0.53, 1.1 and 1.9 ms.)
+// are; but their number grows more slowly. Both take the same between 290 and
+// 580 candidates per column: the line of direct_choice is 450. (In FP64
+// throughout, without the neighbours' test, 1024^2 took 0.53, 1.1 and 1.9 ms.)
 template <int G>
 __global__ void __launch_bounds__(128) k_direct(const BatchVol *__restrict__ vols, int nv) {
   __shared__ BatchVol V;
@@ -1633,8 +1655,10 @@ void fast_prepare(cudaStream_t st, const FastArgs &A, float R, double mean_segs,
   const double most = 2.2 * mean_segs * kTile * std::min(kTile, A.ny);
   const int warps = most <= kPackSort / 32 ? 32 : most <= kPackSort / 16 ? 16 : 8;
   auto *pack = warps == 32 ? &k_pack<32> : warps == 16 ? &k_pack<16> : &k_pack<8>;
-  pack<<<(A.ny + kTile - 1) / kTile, 32 * warps, 0, st>>>(A.nx, A.ny, A.beg, A.end, z, out.par, out.zf, out.code, out.zx,
-                                                          out.cl, out.coff);
+  k_widths<false, false><<<A.ny, kPrepThreads, 0, st>>>(A.nx, A.ny, A.beg, A.end, reinterpret_cast<const longlong2 *>(z),
+                                                        nullptr, nullptr, nullptr, nullptr, out.wide);
+  pack<<<(A.ny + kTile - 1) / kTile, 32 * warps, 0, st>>>(A.nx, A.ny, A.beg, A.end, z, out.par, out.zf, out.wide, out.code,
+                                                          out.zx, out.cl, out.coff);
 }
 
 FastArgs fast_args(int nx, int ny, const DeviceTables &T, const int32_t *beg, const int32_t *end, const double2 *z,
@@ -1656,11 +1680,12 @@ void direct_prepare(cudaStream_t st, const FastArgs &A, const PackOut &out) {
   if (A.ny <= 0) return;
   const longlong2 *z = reinterpret_cast<const longlong2 *>(A.zd);
   if (out.zx)
-    k_direct_prep<true><<<A.ny, kPrepThreads, 0, st>>>(A.nx, A.ny, A.beg, A.end, z, out.rec,
-                                                       reinterpret_cast<longlong2 *>(out.zx), out.rbeg,
-                                                       out.rbeg + (size_t)A.nx * A.ny);
+    k_widths<true, true><<<A.ny, kPrepThreads, 0, st>>>(A.nx, A.ny, A.beg, A.end, z, out.rec,
+                                                        reinterpret_cast<longlong2 *>(out.zx), out.rbeg,
+                                                        out.rbeg + (size_t)A.nx * A.ny, nullptr);
   else
-    k_direct_prep<false><<<A.ny, kPrepThreads, 0, st>>>(A.nx, A.ny, A.beg, A.end, z, out.rec, nullptr, nullptr, nullptr);
+    k_widths<false, true><<<A.ny, kPrepThreads, 0, st>>>(A.nx, A.ny, A.beg, A.end, z, out.rec, nullptr, nullptr, nullptr,
+                                                         nullptr);
 }
 static size_t direct_table(int nx, int ny, int W, int Dy) {
   return sizeof(float2) * (size_t)std::min(W, nx) * (std::min(Dy, ny - 1) + 1);
@@ -1732,6 +1757,7 @@ int dilate_fast(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out, vo_
     int r = patch_plan(ctx, patch_count(g, split), split, T->host.hs, P);
     if (!r) r = dalloc(ctx, &pk.zf, nseg);
     if (!r) r = dalloc(ctx, &pk.code, nseg);
+    if (!r) r = dalloc(ctx, &pk.wide, nseg);
     if (!r) r = dalloc(ctx, &pk.zx, nseg);
     if (!r) r = dalloc(ctx, &pk.cl, nseg);
     if (!r) r = dalloc(ctx, &pk.coff, pack_offsets(g));
@@ -1775,7 +1801,7 @@ int dilate_fast(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out, vo_
     else
       patch_launch(false, P, ctx->stream, dv);
     cudaEventRecord(ctx->ev[5], ctx->stream);
-    ctx->launches += direct ? 2 : 3;
+    ctx->launches += direct ? 2 : 4;
     SlotVol sv;
     sv.grid = g;
     sv.cap = cap;
@@ -1835,7 +1861,7 @@ int dilate_fast(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out, vo_
       tm->kernel_ms[2] += e1;
     }
   }
-  for (void *p : {(void *)misc, (void *)pk.zf, (void *)pk.code, (void *)pk.zx, (void *)pk.cl, (void *)pk.rec,
+  for (void *p : {(void *)misc, (void *)pk.zf, (void *)pk.code, (void *)pk.wide, (void *)pk.zx, (void *)pk.cl, (void *)pk.rec,
                   (void *)pk.coff, (void *)list, (void *)big_list, (void *)scratch[0],
                   (void *)scratch[1], (void *)oz, (void *)big})
     dfree(ctx, p);

@@ -200,10 +200,10 @@ struct FastArgs {
   const int32_t *beg, *end;  // segments [beg[c], end[c]) of column c as given (CSR or slots)
   const double *zd;          // FP64 values as given
   // Packed by 4 x 4 tiles of columns (k_pack in vo_fast.cu): FP32 values
-  // relative to FastPar::base, column in the tile, FP64 values; the clusters
+  // relative to FastPar::base, column in the tile (bits 24 .. 27) with widths (k_widths), FP64 values; the clusters
   // and their offsets [tile rows][tiles per row + 1].
   const float2 *zf;
-  const unsigned char *code;
+  const uint2 *code;
   const double *zx;
   const float4 *cl;
   const int32_t *coff;
@@ -211,7 +211,7 @@ struct FastArgs {
   const double *H64;    // [(Dy + 1) * W]
   const int *Dx;        // [Dy + 1], then the growth of H over a step inwards (Tables::Dx)
   const FastPar *par;
-  // small radii (k_direct_prep): per segment what k_direct needs and its FP64 values, contiguous by rows;
+  // small radii (k_widths): per segment what k_direct needs and its FP64 values, contiguous by rows;
   // [rbeg[c], rend[c]) of column c
   const uint4 *rec;
   const double2 *rz;
@@ -281,7 +281,7 @@ void big_launch(cudaStream_t st, const BatchVol *vols, int nv, double2 *scratch)
 // (with its unused slots), coff pack_offsets(grid).
 struct PackOut {
   float2 *zf = nullptr;
-  unsigned char *code = nullptr;
+  uint2 *code = nullptr, *wide = nullptr;  // wide: widths in the input's order (k_widths)
   double2 *zx = nullptr;
   float4 *cl = nullptr;
   int32_t *coff = nullptr;
