@@ -618,7 +618,7 @@ def main():
             arms["learned_sizing_cyl4096"] = learned_sizing_arm(ctx, sizer, rank, world, timed)
 
     # ---------------- roofline of the dominant kernel
-    kname = {"batched": "k_fast_batched", "fast": "k_fast", "separable": "k_pass2", "brute": "k_brute",
+    kname = {"batched": "k_patch", "fast": "k_patch", "separable": "k_pass2", "brute": "k_brute",
              "envelope": "k_env2"}[args.method]
     per_launch = kernel_ms / args.steps
     alg_bytes = 4 * (ncols + 1) + 16 * int(offs[-1]) + 4 * (ncols + 1) + 16 * int(out_segs)

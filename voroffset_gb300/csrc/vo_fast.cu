@@ -57,7 +57,11 @@
 // whose candidate holds its own, which then reaches them too; and being long they
 // overlap the stretch that its shared entry stands for.
 //
-// What bounds it: issue slots (see the figures at k_patch). The bins' width is
+// What bounds it: dependent latency at 20 warps per SM, with half of the issue
+// slots used (1024^2 spheres, r = 32: 3.1 ms, IPC 2.1, 27 of 32 lanes; 2048^2
+// spheres + cylinders 21.6 ms, 3,098 warp instructions per column). A thread per
+// column, with masks of the segments that a neighbour's candidate holds at each
+// of eleven growths, took 26.9 and 183 ms. The bins' width is
 // a power of two, so that binning is exact (one fused multiply-add that
 // rounds to an integer).
 //
@@ -1302,8 +1306,8 @@ __global__ void __launch_bounds__(kPrepThreads) k_widths(int nx, int ny, const i
 // are compared as integers (Key). Intervals that have come to meet are merged at
 // the end; more than kList of them are inserted into a sorted list at once.
 //
-// What bounds it: instructions (1024^2, 1.5 segments per column, radius 6: 70 of
-// them per candidate and warp, 2.3 per cycle), in inputs of many segments the
+// What bounds it: the ALU pipe (1024^2, 1.5 segments per column, radius 6: 90
+// instructions per candidate and warp, the pipe busy 82 % of its cycles), in inputs of many segments the
 // latency of the lists in local memory, and in small volumes that of a thread's
 // chain. There G = 4 threads share a column, each taking every fourth row, and
 // the first one inserts the others' unions into its own: with four threads 64^2
