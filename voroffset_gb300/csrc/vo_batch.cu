@@ -324,7 +324,7 @@ int plan_dilation_round(vo_ctx *ctx, vo_batch *b, std::vector<DilPlan> &dils, bo
     if (rc) return rc;
     d.A = fast_args(g.nx, g.ny, *d.T, d.in.beg, d.in.end, d.in.z, d.pk);
     const DilPlan c = d;
-    record(b, 3, [c, R](cudaStream_t st) { fast_prepare(st, c.A, R, c.mean_segs, c.mm, c.pk); });
+    record(b, 2, [c, R](cudaStream_t st) { fast_prepare(st, c.A, R, c.mean_segs, c.mm, c.pk); });
   }
   if (ctx->sizer) run_pending(ctx, b);  // features need the dilation inputs
   int *counters = nullptr;

@@ -126,38 +126,15 @@ __device__ __forceinline__ double order_value(unsigned long long o) {
   return __longlong_as_double((long long)(o >> 63 ? o & 0x7fffffffffffffffull : ~o));
 }
 
-// Range of the values and, by the last block to finish, the scalars of the
-// dilation (FastPar). mm (zeroed before): orders of the largest value and of
-// the largest negated value, then the blocks that are done.
+// The scalars of a dilation from the orders of the largest value and of the
+// largest negated value (0: there is none).
 // Guard band: with U bounding the magnitude of every FP32 value (relative to
 // the base), each candidate endpoint is within 1.5 ulp32(U) of its FP64 value
 // (rounding of z, of H and of the sum) and a difference of two adds one more
 // ulp32(U): at most 4 ulp32(U) = 2^-21 U. E = 2^-20 U leaves a factor of two;
 // the rounding of the FP64 endpoints themselves is below 2^-50 times the
 // largest magnitude.
-__global__ void k_range(int ncols, const int32_t *__restrict__ beg, const int32_t *__restrict__ end,
-                        const double2 *__restrict__ z, float R, unsigned long long *mm, FastPar *par) {
-  double hi = -INFINITY, lo = -INFINITY;
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < ncols; c += gridDim.x * blockDim.x)
-    for (int k = beg[c]; k < end[c]; ++k) {
-      const double2 s = z[k];
-      hi = fmax(hi, fmax(s.x, s.y));
-      lo = fmax(lo, -fmin(s.x, s.y));
-    }
-  for (int o = 16; o > 0; o >>= 1) {
-    hi = fmax(hi, __shfl_xor_sync(kFull, hi, o));
-    lo = fmax(lo, __shfl_xor_sync(kFull, lo, o));
-  }
-  if ((threadIdx.x & 31) == 0 && hi > -INFINITY) {
-    atomicMax(&mm[0], order_of(hi));
-    atomicMax(&mm[1], order_of(lo));
-  }
-  __syncthreads();
-  if (threadIdx.x) return;
-  __threadfence();
-  if (atomicAdd(&mm[2], 1ull) + 1 != gridDim.x) return;
-  __threadfence();
-  const unsigned long long a = atomicMax(&mm[0], 0ull), b = atomicMax(&mm[1], 0ull);
+__device__ void set_par(unsigned long long a, unsigned long long b, float R, FastPar *par) {
   const double zmax = a ? order_value(a) : 0.0, zmin = b ? -order_value(b) : 0.0;
   FastPar p;
   p.base = floor(zmin - R - 3.0);
@@ -1215,17 +1192,22 @@ __global__ void __launch_bounds__(32, 20) k_patch(const BatchVol *__restrict__ v
 // included; 1024^2 spheres, r = 32: 5.1 to 4.0), by k_direct on each column's
 // own. For k_direct (RECORDS) with the ends in FP32 and the column, the segments
 // of a row contiguous (CSR inputs are already so: SLOTS false); else the widths
-// alone, in the input's order. A block per row: it loads what it needs of five
+// alone, in the input's order, and the scalars of the dilation from the values'
+// range (mm, zeroed before: orders of the largest value and of the largest
+// negated value, then the blocks that are done); a pass of its own over the
+// values took 0.5 ms at 2048^2. A block per row: it loads what it needs of five
 // columns, and is bound by the latency of that (0.7 ms at 2048^2).
 template <bool SLOTS, bool RECORDS>
 __global__ void __launch_bounds__(kPrepThreads) k_widths(int nx, int ny, const int32_t *__restrict__ beg,
                                                               const int32_t *__restrict__ end,
                                                               const longlong2 *__restrict__ z, uint4 *__restrict__ rec,
                                                               longlong2 *__restrict__ rz, int32_t *__restrict__ rbeg,
-                                                              int32_t *__restrict__ rend, uint2 *__restrict__ wide) {
+                                                              int32_t *__restrict__ rend, uint2 *__restrict__ wide,
+                                                              float R, unsigned long long *mm, FastPar *par) {
   __shared__ int s_sum[kPrepThreads / 32];
   const int y = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int base = SLOTS ? beg[nx * y] : 0;
+  Key top = kKeyMin, bottom = kKeyMax;  // widths alone: the values' range besides (NaN left out)
   for (int x0 = 0; x0 < nx; x0 += kPrepThreads) {
     const int x = x0 + threadIdx.x, c = x + nx * y;
     const int k0 = x < nx ? beg[c] : 0, n = x < nx ? end[c] - k0 : 0;
@@ -1262,6 +1244,15 @@ __global__ void __launch_bounds__(kPrepThreads) k_widths(int nx, int ny, const i
     }
     for (int k = 0; k < n; ++k) {
       const longlong2 v = z[k0 + k];
+      if (!RECORDS) {
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const Key bits = q ? v.y : v.x, key = bits ^ ((bits >> 63) & 0x7fffffffffffffffll);
+          if ((bits & 0x7fffffffffffffffll) > 0x7ff0000000000000ll) continue;
+          top = kmax(top, key);
+          bottom = kmin(bottom, key);
+        }
+      }
       const float lo = trunc32_bits(v.x), hi = trunc32_bits(v.y);
       unsigned w[4];
 #pragma unroll
@@ -1294,6 +1285,21 @@ __global__ void __launch_bounds__(kPrepThreads) k_widths(int nx, int ny, const i
       if (SLOTS) rz[out + k] = v;
     }
   }
+  if (RECORDS) return;
+  for (int o = 16; o > 0; o >>= 1) {
+    top = kmax(top, __shfl_xor_sync(kFull, top, o));
+    bottom = kmin(bottom, __shfl_xor_sync(kFull, bottom, o));
+  }
+  if (lane == 0 && top >= bottom) {
+    atomicMax(&mm[0], order_of(value_of(top)));
+    atomicMax(&mm[1], order_of(-value_of(bottom)));
+  }
+  __syncthreads();
+  if (threadIdx.x) return;
+  __threadfence();
+  if (atomicAdd(&mm[2], 1ull) + 1 != gridDim.x) return;
+  __threadfence();
+  set_par(atomicMax(&mm[0], 0ull), atomicMax(&mm[1], 0ull), R, par);  // the last block to finish
 }
 
 // Dilations by small radii, one thread per column: few columns are in reach, so
@@ -1650,17 +1656,14 @@ size_t pack_offsets(const vo_grid &g) {
 
 void fast_prepare(cudaStream_t st, const FastArgs &A, float R, double mean_segs, unsigned long long *mm,
                   const PackOut &out) {
-  const int ncols = A.nx * A.ny;
   const double2 *z = reinterpret_cast<const double2 *>(A.zd);
   cudaMemsetAsync(mm, 0, 3 * sizeof(unsigned long long), st);
-  const int grid = std::max(1, std::min((ncols + 255) / 256, 8 * sm_count_fast()));
-  k_range<<<grid, 256, 0, st>>>(ncols, A.beg, A.end, z, R, mm, out.par);
   // warps per block by the segments of a tile: twice the mean should fit a warp's share of the sort
   const double most = 2.2 * mean_segs * kTile * std::min(kTile, A.ny);
   const int warps = most <= kPackSort / 32 ? 32 : most <= kPackSort / 16 ? 16 : 8;
   auto *pack = warps == 32 ? &k_pack<32> : warps == 16 ? &k_pack<16> : &k_pack<8>;
   k_widths<false, false><<<A.ny, kPrepThreads, 0, st>>>(A.nx, A.ny, A.beg, A.end, reinterpret_cast<const longlong2 *>(z),
-                                                        nullptr, nullptr, nullptr, nullptr, out.wide);
+                                                        nullptr, nullptr, nullptr, nullptr, out.wide, R, mm, out.par);
   pack<<<(A.ny + kTile - 1) / kTile, 32 * warps, 0, st>>>(A.nx, A.ny, A.beg, A.end, z, out.par, out.zf, out.wide, out.code,
                                                           out.zx, out.cl, out.coff);
 }
@@ -1686,10 +1689,10 @@ void direct_prepare(cudaStream_t st, const FastArgs &A, const PackOut &out) {
   if (out.zx)
     k_widths<true, true><<<A.ny, kPrepThreads, 0, st>>>(A.nx, A.ny, A.beg, A.end, z, out.rec,
                                                         reinterpret_cast<longlong2 *>(out.zx), out.rbeg,
-                                                        out.rbeg + (size_t)A.nx * A.ny, nullptr);
+                                                        out.rbeg + (size_t)A.nx * A.ny, nullptr, 0.f, nullptr, nullptr);
   else
     k_widths<false, true><<<A.ny, kPrepThreads, 0, st>>>(A.nx, A.ny, A.beg, A.end, z, out.rec, nullptr, nullptr, nullptr,
-                                                         nullptr);
+                                                         nullptr, 0.f, nullptr, nullptr);
 }
 static size_t direct_table(int nx, int ny, int W, int Dy) {
   return sizeof(float2) * (size_t)std::min(W, nx) * (std::min(Dy, ny - 1) + 1);
@@ -1706,7 +1709,7 @@ bool direct_choice(const vo_grid &g, const DeviceTables &T, double mean_segs) {
   for (int d = 0; d <= std::min(T.host.Dy, g.ny - 1); ++d)
     cols += (d ? 2.0 : 1.0) * (1.0 - (double)d / g.ny) * std::min(2 * T.host.Dx[d] + 1, g.nx);
   // patches are four rows high: of a grid of fewer rows they use as much less
-  if (g.nx < 1 || g.ny < 1 || g.nx > 65535 || direct_table(g.nx, g.ny, T.host.W, T.host.Dy) > 32 * 1024) return false;
+  if (g.nx < 1 || g.ny < 1 || g.nx > 65535 || direct_table(g.nx, g.ny, T.host.W, T.host.Dy) > 31 * 1024) return false;
   return cols * std::max(mean_segs, 1.0) <= kDirectWork * kPatchY / std::min(g.ny, kPatchY);
 }
 
@@ -1805,7 +1808,7 @@ int dilate_fast(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out, vo_
     else
       patch_launch(false, P, ctx->stream, dv);
     cudaEventRecord(ctx->ev[5], ctx->stream);
-    ctx->launches += direct ? 2 : 4;
+    ctx->launches += direct ? 2 : 3;
     SlotVol sv;
     sv.grid = g;
     sv.cap = cap;

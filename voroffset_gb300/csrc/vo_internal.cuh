@@ -182,7 +182,7 @@ int slot_to_volume(vo_ctx *ctx, const SlotVol &v, vo_volume **out, const int *ex
                    int *extra_host = nullptr, int extra_n = 0);
 
 // Scalars of a dilation's FP32 arithmetic, from the range of its input
-// (k_range in vo_fast.cu): FP32 values are relative to base, E is the guard
+// (set_par in vo_fast.cu): FP32 values are relative to base, E is the guard
 // band, 1 / inv_w the bin width, thr the least length of a long interval.
 struct FastPar {
   double base;
