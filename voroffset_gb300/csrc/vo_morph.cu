@@ -352,9 +352,42 @@ __global__ void __launch_bounds__(kBigThreads) k_pass1_big(int nx, int ny, const
   }
 }
 
+// Column (x, y)'s union by LANES threads of a warp, `cols` columns apart: each takes every LANES-th
+// source column, and the first one (part 0) inserts the others' unions into its own, in A. Returns the
+// count there, or -1 when a list outgrew kCapSmall on the way. The whole warp calls it; threads with
+// inside = false contribute nothing.
+template <int LANES>
+__device__ __forceinline__ int pass2_shared_column(bool inside, int x, int y, int nx, int part, int lane,
+                                                   const int32_t *__restrict__ poffs, const double2 *__restrict__ pz,
+                                                   const uint8_t *__restrict__ pd, const DevTables &t, const double *H,
+                                                   const int *Dx, Key2 *A) {
+  constexpr int kCols = kBX / LANES;
+  int n = inside ? pass2_column(x, y, nx, poffs, pz, pd, t, H, Dx, A, kCapSmall, part, LANES) : 0;
+  // the other lanes' unions into the first one's
+#pragma unroll 1
+  for (int p = 1; p < LANES; ++p) {
+    const int from = lane + p * kCols, m = __shfl_sync(0xffffffffu, n, from);
+    if (part == 0 && m < 0) n = -1;
+    const int most = __reduce_max_sync(0xffffffffu, m);
+#pragma unroll 1
+    for (int i = 0; i < most; ++i) {
+      const Key2 s = A[min(i, kCapSmall - 1)];
+      const Key lo = __shfl_sync(0xffffffffu, s.x, from), hi = __shfl_sync(0xffffffffu, s.y, from);
+      if (part == 0 && n >= 0 && i < m) {
+        const int2 at = union_insert_keys(A, n, kCapSmall, lo, hi);
+        n = at.x < 0 ? -1 : at.y;
+      }
+    }
+  }
+  return n;
+}
+
 // A column's union is found once: up to `nslots` of its intervals wait in its
 // slots (interval i of column c at slots[i * ncols + c]) until the offsets are
-// known, and k_pass2_place moves them. Only a larger union is found again there.
+// known, and k_pass2_place moves them. Only a larger union is found again
+// there, by the same threads in the same order: whether a list outgrows
+// kCapSmall depends on the order in which the chords come, and a column that
+// did not when it was counted must not when it is written.
 //
 // What bounds it is latency: a column is a chain of dependent insertions. With
 // LANES = 4 each of four threads takes every fourth source column, and the first
@@ -388,23 +421,7 @@ __global__ void __launch_bounds__(kBX *kBY) k_pass2(int nx, int ny, const int32_
   const bool inside = x < nx && y < ny;
   const int c = x + nx * y;
   Key2 A[kCapSmall];
-  int n = inside ? pass2_column(x, y, nx, poffs, pz, pd, t, sH, sDx, A, kCapSmall, part, LANES) : 0;
-  // the other lanes' unions into the first one's
-#pragma unroll 1
-  for (int p = 1; p < LANES; ++p) {
-    const int from = lane + p * kCols, m = __shfl_sync(0xffffffffu, n, from);
-    if (part == 0 && m < 0) n = -1;
-    const int most = __reduce_max_sync(0xffffffffu, m);
-#pragma unroll 1
-    for (int i = 0; i < most; ++i) {
-      const Key2 s = A[min(i, kCapSmall - 1)];
-      const Key lo = __shfl_sync(0xffffffffu, s.x, from), hi = __shfl_sync(0xffffffffu, s.y, from);
-      if (part == 0 && n >= 0 && i < m) {
-        const int2 at = union_insert_keys(A, n, kCapSmall, lo, hi);
-        n = at.x < 0 ? -1 : at.y;
-      }
-    }
-  }
+  const int n = pass2_shared_column<LANES>(inside, x, y, nx, part, lane, poffs, pz, pd, t, sH, sDx, A);
   if (part != 0 || !inside) return;
   if (n < 0) record_overflow(ovf, c);
   counts[c] = max(n, 0);
@@ -412,6 +429,9 @@ __global__ void __launch_bounds__(kBX *kBY) k_pass2(int nx, int ny, const int32_
     for (int k = 0; k < n; ++k) slots[(size_t)k * nx * ny + c] = make_double2(value_of(A[k].x), value_of(A[k].y));
 }
 
+// Columns that k_pass2 listed are not written here (or, where their count is small, with what their slots
+// held before): k_pass2_big, launched after this, writes them.
+template <int LANES>
 __global__ void __launch_bounds__(kBX *kBY) k_pass2_place(int nx, int ny, const int32_t *__restrict__ poffs,
                                                           const double2 *__restrict__ pz,
                                                           const uint8_t *__restrict__ pd, DevTables t,
@@ -419,18 +439,21 @@ __global__ void __launch_bounds__(kBX *kBY) k_pass2_place(int nx, int ny, const 
                                                           const double2 *__restrict__ slots, int nslots,
                                                           const int32_t *__restrict__ ooffs,
                                                           double2 *__restrict__ oz) {
-  const int x = blockIdx.x * kBX + threadIdx.x;
+  constexpr int kCols = kBX / LANES;
+  const int part = threadIdx.x / kCols, lane = threadIdx.x % kCols;
+  const int x = blockIdx.x * kCols + lane;
   const int y = blockIdx.y * kBY + threadIdx.y;
-  if (x >= nx || y >= ny) return;
-  const int c = x + nx * y, n = counts[c];
+  const bool inside = x < nx && y < ny;
+  const int c = inside ? x + nx * y : 0, n = inside ? counts[c] : 0;
   double2 *out = oz + ooffs[c];
-  if (n <= nslots) {
-    for (int k = 0; k < n; ++k) out[k] = slots[(size_t)k * nx * ny + c];
-  } else if (n <= kCapSmall) {
-    Key2 A[kCapSmall];
-    const int m = pass2_column(x, y, nx, poffs, pz, pd, t, t.H, t.Dx, A, kCapSmall);
+  if (n <= nslots)
+    for (int k = part; k < n; k += LANES) out[k] = slots[(size_t)k * nx * ny + c];
+  const bool again = n > nslots && n <= kCapSmall;
+  if (!__any_sync(0xffffffffu, again)) return;
+  Key2 A[kCapSmall];
+  const int m = pass2_shared_column<LANES>(again, x, y, nx, part, lane, poffs, pz, pd, t, t.H, t.Dx, A);
+  if (again && part == 0)
     for (int k = 0; k < m; ++k) out[k] = make_double2(value_of(A[k].x), value_of(A[k].y));
-  }
 }
 
 template <bool FILL>
@@ -1257,13 +1280,10 @@ int dilate(vo_ctx *ctx, int method, double R, const vo_volume *in_user, vo_volum
       if (!rc) {
         cudaMemsetAsync(ctx->d_flags, 0, 2 * sizeof(int), ctx->stream);
         cudaEventRecord(ctx->ev[4], ctx->stream);
-        if (split) {
-          const int cols = kBX / kPass2Lanes;
-          k_pass2<kPass2Lanes><<<dim3((nx + cols - 1) / cols, grd.y), blk, sh, ctx->stream>>>(
-              nx, ny, poffs, pz, pd, t, s.counts, slots, nslots, ovf);
-        } else {
-          k_pass2<1><<<grd, blk, sh, ctx->stream>>>(nx, ny, poffs, pz, pd, t, s.counts, slots, nslots, ovf);
-        }
+        const int cols = split ? kBX / kPass2Lanes : kBX;
+        const dim3 grd2((nx + cols - 1) / cols, grd.y);
+        (split ? &k_pass2<kPass2Lanes> : &k_pass2<1>)<<<grd2, blk, sh, ctx->stream>>>(nx, ny, poffs, pz, pd, t, s.counts,
+                                                                                      slots, nslots, ovf);
         k_pass2_big<false><<<gbig, kBigThreads, 0, ctx->stream>>>(nx, ny, poffs, pz, pd, t, s.counts,
                                                                  nullptr, nullptr, ovf, s.big);
         ctx->launches += 2;
@@ -1276,8 +1296,8 @@ int dilate(vo_ctx *ctx, int method, double R, const vo_volume *in_user, vo_volum
         }
         if (!rc) {
           cudaEventRecord(ctx->ev[6], ctx->stream);
-          k_pass2_place<<<grd, blk, 0, ctx->stream>>>(nx, ny, poffs, pz, pd, t, s.counts, slots, nslots, res->offs,
-                                                      res->z);
+          (split ? &k_pass2_place<kPass2Lanes> : &k_pass2_place<1>)<<<grd2, blk, 0, ctx->stream>>>(
+              nx, ny, poffs, pz, pd, t, s.counts, slots, nslots, res->offs, res->z);
           k_pass2_big<true><<<gbig, kBigThreads, 0, ctx->stream>>>(nx, ny, poffs, pz, pd, t, nullptr,
                                                                   res->offs, res->z, ovf, s.big);
           ctx->launches += 2;
