@@ -85,7 +85,7 @@ namespace vo {
 namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
-constexpr int kBins = 1024;       // bins of lower ends (a power of two; indexes are masked into range)
+constexpr int kBins = 1024;       // bins of lower ends (a power of two: bin_of masks its indexes)
 constexpr int kCoverBins = 512;   // bins of the cover: the same, or two in one for inputs that use more
 constexpr int kTile = 4;          // side of a source tile (columns), equal to the patch's height
 constexpr int kGroup = 16;        // most segments of a cluster (half a warp)
@@ -382,9 +382,16 @@ struct PatchState {
 };
 
 // Bin of a lower end: rounds lo / w to an integer (exact scaling, one
-// rounding), masked so that no value can index out of range.
+// rounding), masked below kBins so that no value, NaN included (kBins - 1), can
+// index cmap out of range. The cover has fewer bins: cover_bin_of.
 __device__ __forceinline__ unsigned bin_of(float lo, float inv_w) {
   return __float_as_uint(__fmaf_rn(lo, inv_w, 8388608.f)) & (kBins - 1);
+}
+
+// Bin of the cover for a lower end. Those of numbers lie below kCoverBins (the cover's bins are two in one
+// where the input uses more); a NaN's, which k_widths leaves out of the range, is brought there.
+__device__ __forceinline__ unsigned cover_bin_of(float lo, float inv_w, int cshift) {
+  return min(bin_of(lo, inv_w) >> cshift, (unsigned)kCoverBins - 1);
 }
 
 // New entry for bin b (uniform). False when the entries are used up.
@@ -730,7 +737,7 @@ __device__ __forceinline__ bool sweep(const FastArgs &A, const PatchMem &M, Patc
             const float h = in ? M.hrow1[max(t + kTile - 1, PX - 1 - t)] : -1.f;
             const float lo = c[i].x - h, hi = c[i].y + h;
             if (2.f * h >= S.cthr) {  // every segment of the cluster gives a long interval
-              float2 *bin = M.ml + (bin_of(lo, inv_w) >> S.cshift);
+              float2 *bin = M.ml + cover_bin_of(lo, inv_w, S.cshift);
               // values are positive: their bit patterns are ordered like them
               if (lo < bin->x) atomicMin(reinterpret_cast<int *>(&bin->x), __float_as_int(lo));
               if (hi > bin->y) atomicMax(reinterpret_cast<int *>(&bin->y), __float_as_int(hi));
