@@ -324,7 +324,7 @@ int plan_dilation_round(vo_ctx *ctx, vo_batch *b, std::vector<DilPlan> &dils, bo
     if (!rc) rc = plan_alloc(ctx, b, &d.pk.cl, entries);
     if (!rc) rc = plan_alloc(ctx, b, &d.pk.coff, pack_offsets(g));
     if (!rc) rc = plan_alloc(ctx, b, &d.pk.par, 1);
-    if (!rc) rc = plan_alloc(ctx, b, &d.mm, 3);
+    if (!rc) rc = plan_alloc(ctx, b, &d.mm, 4);
     if (!rc) rc = plan_alloc(ctx, b, &d.big_list, (size_t)ncols);
     if (rc) return rc;
     d.A = fast_args(g.nx, g.ny, *d.T, d.in.beg, d.in.end, d.in.z, d.pk);

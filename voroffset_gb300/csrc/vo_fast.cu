@@ -117,6 +117,8 @@ static_assert(kTile == kPatchY && kPatchX % kTile == 0, "tiles and patches are a
 
 // ------------------------------------------------------------ preparation
 
+constexpr long long kFarBits = 0x46293e5939a08ceall;  // magnitudes beyond this (1e30) stand outside the range
+
 // Doubles as unsigned integers of the same order (zero: below every one).
 __device__ __forceinline__ unsigned long long order_of(double v) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(v);
@@ -127,18 +129,26 @@ __device__ __forceinline__ double order_value(unsigned long long o) {
 }
 
 // The scalars of a dilation from the orders of the largest value and of the
-// largest negated value (0: there is none).
+// largest negated value (0: there is none) of magnitude up to 1e30, and from
+// whether there are others below (bit 0) and above (bit 1): infinite ones, for
+// which no base and no bin width would do. Those keep their order towards every
+// candidate of the others when they stand in FP32 at the nearest places where
+// even their own candidates of any H lie beyond all of those: 2 R and more away.
+// What is decided in FP64 uses their own values.
 // Guard band: with U bounding the magnitude of every FP32 value (relative to
 // the base), each candidate endpoint is within 1.5 ulp32(U) of its FP64 value
 // (rounding of z, of H and of the sum) and a difference of two adds one more
 // ulp32(U): at most 4 ulp32(U) = 2^-21 U. E = 2^-20 U leaves a factor of two;
 // the rounding of the FP64 endpoints themselves is below 2^-50 times the
 // largest magnitude.
-__device__ void set_par(unsigned long long a, unsigned long long b, float R, FastPar *par) {
+__device__ void set_par(unsigned long long a, unsigned long long b, unsigned far, float R, FastPar *par) {
   const double zmax = a ? order_value(a) : 0.0, zmin = b ? -order_value(b) : 0.0;
   FastPar p;
-  p.base = floor(zmin - R - 3.0);
-  const float U = (float)(zmax - p.base + R + 3.0);
+  const double q = 1.8e-15 * fmax(fabs(zmax), fabs(zmin));  // above the rounding of what follows
+  p.base = floor(far & 1 ? zmin - 2.0 * (R + 3.0 + q) : zmin - R - 3.0);
+  p.lo = far & 1 ? R + 2.f : 0.f;
+  p.hi = far & 2 ? (float)(zmax - p.base + 2.0 * (R + 3.0 + q)) : INFINITY;
+  const float U = far & 2 ? p.hi + R + 3.f : (float)(zmax - p.base + R + 3.0);
   p.E = U * 9.5367431640625e-07f + (float)(fmax(fabs(zmax), fabs(zmin)) * 8.8817841970012523e-16);
   // bin width: the power of two at or above a quarter of the radius, wide
   // enough for the range and far above the guard band
@@ -173,7 +183,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_pack(int nx, int ny, const int32
                                                      double2 *__restrict__ zx,
                                                      float4 *__restrict__ cl, int32_t *__restrict__ coff) {
   constexpr int CAP = kPackSort / WARPS;
-  __shared__ __align__(16) int s_key[WARPS][CAP];  // bit patterns of the lower ends: a total order, also of NaNs
+  __shared__ __align__(16) int s_key[WARPS][CAP];  // bit patterns of the lower ends (none is negative)
   __shared__ float s_hi[WARPS][CAP];
   __shared__ unsigned short s_ord[WARPS][CAP];  // segment of rank r
   __shared__ unsigned char s_col[WARPS][CAP];
@@ -182,6 +192,8 @@ __global__ void __launch_bounds__(32 * WARPS) k_pack(int nx, int ny, const int32
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tiles_x = (nx + kTile - 1) / kTile, T = blockIdx.x;
   const double base = par->base;
+  const float least = par->lo, most = par->hi;
+  auto in_fp32 = [=](double v) { return fminf(fmaxf(__double2float_rn(__dsub_rn(v, base)), least), most); };
   int seg0 = beg[T * kTile * nx], cl0 = seg0;  // next free segment and cluster of the tile row
   for (int t0 = 0; t0 < tiles_x; t0 += WARPS) {
     const int tx = t0 + warp;
@@ -207,8 +219,8 @@ __global__ void __launch_bounds__(32 * WARPS) k_pack(int nx, int ny, const int32
       if ((lane & 1) == 0) s_src[warp][c4] = k0 - pre;
       for (int i = lane & 1; i < n; i += 2) {
         const double2 v = z[k0 + i];
-        s_key[warp][pre + i] = __float_as_int(__double2float_rn(__dsub_rn(v.x, base)));
-        s_hi[warp][pre + i] = __double2float_rn(__dsub_rn(v.y, base));
+        s_key[warp][pre + i] = __float_as_int(in_fp32(v.x));
+        s_hi[warp][pre + i] = in_fp32(v.y);
         s_col[warp][pre + i] = (unsigned char)c4;
       }
       // padding up to the next 32: after every segment
@@ -307,7 +319,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_pack(int nx, int ny, const int32
     } else {
       for (int i = lane & 1; i < n; i += 2) {
         const double2 v = z[k0 + i];
-        const float2 f = make_float2(__double2float_rn(__dsub_rn(v.x, base)), __double2float_rn(__dsub_rn(v.y, base)));
+        const float2 f = make_float2(in_fp32(v.x), in_fp32(v.y));
         const int r = pre + i;
         zf[sb + r] = f;
         code[sb + r] = make_uint2(wide[k0 + i].x | (unsigned)c4 << 24, wide[k0 + i].y);
@@ -1201,7 +1213,7 @@ __global__ void __launch_bounds__(32, 20) k_patch(const BatchVol *__restrict__ v
 // of a row contiguous (CSR inputs are already so: SLOTS false); else the widths
 // alone, in the input's order, and the scalars of the dilation from the values'
 // range (mm, zeroed before: orders of the largest value and of the largest
-// negated value, then the blocks that are done); a pass of its own over the
+// negated value, the blocks that are done, whether values lie beyond); a pass of its own over the
 // values took 0.5 ms at 2048^2. A block per row: it loads what it needs of five
 // columns, and is bound by the latency of that (0.7 ms at 2048^2).
 template <bool SLOTS, bool RECORDS>
@@ -1214,7 +1226,9 @@ __global__ void __launch_bounds__(kPrepThreads) k_widths(int nx, int ny, const i
   __shared__ int s_sum[kPrepThreads / 32];
   const int y = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int base = SLOTS ? beg[nx * y] : 0;
-  Key top = kKeyMin, bottom = kKeyMax;  // widths alone: the values' range besides (NaN left out)
+  // widths alone: the values' range besides (NaN left out), and where there are others (set_par)
+  Key top = kKeyMin, bottom = kKeyMax;
+  unsigned far = 0;
   for (int x0 = 0; x0 < nx; x0 += kPrepThreads) {
     const int x = x0 + threadIdx.x, c = x + nx * y;
     const int k0 = x < nx ? beg[c] : 0, n = x < nx ? end[c] - k0 : 0;
@@ -1254,8 +1268,11 @@ __global__ void __launch_bounds__(kPrepThreads) k_widths(int nx, int ny, const i
       if (!RECORDS) {
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
-          const Key bits = q ? v.y : v.x, key = bits ^ ((bits >> 63) & 0x7fffffffffffffffll);
-          if ((bits & 0x7fffffffffffffffll) > 0x7ff0000000000000ll) continue;
+          const Key bits = q ? v.y : v.x, size = bits & 0x7fffffffffffffffll, key = bits ^ (bits < 0 ? 0x7fffffffffffffffll : 0);
+          if (size > kFarBits) {
+            if (size <= 0x7ff0000000000000ll) far |= bits < 0 ? 1u : 2u;
+            continue;
+          }
           top = kmax(top, key);
           bottom = kmin(bottom, key);
         }
@@ -1297,16 +1314,19 @@ __global__ void __launch_bounds__(kPrepThreads) k_widths(int nx, int ny, const i
     top = kmax(top, __shfl_xor_sync(kFull, top, o));
     bottom = kmin(bottom, __shfl_xor_sync(kFull, bottom, o));
   }
+  far = __reduce_or_sync(kFull, far);
   if (lane == 0 && top >= bottom) {
     atomicMax(&mm[0], order_of(value_of(top)));
     atomicMax(&mm[1], order_of(-value_of(bottom)));
   }
+  if (lane == 0 && far) atomicOr(&mm[3], (unsigned long long)far);
   __syncthreads();
   if (threadIdx.x) return;
   __threadfence();
   if (atomicAdd(&mm[2], 1ull) + 1 != gridDim.x) return;
   __threadfence();
-  set_par(atomicMax(&mm[0], 0ull), atomicMax(&mm[1], 0ull), R, par);  // the last block to finish
+  // the last block to finish
+  set_par(atomicMax(&mm[0], 0ull), atomicMax(&mm[1], 0ull), (unsigned)atomicOr(&mm[3], 0ull), R, par);
 }
 
 // Dilations by small radii, one thread per column: few columns are in reach, so
@@ -1664,7 +1684,7 @@ size_t pack_offsets(const vo_grid &g) {
 void fast_prepare(cudaStream_t st, const FastArgs &A, float R, double mean_segs, unsigned long long *mm,
                   const PackOut &out) {
   const double2 *z = reinterpret_cast<const double2 *>(A.zd);
-  cudaMemsetAsync(mm, 0, 3 * sizeof(unsigned long long), st);
+  cudaMemsetAsync(mm, 0, 4 * sizeof(unsigned long long), st);
   // warps per block by the segments of a tile: twice the mean should fit a warp's share of the sort
   const double most = 2.2 * mean_segs * kTile * std::min(kTile, A.ny);
   const int warps = most <= kPackSort / 32 ? 32 : most <= kPackSort / 16 ? 16 : 8;
@@ -1747,7 +1767,7 @@ int dilate_fast(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out, vo_
   unsigned char *misc = nullptr, *scratch[2] = {nullptr, nullptr};
   double2 *oz = nullptr, *big = nullptr;
   BatchVol *dv = nullptr;
-  // misc: range orders (3 x 8 bytes), FastPar at 64, counters at 128 (4 of the queue, FP64-tier columns,
+  // misc: range orders (4 x 8 bytes), FastPar at 64, counters at 128 (4 of the queue, FP64-tier columns,
   // spill used, overflow flags), the launch's BatchVol at 256, then the columns' slots; the first two
   // parts are written by one copy
   struct Head {

@@ -183,11 +183,13 @@ int slot_to_volume(vo_ctx *ctx, const SlotVol &v, vo_volume **out, const int *ex
 
 // Scalars of a dilation's FP32 arithmetic, from the range of its input
 // (set_par in vo_fast.cu): FP32 values are relative to base, E is the guard
-// band, 1 / inv_w the bin width, thr the least length of a long interval.
+// band, 1 / inv_w the bin width, thr the least length of a long interval, and
+// lo and hi bound the FP32 values (infinite ones are brought there).
 struct FastPar {
   double base;
   float E, inv_w, thr;
   int nbins;
+  float lo, hi;
 };
 
 // Columns of a warp of the FP32 kernel: a kPatchX x kPatchY patch, lane l at
@@ -294,7 +296,7 @@ size_t pack_offsets(const vo_grid &g);
 void direct_prepare(cudaStream_t st, const FastArgs &A, const PackOut &out);
 FastArgs fast_args(int nx, int ny, const DeviceTables &T, const int32_t *beg, const int32_t *end, const double2 *z,
                    const PackOut &out);
-// Packs the input of a dilation (CSR or slots in column order). mm: three words of scratch.
+// Packs the input of a dilation (CSR or slots in column order). mm: four words of scratch.
 void fast_prepare(cudaStream_t st, const FastArgs &A, float R, double mean_segs, unsigned long long *mm,
                   const PackOut &out);
 
