@@ -385,14 +385,15 @@ __device__ __forceinline__ void compact_columns(int ncols, const int32_t *__rest
   if (c - lane >= ncols) return;
   const int off = ooffs[min(c, ncols)];
   const long long from = c < ncols ? reinterpret_cast<long long>(src(c)) : 0;
-  const int first = __shfl_sync(0xffffffffu, off, 0), end = ooffs[min(c - lane + 32, ncols)];
-  for (int k0 = first; k0 < end; k0 += 32) {
-    const int k = k0 + lane;
+  // in 64 bits: totals reach 2^31 - 1, and the last turn's positions lie beyond
+  const long long first = __shfl_sync(0xffffffffu, off, 0), end = ooffs[min(c - lane + 32, ncols)];
+  for (long long k0 = first; k0 < end; k0 += 32) {
+    const long long k = k0 + lane;
     int l = 0;  // the last column that starts at or before k (of those that do, the one with segments)
     for (int o = 16; o > 0; o >>= 1)
       if (__shfl_sync(0xffffffffu, off, l + o) <= k) l += o;
     const double2 *p = reinterpret_cast<const double2 *>(__shfl_sync(0xffffffffu, from, l));
-    const int at = k - __shfl_sync(0xffffffffu, off, l);
+    const long long at = k - __shfl_sync(0xffffffffu, off, l);
     if (k < end) oz[k] = p[at];
   }
 }
