@@ -919,7 +919,9 @@ int dilate_envelope(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out,
   // Segments of the lines (pass 1) and rows (pass 2): enough to give every SM `per` of them (the warps of
   // six pass-1 blocks, three times the pass-2 blocks it holds), with at least eight times the halo that
   // each one sweeps beside its own part, so that this costs at most an eighth more steps. Whole lines
-  // remain where there are that many: 512^2, r = 16 gains (see above), 2048^2 has the lines.
+  // remain where there are that many: 512^2, r = 16 gains (see above), 2048^2 has the lines. All lines
+  // together have fewer than `per` segments per SM more than there are lines.
+  constexpr int kE1PerSm = 24, kE2PerSm = 16;
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
   auto segments = [sms](int length, int lines, int halo, int per) {
@@ -930,7 +932,7 @@ int dilate_envelope(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out,
   if (!rc) rc = dalloc(ctx, &nB, (size_t)ncols);
   if (!rc) rc = dalloc(ctx, &counts, (size_t)ncols + 1);
   if (!rc) rc = dalloc(ctx, &bcnt, (size_t)ncols + 1);
-  if (!rc) rc = dalloc(ctx, &list, (size_t)std::max(nx, ny) * (size_t)std::max(1, std::max(nx, ny) / 32 + 1));
+  if (!rc) rc = dalloc(ctx, &list, (size_t)std::max(nx, ny) + (size_t)std::max(kE1PerSm, kE2PerSm) * std::max(sms, 1));
   if (!rc) rc = dalloc(ctx, &rowp, (size_t)ny);
   if (!rc) rc = dalloc(ctx, &slots, (size_t)ncols * kE2Out);
   Key2 *gz1 = nullptr, *gz2 = nullptr;
@@ -951,7 +953,7 @@ int dilate_envelope(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out,
   E1Args a1{nx, ny, 0, ny, Dy, 0, 0, in->offs, in->z, nF, nB, nullptr, nullptr, nullptr, ctx->d_flags, list, nullptr,
             nullptr, 0};
   auto segment_lines = [&](E1Args &a) {
-    const int rows = a.yb1 - a.yb0, segs = segments(rows, nx, Dy, 24);
+    const int rows = a.yb1 - a.yb0, segs = segments(rows, nx, Dy, kE1PerSm);
     a.rows = (rows + segs - 1) / segs;
     a.segs = segs;
     return (nx * segs + kE1Warps - 1) / kE1Warps;
@@ -1053,7 +1055,7 @@ int dilate_envelope(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out,
     const int max_pieces = hflags[3];
     const int hstride = max_pieces > kE2Stage ? max_pieces + 2 : 0;
     // (whole rows then: one range per row, however large a column)
-    const int rows2 = yb1 - yb0, segs2 = hstride > 0 ? 1 : segments(nx, rows2, W - 1, 16), items2 = rows2 * segs2;
+    const int rows2 = yb1 - yb0, segs2 = hstride > 0 ? 1 : segments(nx, rows2, W - 1, kE2PerSm), items2 = rows2 * segs2;
     if (!rc && hstride > 0) rc = dalloc(ctx, &ghist, (size_t)hstride * items2);
     if (!rc) rc = dalloc(ctx, &pz, (size_t)ptotal);
     if (!rc) rc = dalloc(ctx, &pd, (size_t)ptotal);
