@@ -80,6 +80,7 @@
 #include <cuda_fp16.h>
 
 #include "vo_internal.cuh"
+#include "vo_slots.h"
 
 namespace vo {
 namespace {
@@ -1740,12 +1741,6 @@ bool direct_choice(const vo_grid &g, const DeviceTables &T, double mean_segs) {
   return cols * std::max(mean_segs, 1.0) <= kDirectWork * kPatchY / std::min(g.ny, kPatchY);
 }
 
-// Slots per column of a single dilation's output (the rest goes to the spill
-// region), from the input's mean segment count per column.
-static int slot_cap(double mean_segs) {
-  return mean_segs > 24.0 ? 64 : mean_segs > 10.0 ? 48 : mean_segs > 6.0 ? 32 : 24;
-}
-
 int dilate_fast(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out, vo_timings *tm) {
   const vo_grid g = in->grid;
   const int nx = g.nx, ny = g.ny, ncols = nx * ny;
@@ -1755,11 +1750,7 @@ int dilate_fast(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out, vo_
   const double mean_segs = (double)in->nseg / std::max(ncols, 1);
   bool direct = direct_choice(g, *T, mean_segs);
   PatchPlan P;
-  // slot indices are unsigned 32-bit: columns and spill together below 2^32
-  const int64_t most = 4294967295LL;
-  int cap = slot_cap(mean_segs);
-  cap = (int)std::max<int64_t>(1, std::min<int64_t>(cap, most / 9 * 8 / std::max(ncols, 1)));
-  int64_t spill = std::max<int64_t>(4096, (int64_t)ncols * cap / 8);
+  SlotLayout slots = slots_first(ncols, mean_segs);
   const size_t nseg = (size_t)std::max<int64_t>(in->nseg, 1);
   PackOut pk;
   int32_t *obeg = nullptr, *big_list = nullptr;
@@ -1806,7 +1797,7 @@ int dilate_fast(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out, vo_
   vo_volume *res = nullptr;
   int cols2 = 0;
   for (int attempt = 0; !rc; ++attempt) {
-    rc = dalloc(ctx, &oz, (size_t)ncols * cap + (size_t)spill);
+    rc = dalloc(ctx, &oz, (size_t)ncols * slots.cap + (size_t)slots.spill);
     if (rc) break;
     std::memset(&head, 0, sizeof head);
     BatchVol &V = head.V;
@@ -1814,10 +1805,10 @@ int dilate_fast(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out, vo_
     V.obeg = obeg;
     V.oend = obeg + ncols;
     V.oz = oz;
-    V.cap = cap;
+    V.cap = slots.cap;
     V.item1 = direct ? direct_blocks(g, ncols) : P.nitems;
-    V.spill_base = (unsigned)((int64_t)ncols * cap);
-    V.spill_cap = (unsigned)spill;
+    V.spill_base = (unsigned)((int64_t)ncols * slots.cap);
+    V.spill_cap = (unsigned)slots.spill;
     V.big_list = big_list;
     V.big_count = cnt + 4;
     V.spill_used = reinterpret_cast<unsigned *>(cnt + 5);
@@ -1838,7 +1829,7 @@ int dilate_fast(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out, vo_
     ctx->launches += direct ? 2 : 3;
     SlotVol sv;
     sv.grid = g;
-    sv.cap = cap;
+    sv.cap = slots.cap;
     sv.beg = obeg;
     sv.end = obeg + ncols;
     sv.z = oz;
@@ -1876,8 +1867,7 @@ int dilate_fast(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out, vo_
       res = nullptr;
       dfree(ctx, oz);
       oz = nullptr;
-      spill = (int64_t)(unsigned)hc[5] + 4096;
-      if (attempt >= 2 || (int64_t)ncols * cap + spill > most)
+      if (attempt >= 2 || !slots_next(ncols, (int64_t)(unsigned)hc[5], slots))
         rc = set_error(ctx, VO_ERANGE, "dilation: the result exceeds the slot range");
       continue;
     }
