@@ -174,7 +174,7 @@ typedef struct {
   int32_t reruns;       /* volumes re-run by the last vo_batch_run */
   int32_t rerun_first;  /* index of the first of them (-1: none) */
   int32_t rerun_cause;  /* its overflow flags: 1 union beyond the FP64 list, 2 complement slot, 4 spill exhausted,
-                           8 union beyond the list of the small-radius kernel */
+                           8 more unions beyond the kernels' lists than a replay takes */
   double spill_peak;    /* largest fraction of a dilation's spill region used by the last run (> 1: exhausted) */
   int32_t spill_peak_round; /* its dilation round */
   double plan_ms;       /* host time of vo_batch_create */

@@ -94,6 +94,16 @@ int build_tables(double R, int kmax, Tables &t) {
   return VO_OK;
 }
 
+int column_tables(vo_ctx *ctx, const DeviceTables *T) {
+  if (T->prec) return VO_OK;
+  DeviceTables *d = const_cast<DeviceTables *>(T);  // a cached entry of the context
+  const std::vector<float4> pairs = column_pairs(d->host, d->dom);
+  VO_CK(ctx, cudaMalloc(&d->prec, sizeof(float4) * pairs.size()));
+  d->npairs = (int)pairs.size();
+  VO_CK(ctx, cudaMemcpy(d->prec, pairs.data(), sizeof(float4) * pairs.size(), cudaMemcpyHostToDevice));
+  return VO_OK;
+}
+
 int get_tables(vo_ctx *ctx, double R, int kmax, const DeviceTables **out) {
   for (DeviceTables *d : ctx->tables)
     if (d->R == R && d->kmax >= kmax) {
@@ -142,6 +152,7 @@ int get_tables(vo_ctx *ctx, double R, int kmax, const DeviceTables **out) {
     cudaFree(old->Hp);
     cudaFree(old->Dx);
     cudaFree(old->HB);
+    cudaFree(old->prec);
     delete old;
     ctx->tables.erase(ctx->tables.begin());
   }
@@ -262,6 +273,7 @@ void vo_destroy(vo_ctx *ctx) {
     cudaFree(d->Hp);
     cudaFree(d->Dx);
     cudaFree(d->HB);
+    cudaFree(d->prec);
     delete d;
   }
   for (auto &e : ctx->ev)

@@ -61,6 +61,10 @@ std::vector<StepKind> steps_of(int op) {
 
 using Launch = std::function<void(cudaStream_t)>;
 
+// Counters of a dilation: spill space used, FP64-tier columns, columns for k_column_list, patches listed, large unions.
+constexpr int kDilCounters = 5;
+constexpr int kRoundCounters = 5;  // of a round before them: four of the patch queue, lists of the pool taken
+
 struct DilPlan {
   int vol = 0;
   SlotVol in, out;
@@ -69,14 +73,17 @@ struct DilPlan {
   PackOut pk;
   unsigned long long *mm = nullptr;
   int *big_list = nullptr;
-  int *counters = nullptr;  // spill used, third-tier columns (zeroed before every replay)
+  int *counters = nullptr;  // kDilCounters of them (zeroed before every replay)
   int32_t *tcap = nullptr, *toff = nullptr;
   int tiles32_x = 0, tiles32 = 0;
   std::vector<float> tile_work;  // predicted candidates per column of each sizing tile
   int spill_base = 0, spill_cap = 0;
   double cost = 0;  // mean candidates per column (no sizer)
   double mean_segs = 0;
-  bool direct = false;  // small radius, small columns: k_direct
+  Engine engine = Engine::kPatches;
+  ColumnPrep cp;  // kColumns
+  ColumnArgs C{};
+  int *over_list = nullptr;
   int64_t slot_entries = 0;
 };
 
@@ -98,8 +105,8 @@ struct vo_batch {
   double2 *big_scratch = nullptr;  // working lists of the FP64 tier
   unsigned char *scratch[2] = {nullptr, nullptr};  // working memory of the patch kernel's tiers
   size_t scratch_bytes[2] = {0, 0};
-  // Per dilation round: its counters (4, then 2 per dilation: spill space used, FP64-tier columns) and
-  // the dilations' spill capacities.
+  // Per dilation round: its counters (kRoundCounters, then kDilCounters per dilation) and the dilations' spill
+  // capacities.
   struct Round {
     const int *counters;
     std::vector<int> caps;
@@ -233,6 +240,11 @@ BatchVol batch_vol(const DilPlan &d, int *ovf) {
   v.spill_used = reinterpret_cast<unsigned *>(d.counters);
   v.big_list = d.big_list;
   v.big_count = d.counters + 1;
+  v.over_list = d.over_list;
+  v.over_count = d.counters + 2;
+  v.listed = d.engine == Engine::kDirect ? v.big_count : d.counters + 3;
+  v.most = d.engine == Engine::kDirect ? kFewColumns : kFewPatches;
+  v.large = d.counters + 4;
   v.ovf = ovf;
   return v;
 }
@@ -256,10 +268,6 @@ int sm_count() {
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   return sms > 0 ? sms : 1;
 }
-
-// Largest column of an input up to which its dilation may go column by column:
-// a union beyond that kernel's list re-runs the volume at every replay.
-constexpr int kDirectColumn = 16;
 
 // Autotuner: rounds of kTuneFrom to kTuneTo patches per SM lie where one lane
 // per column (throughput) and four (the longest patch's latency) cross, at a
@@ -295,6 +303,22 @@ int tune_split(vo_ctx *ctx, vo_batch *b, const std::vector<DilPlan> &dils, int64
   return VO_OK;
 }
 
+// Order of a round's dilations in its launches.
+int launch_order(Engine e) { return e == Engine::kPatches ? 0 : e == Engine::kColumns ? 1 : 2; }
+
+// The pair records of plan-owned tables (the context's own entry may be evicted).
+int plan_column_tables(vo_ctx *ctx, vo_batch *b, const DeviceTables *T) {
+  if (T->prec) return VO_OK;
+  DeviceTables *own = const_cast<DeviceTables *>(T);
+  const std::vector<float4> pairs = column_pairs(T->host, own->dom);
+  int rc = plan_alloc(ctx, b, &own->prec, pairs.size());
+  if (rc) return rc;
+  own->npairs = (int)pairs.size();
+  cudaMemcpyAsync(own->prec, pairs.data(), sizeof(float4) * pairs.size(), cudaMemcpyHostToDevice, ctx->stream);
+  VO_CK(ctx, cudaStreamSynchronize(ctx->stream));
+  return VO_OK;
+}
+
 int plan_dilation_round(vo_ctx *ctx, vo_batch *b, std::vector<DilPlan> &dils, bool later_rounds) {
   int rc = VO_OK;
   for (DilPlan &d : dils) {
@@ -306,8 +330,10 @@ int plan_dilation_round(vo_ctx *ctx, vo_batch *b, std::vector<DilPlan> &dils, bo
     const float R = (float)b->radii[d.vol];
     // candidates per column: lattice points of the disc x mean segments of the input (no sizer)
     d.cost = 3.14159 * (R + 0.5) * (R + 0.5) * (d.mean_segs + 0.5);
-    d.direct = (d.in.owns || d.in.end == d.in.beg + 1) && d.in.cap <= kDirectColumn && direct_choice(g, *d.T, d.mean_segs);
-    if (d.direct) {
+    d.engine = (d.in.owns || d.in.end == d.in.beg + 1) && direct_choice(g, *d.T, d.mean_segs) ? Engine::kDirect : Engine::kPatches;
+    if (!rc) rc = plan_alloc(ctx, b, &d.big_list, (size_t)ncols);
+    if (rc) return rc;
+    if (d.engine == Engine::kDirect) {
       rc = plan_alloc(ctx, b, &d.pk.rec, entries);
       if (!rc && d.in.owns) rc = plan_alloc(ctx, b, &d.pk.zx, entries);
       if (!rc && d.in.owns) rc = plan_alloc(ctx, b, &d.pk.rbeg, 2 * (size_t)ncols);
@@ -315,6 +341,23 @@ int plan_dilation_round(vo_ctx *ctx, vo_batch *b, std::vector<DilPlan> &dils, bo
       d.A = fast_args(g.nx, g.ny, *d.T, d.in.beg, d.in.end, d.in.z, d.pk);
       const DilPlan c = d;
       record(b, 1, [c](cudaStream_t st) { direct_prepare(st, c.A, c.pk); });
+      continue;
+    }
+    if (d.engine == Engine::kColumns) {
+      rc = plan_column_tables(ctx, b, d.T);
+      auto take = [&](void **p, size_t bytes) {
+        unsigned char *q = nullptr;
+        const int r = plan_alloc(ctx, b, &q, bytes);
+        *p = q;
+        return r;
+      };
+      if (!rc) rc = column_alloc(g, entries, d.mean_segs, take, d.cp);
+      if (!rc) rc = plan_alloc(ctx, b, &d.over_list, (size_t)ncols);
+      if (rc) return rc;
+      d.A = fast_args(g.nx, g.ny, *d.T, d.in.beg, d.in.end, d.in.z, d.pk);
+      d.C = column_args(g.nx, g.ny, *d.T, d.in.beg, d.in.end, d.in.z, d.cp);
+      const DilPlan c = d;
+      record(b, 3, [c, R](cudaStream_t st) { column_prepare(st, c.C, R, c.T->dom, c.cp); });
       continue;
     }
     rc = plan_alloc(ctx, b, &d.pk.zf, entries);
@@ -325,7 +368,6 @@ int plan_dilation_round(vo_ctx *ctx, vo_batch *b, std::vector<DilPlan> &dils, bo
     if (!rc) rc = plan_alloc(ctx, b, &d.pk.coff, pack_offsets(g));
     if (!rc) rc = plan_alloc(ctx, b, &d.pk.par, 1);
     if (!rc) rc = plan_alloc(ctx, b, &d.mm, 4);
-    if (!rc) rc = plan_alloc(ctx, b, &d.big_list, (size_t)ncols);
     if (rc) return rc;
     d.A = fast_args(g.nx, g.ny, *d.T, d.in.beg, d.in.end, d.in.z, d.pk);
     const DilPlan c = d;
@@ -333,11 +375,11 @@ int plan_dilation_round(vo_ctx *ctx, vo_batch *b, std::vector<DilPlan> &dils, bo
   }
   if (ctx->sizer) run_pending(ctx, b);  // features need the dilation inputs
   int *counters = nullptr;
-  rc = plan_alloc(ctx, b, &counters, 4 + 2 * dils.size());
+  rc = plan_alloc(ctx, b, &counters, kRoundCounters + kDilCounters * dils.size());
   if (rc) return rc;
   for (size_t i = 0; i < dils.size(); ++i) {
     DilPlan &d = dils[i];
-    d.counters = counters + 4 + 2 * i;
+    d.counters = counters + kRoundCounters + kDilCounters * i;
     rc = size_output(ctx, b, d, b->radii[d.vol]);
     if (rc) return rc;
     b->stats.slot_bytes += d.slot_entries * (int64_t)sizeof(double2);
@@ -349,48 +391,71 @@ int plan_dilation_round(vo_ctx *ctx, vo_batch *b, std::vector<DilPlan> &dils, bo
   std::stable_sort(order.begin(), order.end(), [](const std::pair<double, int> &x, const std::pair<double, int> &y) {
     return x.first > y.first;
   });
-  // those by patches first
-  std::stable_partition(order.begin(), order.end(), [&](const std::pair<double, int> &x) { return !dils[x.second].direct; });
-  int np = 0;
+  // those by patches first, then those by columns
+  std::stable_sort(order.begin(), order.end(), [&](const std::pair<double, int> &x, const std::pair<double, int> &y) {
+    return launch_order(dils[x.second].engine) < launch_order(dils[y.second].engine);
+  });
+  int np = 0, nc = 0, slots = 0;
   int64_t direct_cols = 0;
   size_t direct_shared = 0;
   for (const DilPlan &d : dils) {
-    np += !d.direct;
-    if (d.direct) direct_cols += (int64_t)d.in.grid.nx * d.in.grid.ny;
-    if (d.direct) direct_shared = std::max(direct_shared, direct_smem(d.A));
+    if (d.engine == Engine::kDirect) {
+      direct_cols += (int64_t)d.in.grid.nx * d.in.grid.ny;
+      direct_shared = std::max(direct_shared, direct_smem(d.A));
+    } else if (d.engine == Engine::kColumns) {
+      ++nc;
+      slots = std::max(slots, column_slots(d.mean_segs));
+    } else {
+      ++np;
+    }
   }
-  const int nd = (int)dils.size() - np;
-  if (np > 0 && !b->big_scratch) rc = plan_alloc(ctx, b, &b->big_scratch, big_scratch_elems());
+  // FP64 lists: of the last tier's threads, or of k_direct's columns (a union beyond kPoolCap runs the volume again)
+  const int nd = (int)dils.size() - np - nc, big_grid = big_blocks(1 << 30);
+  const size_t big_elems = std::max(big_scratch_elems(big_grid, kPoolCap), (size_t)kFewColumns * kPoolCap);
+  if (!b->big_scratch) rc = plan_alloc(ctx, b, &b->big_scratch, big_elems);
+  ColumnArgs *dcolumns = nullptr;
+  if (!rc && nc > 0) rc = plan_alloc(ctx, b, &dcolumns, (size_t)nc);
   if (rc) return rc;
-  const size_t counter_bytes = sizeof(int) * (4 + 2 * dils.size());
+  const size_t counter_bytes = sizeof(int) * (kRoundCounters + kDilCounters * dils.size());
   double2 *big_scratch = b->big_scratch;
   // the round's launch with `split` lanes per column
   struct RoundLaunch {
     PatchPlan P;
-    BatchVol *dvols = nullptr;  // those by patches, then the direct ones
-    int direct_items = 0;
+    BatchVol *dvols = nullptr;  // in the order above
+    int column_items = 0, direct_items = 0;
+    ColumnArgs column{};  // of the first dilation by columns
   };
   auto prepare = [&](int split, RoundLaunch &L) -> int {
     std::vector<BatchVol> hv;
-    int64_t items = 0;
+    std::vector<ColumnArgs> hc;
+    int64_t items = 0, column_items = 0;
     int hs = 0;
     for (const auto &o : order) {
       const DilPlan &d = dils[o.second];
       BatchVol v = batch_vol(d, b->d_flags + d.vol);
-      if (d.direct) {
+      if (d.engine == Engine::kDirect) {
         v.item0 = L.direct_items;
         L.direct_items += direct_blocks(d.in.grid, direct_cols);
         v.item1 = L.direct_items;
-        hv.push_back(v);
-        continue;
+        v.pool = big_scratch;
+        v.pool_used = counters + 4;
+      } else if (d.engine == Engine::kColumns) {
+        v.item0 = (int)column_items;
+        column_items += patch_count(d.in.grid, 1);
+        v.item1 = (int)column_items;
+        v.column = dcolumns + hc.size();
+        hc.push_back(d.C);
+      } else {
+        v.item0 = (int)items;
+        items += patch_count(d.in.grid, split);
+        v.item1 = (int)items;
+        hs = std::max(hs, d.T->host.hs);
       }
-      v.item0 = (int)items;
-      items += patch_count(d.in.grid, split);
-      if (items > 2147483647LL) return set_error(ctx, VO_ERANGE, "batch: too many columns");
-      v.item1 = (int)items;
+      if (items > 2147483647LL || column_items > 2147483647LL) return set_error(ctx, VO_ERANGE, "batch: too many columns");
       hv.push_back(v);
-      hs = std::max(hs, d.T->host.hs);
     }
+    L.column_items = (int)column_items;
+    if (nc > 0) L.column = hc[0];
     int r = plan_alloc(ctx, b, &L.dvols, hv.size());
     int *list = nullptr;
     if (!r && np > 0) r = patch_plan(ctx, (int)items, split, hs, L.P);
@@ -407,22 +472,26 @@ int plan_dilation_round(vo_ctx *ctx, vo_batch *b, std::vector<DilPlan> &dils, bo
     if (r) return r;
     L.P.Q = PatchQueue{counters, list};
     cudaMemcpyAsync(L.dvols, hv.data(), sizeof(BatchVol) * hv.size(), cudaMemcpyHostToDevice, ctx->stream);
+    if (nc > 0) cudaMemcpyAsync(dcolumns, hc.data(), sizeof(ColumnArgs) * hc.size(), cudaMemcpyHostToDevice, ctx->stream);
     VO_CK(ctx, cudaStreamSynchronize(ctx->stream));
     return VO_OK;
   };
-  auto launch = [counters, counter_bytes, np, nd, direct_cols, direct_shared, big_scratch](const RoundLaunch &L,
-                                                                                           cudaStream_t st) {
+  auto launch = [=](const RoundLaunch &L, cudaStream_t st) {
     cudaMemsetAsync(counters, 0, counter_bytes, st);
     if (np > 0) {
       patch_launch(false, L.P, st, L.dvols);
       patch_launch(true, L.P, st, L.dvols);
-      big_launch(st, L.dvols, np, big_scratch);
     }
-    if (nd > 0) direct_launch(st, L.dvols + np, nd, L.direct_items, direct_cols, direct_shared);
+    if (nc > 0) {
+      column_launch(st, L.dvols + np, nc, L.column_items, slots, L.column);
+      column_list_launch(st, L.dvols + np, nc);
+    }
+    if (np + nc > 0) big_launch(st, L.dvols, np + nc, big_scratch, big_grid, kPoolCap);
+    if (nd > 0) direct_launch(st, L.dvols + np + nc, nd, L.direct_items, direct_cols, direct_shared);
   };
   std::vector<const vo_grid *> grids;
   for (const DilPlan &d : dils)
-    if (!d.direct) grids.push_back(&d.in.grid);
+    if (d.engine == Engine::kPatches) grids.push_back(&d.in.grid);
   int split = patch_split(grids.data(), (int)grids.size());
   RoundLaunch L;
   const int64_t patches = patch_total(grids.data(), (int)grids.size());
@@ -448,14 +517,14 @@ int plan_dilation_round(vo_ctx *ctx, vo_batch *b, std::vector<DilPlan> &dils, bo
     if (!rc) rc = prepare(split, L);
   }
   if (rc) return rc;
-  record(b, (np > 0 ? 3 : 0) + (nd > 0 ? 1 : 0), [launch, L](cudaStream_t st) { launch(L, st); });
+  record(b, (np > 0 ? 2 : 0) + (nc > 0 ? 2 : 0) + (np + nc > 0 ? 1 : 0) + (nd > 0 ? 1 : 0), [launch, L](cudaStream_t st) { launch(L, st); });
   b->rounds.push_back({counters, {}});
   for (const DilPlan &d : dils) b->rounds.back().caps.push_back(d.spill_cap);
   b->stats.tile_rows = split;
   b->stats.union_cap = kUnionCapMid / 2;
   b->stats.persistent = 1;
   b->stats.regs = 96;
-  b->stats.tiles += L.P.nitems + L.direct_items;
+  b->stats.tiles += L.P.nitems + L.column_items + L.direct_items;
   if (later_rounds) run_pending(ctx, b);
   return VO_OK;
 }
@@ -704,7 +773,7 @@ int vo_batch_run(vo_ctx *ctx, vo_batch *b, vo_timings *tm) {
   cudaEventRecord(ctx->ev[1], ctx->stream);
   cudaMemcpyAsync(flags.data(), b->d_flags, sizeof(int) * (n + 1), cudaMemcpyDeviceToHost, ctx->stream);
   for (const vo_batch::Round &r : b->rounds) {
-    counters.emplace_back(4 + 2 * r.caps.size());
+    counters.emplace_back(kRoundCounters + kDilCounters * r.caps.size());
     cudaMemcpyAsync(counters.back().data(), r.counters, sizeof(int) * counters.back().size(), cudaMemcpyDeviceToHost,
                     ctx->stream);
   }
@@ -717,7 +786,7 @@ int vo_batch_run(vo_ctx *ctx, vo_batch *b, vo_timings *tm) {
   for (size_t r = 0; r < b->rounds.size(); ++r)
     for (size_t i = 0; i < b->rounds[r].caps.size(); ++i) {
       const int cap = b->rounds[r].caps[i];
-      const double f = cap > 0 ? (double)counters[r][4 + 2 * i] / cap : 0.0;
+      const double f = cap > 0 ? (double)counters[r][kRoundCounters + kDilCounters * i] / cap : 0.0;
       if (f > b->stats.spill_peak) {
         b->stats.spill_peak = f;
         b->stats.spill_peak_round = (int)r;

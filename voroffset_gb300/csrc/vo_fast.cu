@@ -68,9 +68,12 @@
 // Small radii take another way (k_direct).
 //
 // Capacities: a patch that needs more entries, kept-aside intervals or union
-// intervals than the launch has re-runs with larger lists (second tier), and a
-// column that outgrows those too goes to an FP64 kernel with an 8,192-interval
-// list.
+// intervals than the launch has re-runs with larger lists (second tier), if those
+// are few; if they are many their columns go to the columns kernel
+// (vo_column.cu), and if they are most, all of the dilation does: patches of
+// scattered short intervals spend their time on intervals kept aside. A column
+// that outgrows the larger lists too goes to an FP64 kernel with an
+// 8,192-interval list.
 #include <algorithm>
 #include <cmath>
 #include <cstddef>
@@ -80,13 +83,13 @@
 #include <cuda_fp16.h>
 
 #include "vo_internal.cuh"
+#include "vo_range.cuh"
 #include "vo_slots.h"
 
 namespace vo {
 namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
-constexpr int kBins = 1024;       // bins of lower ends (a power of two: bin_of masks its indexes)
 constexpr int kCoverBins = 512;   // bins of the cover: the same, or two in one for inputs that use more
 constexpr int kTile = 4;          // side of a source tile (columns), equal to the patch's height
 constexpr int kGroup = 16;        // most segments of a cluster (half a warp)
@@ -112,57 +115,10 @@ constexpr int kHot = 2;           // intervals that each candidate is compared w
 constexpr int kDirectCap = 48;    // union intervals per column there
 constexpr int kBigCap = 8192;     // last tier (FP64): intervals of a column's working list
 constexpr int kBigThreads = 32;
-constexpr int kBigBlocks = 16;      // last tier: blocks
 constexpr int kPatchBigBlocks = 76; // second tier: warps
 static_assert(kTile == kPatchY && kPatchX % kTile == 0, "tiles and patches are aligned to each other");
 
 // ------------------------------------------------------------ preparation
-
-constexpr long long kFarBits = 0x46293e5939a08ceall;  // magnitudes beyond this (1e30) stand outside the range
-
-// Doubles as unsigned integers of the same order (zero: below every one).
-__device__ __forceinline__ unsigned long long order_of(double v) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
-  return b >> 63 ? ~b : b | 0x8000000000000000ull;
-}
-__device__ __forceinline__ double order_value(unsigned long long o) {
-  return __longlong_as_double((long long)(o >> 63 ? o & 0x7fffffffffffffffull : ~o));
-}
-
-// The scalars of a dilation from the orders of the largest value and of the
-// largest negated value (0: there is none) of magnitude up to 1e30, and from
-// whether there are others below (bit 0) and above (bit 1): infinite ones, for
-// which no base and no bin width would do. Those keep their order towards every
-// candidate of the others when they stand in FP32 at the nearest places where
-// even their own candidates of any H lie beyond all of those: 2 R and more away.
-// What is decided in FP64 uses their own values.
-// Guard band: with U bounding the magnitude of every FP32 value (relative to
-// the base), each candidate endpoint is within 1.5 ulp32(U) of its FP64 value
-// (rounding of z, of H and of the sum) and a difference of two adds one more
-// ulp32(U): at most 4 ulp32(U) = 2^-21 U. E = 2^-20 U leaves a factor of two;
-// the rounding of the FP64 endpoints themselves is below 2^-50 times the
-// largest magnitude.
-__device__ void set_par(unsigned long long a, unsigned long long b, unsigned far, float R, FastPar *par) {
-  const double zmax = a ? order_value(a) : 0.0, zmin = b ? -order_value(b) : 0.0;
-  FastPar p;
-  const double q = 1.8e-15 * fmax(fabs(zmax), fabs(zmin));  // above the rounding of what follows
-  p.base = floor(far & 1 ? zmin - 2.0 * (R + 3.0 + q) : zmin - R - 3.0);
-  p.lo = far & 1 ? R + 2.f : 0.f;
-  p.hi = far & 2 ? (float)(zmax - p.base + 2.0 * (R + 3.0 + q)) : INFINITY;
-  const float U = far & 2 ? p.hi + R + 3.f : (float)(zmax - p.base + R + 3.0);
-  p.E = U * 9.5367431640625e-07f + (float)(fmax(fabs(zmax), fabs(zmin)) * 8.8817841970012523e-16);
-  // bin width: the power of two at or above a quarter of the radius, wide
-  // enough for the range and far above the guard band
-  const float w0 = fmaxf(fmaxf(U / (float)(kBins - 8), 0.25f * R), fmaxf(64.f * p.E, 1e-20f));
-  int e;
-  const float m = frexpf(fminf(w0, 1e30f), &e);
-  if (m == 0.5f) --e;
-  const float w = ldexpf(1.f, e);
-  p.inv_w = ldexpf(1.f, -e);
-  p.thr = w + 4.f * p.E;
-  p.nbins = (int)fminf((float)kBins, U * p.inv_w + 3.f);
-  *par = p;
-}
 
 // Packs the segments by 4 x 4 tiles of columns into clusters: runs of at most
 // kGroup segments, in order of their lower ends, whose union is one interval
@@ -1063,32 +1019,6 @@ __device__ __forceinline__ int patch_union(const FastArgs &A, const PatchMem &M,
   return bad ? -2 : n;
 }
 
-// Output slot of column (x, y) for an n-interval union: the column's own slot
-// when its capacity allows, else spill space, else false (the dilation's
-// overflow flag is then set). Slot indices are unsigned 32-bit.
-__device__ __forceinline__ bool place_union(const BatchVol &V, int x, int y, int n, unsigned &dst) {
-  const int nx = V.A.nx;
-  int cap = V.cap;
-  if (V.tcap) {
-    const int tx = x / kSizerTile, ty = y / kSizerTile, t = tx + V.tiles32_x * ty;
-    const int w = min(kSizerTile, nx - tx * kSizerTile);
-    cap = V.tcap[t];
-    dst = (unsigned)V.toff[t] + (unsigned)(((x - tx * kSizerTile) + w * (y - ty * kSizerTile)) * cap);
-  } else {
-    dst = (unsigned)(x + nx * y) * (unsigned)cap;
-  }
-  if (n > cap) {
-    const unsigned off = atomicAdd(V.spill_used, (unsigned)n);
-    if (off + (unsigned)n <= V.spill_cap) {
-      dst = V.spill_base + off;
-      return true;
-    }
-    atomicOr(V.ovf, 4);  // spill region exhausted
-    return false;
-  }
-  return true;
-}
-
 // Persistent: a warp per block takes patches of the launch's dilations from a
 // queue (dilations in the order of vols; each one's patches in bands of 512
 // columns, all rows of a band before the next, so that the patches in flight
@@ -1167,14 +1097,21 @@ __global__ void __launch_bounds__(32, 20) k_patch(const BatchVol *__restrict__ v
     S.E = par->E;
     S.inv_w = par->inv_w;
     S.thr = par->thr;
-    const int n = patch_union<G>(V.A, M, S, par->nbins);
+    // beyond `most` listed patches the dilation is left undone (one lane looks: the answer may change meanwhile)
+    const bool undone = __shfl_sync(kFull, S.lane == 0 && *(volatile int *)V.listed > V.most ? 1 : 0, 0);
+    if (BIG && undone) {
+      if (S.lane == 0) atomicOr(V.ovf, 8);
+      continue;
+    }
+    const int n = undone ? -1 : patch_union<G>(V.A, M, S, par->nbins);
     const int x = S.X0 + S.lx, y = S.Y0 + S.ly;
     const bool in = S.g == 0 && x < nx && y < ny;
     const bool over = __any_sync(kFull, n == -1);
     if (over && !BIG) {  // the whole patch goes to the next tier
       const int cols = __popc(__ballot_sync(kFull, in));
       if (S.lane == 0) {
-        Q.list[atomicAdd(&Q.count[1], 1)] = item;
+        atomicAdd(V.listed, 1);
+        if (!undone) Q.list[atomicAdd(&Q.count[1], 1)] = item;
         atomicAdd(&Q.count[3], cols);
       }
       if (in) V.obeg[x + nx * y] = V.oend[x + nx * y] = 0;
@@ -1199,6 +1136,70 @@ __global__ void __launch_bounds__(32, 20) k_patch(const BatchVol *__restrict__ v
     }
     __syncwarp();
   }
+}
+
+// ------------------------------------------------------------ FP64 lists
+
+// Inserts [lo, hi] into the sorted list L of n disjoint closed intervals.
+__device__ bool big_insert(double2 *L, int &n, int cap, double lo, double hi) {
+  int l = 0, r = n;
+  while (l < r) {
+    const int m = (l + r) >> 1;
+    if (L[m].y >= lo)
+      r = m;
+    else
+      l = m + 1;
+  }
+  const int i = l;
+  if (i == n || L[i].x > hi) {
+    if (n >= cap) return false;
+    for (int k = n; k > i; --k) L[k] = L[k - 1];
+    L[i] = make_double2(lo, hi);
+    ++n;
+    return true;
+  }
+  int j = i;
+  while (j + 1 < n && L[j + 1].x <= hi) ++j;
+  L[i] = make_double2(L[i].x < lo ? L[i].x : lo, L[j].y > hi ? L[j].y : hi);
+  if (j > i) {
+    const int sh = j - i;
+    for (int k = i + 1; k + sh < n; ++k) L[k] = L[k + sh];
+    n -= sh;
+  }
+  return true;
+}
+
+// A column's union in a list of `cap` intervals: their count, or -1 beyond it.
+// Source columns come ring by ring from the column's own outwards: the nearest
+// give the longest intervals, in which most of the others then lie (row by row,
+// the list holds far more intervals on the way: scattered segments, 256^2
+// columns, 12 of them each over 30000, radius 16: 5.2 s against 1.7).
+__device__ __noinline__ int big_union(const FastArgs &A, int x, int y, double2 *L, int cap) {
+  // (copies: the list's stores would have the members loaded again after each)
+  const int nx = A.nx, ny = A.ny, W = A.W, Dy = A.Dy;
+  const int32_t *__restrict__ beg = A.beg, *__restrict__ end = A.end;
+  const double2 *__restrict__ z = reinterpret_cast<const double2 *>(A.zd);
+  const double *__restrict__ H = A.H64;
+  const int *__restrict__ Dx = A.Dx;
+  int n = 0;
+  bool ok = true;
+  auto column = [&](int d, int a) {
+    if (d > Dy || a > Dx[d]) return;
+    const double h = H[d * W + a];
+    for (int s = 0; s < 4; ++s) {
+      if (((s & 1) && a == 0) || ((s & 2) && d == 0)) continue;
+      const int xs = s & 1 ? x + a : x - a, ys = s & 2 ? y + d : y - d;
+      if (xs < 0 || xs >= nx || ys < 0 || ys >= ny) continue;
+      const int cs = xs + nx * ys;
+      for (int k = beg[cs], e = end[cs]; k < e && ok; ++k) {
+        const double2 v = z[k];
+        ok = big_insert(L, n, cap, __dsub_rn(v.x, h), __dadd_rn(v.y, h));
+      }
+    }
+  };
+  for (int ring = 0; ring < max(Dy + 1, W) && ok; ++ring)
+    for (int i = 0; i < 2 * ring + 1 && ok; ++i) column(min(i, ring), min(ring, 2 * ring - i));
+  return ok ? n : -1;
 }
 
 // ------------------------------------------------------------ small radii
@@ -1227,9 +1228,7 @@ __global__ void __launch_bounds__(kPrepThreads) k_widths(int nx, int ny, const i
   __shared__ int s_sum[kPrepThreads / 32];
   const int y = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int base = SLOTS ? beg[nx * y] : 0;
-  // widths alone: the values' range besides (NaN left out), and where there are others (set_par)
-  Key top = kKeyMin, bottom = kKeyMax;
-  unsigned far = 0;
+  ValueRange range;  // widths alone: the values' range besides
   for (int x0 = 0; x0 < nx; x0 += kPrepThreads) {
     const int x = x0 + threadIdx.x, c = x + nx * y;
     const int k0 = x < nx ? beg[c] : 0, n = x < nx ? end[c] - k0 : 0;
@@ -1267,16 +1266,8 @@ __global__ void __launch_bounds__(kPrepThreads) k_widths(int nx, int ny, const i
     for (int k = 0; k < n; ++k) {
       const longlong2 v = z[k0 + k];
       if (!RECORDS) {
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          const Key bits = q ? v.y : v.x, size = bits & 0x7fffffffffffffffll, key = bits ^ (bits < 0 ? 0x7fffffffffffffffll : 0);
-          if (size > kFarBits) {
-            if (size <= 0x7ff0000000000000ll) far |= bits < 0 ? 1u : 2u;
-            continue;
-          }
-          top = kmax(top, key);
-          bottom = kmin(bottom, key);
-        }
+        range.take(v.x);
+        range.take(v.y);
       }
       const float lo = trunc32_bits(v.x), hi = trunc32_bits(v.y);
       unsigned w[4];
@@ -1310,24 +1301,29 @@ __global__ void __launch_bounds__(kPrepThreads) k_widths(int nx, int ny, const i
       if (SLOTS) rz[out + k] = v;
     }
   }
-  if (RECORDS) return;
-  for (int o = 16; o > 0; o >>= 1) {
-    top = kmax(top, __shfl_xor_sync(kFull, top, o));
-    bottom = kmin(bottom, __shfl_xor_sync(kFull, bottom, o));
+  if (!RECORDS) range.finish(mm, R, par);
+}
+
+// A column beyond k_direct's list: for the caller's last tier, or, with a pool of FP64 lists, here and now.
+__device__ __noinline__ void beyond_list(const BatchVol &V, int x, int y) {
+  const int c = x + V.A.nx * y, i = atomicAdd(V.big_count, 1);
+  int n = 0;
+  unsigned dst = 0;
+  if (!V.pool) {
+    V.big_list[i] = c;
+  } else {
+    const int slot = atomicAdd(V.pool_used, 1);
+    double2 *L = V.pool + (size_t)slot * kPoolCap;
+    n = slot < kFewColumns ? big_union(V.A, x, y, L, kPoolCap) : -1;
+    if (n < 0 || !place_union(V, x, y, n, dst)) {
+      if (n < 0) atomicOr(V.ovf, 8);
+      n = 0;
+      dst = 0;
+    }
+    for (int k = 0; k < n; ++k) V.oz[dst + k] = L[k];
   }
-  far = __reduce_or_sync(kFull, far);
-  if (lane == 0 && top >= bottom) {
-    atomicMax(&mm[0], order_of(value_of(top)));
-    atomicMax(&mm[1], order_of(-value_of(bottom)));
-  }
-  if (lane == 0 && far) atomicOr(&mm[3], (unsigned long long)far);
-  __syncthreads();
-  if (threadIdx.x) return;
-  __threadfence();
-  if (atomicAdd(&mm[2], 1ull) + 1 != gridDim.x) return;
-  __threadfence();
-  // the last block to finish
-  set_par(atomicMax(&mm[0], 0ull), atomicMax(&mm[1], 0ull), (unsigned)atomicOr(&mm[3], 0ull), R, par);
+  V.obeg[c] = (int32_t)dst;
+  V.oend[c] = (int32_t)(dst + (unsigned)n);
 }
 
 // Dilations by small radii, one thread per column: few columns are in reach, so
@@ -1359,8 +1355,9 @@ __global__ void __launch_bounds__(kPrepThreads) k_widths(int nx, int ny, const i
 // 580 candidates per column: the line of direct_choice is 450. (In FP64
 // throughout, without the neighbours' test, 1024^2 took 0.53, 1.1 and 1.9 ms.)
 template <int G>
-__global__ void __launch_bounds__(128) k_direct(const BatchVol *__restrict__ vols, int nv) {
+__global__ void __launch_bounds__(128, 8) k_direct(const BatchVol *__restrict__ vols, int nv) {
   __shared__ BatchVol V;
+  __shared__ bool s_undone;
   extern __shared__ float2 s_tab[];
   int v = 0;
   for (int r = nv - 1; v < r;) {
@@ -1370,6 +1367,7 @@ __global__ void __launch_bounds__(128) k_direct(const BatchVol *__restrict__ vol
   for (int i = threadIdx.x; i < (int)(sizeof(BatchVol) / sizeof(int)); i += 128)
     reinterpret_cast<int *>(&V)[i] = reinterpret_cast<const int *>(&vols[v])[i];
   __syncthreads();
+  if (threadIdx.x == 0) s_undone = *(volatile int *)V.listed > V.most;
   constexpr int COLS = 32 / G;
   const int nx = V.A.nx, ny = V.A.ny, W = V.A.W, tw = min(W, nx);
   // H in FP32 and its growth inwards, for the distances that occur
@@ -1382,6 +1380,10 @@ __global__ void __launch_bounds__(128) k_direct(const BatchVol *__restrict__ vol
   const int lane = threadIdx.x & 31, part = lane / COLS;
   const int x = blk % blocks_x * COLS + lane % COLS, y = blk / blocks_x * 4 + (threadIdx.x >> 5);
   const bool inside = x < nx && y < ny;
+  if (s_undone) {  // too many columns listed: the dilation is left undone
+    if (inside && part == 0) V.obeg[x + nx * y] = V.oend[x + nx * y] = 0;
+    return;
+  }
   Key2 A[kDirectCap];
   Key2 found[kList];  // intervals found so far; those that have come to meet are merged at the end
   float2 sure[kHot];  // of the first ones, inside which an FP32 candidate is certain to lie in them
@@ -1494,9 +1496,10 @@ __global__ void __launch_bounds__(128) k_direct(const BatchVol *__restrict__ vol
   const int c = x + nx * y;
   unsigned dst = 0;
   if (n < 0) {
-    atomicOr(V.ovf, 8);
-    n = 0;
-  } else if (!place_union(V, x, y, n, dst)) {
+    beyond_list(V, x, y);
+    return;
+  }
+  if (!place_union(V, x, y, n, dst)) {
     n = 0;
     dst = 0;
   }
@@ -1505,43 +1508,30 @@ __global__ void __launch_bounds__(128) k_direct(const BatchVol *__restrict__ vol
   V.oend[c] = (int32_t)(dst + (unsigned)n);
 }
 
-// ------------------------------------------------------------ last tier
+// ------------------------------------------------------------ last tiers
 
-// Inserts [lo, hi] into the sorted list L of n disjoint closed intervals.
-__device__ bool big_insert(double2 *L, int &n, int cap, double lo, double hi) {
-  int l = 0, r = n;
-  while (l < r) {
-    const int m = (l + r) >> 1;
-    if (L[m].y >= lo)
-      r = m;
-    else
-      l = m + 1;
+// The patches of `list` (items of a launch of one dilation, with G lanes per column) as columns of its over_list.
+__global__ void k_patch_columns(const BatchVol *vols, const int *list, const int *count, int px) {
+  const BatchVol &V = vols[0];
+  const int nx = V.A.nx, ny = V.A.ny, band_most = 512 / px;
+  const int tiles_x = (nx + px - 1) / px, tiles_y = (ny + kPatchY - 1) / kPatchY;
+  for (int i = blockIdx.x; i < *count; i += gridDim.x) {
+    const int item = list[i], band = item / (band_most * tiles_y), rb = item - band * band_most * tiles_y;
+    const int bw = min(band_most, tiles_x - band * band_most);
+    const int x = (band * band_most + rb % bw) * px + threadIdx.x % px, y = (rb / bw) * kPatchY + threadIdx.x / px;
+    const bool in = (int)threadIdx.x < px * kPatchY && x < nx && y < ny;
+    if (in) V.over_list[atomicAdd(V.over_count, 1)] = x + nx * y;
   }
-  const int i = l;
-  if (i == n || L[i].x > hi) {
-    if (n >= cap) return false;
-    for (int k = n; k > i; --k) L[k] = L[k - 1];
-    L[i] = make_double2(lo, hi);
-    ++n;
-    return true;
-  }
-  int j = i;
-  while (j + 1 < n && L[j + 1].x <= hi) ++j;
-  L[i] = make_double2(L[i].x < lo ? L[i].x : lo, L[j].y > hi ? L[j].y : hi);
-  if (j > i) {
-    const int sh = j - i;
-    for (int k = i + 1; k + sh < n; ++k) L[k] = L[k + sh];
-    n -= sh;
-  }
-  return true;
 }
 
 // The listed columns of every dilation in FP64 (grid-stride), each built in a
-// kBigCap-interval list in global scratch and placed like the other tiers; a
-// union beyond kBigCap sets the overflow flag.
-__global__ void __launch_bounds__(kBigThreads) k_big(const BatchVol *vols, int nv, double2 *scratch) {
+// list of `cap` intervals in global scratch and placed like the other tiers; a
+// union beyond it sets the overflow flag. Every SM has a block: with 16 in all the
+// scattered segments of k_column's comment took 77 ms at radius 2 and 1,300 at 4,
+// with one per SM 21 and 178 (two: 20 and 177).
+__global__ void __launch_bounds__(kBigThreads) k_big(const BatchVol *vols, int nv, double2 *scratch, int cap) {
   const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
-  double2 *L = scratch + (size_t)tid * kBigCap;
+  double2 *L = scratch + (size_t)tid * cap;
   for (int v = 0; v < nv; ++v) {
     const BatchVol &V = vols[v];
     const FastArgs &A = V.A;
@@ -1549,19 +1539,10 @@ __global__ void __launch_bounds__(kBigThreads) k_big(const BatchVol *vols, int n
     for (int i = tid; i < m; i += nth) {
       const int c = V.big_list[i];
       const int x = c % A.nx, y = c / A.nx;
-      int n = 0;
-      bool ok = true;
-      for (int ys = max(0, y - A.Dy); ys <= min(A.ny - 1, y + A.Dy) && ok; ++ys) {
-        const int d = abs(ys - y), reach = A.Dx[d];
-        for (int xs = max(0, x - reach); xs <= min(A.nx - 1, x + reach) && ok; ++xs) {
-          const double h = A.H64[d * A.W + abs(xs - x)];
-          const int cs = xs + A.nx * ys;
-          for (int k = A.beg[cs]; k < A.end[cs] && ok; ++k)
-            ok = big_insert(L, n, kBigCap, __dsub_rn(A.zd[2 * k], h), __dadd_rn(A.zd[2 * k + 1], h));
-        }
-      }
+      int n = big_union(A, x, y, L, cap);
       unsigned dst = 0;
-      if (!ok) {
+      if (n > kUnionLarge) atomicAdd(V.large, 1);
+      if (n < 0) {
         atomicOr(V.ovf, 1);
         n = 0;
       } else if (!place_union(V, x, y, n, dst)) {
@@ -1672,10 +1653,13 @@ void patch_scratch_set(PatchPlan &P, bool big, void *mem) {
   S.cids = reinterpret_cast<int2 *>(p);
 }
 
-size_t big_scratch_elems() { return (size_t)kBigBlocks * kBigThreads * kBigCap; }
+int big_blocks(int64_t columns) {
+  return (int)std::max<int64_t>(1, std::min<int64_t>(sm_count_fast(), (columns + kBigThreads - 1) / kBigThreads));
+}
+size_t big_scratch_elems(int blocks, int cap) { return (size_t)blocks * kBigThreads * cap; }
 
-void big_launch(cudaStream_t st, const BatchVol *vols, int nv, double2 *scratch) {
-  k_big<<<kBigBlocks, kBigThreads, 0, st>>>(vols, nv, scratch);
+void big_launch(cudaStream_t st, const BatchVol *vols, int nv, double2 *scratch, int blocks, int cap) {
+  k_big<<<blocks, kBigThreads, 0, st>>>(vols, nv, scratch, cap);
 }
 
 size_t pack_offsets(const vo_grid &g) {
@@ -1731,11 +1715,15 @@ void direct_launch(cudaStream_t st, const BatchVol *vols, int nv, int blocks, in
   (split == 1 ? &k_direct<1> : &k_direct<kSplit>)<<<blocks, 128, smem + sizeof(float2) * kList * 128, st>>>(vols, nv);
 }
 
-bool direct_choice(const vo_grid &g, const DeviceTables &T, double mean_segs) {
-  // source columns in reach of a column, on average over the grid
+double reach_columns(const vo_grid &g, const DeviceTables &T) {
   double cols = 0;
   for (int d = 0; d <= std::min(T.host.Dy, g.ny - 1); ++d)
     cols += (d ? 2.0 : 1.0) * (1.0 - (double)d / g.ny) * std::min(2 * T.host.Dx[d] + 1, g.nx);
+  return cols;
+}
+
+bool direct_choice(const vo_grid &g, const DeviceTables &T, double mean_segs) {
+  const double cols = reach_columns(g, T);
   // patches are four rows high: of a grid of fewer rows they use as much less
   if (g.nx < 1 || g.ny < 1 || g.nx > 65535 || direct_table(g.nx, g.ny, T.host.W, T.host.Dy) > 31 * 1024) return false;
   return cols * std::max(mean_segs, 1.0) <= kDirectWork * kPatchY / std::min(g.ny, kPatchY);
@@ -1748,118 +1736,198 @@ int dilate_fast(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out, vo_
   int rc = get_tables(ctx, R, std::max(nx, ny), &T);
   if (rc) return rc;
   const double mean_segs = (double)in->nseg / std::max(ncols, 1);
-  bool direct = direct_choice(g, *T, mean_segs);
-  PatchPlan P;
+  Engine engine = direct_choice(g, *T, mean_segs) ? Engine::kDirect : Engine::kPatches;
+  int union_slots = column_slots(mean_segs);
   SlotLayout slots = slots_first(ncols, mean_segs);
+  std::vector<void *> mem;
+  auto take = [&](void **p, size_t bytes) -> int {
+    unsigned char *q = nullptr;
+    const int r = dalloc(ctx, &q, bytes);
+    *p = q;
+    if (!r) mem.push_back(q);
+    return r;
+  };
+  auto take_n = [&](auto **p, size_t n) -> int { return *p ? VO_OK : take((void **)p, n * sizeof(**p)); };
   const size_t nseg = (size_t)std::max<int64_t>(in->nseg, 1);
-  PackOut pk;
-  int32_t *obeg = nullptr, *big_list = nullptr;
-  int *list = nullptr;
-  unsigned char *misc = nullptr, *scratch[2] = {nullptr, nullptr};
-  double2 *oz = nullptr, *big = nullptr;
-  BatchVol *dv = nullptr;
   // misc: range orders (4 x 8 bytes), FastPar at 64, counters at 128 (4 of the queue, FP64-tier columns,
-  // spill used, overflow flags), the launch's BatchVol at 256, then the columns' slots; the first two
-  // parts are written by one copy
+  // spill used, overflow flags, columns for k_column_list, listed patches, large unions), the launch's BatchVol at 256 and
+  // its ColumnArgs, then the columns' slots and the FP64 tier's list; all up to the slots is written by one copy
   struct Head {
     unsigned char zeros[256];
     BatchVol V;
+    ColumnArgs C;
   } head;
   static_assert(offsetof(Head, V) == 256, "the counters lie before the launch's description");
+  constexpr int kCounters = 10;
   const size_t head_bytes = (sizeof(Head) + 255) / 256 * 256;
-  rc = dalloc(ctx, &misc, head_bytes + sizeof(int32_t) * 2 * (size_t)ncols);
+  unsigned char *misc = nullptr;
+  rc = take((void **)&misc, head_bytes + sizeof(int32_t) * 3 * (size_t)ncols);
+  BatchVol *dv = nullptr;
+  int32_t *obeg = nullptr;
+  int *cnt = nullptr;
+  PackOut pk;
   if (!rc) {
     dv = reinterpret_cast<BatchVol *>(misc + offsetof(Head, V));
     obeg = reinterpret_cast<int32_t *>(misc + head_bytes);
+    pk.par = reinterpret_cast<FastPar *>(misc + 64);
+    cnt = reinterpret_cast<int *>(misc + 128);
   }
-  unsigned long long *mm = reinterpret_cast<unsigned long long *>(misc);
-  pk.par = reinterpret_cast<FastPar *>(misc + 64);
-  int *cnt = reinterpret_cast<int *>(misc + 128);
-  // what the patches need beside that
-  auto patch_memory = [&]() -> int {
-    const vo_grid *const gp = &g;
-    const int split = patch_split(&gp, 1);
-    int r = patch_plan(ctx, patch_count(g, split), split, T->host.hs, P);
-    if (!r) r = dalloc(ctx, &pk.zf, nseg);
-    if (!r) r = dalloc(ctx, &pk.code, nseg);
-    if (!r) r = dalloc(ctx, &pk.wide, nseg);
-    if (!r) r = dalloc(ctx, &pk.zx, nseg);
-    if (!r) r = dalloc(ctx, &pk.cl, nseg);
-    if (!r) r = dalloc(ctx, &pk.coff, pack_offsets(g));
-    if (!r) r = dalloc(ctx, &list, (size_t)P.nitems);
-    if (!r) r = dalloc(ctx, &big_list, (size_t)ncols);
-    if (!r) r = dalloc(ctx, &scratch[0], patch_scratch_bytes(P, false));
-    if (!r) patch_scratch_set(P, false, scratch[0]);
-    P.Q = PatchQueue{cnt, list};
+  PatchPlan P;
+  ColumnPrep cp;
+  int *list = nullptr, *over_list = nullptr;
+  unsigned char *scratch[2] = {nullptr, nullptr};
+  double2 *oz = nullptr, *big = nullptr;
+  // what an engine needs beside that
+  int *const big_list = obeg ? obeg + 2 * (size_t)ncols : nullptr;
+  auto memory = [&](Engine e) -> int {
+    int r = VO_OK;
+    if (e == Engine::kDirect) {
+      if (!r) r = take_n(&pk.rec, nseg);
+    } else if (e == Engine::kPatches) {
+      const vo_grid *const gp = &g;
+      const int split = patch_split(&gp, 1);
+      if (!r) r = patch_plan(ctx, patch_count(g, split), split, T->host.hs, P);
+      if (!r) r = take_n(&pk.zf, nseg);
+      if (!r) r = take_n(&pk.code, nseg);
+      if (!r) r = take_n(&pk.wide, nseg);
+      if (!r) r = take_n(&pk.zx, nseg);
+      if (!r) r = take_n(&pk.cl, nseg);
+      if (!r) r = take_n(&pk.coff, pack_offsets(g));
+      if (!r) r = take_n(&list, (size_t)P.nitems);
+      if (!r) r = take_n(&scratch[0], patch_scratch_bytes(P, false));
+      if (!r) patch_scratch_set(P, false, scratch[0]);
+      P.Q = PatchQueue{cnt, list};
+    } else if (!cp.zf) {
+      if (!r) r = column_tables(ctx, T);
+      if (!r) r = column_alloc(g, nseg, mean_segs, take, cp);
+      if (!r) r = take_n(&over_list, (size_t)ncols);
+    }
     return r;
   };
-  if (!rc) rc = direct ? dalloc(ctx, &pk.rec, nseg) : patch_memory();
-  vo_volume *res = nullptr;
-  int cols2 = 0;
-  for (int attempt = 0; !rc; ++attempt) {
-    rc = dalloc(ctx, &oz, (size_t)ncols * slots.cap + (size_t)slots.spill);
-    if (rc) break;
-    std::memset(&head, 0, sizeof head);
+  auto prepare_columns = [&]() {
+    column_prepare(ctx->stream, head.C, (float)R, T->dom, cp);
+    ctx->launches += 3;
+  };
+  auto last_tier = [&](int64_t columns) -> int {
+    const int blocks = big_blocks(columns);
+    const int r = take_n(&big, big_scratch_elems(big_blocks(ncols), kBigCap));
+    if (r) return r;
+    big_launch(ctx->stream, dv, 1, big, blocks, kBigCap);
+    ctx->launches += 1;
+    return VO_OK;
+  };
+  auto describe = [&](Engine e) {
     BatchVol &V = head.V;
     V.A = fast_args(nx, ny, *T, in->offs, in->offs + 1, in->z, pk);
     V.obeg = obeg;
     V.oend = obeg + ncols;
     V.oz = oz;
     V.cap = slots.cap;
-    V.item1 = direct ? direct_blocks(g, ncols) : P.nitems;
+    V.item1 = e == Engine::kDirect ? direct_blocks(g, ncols) : e == Engine::kPatches ? P.nitems : patch_count(g, 1);
     V.spill_base = (unsigned)((int64_t)ncols * slots.cap);
     V.spill_cap = (unsigned)slots.spill;
     V.big_list = big_list;
     V.big_count = cnt + 4;
     V.spill_used = reinterpret_cast<unsigned *>(cnt + 5);
     V.ovf = cnt + 6;
+    V.column = reinterpret_cast<const ColumnArgs *>(misc + offsetof(Head, C));
+    V.over_list = over_list;
+    V.over_count = cnt + 7;
+    V.listed = e == Engine::kDirect ? V.big_count : cnt + 8;
+    V.most = e == Engine::kDirect ? kFewColumns + ncols / 64 : kFewPatches + P.nitems / 64;
+    V.large = cnt + 9;
+    if (cp.zf) head.C = column_args(nx, ny, *T, in->offs, in->offs + 1, in->z, cp);
+  };
+  if (!rc) rc = memory(engine);
+  vo_volume *res = nullptr;
+  int cols2 = 0;
+  for (int attempt = 0; !rc; ++attempt) {
+    rc = dalloc(ctx, &oz, (size_t)ncols * slots.cap + (size_t)slots.spill);
+    if (rc) break;
+    std::memset(&head, 0, sizeof head);
+    describe(engine);
     cudaMemcpyAsync(misc, &head, sizeof head, cudaMemcpyHostToDevice, ctx->stream);
     cudaEventRecord(ctx->ev[0], ctx->stream);
-    if (direct)
-      direct_prepare(ctx->stream, V.A, pk);
+    if (engine == Engine::kDirect)
+      direct_prepare(ctx->stream, head.V.A, pk);
+    else if (engine == Engine::kPatches)
+      fast_prepare(ctx->stream, head.V.A, (float)R, mean_segs, reinterpret_cast<unsigned long long *>(misc), pk);
     else
-      fast_prepare(ctx->stream, V.A, (float)R, mean_segs, mm, pk);
+      prepare_columns();
     cudaEventRecord(ctx->ev[1], ctx->stream);
     cudaEventRecord(ctx->ev[4], ctx->stream);
-    if (direct)
-      direct_launch(ctx->stream, dv, 1, V.item1, ncols, direct_smem(V.A));
-    else
+    if (engine == Engine::kDirect)
+      direct_launch(ctx->stream, dv, 1, head.V.item1, ncols, direct_smem(head.V.A));
+    else if (engine == Engine::kPatches)
       patch_launch(false, P, ctx->stream, dv);
+    else
+      column_launch(ctx->stream, dv, 1, head.V.item1, union_slots, head.C);
     cudaEventRecord(ctx->ev[5], ctx->stream);
-    ctx->launches += direct ? 2 : 3;
+    ctx->launches += engine == Engine::kDirect ? 2 : engine == Engine::kPatches ? 3 : 1;
     SlotVol sv;
     sv.grid = g;
     sv.cap = slots.cap;
     sv.beg = obeg;
     sv.end = obeg + ncols;
     sv.z = oz;
-    int hc[7] = {0};
-    rc = slot_to_volume(ctx, sv, &res, cnt, hc, 7);
-    if (!rc && hc[1] + hc[4] > 0) {  // patches and columns for the last tiers
-      vo_volume_free(ctx, res);
-      res = nullptr;
-      if (!scratch[1]) rc = dalloc(ctx, &scratch[1], patch_scratch_bytes(P, true));
-      if (!rc && !big) rc = dalloc(ctx, &big, big_scratch_elems());
-      if (!rc) {
-        patch_scratch_set(P, true, scratch[1]);
-        patch_launch(true, P, ctx->stream, dv);
-        big_launch(ctx->stream, dv, 1, big);
-        ctx->launches += 2;
-        rc = slot_to_volume(ctx, sv, &res, cnt, hc, 7);
-      }
-    }
+    int hc[kCounters] = {0};
+    rc = slot_to_volume(ctx, sv, &res, cnt, hc, kCounters);
     if (rc) break;
-    if (hc[6] & 8) {  // a union beyond the small list: by patches
+    const int patches = hc[1], fp64 = hc[4], over = hc[7], listed = engine == Engine::kDirect ? fp64 : hc[8];
+    if (engine != Engine::kColumns && listed > head.V.most) {  // left undone: all of it by columns, with room for large unions
       vo_volume_free(ctx, res);
       res = nullptr;
       dfree(ctx, oz);
       oz = nullptr;
-      direct = false;
-      rc = patch_memory();
+      engine = Engine::kColumns;
+      union_slots = 24;  // few of its columns have so few, and the more lists it keeps the longer they take to outgrow them
+      slots_many(ncols, slots);
+      rc = memory(engine);
       --attempt;
       continue;
     }
-    cols2 = hc[3] + (hc[3] == 0 ? hc[4] : 0);
+    cols2 = engine == Engine::kPatches ? std::max(hc[3], fp64) : over;
+    if (patches + fp64 + over > 0) {  // what the later tiers take
+      vo_volume_free(ctx, res);
+      res = nullptr;
+      const bool many = (engine == Engine::kDirect && fp64 > kFewColumns) || (engine == Engine::kPatches && patches > kFewPatches);
+      if (many) {  // by k_column_list
+        rc = memory(Engine::kColumns);
+        describe(engine);
+        BatchVol &V = head.V;
+        if (engine == Engine::kDirect) {  // its list becomes that kernel's
+          V.over_list = big_list;
+          V.over_count = cnt + 4;
+          V.big_list = over_list;
+          V.big_count = cnt + 7;
+        }
+        V.listed = cnt + 8;  // no limit from here on
+        V.most = 2147483647;
+        if (!rc) {
+          cudaMemcpyAsync(dv, &head.V, sizeof head.V + sizeof head.C, cudaMemcpyHostToDevice, ctx->stream);
+          prepare_columns();
+          if (engine == Engine::kPatches) {
+            k_patch_columns<<<std::min(patches, 4096), 32, 0, ctx->stream>>>(dv, list, cnt + 1, kPatchX / P.split);
+            ctx->launches += 1;
+          }
+        }
+      } else if (patches > 0) {
+        rc = take_n(&scratch[1], patch_scratch_bytes(P, true));
+        if (!rc) {
+          patch_scratch_set(P, true, scratch[1]);
+          patch_launch(true, P, ctx->stream, dv);
+          ctx->launches += 1;
+        }
+      }
+      if (!rc && (many || over > 0)) {
+        column_list_launch(ctx->stream, dv, 1);
+        ctx->launches += 1;
+      }
+      if (!rc) rc = last_tier(many || patches + over > 0 ? ncols : fp64);
+      if (!rc) rc = slot_to_volume(ctx, sv, &res, cnt, hc, kCounters);
+      if (rc) break;
+      if (engine == Engine::kDirect) cols2 = hc[9];
+    }
     if (hc[6] & 1) {
       rc = set_error(ctx, VO_EINTERNAL, "a column exceeds the fallback union capacity");
     } else if (hc[6] & 4) {  // the spill region was too small: its counter says what it takes
@@ -1885,10 +1953,8 @@ int dilate_fast(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out, vo_
       tm->kernel_ms[2] += e1;
     }
   }
-  for (void *p : {(void *)misc, (void *)pk.zf, (void *)pk.code, (void *)pk.wide, (void *)pk.zx, (void *)pk.cl, (void *)pk.rec,
-                  (void *)pk.coff, (void *)list, (void *)big_list, (void *)scratch[0],
-                  (void *)scratch[1], (void *)oz, (void *)big})
-    dfree(ctx, p);
+  dfree(ctx, oz);
+  for (void *p : mem) dfree(ctx, p);
   if (rc) {
     if (res) vo_volume_free(ctx, res);
     return rc;

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -50,6 +51,11 @@ struct DevTables {
 // VO_EINVAL or VO_ERADIUS.
 int build_tables(double R, int kmax, Tables &t);
 
+constexpr int kDomLevels = 11;  // growths of H whose dominance masks are kept (15 in a pair record: none)
+struct DomLevels {
+  float t[kDomLevels];
+};
+
 struct DeviceTables {
   double R = -1;
   int kmax = 0;
@@ -57,6 +63,10 @@ struct DeviceTables {
   float *Hp = nullptr;
   int *Dx = nullptr;
   double *HB = nullptr;
+  // for the columns kernel, made when it is first used (column_tables)
+  float4 *prec = nullptr;
+  int npairs = 0;
+  DomLevels dom{};
   Tables host;
   DevTables view() const { return DevTables{host.Dy, host.W, H, Dx, HB}; }
 };
@@ -190,6 +200,7 @@ struct FastPar {
   float E, inv_w, thr;
   int nbins;
   float lo, hi;
+  float q;  // bounds the error of a difference of two values less the base
 };
 
 // Columns of a warp of the FP32 kernel: a kPatchX x kPatchY patch, lane l at
@@ -220,9 +231,26 @@ struct FastArgs {
   const int32_t *rbeg, *rend;
 };
 
+// Arguments of the columns kernel for one volume (vo_column.cu).
+struct ColumnArgs {
+  int nx, ny, W, npairs, mask_bits, unused;
+  const int32_t *beg, *end;  // segments [beg[c], end[c]) of column c (CSR or slots)
+  const double *zd;          // FP64 values
+  const float *zf;           // FP32 copies relative to FastPar::base
+  const double *H64;         // [(Dy + 1) * W]
+  const float4 *prec;        // pair records (column_pairs)
+  const FastPar *par;
+  // (beg, end, widths x- | x+ << 16, y- | y+ << 16 as FP16) per column
+  const int4 *col;
+  // Segment dominance masks [4 directions][kDomLevels][ncols] of mask_bits bits: bit j of a column with at most
+  // mask_bits segments is set when its segment j lies in a neighbour segment widened by the level's threshold.
+  const void *dmask;
+};
+
 constexpr int kSizerTile = 32;     // side of a sizing tile (columns)
 constexpr int kUnionCap = 32;      // output slots per column of a batch dilation without a sizer
 constexpr int kUnionCapMid = 128;  // most output slots per column of a sized tile
+constexpr int kUnionLarge = 63;    // intervals of the first tiers' largest unions
 // One dilation of a launch (device array element).
 struct BatchVol {
   FastArgs A;
@@ -235,9 +263,50 @@ struct BatchVol {
   int item0, item1;      // its patches in the launch's queue
   unsigned spill_base, spill_cap;
   unsigned *spill_used;
-  int *big_list, *big_count;  // columns for the third tier (FP64)
-  int *ovf;  // flags: 1 a union beyond the FP64 list, 4 spill region exhausted, 8 a union beyond k_direct's list
+  int *big_list, *big_count;  // columns for the last tier (FP64)
+  int *ovf;  // flags: 1 a union beyond the FP64 list, 4 spill region exhausted, 8 more unions beyond the lists than the tiers take
+  // The columns kernel: its arguments, and the columns with more intervals than it (or k_column_list's caller) holds.
+  const ColumnArgs *column;
+  int *over_list, *over_count;
+  // More columns (k_direct) or patches (k_patch) than this beyond the first tier's lists: the rest of the dilation
+  // is left undone, for the caller to do it all by columns.
+  int *listed, most;
+  int *large;  // columns of the later tiers with more than kUnionLarge intervals
+  // k_direct: kFewColumns lists of kPoolCap intervals for columns beyond its own, shared by the launch's dilations
+  // (how many are taken: pool_used); nullptr: those columns are listed.
+  double2 *pool;
+  int *pool_used;
 };
+constexpr int kPoolCap = 1024;
+
+// Masks of 16 bits per column and level where the input averages at most this many segments per column, else of
+// 32; a column with more segments than bits takes part with all of them (2048^2 spheres + cylinders: 0.02 % of the
+// columns have more than 16).
+constexpr double kMask16MeanSegs = 8.0;
+
+// Working memory of column_prepare.
+struct ColumnPrep {
+  int mask_bits = 16;
+  float2 *zf = nullptr;
+  int4 *col = nullptr;
+  void *dmask = nullptr;
+  FastPar *par = nullptr;
+  unsigned long long *mm = nullptr;
+};
+// Allocates it for a grid with an input of `entries` segments (unused slots included), by alloc(pointer, bytes).
+int column_alloc(const vo_grid &g, size_t entries, double mean_segs, const std::function<int(void **, size_t)> &alloc,
+                 ColumnPrep &P);
+ColumnArgs column_args(int nx, int ny, const DeviceTables &T, const int32_t *beg, const int32_t *end, const double2 *z,
+                       const ColumnPrep &P);
+void column_prepare(cudaStream_t st, const ColumnArgs &A, float R, const DomLevels &L, const ColumnPrep &P);
+// The launch over the nv dilations vols, items as patches (patch_count with split 1), and the one over the columns
+// that they list. A: of the first one.
+int column_slots(double mean_segs);
+void column_launch(cudaStream_t st, const BatchVol *vols, int nv, int blocks, int slots, const ColumnArgs &A);
+void column_list_launch(cudaStream_t st, const BatchVol *vols, int nv);
+// A radius' pair records and dominance levels (DeviceTables::prec, ::dom).
+std::vector<float4> column_pairs(const Tables &h, DomLevels &L);
+int column_tables(vo_ctx *ctx, const DeviceTables *T);
 
 // Queue of a launch. count: the first tier's next item, the items it listed
 // for the second tier, that tier's next one, columns of the listed items.
@@ -265,6 +334,7 @@ int patch_split(const vo_grid *const *grids, int n);
 // (k_direct; its prepared inputs are not needed then), the launch over the nv
 // dilations vols and its blocks for a grid. launch_cols: columns of all of them.
 bool direct_choice(const vo_grid &g, const DeviceTables &T, double mean_segs);
+double reach_columns(const vo_grid &g, const DeviceTables &T);  // source columns in reach of a column, on average
 int direct_blocks(const vo_grid &g, int64_t launch_cols);
 size_t direct_smem(const FastArgs &A);
 void direct_launch(cudaStream_t st, const BatchVol *vols, int nv, int blocks, int64_t launch_cols, size_t smem);
@@ -276,9 +346,11 @@ int patch_plan(vo_ctx *ctx, int nitems, int split, int hs_max, PatchPlan &P);
 size_t patch_scratch_bytes(const PatchPlan &P, bool big);
 void patch_scratch_set(PatchPlan &P, bool big, void *mem);
 void patch_launch(bool big, const PatchPlan &P, cudaStream_t st, const BatchVol *vols);
-// Last tier (FP64) over the dilations vols[0..nv); scratch holds big_scratch_elems() intervals.
-size_t big_scratch_elems();
-void big_launch(cudaStream_t st, const BatchVol *vols, int nv, double2 *scratch);
+// Last tier (FP64) over the dilations vols[0..nv), with unions of up to `cap` intervals; scratch holds
+// big_scratch_elems(blocks, cap) of them. big_blocks: for up to so many columns.
+int big_blocks(int64_t columns);
+size_t big_scratch_elems(int blocks, int cap);
+void big_launch(cudaStream_t st, const BatchVol *vols, int nv, double2 *scratch, int blocks, int cap);
 // Outputs of the packing step, each as long as the input's segment array
 // (with its unused slots), coff pack_offsets(grid).
 struct PackOut {
@@ -300,6 +372,11 @@ FastArgs fast_args(int nx, int ny, const DeviceTables &T, const int32_t *beg, co
 void fast_prepare(cudaStream_t st, const FastArgs &A, float R, double mean_segs, unsigned long long *mm,
                   const PackOut &out);
 
+// Which kernel a dilation takes first: k_direct, k_patch or k_column.
+enum class Engine { kDirect, kPatches, kColumns };
+constexpr int kFewColumns = 4096;  // columns beyond k_direct's list up to which the FP64 tier takes them as they are
+constexpr int kFewPatches = 608;   // patches that the patch kernel's second tier takes (eight rounds of its warps)
+
 // Batch plans (vo_batch.cu).
 int morph_batched_fast(vo_ctx *ctx, int n, const int *ops, const double *radii, const vo_volume *const *ins,
                        vo_volume **outs, vo_timings *tm);
@@ -313,6 +390,32 @@ int sizer_predict_device(vo_ctx *ctx, const vo_sizer *s, const float *feats, int
 int volume_alloc(vo_ctx *ctx, const vo_grid &g, int64_t nseg, vo_volume **out);
 
 #ifdef __CUDACC__
+// Output slot of column (x, y) for an n-interval union: the column's own slot
+// when its capacity allows, else spill space, else false (the dilation's
+// overflow flag is then set). Slot indices are unsigned 32-bit.
+static __device__ __forceinline__ bool place_union(const BatchVol &V, int x, int y, int n, unsigned &dst) {
+  const int nx = V.A.nx;
+  int cap = V.cap;
+  if (V.tcap) {
+    const int tx = x / kSizerTile, ty = y / kSizerTile, t = tx + V.tiles32_x * ty;
+    const int w = min(kSizerTile, nx - tx * kSizerTile);
+    cap = V.tcap[t];
+    dst = (unsigned)V.toff[t] + (unsigned)(((x - tx * kSizerTile) + w * (y - ty * kSizerTile)) * cap);
+  } else {
+    dst = (unsigned)(x + nx * y) * (unsigned)cap;
+  }
+  if (n > cap) {
+    const unsigned off = atomicAdd(V.spill_used, (unsigned)n);
+    if (off + (unsigned)n <= V.spill_cap) {
+      dst = V.spill_base + off;
+      return true;
+    }
+    atomicOr(V.ovf, 4);  // spill region exhausted
+    return false;
+  }
+  return true;
+}
+
 // The FP64 methods compare and select values far more often than they add them,
 // and an FP64 comparison occupies the SM for as long as sixteen integer ones.
 // So they hold ends as signed integers of the same order: the bit pattern, its

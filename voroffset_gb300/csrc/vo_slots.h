@@ -25,6 +25,14 @@ inline SlotLayout slots_first(int64_t ncols, double mean_segs) {
   return s;
 }
 
+// For a run most of whose columns have unions beyond the first tiers' lists: slots for 128 intervals each and as many
+// again to spill, up to 4 GB of either.
+inline void slots_many(int64_t ncols, SlotLayout &s) {
+  const int64_t n = std::max<int64_t>(ncols, 1);
+  s.cap = (int)std::max<int64_t>(s.cap, std::min<int64_t>(128, (1LL << 28) / n));
+  s.spill = std::max<int64_t>(s.spill, std::min<int64_t>(n * s.cap, std::min<int64_t>(1LL << 28, kSlotMost - n * s.cap)));
+}
+
 // After a run whose columns asked for `need` intervals of spill space, more than there was. Where that and
 // the columns' slots together pass the slot range, the slots shrink until any result that is not refused
 // fits: with it all in the spill region. False when the result is refused.
