@@ -1068,8 +1068,11 @@ __global__ void __launch_bounds__(32, 20) k_patch(const BatchVol *__restrict__ v
   int cur = -1;
   const int todo = BIG ? min(Q.count[1], nitems) : nitems;
   for (;;) {
-    int item = 0;
-    if (S.lane == 0) item = atomicAdd(&Q.count[BIG ? 2 : 0], 1);
+    int item = 0, listed = 0;  // (of the patch before: its load and the queue's overlap)
+    if (S.lane == 0) {
+      item = atomicAdd(&Q.count[BIG ? 2 : 0], 1);
+      if (!BIG && cur >= 0) listed = *(volatile int *)V.listed;
+    }
     item = __shfl_sync(kFull, item, 0);
     if (item >= todo) return;
     if (BIG) item = Q.list[item];
@@ -1082,6 +1085,7 @@ __global__ void __launch_bounds__(32, 20) k_patch(const BatchVol *__restrict__ v
       for (int i = S.lane; i < (int)(sizeof(BatchVol) / sizeof(int)); i += 32)
         reinterpret_cast<int *>(&V)[i] = reinterpret_cast<const int *>(&vols[v])[i];
       cur = v;
+      listed = 0;
       __syncwarp();
     }
     constexpr int kBand = 512 / PX;
@@ -1098,7 +1102,8 @@ __global__ void __launch_bounds__(32, 20) k_patch(const BatchVol *__restrict__ v
     S.inv_w = par->inv_w;
     S.thr = par->thr;
     // beyond `most` listed patches the dilation is left undone (one lane looks: the answer may change meanwhile)
-    const bool undone = __shfl_sync(kFull, S.lane == 0 && *(volatile int *)V.listed > V.most ? 1 : 0, 0);
+    if (BIG && S.lane == 0) listed = *(volatile int *)V.listed;
+    const bool undone = __shfl_sync(kFull, listed, 0) > V.most;
     if (BIG && undone) {
       if (S.lane == 0) atomicOr(V.ovf, 8);
       continue;
