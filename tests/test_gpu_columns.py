@@ -1,6 +1,7 @@
-"""The columns kernel: unions of more intervals than the lists of the small-radius and patch kernels hold, in few
-columns, in many and in most: by its second launch, by the FP64 tier, or all over again. Single calls, replayed plans
-and batches against the oracle's own FP64 candidates, so equality is exact."""
+"""The columns kernel: inputs that take it first (smooth, dense, small radius, at least 2^18 columns), and unions
+of more intervals than the lists of the small-radius and patch kernels hold, in few columns, in many and in most:
+by its second launch, by the FP64 tier, or all over again. Single calls, replayed plans and batches against the
+oracle's own FP64 candidates, so equality is exact."""
 from __future__ import annotations
 
 import numpy as np
@@ -46,6 +47,14 @@ def check(ctx, oracle, grid, offs, z, r, op="dilation", what=""):
     out.free()
     v.free()
     return t
+
+
+# sides that leave remainders of the 8 x 4 patches and of the 512-column bands
+@pytest.mark.parametrize("nx,ny,spheres,r", [(513, 515, 1300, 5.0), (1030, 261, 1500, 6.25), (512, 512, 1600, 4.5), (4097, 66, 1200, 7.0)])
+def test_smooth_dense_volumes(ctx, vo, oracle, nx, ny, spheres, r):
+    grid, offs, z = vo.synth_volume(vo.SynthSpec(nx, ny=ny, zmax=512.0, n_spheres=spheres, s_rmin=3, s_rmax=38, seed=nx))
+    for op in ("dilation", "closing"):
+        check(ctx, oracle, grid, offs, z, r, op, what=f"{nx}x{ny}")
 
 
 @pytest.mark.parametrize("nx,ny", [(64, 64), (131, 97), (300, 5), (1, 700)])

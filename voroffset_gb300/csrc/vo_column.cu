@@ -12,13 +12,16 @@
 // per column hold that for eleven growths, so that a source column costs one load
 // of its record and two of its masks however many of its segments are held.
 //
-// It takes unions of many intervals: the patch kernel's bins and the lists of
-// k_direct hold some fifty per column. Columns beyond them (or whole inputs of
-// such columns) come here: unions of up to kUnionCapMid - 1 in a second launch
-// over the listed columns, larger ones in the FP64 tier. Scattered segments, 256^2
-// columns, 12 of 1 dexel each over 3000: 21 ms at radius 2 (131 intervals per
-// column) and 178 at 4, where the patch kernel's second tier and a small FP64
-// tier took 820 and 1,100.
+// It is the better kernel in two places.
+// - Smooth dense inputs at small radii, where most segments are held
+//   (column_choice has the measured line).
+// - Unions of many intervals: the patch kernel's bins and the lists of k_direct
+//   hold some fifty per column. Columns beyond them (or whole inputs of such
+//   columns) come here: unions of up to kUnionCapMid - 1 in a second launch over
+//   the listed columns, larger ones in the FP64 tier. Scattered segments, 256^2
+//   columns, 12 of 1 dexel each over 3000: 21 ms at radius 2 (131 intervals per
+//   column) and 178 at 4, where the patch kernel's second tier and a small FP64
+//   tier took 820 and 1,100.
 // Issue slots and divergence bound it: lanes wait for the longest candidate list of
 // their warp (1024^2 spheres, r = 32: 73 % of the issue slots, 16 of 32 lanes).
 #include <algorithm>
@@ -522,6 +525,43 @@ __global__ void k_dominance(int nx, int ny, const int32_t *__restrict__ beg, con
   col[c] = make_int4(k0, k1, (int)(h[0] | (h[1] << 16)), (int)(h[2] | (h[3] << 16)));
 }
 
+// Of kSampleColumns columns spread over the grid: their segments, times four, and how many of those (segment,
+// neighbour column) lie in a segment of that column widened by `growth`.
+constexpr int kSampleColumns = 8192;
+__global__ void __launch_bounds__(128) k_sample_held(int nx, int ny, const int32_t *__restrict__ beg,
+                                                     const int32_t *__restrict__ end, const double2 *__restrict__ z,
+                                                     double growth, int *out) {
+  const int i = blockIdx.x * 128 + threadIdx.x;
+  const long long ncols = (long long)nx * ny;
+  // evenly spread, with a step that shares no period with the rows
+  const int c = (int)(((unsigned long long)i * 0x9e3779b97f4a7c15ull >> 32) * ncols >> 32);
+  const int x = c % nx, y = c / nx;
+  int all = 0, held = 0;
+  if (x > 0 && y > 0 && x + 1 < nx && y + 1 < ny) {
+    const int step[4] = {-1, 1, -nx, nx};
+    int at[4];
+    for (int d = 0; d < 4; ++d) at[d] = beg[c + step[d]];
+    for (int k = beg[c]; k < end[c]; ++k) {
+      const double2 s = z[k];
+      all += 4;
+      for (int d = 0; d < 4; ++d) {
+        // of the neighbour's segments the first that reaches this one, or the next
+        const int e = end[c + step[d]];
+        while (at[d] < e && z[at[d]].y < s.x) ++at[d];
+        bool in = false;
+        for (int j = at[d]; j < min(at[d] + 2, e); ++j) in |= z[j].x - s.x <= growth && s.y - z[j].y <= growth;
+        held += in;
+      }
+    }
+  }
+  all = __reduce_add_sync(0xffffffffu, all);
+  held = __reduce_add_sync(0xffffffffu, held);
+  if ((threadIdx.x & 31) == 0) {
+    atomicAdd(&out[0], all);
+    atomicAdd(&out[1], held);
+  }
+}
+
 static_assert(kDomLevels <= 15, "pair records hold a level in 4 bits, 15 meaning none");
 static_assert(sizeof(BatchVol) % sizeof(int) == 0 && sizeof(ColumnArgs) % sizeof(int) == 0, "copied as ints");
 
@@ -650,6 +690,47 @@ void column_list_launch(cudaStream_t st, const BatchVol *vols, int nv) {
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   k_column_list<<<16 * std::max(sms, 1), kMidThreads, 0, st>>>(vols, nv);
+}
+
+// Against k_direct and the patch kernel, preparation and copy included (ms; segments per column; radius; the better
+// of those two, this kernel):
+//   spheres     512^2    4.0   r 4   0.52 / 0.53     r 6   0.86 / 0.74     r 8   1.04 / 1.00     r 10  1.02 / 1.30
+//               1024^2   2.9         1.13 / 1.08           1.97 / 1.64           2.71 / 2.33           2.83 / 3.20
+//               1024^2   5.1         2.01 / 1.75           3.59 / 2.66           4.17 / 3.76           4.20 / 5.01
+//               2048^2   6.1         8.89 / 8.00           15.7 / 12.6           18.1 / 17.9           19.5 / 24.6
+//               1024^2   9.6         4.27 / 4.01           7.35 / 5.70           6.72 / 7.35
+//               1024^2   1.0         0.63 / 0.75           1.04 / 1.21           1.53 / 1.77
+//   cylinders   1024^2   4.4         3.75 / 5.56           6.30 / 8.61           6.74 / 10.8
+//                        16.2        17.0 / 25.0           21.7 / 31.9           17.9 / 36.6
+// Below 2^18 columns four threads share one in k_direct, which is the best there (256^2, 4.1 segments, r = 6: 0.39 /
+// 0.48). What tells the inputs apart is how many segments a neighbour column holds at the median growth of H: 0.63
+// to 0.71 of them for spheres (with some cylinders among them 0.63 to 0.65), 0.48 to 0.52 for thin cylinders, none
+// for scattered segments. The line is 0.55; the sample takes 15 us.
+constexpr double kHeldShare = 0.55, kColumnWorkFrom = 190, kColumnWorkTo = 1050;
+constexpr int64_t kColumnCols = 1 << 18;
+constexpr double kColumnSegs = 2.0, kColumnRadiusFrom = 3.5, kColumnRadiusMid = 7.5, kColumnRadiusTo = 9.0;
+
+int column_choice(vo_ctx *ctx, const vo_grid &g, const DeviceTables &T, double mean_segs, const int32_t *beg,
+                  const int32_t *end, const double2 *z, const std::function<int()> &tables, bool *columns) {
+  *columns = false;
+  const double work = reach_columns(g, T) * mean_segs;
+  if ((int64_t)g.nx * g.ny < kColumnCols || std::min(g.nx, g.ny) < kPatchY || mean_segs < kColumnSegs ||
+      T.host.R < kColumnRadiusFrom || T.host.R >= kColumnRadiusTo || work < kColumnWorkFrom ||
+      (T.host.R >= kColumnRadiusMid && work > kColumnWorkTo))
+    return VO_OK;
+  int rc = tables();
+  if (rc) return rc;
+  int *d = nullptr, h[2] = {0, 0};
+  rc = dalloc(ctx, &d, 2);
+  if (rc) return rc;
+  cudaMemsetAsync(d, 0, sizeof h, ctx->stream);
+  k_sample_held<<<kSampleColumns / 128, 128, 0, ctx->stream>>>(g.nx, g.ny, beg, end, z, T.dom.t[kDomLevels / 2], d);
+  ctx->launches += 1;
+  cudaMemcpyAsync(h, d, sizeof h, cudaMemcpyDeviceToHost, ctx->stream);
+  dfree(ctx, d);
+  VO_CK(ctx, cudaStreamSynchronize(ctx->stream));
+  *columns = h[1] >= kHeldShare * h[0];
+  return VO_OK;
 }
 
 }  // namespace vo

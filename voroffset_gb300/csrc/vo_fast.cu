@@ -1742,6 +1742,12 @@ int dilate_fast(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out, vo_
   if (rc) return rc;
   const double mean_segs = (double)in->nseg / std::max(ncols, 1);
   Engine engine = direct_choice(g, *T, mean_segs) ? Engine::kDirect : Engine::kPatches;
+  {
+    bool columns = false;
+    rc = column_choice(ctx, g, *T, mean_segs, in->offs, in->offs + 1, in->z, [&] { return column_tables(ctx, T); }, &columns);
+    if (rc) return rc;
+    if (columns) engine = Engine::kColumns;
+  }
   int union_slots = column_slots(mean_segs);
   SlotLayout slots = slots_first(ncols, mean_segs);
   std::vector<void *> mem;
