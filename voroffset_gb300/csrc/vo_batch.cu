@@ -345,7 +345,7 @@ int plan_dilation_round(vo_ctx *ctx, vo_batch *b, std::vector<DilPlan> &dils, bo
       if (!rc && d.in.owns) rc = plan_alloc(ctx, b, &d.pk.zx, entries);
       if (!rc && d.in.owns) rc = plan_alloc(ctx, b, &d.pk.rbeg, 2 * (size_t)ncols);
       if (rc) return rc;
-      d.A = fast_args(g.nx, g.ny, *d.T, d.in.beg, d.in.end, d.in.z, d.pk);
+      d.A = fast_args(g, *d.T, d.in.beg, d.in.end, d.in.z, d.pk);
       const DilPlan c = d;
       record(b, 1, [c](cudaStream_t st) { direct_prepare(st, c.A, c.pk); });
       continue;
@@ -361,7 +361,7 @@ int plan_dilation_round(vo_ctx *ctx, vo_batch *b, std::vector<DilPlan> &dils, bo
       if (!rc) rc = column_alloc(g, entries, d.mean_segs, take, d.cp);
       if (!rc) rc = plan_alloc(ctx, b, &d.over_list, (size_t)ncols);
       if (rc) return rc;
-      d.A = fast_args(g.nx, g.ny, *d.T, d.in.beg, d.in.end, d.in.z, d.pk);
+      d.A = fast_args(g, *d.T, d.in.beg, d.in.end, d.in.z, d.pk);
       d.C = column_args(g.nx, g.ny, *d.T, d.in.beg, d.in.end, d.in.z, d.cp);
       const DilPlan c = d;
       record(b, 3, [c, R](cudaStream_t st) { column_prepare(st, c.C, R, c.T->dom, c.cp); });
@@ -376,7 +376,7 @@ int plan_dilation_round(vo_ctx *ctx, vo_batch *b, std::vector<DilPlan> &dils, bo
     if (!rc) rc = plan_alloc(ctx, b, &d.pk.par, 1);
     if (!rc) rc = plan_alloc(ctx, b, &d.mm, 4);
     if (rc) return rc;
-    d.A = fast_args(g.nx, g.ny, *d.T, d.in.beg, d.in.end, d.in.z, d.pk);
+    d.A = fast_args(g, *d.T, d.in.beg, d.in.end, d.in.z, d.pk);
     const DilPlan c = d;
     record(b, 2, [c, R](cudaStream_t st) { fast_prepare(st, c.A, R, c.mean_segs, c.mm, c.pk); });
   }
@@ -405,10 +405,12 @@ int plan_dilation_round(vo_ctx *ctx, vo_batch *b, std::vector<DilPlan> &dils, bo
   int np = 0, nc = 0, slots = 0;
   int64_t direct_cols = 0;
   size_t direct_shared = 0;
+  bool direct_shift = false;
   for (const DilPlan &d : dils) {
     if (d.engine == Engine::kDirect) {
       direct_cols += (int64_t)d.in.grid.nx * d.in.grid.ny;
       direct_shared = std::max(direct_shared, direct_smem(d.A));
+      direct_shift |= d.A.off != 0.0;
     } else if (d.engine == Engine::kColumns) {
       ++nc;
       slots = std::max(slots, column_slots(d.mean_segs));
@@ -494,7 +496,7 @@ int plan_dilation_round(vo_ctx *ctx, vo_batch *b, std::vector<DilPlan> &dils, bo
       column_list_launch(st, L.dvols + np, nc);
     }
     if (np + nc > 0) big_launch(st, L.dvols, np + nc, big_scratch, big_grid, kPoolCap);
-    if (nd > 0) direct_launch(st, L.dvols + np + nc, nd, L.direct_items, direct_cols, direct_shared);
+    if (nd > 0) direct_launch(st, L.dvols + np + nc, nd, L.direct_items, direct_cols, direct_shared, direct_shift);
   };
   std::vector<const vo_grid *> grids;
   for (const DilPlan &d : dils)

@@ -437,6 +437,7 @@ struct E2Args {
   Key2 *gz;              // re-run: 2 * kE2CapBig per block
   uint32_t *gk;          // re-run: keys, 2 * kE2CapBig per block
   int cap_small;         // stadium capacity of the first launch (<= kE2CapSmall)
+  double off;            // value_offset of the grid
   int *ghist;            // placement counts of columns with more than kE2Stage pieces (per block)
   int ghist_stride;      // ints per block of ghist (the band's most pieces per column + 2)
 };
@@ -466,7 +467,7 @@ __device__ __forceinline__ bool live(uint32_t k, int x, int dir, const E2Args &A
 // M' = M + 4 table errors, the tables' chords at every later column satisfy
 // [a_v - H_v, b_v + H_v] inside [a_p - H_p, b_p + H_p] in exact arithmetic on
 // the FP64 values, hence also after each endpoint's rounding. The test runs in
-// FP32 on values within 2^-23 of theirs (trunc32) and tables within 2^-24; eps
+// FP32 on values less the grid's offset, within 2^-23 of theirs (trunc32), and tables within 2^-24; eps
 // bounds those errors, the roundings of the differences and the table errors
 // four times over.
 __device__ __forceinline__ bool covers_for_life(Key2 pk, int dp, float vx, float vy, uint32_t k, float hv, int reach,
@@ -476,7 +477,7 @@ __device__ __forceinline__ bool covers_for_life(Key2 pk, int dp, float vx, float
   if (dir == 0 ? x + lj < xi + reach : x - lj > xi - reach) return false;  // the piece expires first
   const float hp = __ldg(&A.Hf[dp * A.hs]);
   if (!(hp > hv)) return false;
-  const float px = trunc32(pk.x), py = trunc32(pk.y);
+  const float px = trunc32(pk.x, A.off), py = trunc32(pk.y, A.off);
   const float m = fmaxf(fmaxf(px - vx, vy - py), 0.f);
   const float eps = 4.76837158203125e-7f * (fabsf(px) + fabsf(vx) + fabsf(py) + fabsf(vy) + hp + hv);
   return hp - hv - m >= eps;
@@ -695,7 +696,7 @@ __global__ void __launch_bounds__(kE2Threads, BIG ? 5 : 1) k_env2(E2Args A, int 
             // column, 3.34 s every other one, 3.41 s every fourth; two candidates instead of four: 3.55 s)
             bool dom = false;
             if ((x & 1) == 0) {
-              const float vx = trunc32(v.x), vy = trunc32(v.y);
+              const float vx = trunc32(v.x, A.off), vy = trunc32(v.y, A.off);
               const int di = (int)(k >> 24), xi = (int)(k & 0xffffffu);
               const float hv = __ldg(&A.Hf[di * A.hs + (dir == 0 ? x - xi : xi - x)]);
               const int reach = __ldg(&A.Dx[di]);
@@ -1082,7 +1083,7 @@ int dilate_envelope(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out,
     cudaEventRecord(e1, ctx->stream);
     if (!rc && !fallback) {
       E2Args a2{nx, yb0, Dy, W, (nx + segs2 - 1) / segs2, segs2, T->Hp, T->host.hs, T->H, T->Dx, poff, nF, pz, pd,
-                slots, counts, ctx->d_flags, list, nullptr, nullptr, cap2, ghist, hstride};
+                slots, counts, ctx->d_flags, list, nullptr, nullptr, cap2, value_offset(g), ghist, hstride};
       cudaMemsetAsync(ctx->d_flags, 0, 3 * sizeof(int), ctx->stream);
       // The global-memory sweep runs five row segments per SM against one in shared memory (227 KB per
       // block); with at least two per SM to run it is the faster one (1024^2 spheres, r = 16, whole rows:

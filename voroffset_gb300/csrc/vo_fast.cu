@@ -1223,13 +1223,15 @@ __device__ __noinline__ int big_union(const FastArgs &A, int x, int y, double2 *
 // negated value, the blocks that are done, whether values lie beyond); a pass of its own over the
 // values took 0.5 ms at 2048^2. A block per row: it loads what it needs of five
 // columns, and is bound by the latency of that (0.7 ms at 2048^2).
-template <bool SLOTS, bool RECORDS>
+template <bool SLOTS, bool RECORDS, bool SHIFT>
 __global__ void __launch_bounds__(kPrepThreads) k_widths(int nx, int ny, const int32_t *__restrict__ beg,
                                                               const int32_t *__restrict__ end,
                                                               const longlong2 *__restrict__ z, uint4 *__restrict__ rec,
                                                               longlong2 *__restrict__ rz, int32_t *__restrict__ rbeg,
                                                               int32_t *__restrict__ rend, uint2 *__restrict__ wide,
-                                                              float R, unsigned long long *mm, FastPar *par) {
+                                                              float R, unsigned long long *mm, FastPar *par,
+                                                              const double offset) {
+  const double off = SHIFT ? offset : 0.0;
   __shared__ int s_sum[kPrepThreads / 32];
   const int y = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int base = SLOTS ? beg[nx * y] : 0;
@@ -1274,7 +1276,7 @@ __global__ void __launch_bounds__(kPrepThreads) k_widths(int nx, int ny, const i
         range.take(v.x);
         range.take(v.y);
       }
-      const float lo = trunc32_bits(v.x), hi = trunc32_bits(v.y);
+      const float lo = trunc32_bits(v.x, off), hi = trunc32_bits(v.y, off);
       unsigned w[4];
 #pragma unroll
       for (int d = 0; d < 4; ++d) {
@@ -1284,14 +1286,14 @@ __global__ void __launch_bounds__(kPrepThreads) k_widths(int nx, int ny, const i
         longlong2 u = make_longlong2(0, 0);
         for (; j < ne[d]; ++j) {
           u = z[j];
-          if (!(trunc32_bits(u.y) < lo)) break;
+          if (!(trunc32_bits(u.y, off) < lo)) break;
         }
         nb[d] = j;
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
           if (j + q < ne[d]) {
             if (q) u = z[j + q];
-            const float a = trunc32_bits(u.x), b = trunc32_bits(u.y);
+            const float a = trunc32_bits(u.x, off), b = trunc32_bits(u.y, off);
             const float e = 4.76837158203125e-7f * (fabsf(a) + fabsf(b) + fabsf(lo) + fabsf(hi)) + 1e-30f;
             best = fminf(best, fmaxf(fmaxf(a - lo, hi - b), 0.f) + e);
           }
@@ -1359,7 +1361,7 @@ __device__ __noinline__ void beyond_list(const BatchVol &V, int x, int y) {
 // are; but their number grows more slowly. Both take the same between 290 and
 // 580 candidates per column: the line of direct_choice is 450. (In FP64
 // throughout, without the neighbours' test, 1024^2 took 0.53, 1.1 and 1.9 ms.)
-template <int G>
+template <int G, bool SHIFT>
 __global__ void __launch_bounds__(128, 8) k_direct(const BatchVol *__restrict__ vols, int nv) {
   __shared__ BatchVol V;
   __shared__ bool s_undone;
@@ -1403,7 +1405,7 @@ __global__ void __launch_bounds__(128, 8) k_direct(const BatchVol *__restrict__ 
     n = at.x < 0 ? -1 : at.y;
   };
   auto inner = [&](Key2 u) {
-    const float lo = trunc32(u.x), hi = trunc32(u.y);
+    const float lo = SHIFT ? trunc32(u.x, V.A.off) : trunc32(u.x), hi = SHIFT ? trunc32(u.y, V.A.off) : trunc32(u.y);
     const float e = 9.5367431640625e-07f * (fabsf(lo) + fabsf(hi) + reach);
     return make_float2(lo + e, hi - e);
   };
@@ -1679,17 +1681,19 @@ void fast_prepare(cudaStream_t st, const FastArgs &A, float R, double mean_segs,
   const double most = 2.2 * mean_segs * kTile * std::min(kTile, A.ny);
   const int warps = most <= kPackSort / 32 ? 32 : most <= kPackSort / 16 ? 16 : 8;
   auto *pack = warps == 32 ? &k_pack<32> : warps == 16 ? &k_pack<16> : &k_pack<8>;
-  k_widths<false, false><<<A.ny, kPrepThreads, 0, st>>>(A.nx, A.ny, A.beg, A.end, reinterpret_cast<const longlong2 *>(z),
-                                                        nullptr, nullptr, nullptr, nullptr, out.wide, R, mm, out.par);
+  (A.off != 0.0 ? &k_widths<false, false, true> : &k_widths<false, false, false>)<<<A.ny, kPrepThreads, 0, st>>>(
+      A.nx, A.ny, A.beg, A.end, reinterpret_cast<const longlong2 *>(z), nullptr, nullptr, nullptr, nullptr, out.wide, R, mm,
+      out.par, A.off);
   pack<<<(A.ny + kTile - 1) / kTile, 32 * warps, 0, st>>>(A.nx, A.ny, A.beg, A.end, z, out.par, out.zf, out.wide, out.code,
                                                           out.zx, out.cl, out.coff);
 }
 
-FastArgs fast_args(int nx, int ny, const DeviceTables &T, const int32_t *beg, const int32_t *end, const double2 *z,
+FastArgs fast_args(const vo_grid &g, const DeviceTables &T, const int32_t *beg, const int32_t *end, const double2 *z,
                    const PackOut &out) {
+  const int nx = g.nx, ny = g.ny;
   return FastArgs{nx,  ny,  T.host.W, T.host.Dy, T.host.hs, beg, end, (const double *)z, out.zf, out.code,
                   (const double *)out.zx, out.cl, out.coff, T.Hp, T.H, T.Dx, out.par, out.rec, out.zx ? out.zx : z,
-                  out.zx ? out.rbeg : beg, out.zx ? out.rbeg + (size_t)nx * ny : end};
+                  out.zx ? out.rbeg : beg, out.zx ? out.rbeg + (size_t)nx * ny : end, value_offset(g)};
 }
 
 // Threads per column: the line is explained at k_direct.
@@ -1703,21 +1707,21 @@ int direct_blocks(const vo_grid &g, int64_t launch_cols) {
 void direct_prepare(cudaStream_t st, const FastArgs &A, const PackOut &out) {
   if (A.ny <= 0) return;
   const longlong2 *z = reinterpret_cast<const longlong2 *>(A.zd);
-  if (out.zx)
-    k_widths<true, true><<<A.ny, kPrepThreads, 0, st>>>(A.nx, A.ny, A.beg, A.end, z, out.rec,
-                                                        reinterpret_cast<longlong2 *>(out.zx), out.rbeg,
-                                                        out.rbeg + (size_t)A.nx * A.ny, nullptr, 0.f, nullptr, nullptr);
-  else
-    k_widths<false, true><<<A.ny, kPrepThreads, 0, st>>>(A.nx, A.ny, A.beg, A.end, z, out.rec, nullptr, nullptr, nullptr,
-                                                         nullptr, 0.f, nullptr, nullptr);
+  const bool shift = A.off != 0.0;
+  auto *widths = out.zx ? (shift ? &k_widths<true, true, true> : &k_widths<true, true, false>)
+                        : (shift ? &k_widths<false, true, true> : &k_widths<false, true, false>);
+  widths<<<A.ny, kPrepThreads, 0, st>>>(A.nx, A.ny, A.beg, A.end, z, out.rec, reinterpret_cast<longlong2 *>(out.zx), out.rbeg,
+                                        out.zx ? out.rbeg + (size_t)A.nx * A.ny : nullptr, nullptr, 0.f, nullptr, nullptr,
+                                        A.off);
 }
 static size_t direct_table(int nx, int ny, int W, int Dy) {
   return sizeof(float2) * (size_t)std::min(W, nx) * (std::min(Dy, ny - 1) + 1);
 }
 size_t direct_smem(const FastArgs &A) { return direct_table(A.nx, A.ny, A.W, A.Dy); }
-void direct_launch(cudaStream_t st, const BatchVol *vols, int nv, int blocks, int64_t launch_cols, size_t smem) {
-  const int split = direct_split(launch_cols);
-  (split == 1 ? &k_direct<1> : &k_direct<kSplit>)<<<blocks, 128, smem + sizeof(float2) * kList * 128, st>>>(vols, nv);
+void direct_launch(cudaStream_t st, const BatchVol *vols, int nv, int blocks, int64_t launch_cols, size_t smem, bool shift) {
+  auto *f = direct_split(launch_cols) == 1 ? (shift ? &k_direct<1, true> : &k_direct<1, false>)
+                                           : (shift ? &k_direct<kSplit, true> : &k_direct<kSplit, false>);
+  f<<<blocks, 128, smem + sizeof(float2) * kList * 128, st>>>(vols, nv);
 }
 
 double reach_columns(const vo_grid &g, const DeviceTables &T) {
@@ -1829,7 +1833,7 @@ int dilate_fast(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out, vo_
   };
   auto describe = [&](Engine e) {
     BatchVol &V = head.V;
-    V.A = fast_args(nx, ny, *T, in->offs, in->offs + 1, in->z, pk);
+    V.A = fast_args(g, *T, in->offs, in->offs + 1, in->z, pk);
     V.obeg = obeg;
     V.oend = obeg + ncols;
     V.oz = oz;
@@ -1868,7 +1872,7 @@ int dilate_fast(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out, vo_
     cudaEventRecord(ctx->ev[1], ctx->stream);
     cudaEventRecord(ctx->ev[4], ctx->stream);
     if (engine == Engine::kDirect)
-      direct_launch(ctx->stream, dv, 1, head.V.item1, ncols, direct_smem(head.V.A));
+      direct_launch(ctx->stream, dv, 1, head.V.item1, ncols, direct_smem(head.V.A), head.V.A.off != 0.0);
     else if (engine == Engine::kPatches)
       patch_launch(false, P, ctx->stream, dv);
     else

@@ -229,6 +229,7 @@ struct FastArgs {
   const uint4 *rec;
   const double2 *rz;
   const int32_t *rbeg, *rend;
+  double off;  // value_offset of the grid
 };
 
 // Arguments of the columns kernel for one volume (vo_column.cu).
@@ -336,12 +337,13 @@ struct PatchPlan {
 int patch_split(const vo_grid *const *grids, int n);
 // Small radii: whether a dilation meets its candidates column by column
 // (k_direct; its prepared inputs are not needed then), the launch over the nv
-// dilations vols and its blocks for a grid. launch_cols: columns of all of them.
+// dilations vols and its blocks for a grid. launch_cols: columns of all of them;
+// shift: whether one of them has an offset (FastArgs::off).
 bool direct_choice(const vo_grid &g, const DeviceTables &T, double mean_segs);
 double reach_columns(const vo_grid &g, const DeviceTables &T);  // source columns in reach of a column, on average
 int direct_blocks(const vo_grid &g, int64_t launch_cols);
 size_t direct_smem(const FastArgs &A);
-void direct_launch(cudaStream_t st, const BatchVol *vols, int nv, int blocks, int64_t launch_cols, size_t smem);
+void direct_launch(cudaStream_t st, const BatchVol *vols, int nv, int blocks, int64_t launch_cols, size_t smem, bool shift);
 int64_t patch_total(const vo_grid *const *grids, int n);  // with one lane per column
 int patch_count(const vo_grid &g, int split);
 // Grids of a launch over nitems patches; the working memory of each tier is
@@ -370,7 +372,7 @@ struct PackOut {
 size_t pack_offsets(const vo_grid &g);
 // Prepares the input of k_direct (pk.rec).
 void direct_prepare(cudaStream_t st, const FastArgs &A, const PackOut &out);
-FastArgs fast_args(int nx, int ny, const DeviceTables &T, const int32_t *beg, const int32_t *end, const double2 *z,
+FastArgs fast_args(const vo_grid &g, const DeviceTables &T, const int32_t *beg, const int32_t *end, const double2 *z,
                    const PackOut &out);
 // Packs the input of a dilation (CSR or slots in column order). mm: four words of scratch.
 void fast_prepare(cudaStream_t st, const FastArgs &A, float R, double mean_segs, unsigned long long *mm,
@@ -389,6 +391,14 @@ int morph_batched_fast(vo_ctx *ctx, int n, const int *ops, const double *radii, 
 // array of ntiles x VO_SIZER_FEATURES, and predictions (ntiles x 4, three used).
 int sizer_features_device(vo_ctx *ctx, const SlotVol &in, double radius, float *feats, int *ntiles);
 int sizer_predict_device(vo_ctx *ctx, const vo_sizer *s, const float *feats, int n, float *out4);
+
+// A value near those of a volume over the grid, from its origin: 0 below the magnitude from which taking it off pays
+// (1024^2 spheres, r = 32, at 1e4: 3.83 ms without and 4.02 with it, at 1e5 4.17 and 4.01). It only makes filters
+// sharper, never decides a result.
+inline double value_offset(const vo_grid &g) {
+  const double z = g.origin[2] / g.spacing;
+  return z >= 32768.0 || z <= -32768.0 ? (z >= 1e15 || z <= -1e15 ? 0.0 : (double)(long long)z) : 0.0;
+}
 
 // Volume allocation (vo_api.cu).
 int volume_alloc(vo_ctx *ctx, const vo_grid &g, int64_t nseg, vo_volume **out);
@@ -447,6 +457,16 @@ __device__ __forceinline__ float trunc32_bits(Key b) {
   return __uint_as_float((hi & 0x80000000u) | f);
 }
 __device__ __forceinline__ float trunc32(Key k) { return trunc32_bits(k ^ ((k >> 63) & 0x7fffffffffffffffll)); }
+// The same of the value less `off` (value_offset): FP32 margins are parts of the
+// magnitude, and values far from zero leave none at all of a filter without it
+// (1024^2 spheres, r = 5: 2.8 ms at z = 0, 6.2 at 1e6). The difference is within
+// 2^-53 of itself, which the margins cover. Without an offset, integer operations only.
+__device__ __forceinline__ float trunc32_bits(Key b, double off) {
+  return trunc32_bits(off == 0.0 ? b : __double_as_longlong(__dsub_rn(__longlong_as_double(b), off)));
+}
+__device__ __forceinline__ float trunc32(Key k, double off) {
+  return trunc32_bits(k ^ ((k >> 63) & 0x7fffffffffffffffll), off);
+}
 __device__ __forceinline__ Key kmax(Key a, Key b) { return a > b ? a : b; }
 __device__ __forceinline__ Key kmin(Key a, Key b) { return a < b ? a : b; }
 
