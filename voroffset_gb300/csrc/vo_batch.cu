@@ -113,6 +113,7 @@ struct vo_batch {
   };
   std::vector<Round> rounds;
   bool once = false;  // a plan for one run: its steps run as they are recorded, with no graph
+  std::vector<std::pair<cudaEvent_t, cudaEvent_t>> stretches;  // when they did (run_pending)
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   std::vector<vo_volume *> rerun;
@@ -131,9 +132,22 @@ int plan_alloc(vo_ctx *ctx, vo_batch *b, T **p, size_t n) {
   return rc;
 }
 
-// Runs the recorded closures not yet run.
+// Runs the recorded closures not yet run. Of a plan for one run each such stretch is timed: its run reports the
+// steps' time on the device, without the planning between them.
 void run_pending(vo_ctx *ctx, vo_batch *b) {
+  if (b->executed == b->rec.size()) return;
+  cudaEvent_t from = nullptr, to = nullptr;
+  if (b->once && (cudaEventCreate(&from) != cudaSuccess || cudaEventCreate(&to) != cudaSuccess)) {
+    cudaGetLastError();  // a stretch without its time
+    if (from) cudaEventDestroy(from);
+    from = nullptr;
+  }
+  if (from) cudaEventRecord(from, ctx->stream);
   for (; b->executed < b->rec.size(); ++b->executed) b->rec[b->executed](ctx->stream);
+  if (from) {
+    cudaEventRecord(to, ctx->stream);
+    b->stretches.push_back({from, to});
+  }
 }
 
 void record(vo_batch *b, int kernels, Launch f) {
@@ -539,6 +553,10 @@ int plan_dilation_round(vo_ctx *ctx, vo_batch *b, std::vector<DilPlan> &dils, bo
 }
 
 void plan_free(vo_ctx *ctx, vo_batch *b) {
+  for (const auto &s : b->stretches) {
+    cudaEventDestroy(s.first);
+    cudaEventDestroy(s.second);
+  }
   if (b->exec) cudaGraphExecDestroy(b->exec);
   if (b->graph) cudaGraphDestroy(b->graph);
   for (SlotVol &s : b->owned) slot_free(ctx, s);
@@ -731,7 +749,6 @@ int create(vo_ctx *ctx, int n, const int *ops, const double *radii, int method, 
   cudaSetDevice(ctx->device);
   for (int i = 0; i < n; ++i) vol_wait(ctx, ins[i]);  // before any capture: the plan then reads them in order
   ctx->err.clear();
-  cudaEventRecord(ctx->ev[0], ctx->stream);
   const auto t0 = std::chrono::steady_clock::now();
   vo_batch *b = new vo_batch();
   b->n = n;
@@ -778,8 +795,8 @@ int vo_batch_run(vo_ctx *ctx, vo_batch *b, vo_timings *tm) {
   if (!b->once) {
     cudaEventRecord(ctx->ev[0], ctx->stream);
     VO_CK(ctx, cudaGraphLaunch(b->exec, ctx->stream));
+    cudaEventRecord(ctx->ev[1], ctx->stream);
   }
-  cudaEventRecord(ctx->ev[1], ctx->stream);
   cudaMemcpyAsync(flags.data(), b->d_flags, sizeof(int) * (n + 1), cudaMemcpyDeviceToHost, ctx->stream);
   for (const vo_batch::Round &r : b->rounds) {
     counters.emplace_back(kRoundCounters + kDilCounters * r.caps.size());
@@ -788,7 +805,11 @@ int vo_batch_run(vo_ctx *ctx, vo_batch *b, vo_timings *tm) {
   }
   VO_CK(ctx, cudaStreamSynchronize(ctx->stream));
   float graph_ms = 0;
-  cudaEventElapsedTime(&graph_ms, ctx->ev[0], ctx->ev[1]);
+  if (!b->once) cudaEventElapsedTime(&graph_ms, ctx->ev[0], ctx->ev[1]);
+  for (const auto &s : b->stretches) {
+    float ms = 0;
+    if (cudaEventElapsedTime(&ms, s.first, s.second) == cudaSuccess) graph_ms += ms;
+  }
   // spill use of every dilation (the largest fraction and its round)
   b->stats.spill_peak = 0;
   b->stats.spill_peak_round = -1;
