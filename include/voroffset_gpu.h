@@ -164,10 +164,12 @@ typedef struct vo_batch vo_batch;
 typedef struct {
   int64_t slot_bytes;   /* output slot memory of the dilations */
   int32_t tiles;        /* work-queue items over all rounds */
-  int32_t tile_rows;    /* lanes per column of the patch kernel (last round): 1 or 4 */
-  int32_t union_cap;    /* union slots per column of the patch kernel's first tier: 64, one of them spare */
-  int32_t persistent;   /* 1: one wave of blocks pulling queue items */
-  int32_t regs;         /* register budget per thread of the patch kernel */
+  /* of the last round's main kernel: the patch kernel if any dilation takes it, else the per-column kernel, else the
+   * small-radius kernel */
+  int32_t tile_rows;    /* lanes that share a column: 1 or 4 */
+  int32_t union_cap;    /* union slots per column */
+  int32_t persistent;   /* 1: one wave of blocks pulling queue items (the patch kernel), 0: a block per item */
+  int32_t regs;         /* registers per thread, as compiled */
   int32_t graph_nodes;  /* nodes of the captured graph */
   int32_t graph_kernels;/* kernel launches per replay */
   int32_t learned;      /* 1 when slots and queue came from a sizer */

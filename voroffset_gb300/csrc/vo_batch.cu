@@ -543,10 +543,13 @@ int plan_dilation_round(vo_ctx *ctx, vo_batch *b, std::vector<DilPlan> &dils, bo
   record(b, (np > 0 ? 2 : 0) + (nc > 0 ? 2 : 0) + (np + nc > 0 ? 1 : 0) + (nd > 0 ? 1 : 0), [launch, L](cudaStream_t st) { launch(L, st); });
   b->rounds.push_back({counters, {}});
   for (const DilPlan &d : dils) b->rounds.back().caps.push_back(d.spill_cap);
-  b->stats.tile_rows = split;
-  b->stats.union_cap = kUnionCapMid / 2;
-  b->stats.persistent = 1;
-  b->stats.regs = 96;
+  if (!b->once) {
+    const KernelShape s = np > 0 ? patch_shape(split) : nc > 0 ? column_shape(slots, nc == 1) : direct_shape(direct_cols, direct_shift);
+    b->stats.tile_rows = s.lanes;
+    b->stats.union_cap = s.slots;
+    b->stats.persistent = np > 0 ? 1 : 0;
+    b->stats.regs = s.regs;
+  }
   b->stats.tiles += L.P.nitems + L.column_items + L.direct_items;
   if (later_rounds) run_pending(ctx, b);
   return VO_OK;

@@ -680,6 +680,11 @@ static auto *column_kernel(int slots) {
   return slots == 64 ? &k_column<64, SINGLE>
          : slots == 48 ? &k_column<48, SINGLE> : slots == 32 ? &k_column<32, SINGLE> : &k_column<24, SINGLE>;
 }
+KernelShape column_shape(int slots, bool single) {
+  cudaFuncAttributes a{};
+  cudaFuncGetAttributes(&a, single ? column_kernel<true>(slots) : column_kernel<false>(slots));
+  return KernelShape{1, slots, a.numRegs};
+}
 void column_launch(cudaStream_t st, const BatchVol *vols, int nv, int blocks, int slots, const ColumnArgs &A) {
   (nv == 1 ? column_kernel<true>(slots) : column_kernel<false>(slots))<<<blocks, kBlockCols,
                                                                         sizeof(float2) * slots * kBlockCols, st>>>(vols, nv, A);

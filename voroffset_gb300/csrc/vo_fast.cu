@@ -1615,6 +1615,12 @@ PatchFn patch_fn(bool big, int split) {
 }
 }  // namespace
 
+KernelShape patch_shape(int split) {
+  cudaFuncAttributes a{};
+  cudaFuncGetAttributes(&a, patch_fn(false, split));
+  return KernelShape{split, kUnion, a.numRegs};
+}
+
 void patch_launch(bool big, const PatchPlan &P, cudaStream_t st, const BatchVol *vols) {
   patch_fn(big, P.split)<<<P.grid[big], 32, patch_smem(P.hs_max), st>>>(vols, P.nitems, P.Q, P.hs_max, P.scratch[big]);
 }
@@ -1718,10 +1724,17 @@ static size_t direct_table(int nx, int ny, int W, int Dy) {
   return sizeof(float2) * (size_t)std::min(W, nx) * (std::min(Dy, ny - 1) + 1);
 }
 size_t direct_smem(const FastArgs &A) { return direct_table(A.nx, A.ny, A.W, A.Dy); }
+static auto *direct_kernel(int64_t launch_cols, bool shift) {
+  return direct_split(launch_cols) == 1 ? (shift ? &k_direct<1, true> : &k_direct<1, false>)
+                                        : (shift ? &k_direct<kSplit, true> : &k_direct<kSplit, false>);
+}
+KernelShape direct_shape(int64_t launch_cols, bool shift) {
+  cudaFuncAttributes a{};
+  cudaFuncGetAttributes(&a, direct_kernel(launch_cols, shift));
+  return KernelShape{direct_split(launch_cols), kDirectCap, a.numRegs};
+}
 void direct_launch(cudaStream_t st, const BatchVol *vols, int nv, int blocks, int64_t launch_cols, size_t smem, bool shift) {
-  auto *f = direct_split(launch_cols) == 1 ? (shift ? &k_direct<1, true> : &k_direct<1, false>)
-                                           : (shift ? &k_direct<kSplit, true> : &k_direct<kSplit, false>);
-  f<<<blocks, 128, smem + sizeof(float2) * kList * 128, st>>>(vols, nv);
+  direct_kernel(launch_cols, shift)<<<blocks, 128, smem + sizeof(float2) * kList * 128, st>>>(vols, nv);
 }
 
 double reach_columns(const vo_grid &g, const DeviceTables &T) {

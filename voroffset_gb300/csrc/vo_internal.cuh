@@ -378,6 +378,14 @@ FastArgs fast_args(const vo_grid &g, const DeviceTables &T, const int32_t *beg, 
 void fast_prepare(cudaStream_t st, const FastArgs &A, float R, double mean_segs, unsigned long long *mm,
                   const PackOut &out);
 
+// What a launch of one of them is like: lanes that share a column, union slots per column, registers per thread.
+struct KernelShape {
+  int lanes = 0, slots = 0, regs = 0;
+};
+KernelShape patch_shape(int split);
+KernelShape direct_shape(int64_t launch_cols, bool shift);
+KernelShape column_shape(int slots, bool single);
+
 // Which kernel a dilation takes first: k_direct, k_patch or k_column.
 enum class Engine { kDirect, kPatches, kColumns };
 constexpr int kFewColumns = 4096;  // columns beyond k_direct's list up to which the FP64 tier takes them as they are
