@@ -470,6 +470,7 @@ __device__ __forceinline__ bool live(uint32_t k, int x, int dir, const E2Args &A
 // FP32 on values less the grid's offset, within 2^-23 of theirs (trunc32), and tables within 2^-24; eps
 // bounds those errors, the roundings of the differences and the table errors
 // four times over.
+template <bool SHIFT>
 __device__ __forceinline__ bool covers_for_life(Key2 pk, int dp, float vx, float vy, uint32_t k, float hv, int reach,
                                                 int x, int dir, const E2Args &A) {
   const int xi = (int)(k & 0xffffffu);
@@ -477,7 +478,7 @@ __device__ __forceinline__ bool covers_for_life(Key2 pk, int dp, float vx, float
   if (dir == 0 ? x + lj < xi + reach : x - lj > xi - reach) return false;  // the piece expires first
   const float hp = __ldg(&A.Hf[dp * A.hs]);
   if (!(hp > hv)) return false;
-  const float px = trunc32(pk.x, A.off), py = trunc32(pk.y, A.off);
+  const float px = SHIFT ? trunc32(pk.x, A.off) : trunc32(pk.x), py = SHIFT ? trunc32(pk.y, A.off) : trunc32(pk.y);
   const float m = fmaxf(fmaxf(px - vx, vy - py), 0.f);
   const float eps = 4.76837158203125e-7f * (fabsf(px) + fabsf(vx) + fabsf(py) + fabsf(vy) + hp + hv);
   return hp - hv - m >= eps;
@@ -572,7 +573,7 @@ __device__ int warp_union_two(const Key2 *U1, int n1, const Key2 *U2, int n2, Ke
   return outn > cap ? -1 : outn;
 }
 
-template <bool BIG>
+template <bool BIG, bool SHIFT>
 __global__ void __launch_bounds__(kE2Threads, BIG ? 5 : 1) k_env2(E2Args A, int nitems) {
   extern __shared__ __align__(16) unsigned char e2_smem[];
   __shared__ uint64_t bar[2];
@@ -696,14 +697,14 @@ __global__ void __launch_bounds__(kE2Threads, BIG ? 5 : 1) k_env2(E2Args A, int 
             // column, 3.34 s every other one, 3.41 s every fourth; two candidates instead of four: 3.55 s)
             bool dom = false;
             if ((x & 1) == 0) {
-              const float vx = trunc32(v.x, A.off), vy = trunc32(v.y, A.off);
+              const float vx = SHIFT ? trunc32(v.x, A.off) : trunc32(v.x), vy = SHIFT ? trunc32(v.y, A.off) : trunc32(v.y);
               const int di = (int)(k >> 24), xi = (int)(k & 0xffffffu);
               const float hv = __ldg(&A.Hf[di * A.hs + (dir == 0 ? x - xi : xi - x)]);
               const int reach = __ldg(&A.Dx[di]);
-              dom = cF > 0 && covers_for_life(F[cF - 1], Fd[cF - 1], vx, vy, k, hv, reach, x, dir, A);
-              dom = dom || (cF < f && covers_for_life(F[cF], Fd[cF], vx, vy, k, hv, reach, x, dir, A));
-              dom = dom || (cB > 0 && covers_for_life(B[cB - 1], Bd[cB - 1], vx, vy, k, hv, reach, x, dir, A));
-              dom = dom || (cB < b && covers_for_life(B[cB], Bd[cB], vx, vy, k, hv, reach, x, dir, A));
+              dom = cF > 0 && covers_for_life<SHIFT>(F[cF - 1], Fd[cF - 1], vx, vy, k, hv, reach, x, dir, A);
+              dom = dom || (cF < f && covers_for_life<SHIFT>(F[cF], Fd[cF], vx, vy, k, hv, reach, x, dir, A));
+              dom = dom || (cB > 0 && covers_for_life<SHIFT>(B[cB - 1], Bd[cB - 1], vx, vy, k, hv, reach, x, dir, A));
+              dom = dom || (cB < b && covers_for_life<SHIFT>(B[cB], Bd[cB], vx, vy, k, hv, reach, x, dir, A));
             }
             Tz[pos] = v;
             Tk[pos] = dom ? kDeadKey : k;
@@ -913,7 +914,10 @@ int dilate_envelope(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out,
   }
   cudaFuncSetAttribute(k_env1<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e1_smem_bytes(false));
   cudaFuncSetAttribute(k_env1<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e1_smem_bytes(false));
-  cudaFuncSetAttribute(k_env2<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e2_smem_bytes(false));
+  const double off = value_offset(g);
+  auto *const env2_small = off != 0.0 ? &k_env2<false, true> : &k_env2<false, false>;
+  auto *const env2_big = off != 0.0 ? &k_env2<true, true> : &k_env2<true, false>;
+  cudaFuncSetAttribute(env2_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e2_smem_bytes(false));
   int32_t *nF = nullptr, *nB = nullptr, *counts = nullptr, *bcnt = nullptr, *list = nullptr;
   long long *rowp = nullptr;
   double2 *slots = nullptr;
@@ -1083,7 +1087,7 @@ int dilate_envelope(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out,
     cudaEventRecord(e1, ctx->stream);
     if (!rc && !fallback) {
       E2Args a2{nx, yb0, Dy, W, (nx + segs2 - 1) / segs2, segs2, T->Hp, T->host.hs, T->H, T->Dx, poff, nF, pz, pd,
-                slots, counts, ctx->d_flags, list, nullptr, nullptr, cap2, value_offset(g), ghist, hstride};
+                slots, counts, ctx->d_flags, list, nullptr, nullptr, cap2, off, ghist, hstride};
       cudaMemsetAsync(ctx->d_flags, 0, 3 * sizeof(int), ctx->stream);
       // The global-memory sweep runs five row segments per SM against one in shared memory (227 KB per
       // block); with at least two per SM to run it is the faster one (1024^2 spheres, r = 16, whole rows:
@@ -1094,7 +1098,7 @@ int dilate_envelope(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out,
       if (items2 >= 2 * std::max(sms, 1) || mean_pieces * (Dy + 1) / 3.0 > 0.6 * cap2) {
         k_list_rows<<<(items2 + 255) / 256, 256, 0, ctx->stream>>>(items2, list, ctx->d_flags);
       } else {
-        k_env2<false><<<items2, kE2Threads, e2_smem_bytes(false), ctx->stream>>>(a2, items2);
+        env2_small<<<items2, kE2Threads, e2_smem_bytes(false), ctx->stream>>>(a2, items2);
       }
       ctx->launches += 1;
       rc = flags_now();
@@ -1119,7 +1123,7 @@ int dilate_envelope(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out,
           ab.gz = gz2;
           ab.gk = gk2;
           ab.list = list + r0;
-          k_env2<true><<<cnt, kE2Threads, e2_smem_bytes(true), ctx->stream>>>(ab, cnt);
+          env2_big<<<cnt, kE2Threads, e2_smem_bytes(true), ctx->stream>>>(ab, cnt);
           ctx->launches += 1;
           rc = flags_now();
         }
