@@ -22,6 +22,7 @@ int main(int, char **argv) {
   const int64_t rich = atoll(argv[5]);                        // how many have many
   if (rich * many + (ncols - rich) * few > kSegmentsMost) return 3;
   SlotLayout s = slots_first(ncols, mean);
+  if (atoi(argv[6])) slots_many(ncols, s);
   for (int run = 0; run < 3; ++run) {
     if (s.cap < 1 || s.cap * ncols + s.spill > kSlotMost) return 4;
     const int64_t need = (many > s.cap ? rich * many : 0) + (few > s.cap ? (ncols - rich) * few : 0);
@@ -48,7 +49,9 @@ CASES = [(1, 1.0, 500, 0, 1), (4096, 3.0, 8000, 1, 4096), (LARGEST, 1.0, 31, 31,
          (LARGEST - 1, 30.0, 65, 0, 33_000_000), (LARGEST, 6.5, 33, 31, 1_000_000), (50_000_000, 40.0, 60, 42, 600_000)]
 
 
+# `large`: from the layout for inputs most of whose columns have large unions
+@pytest.mark.parametrize("large", [0, 1])
 @pytest.mark.parametrize("ncols,mean,many,few,rich", CASES)
-def test_any_result_gets_its_slots(program, ncols, mean, many, few, rich):
-    r = subprocess.run([program, str(ncols), str(mean), str(many), str(few), str(rich)])
+def test_any_result_gets_its_slots(program, ncols, mean, many, few, rich, large):
+    r = subprocess.run([program, str(ncols), str(mean), str(many), str(few), str(rich), str(large)])
     assert r.returncode == 0
