@@ -10,6 +10,8 @@
 // eagerly only when a later step needs the data (the input features of a
 // learned-sized dilation, the capacity of a complement of a dilation result).
 // Per dilation:
+//   * the kernel: patches, the small-radius kernel or the per-column kernel, as
+//     a single dilation chooses it (a sample of the input may be taken);
 //   * output slots: with a sizer attached, every 32 x 32 tile of output
 //     columns gets the capacity the network predicts for its largest union
 //     (plus a margin, at most kUnionCapMid); without one, every column gets
@@ -23,12 +25,12 @@
 //     context).
 // Then the closures are captured into one graph. vo_batch_run replays it and
 // re-runs, through the single-volume path, every volume whose overflow flag
-// is set (a union larger than its slot with the spill region exhausted, or
-// beyond the FP64 tier's or the small-radius kernel's list), so results never
-// depend on the predictions. vo_morph_batched, which runs a plan once, runs each
+// is set (a union larger than its slot with the spill region exhausted, beyond the
+// FP64 lists, or more unions beyond the first kernel's lists than the round's tiers
+// take), so results never depend on the predictions. vo_morph_batched, which runs a plan once, runs each
 // step once, as it is planned, without a graph (24 mixed volumes: 18.1 ms
 // against 26.8 with a capture and a replay; one of 1001^2 columns and 19 segments
-// each: 18.9 against 23.1).
+// each: 18.9 against 23.1); its stretches of steps are timed one by one.
 #include <algorithm>
 #include <chrono>
 #include <cmath>

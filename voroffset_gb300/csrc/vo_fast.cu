@@ -69,7 +69,7 @@
 //
 // Capacities: a patch that needs more entries, kept-aside intervals or union
 // intervals than the launch has re-runs with larger lists (second tier), if those
-// are few; if they are many their columns go to the columns kernel
+// are few; if they are many their columns go to the per-column kernel
 // (vo_column.cu), and if they are most, all of the dilation does: patches of
 // scattered short intervals spend their time on intervals kept aside. A column
 // that outgrows the larger lists too goes to an FP64 kernel with an

@@ -63,7 +63,7 @@ struct DeviceTables {
   float *Hp = nullptr;
   int *Dx = nullptr;
   double *HB = nullptr;
-  // for the columns kernel, made when it is first used (column_tables)
+  // for the per-column kernel, made when it is first used (column_tables)
   float4 *prec = nullptr;
   int npairs = 0;
   DomLevels dom{};
@@ -232,7 +232,7 @@ struct FastArgs {
   double off;  // value_offset of the grid
 };
 
-// Arguments of the columns kernel for one volume (vo_column.cu).
+// Arguments of the per-column kernel for one volume (vo_column.cu).
 struct ColumnArgs {
   int nx, ny, W, npairs, mask_bits, unused;
   const int32_t *beg, *end;  // segments [beg[c], end[c]) of column c (CSR or slots)
@@ -266,7 +266,8 @@ struct BatchVol {
   unsigned *spill_used;
   int *big_list, *big_count;  // columns for the last tier (FP64)
   int *ovf;  // flags: 1 a union beyond the FP64 list, 4 spill region exhausted, 8 more unions beyond the lists than the tiers take
-  // The columns kernel: its arguments, and the columns with more intervals than it (or k_column_list's caller) holds.
+  // The per-column kernel: its arguments, and the columns for k_column_list: those with more intervals than it holds,
+  // or those of the first tier that the caller lists there.
   const ColumnArgs *column;
   int *over_list, *over_count;
   // More columns (k_direct) or patches (k_patch) than this beyond the first tier's lists: the rest of the dilation
@@ -308,7 +309,7 @@ void column_list_launch(cudaStream_t st, const BatchVol *vols, int nv);
 // A radius' pair records and dominance levels (DeviceTables::prec, ::dom).
 std::vector<float4> column_pairs(const Tables &h, DomLevels &L);
 int column_tables(vo_ctx *ctx, const DeviceTables *T);
-// Whether a dilation by that radius is to take the columns kernel first: where the sizes leave it open, a sample of
+// Whether a dilation by that radius is to take the per-column kernel first: where the sizes leave it open, a sample of
 // the input decides (synchronising). tables(T) makes T->prec and T->dom.
 int column_choice(vo_ctx *ctx, const vo_grid &g, const DeviceTables &T, double mean_segs, const int32_t *beg,
                   const int32_t *end, const double2 *z, const std::function<int()> &tables, bool *columns);
