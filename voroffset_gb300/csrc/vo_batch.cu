@@ -40,6 +40,7 @@
 #include <vector>
 
 #include "vo_internal.cuh"
+#include "vo_slots.h"
 
 using namespace vo;
 
@@ -353,7 +354,7 @@ int plan_dilation_round(vo_ctx *ctx, vo_batch *b, std::vector<DilPlan> &dils, bo
       return plan_column_tables(ctx, b, d.T);
     };
     rc = column_choice(ctx, g, *d.T, d.mean_segs, d.in.beg, d.in.end, d.in.z, tables, &columns);
-    if (columns) d.engine = Engine::kColumns;
+    if (columns || (d.engine == Engine::kPatches && (int64_t)entries > kPatchSegments)) d.engine = Engine::kColumns;
     if (!rc) rc = plan_alloc(ctx, b, &d.big_list, (size_t)ncols);
     if (rc) return rc;
     if (d.engine == Engine::kDirect) {

@@ -45,13 +45,19 @@ constexpr int kMidThreads = 32;
 // FP32 comparison falls inside the guard band or the output is written.
 template <int KA>
 struct UnionIds {
-  // (input value index, d | a << 8) of the lower / upper endpoint
+  // (input value index as unsigned bits, d | a << 8) of the lower / upper endpoint
   int2 lo[KA], hi[KA];
 };
 
+// The index of a segment's value among all: unsigned, an input has up to 2^31 - 1 segments.
+__device__ __forceinline__ int value_index(int k, bool upper) { return (int)(2u * (unsigned)k + (upper ? 1u : 0u)); }
+__device__ __forceinline__ double value_at(const double *z, int index) { return z[(unsigned)index]; }
+// FP32 copies of a segment's ends.
+__device__ __forceinline__ float2 copies_at(const float *zf, int k) { return reinterpret_cast<const float2 *>(zf)[k]; }
+
 __device__ __forceinline__ double exact_val(const ColumnArgs &A, int idx, int da, bool plus) {
   const double h = A.H64[(da & 255) * A.W + (da >> 8)];
-  const double z = A.zd[idx];
+  const double z = value_at(A.zd, idx);
   return plus ? __dadd_rn(z, h) : __dsub_rn(z, h);
 }
 
@@ -214,13 +220,13 @@ __device__ int fast_column(const ColumnArgs &A, float E, int x, int y, float2 *s
     float2 cv = make_float2(0.f, 0.f);
     int kn, sn;
     NEXT(kn, sn)
-    float2 znext = kn >= 0 ? *reinterpret_cast<const float2 *>(A.zf + 2 * kn) : make_float2(0.f, 0.f);
+    float2 znext = kn >= 0 ? copies_at(A.zf, kn) : make_float2(0.f, 0.f);
     for (int it = 0; it < iters; ++it) {
       if (it < total && !overflow) {
         const int k = kn, src = sn;
         const float2 zf = znext;
         NEXT(kn, sn)
-        if (kn >= 0) znext = *reinterpret_cast<const float2 *>(A.zf + 2 * kn);
+        if (kn >= 0) znext = copies_at(A.zf, kn);
         if (src != cur_src) {  // first candidate of a new source column: restart the cursor
           cur_src = src;
           cur = 0;
@@ -228,7 +234,7 @@ __device__ int fast_column(const ColumnArgs &A, float E, int x, int y, float2 *s
         }
         {
           const float lo = zf.x - h, hi = zf.y + h;
-          const int il = 2 * k, ih = 2 * k + 1;
+          const int il = value_index(k, false), ih = value_index(k, true);
           // skip union intervals that end strictly below the candidate: U.hi[cur] < lo
           // (the next interval's values are loaded one step ahead)
           if (lo - cv.y > E) {  // two intervals per step: cur < n here, so cur + 1 <= n

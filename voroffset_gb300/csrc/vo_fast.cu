@@ -1763,7 +1763,7 @@ int dilate_fast(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out, vo_
     bool columns = false;
     rc = column_choice(ctx, g, *T, mean_segs, in->offs, in->offs + 1, in->z, [&] { return column_tables(ctx, T); }, &columns);
     if (rc) return rc;
-    if (columns) engine = Engine::kColumns;
+    if (columns || (engine == Engine::kPatches && in->nseg > kPatchSegments)) engine = Engine::kColumns;
   }
   int union_slots = column_slots(mean_segs);
   SlotLayout slots = slots_first(ncols, mean_segs);

@@ -1,5 +1,5 @@
 // Output slots of a single dilation (dilate_fast): `cap` intervals for every
-// column, then a spill region for the columns with more. Host only.
+// column, then a spill region for the columns with more; and the largest input of patches. Host only.
 #pragma once
 #include <stdint.h>
 
@@ -15,6 +15,10 @@ struct SlotLayout {
 constexpr int64_t kSlotSpare = 4096;         // spill space beyond what is asked for
 constexpr int64_t kSlotMost = 4294967295LL;  // slot indices are unsigned 32-bit: columns and spill together
 constexpr int64_t kSegmentsMost = 2147483647LL;  // a result of more segments is refused
+
+// Inputs of up to so many segments (or slots) may go by patches, whose entries hold the index of a value, two per segment,
+// in a signed 32-bit integer; larger ones go by columns.
+constexpr int64_t kPatchSegments = 1LL << 30;
 
 // At first: from the input's mean segment count per column, with an eighth of the columns' slots to spill.
 inline SlotLayout slots_first(int64_t ncols, double mean_segs) {
