@@ -349,11 +349,7 @@ int plan_dilation_round(vo_ctx *ctx, vo_batch *b, std::vector<DilPlan> &dils, bo
     d.cost = 3.14159 * (R + 0.5) * (R + 0.5) * (d.mean_segs + 0.5);
     d.engine = (d.in.owns || d.in.end == d.in.beg + 1) && direct_choice(g, *d.T, d.mean_segs) ? Engine::kDirect : Engine::kPatches;
     bool columns = false;
-    auto tables = [&] {
-      run_pending(ctx, b);  // a sample is about to be taken of the input
-      return plan_column_tables(ctx, b, d.T);
-    };
-    rc = column_choice(ctx, g, *d.T, d.mean_segs, d.in.beg, d.in.end, d.in.z, tables, &columns);
+    rc = column_choice(ctx, g, *d.T, d.mean_segs, d.in.beg, d.in.end, d.in.z, [&] { run_pending(ctx, b); }, &columns);
     if (columns || (d.engine == Engine::kPatches && (int64_t)entries > kPatchSegments)) d.engine = Engine::kColumns;
     if (!rc) rc = plan_alloc(ctx, b, &d.big_list, (size_t)ncols);
     if (rc) return rc;

@@ -531,41 +531,47 @@ __global__ void k_dominance(int nx, int ny, const int32_t *__restrict__ beg, con
   col[c] = make_int4(k0, k1, (int)(h[0] | (h[1] << 16)), (int)(h[2] | (h[3] << 16)));
 }
 
-// Of kSampleColumns columns spread over the grid: their segments, times four, and how many of those (segment,
-// neighbour column) lie in a segment of that column widened by `growth`.
-constexpr int kSampleColumns = 8192;
-__global__ void __launch_bounds__(128) k_sample_held(int nx, int ny, const int32_t *__restrict__ beg,
-                                                     const int32_t *__restrict__ end, const double2 *__restrict__ z,
-                                                     double growth, int *out) {
-  const int i = blockIdx.x * 128 + threadIdx.x;
+// Of kSampleColumns columns spread over the grid the first kSampleSegs segments: how many pairs (segment, neighbour
+// column) there are and how many of those segments lie in one of that column widened by kSampleGrowth, block by block
+// to page-locked host memory. A thread per column and neighbour: the latency of its loads is what it takes.
+constexpr int kSampleColumns = 2048, kSampleThreads = 1024, kSampleBlocks = 4 * kSampleColumns / kSampleThreads;
+constexpr int kSampleSegs = 64;
+constexpr double kSampleGrowth = 0.45;
+static_assert(2 * kSampleBlocks <= kScanExtra, "h_total holds the blocks' counts");
+__global__ void __launch_bounds__(kSampleThreads) k_sample_held(int nx, int ny, const int32_t *__restrict__ beg,
+                                                                const int32_t *__restrict__ end,
+                                                                const double2 *__restrict__ z, int2 *out) {
+  __shared__ int s_all, s_held;
+  if (threadIdx.x == 0) s_all = s_held = 0;
+  __syncthreads();
+  const unsigned t = blockIdx.x * kSampleThreads + threadIdx.x, i = t >> 2, d = t & 3;
   const long long ncols = (long long)nx * ny;
   // evenly spread, with a step that shares no period with the rows
   const int c = (int)(((unsigned long long)i * 0x9e3779b97f4a7c15ull >> 32) * ncols >> 32);
   const int x = c % nx, y = c / nx;
   int all = 0, held = 0;
   if (x > 0 && y > 0 && x + 1 < nx && y + 1 < ny) {
-    const int step[4] = {-1, 1, -nx, nx};
-    int at[4];
-    for (int d = 0; d < 4; ++d) at[d] = beg[c + step[d]];
-    for (int k = beg[c]; k < end[c]; ++k) {
-      const double2 s = z[k];
-      all += 4;
-      for (int d = 0; d < 4; ++d) {
-        // of the neighbour's segments the first that reaches this one, or the next
-        const int e = end[c + step[d]];
-        while (at[d] < e && z[at[d]].y < s.x) ++at[d];
-        bool in = false;
-        for (int j = at[d]; j < min(at[d] + 2, e); ++j) in |= z[j].x - s.x <= growth && s.y - z[j].y <= growth;
-        held += in;
-      }
+    const int cn = c + (d == 0 ? -1 : d == 1 ? 1 : d == 2 ? -nx : nx), e = end[cn];
+    const int k0 = beg[c], n = min(end[c] - k0, kSampleSegs);
+    all = n;
+    int at = beg[cn];
+    for (int k = 0; k < n; ++k) {
+      const double2 s = z[k0 + k];
+      // of the neighbour's segments the first that reaches this one, or the next
+      while (at < e && z[at].y < s.x) ++at;
+      bool in = false;
+      for (int j = 0; j < 2 && at + j < e; ++j) in |= z[at + j].x - s.x <= kSampleGrowth && s.y - z[at + j].y <= kSampleGrowth;
+      held += in;
     }
   }
   all = __reduce_add_sync(0xffffffffu, all);
   held = __reduce_add_sync(0xffffffffu, held);
   if ((threadIdx.x & 31) == 0) {
-    atomicAdd(&out[0], all);
-    atomicAdd(&out[1], held);
+    atomicAdd(&s_all, all);
+    atomicAdd(&s_held, held);
   }
+  __syncthreads();
+  if (threadIdx.x == 0) out[blockIdx.x] = make_int2(s_all, s_held);
 }
 
 static_assert(kDomLevels <= 15, "pair records hold a level in 4 bits, 15 meaning none");
@@ -714,33 +720,37 @@ void column_list_launch(cudaStream_t st, const BatchVol *vols, int nv) {
 //   cylinders   1024^2   4.4         3.75 / 5.56           6.30 / 8.61           6.74 / 10.8
 //                        16.2        17.0 / 25.0           21.7 / 31.9           17.9 / 36.6
 // Below 2^18 columns four threads share one in k_direct, which is the best there (256^2, 4.1 segments, r = 6: 0.39 /
-// 0.48). What tells the inputs apart is how many segments a neighbour column holds at the median growth of H: 0.63
-// to 0.71 of them for spheres (with some cylinders among them 0.63 to 0.65), 0.48 to 0.52 for thin cylinders, none
-// for scattered segments. The line is 0.55; the sample takes 15 us.
-constexpr double kHeldShare = 0.55, kColumnWorkFrom = 190, kColumnWorkTo = 1050;
+// 0.48). What tells the inputs apart is how many segments a neighbour column holds when widened by what H grows in
+// a step, its median at any of these radii (0.41 to 0.49 dexels; 0.58 at radius 5, where many growths are alike, so that
+// the growth is a constant here): 0.64 to 0.66 of them for spheres, with some cylinders among them 0.59 to 0.63, 0.49
+// for thin cylinders, none for scattered segments. The line is 0.55. The sample takes 15 to 30 us with the wait for it, so it
+// is not taken where there is less to gain: calls of about a millisecond (work over all columns; 512^2 thin cylinders,
+// 2.5 segments, r = 6, lie below: 1.05 ms, with a sample 1.13 before it was made shorter), and from radius 7.5 fewer
+// than 2^19 columns (513^2 spheres, 3.4 segments, r = 8: 0.85 / 0.88).
+constexpr double kHeldShare = 0.55, kColumnWorkFrom = 190, kColumnWorkTo = 1050, kSampleWork = 8e7;
 constexpr int64_t kColumnCols = 1 << 18;
 constexpr double kColumnSegs = 2.0, kColumnRadiusFrom = 3.5, kColumnRadiusMid = 7.5, kColumnRadiusTo = 9.0;
 
 int column_choice(vo_ctx *ctx, const vo_grid &g, const DeviceTables &T, double mean_segs, const int32_t *beg,
-                  const int32_t *end, const double2 *z, const std::function<int()> &tables, bool *columns) {
+                  const int32_t *end, const double2 *z, const std::function<void()> &ready, bool *columns) {
   *columns = false;
-  const double work = reach_columns(g, T) * mean_segs;
-  if ((int64_t)g.nx * g.ny < kColumnCols || std::min(g.nx, g.ny) < kPatchY || mean_segs < kColumnSegs ||
-      T.host.R < kColumnRadiusFrom || T.host.R >= kColumnRadiusTo || work < kColumnWorkFrom ||
-      (T.host.R >= kColumnRadiusMid && work > kColumnWorkTo))
+  const double work = reach_columns(g, T) * mean_segs, ncols = (double)g.nx * g.ny;
+  if (ncols < kColumnCols || std::min(g.nx, g.ny) < kPatchY || mean_segs < kColumnSegs || T.host.R < kColumnRadiusFrom ||
+      T.host.R >= kColumnRadiusTo || work < kColumnWorkFrom || ncols * work < kSampleWork ||
+      (T.host.R >= kColumnRadiusMid && (work > kColumnWorkTo || ncols < 2 * kColumnCols)))
     return VO_OK;
-  int rc = tables();
-  if (rc) return rc;
-  int *d = nullptr, h[2] = {0, 0};
-  rc = dalloc(ctx, &d, 2);
-  if (rc) return rc;
-  cudaMemsetAsync(d, 0, sizeof h, ctx->stream);
-  k_sample_held<<<kSampleColumns / 128, 128, 0, ctx->stream>>>(g.nx, g.ny, beg, end, z, T.dom.t[kDomLevels / 2], d);
+  ready();
+  int2 *h = reinterpret_cast<int2 *>(ctx->h_total + 1);
+  k_sample_held<<<kSampleBlocks, kSampleThreads, 0, ctx->stream>>>(g.nx, g.ny, beg, end, z, h);
   ctx->launches += 1;
-  cudaMemcpyAsync(h, d, sizeof h, cudaMemcpyDeviceToHost, ctx->stream);
-  dfree(ctx, d);
+  VO_CK(ctx, cudaGetLastError());
   VO_CK(ctx, cudaStreamSynchronize(ctx->stream));
-  *columns = h[1] >= kHeldShare * h[0];
+  double all = 0, held = 0;
+  for (int i = 0; i < kSampleBlocks; ++i) {
+    all += h[i].x;
+    held += h[i].y;
+  }
+  *columns = all > 0 && held >= kHeldShare * all;
   return VO_OK;
 }
 

@@ -1761,7 +1761,7 @@ int dilate_fast(vo_ctx *ctx, double R, const vo_volume *in, vo_volume **out, vo_
   Engine engine = direct_choice(g, *T, mean_segs) ? Engine::kDirect : Engine::kPatches;
   {
     bool columns = false;
-    rc = column_choice(ctx, g, *T, mean_segs, in->offs, in->offs + 1, in->z, [&] { return column_tables(ctx, T); }, &columns);
+    rc = column_choice(ctx, g, *T, mean_segs, in->offs, in->offs + 1, in->z, [] {}, &columns);
     if (rc) return rc;
     if (columns || (engine == Engine::kPatches && in->nseg > kPatchSegments)) engine = Engine::kColumns;
   }

@@ -310,9 +310,9 @@ void column_list_launch(cudaStream_t st, const BatchVol *vols, int nv);
 std::vector<float4> column_pairs(const Tables &h, DomLevels &L);
 int column_tables(vo_ctx *ctx, const DeviceTables *T);
 // Whether a dilation by that radius is to take the per-column kernel first: where the sizes leave it open, a sample of
-// the input decides (synchronising). tables(T) makes T->prec and T->dom.
+// the input, there after ready(), decides (synchronising).
 int column_choice(vo_ctx *ctx, const vo_grid &g, const DeviceTables &T, double mean_segs, const int32_t *beg,
-                  const int32_t *end, const double2 *z, const std::function<int()> &tables, bool *columns);
+                  const int32_t *end, const double2 *z, const std::function<void()> &ready, bool *columns);
 
 // Queue of a launch. count: the first tier's next item, the items it listed
 // for the second tier, that tier's next one, columns of the listed items.
