@@ -12,7 +12,8 @@
 // per column hold that for eleven growths, so that a source column costs one load
 // of its record and two of its masks however many of its segments are held.
 //
-// It is the better kernel in two places.
+// It is the better kernel in two places, and the one for inputs of more than 2^30
+// segments (kPatchSegments).
 // - Smooth dense inputs at small radii, where most segments are held
 //   (column_choice has the measured line).
 // - Unions of many intervals: the patch kernel's bins and the lists of k_direct
